@@ -28,7 +28,7 @@ DECODER_LIB = os.path.join(LIBDIR, "libgptb200_decoder.so")
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 DECODER_SOURCES = ["capi.cu", "decoder_model.cu"]
-SOURCES = ["capi.cu", "backend_capi.cu", "b200_backend.cu", "gpt_model.cu", "noalloc.cu", "decoder_model.cu", "loader.cpp"]
+SOURCES = ["capi.cu", "backend_capi.cu", "b200_backend.cu", "gpt_model.cu", "gpt_step.cu", "noalloc.cu", "decoder_model.cu", "loader.cpp"]
 
 
 def _nvcc() -> str:

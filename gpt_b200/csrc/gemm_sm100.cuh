@@ -45,6 +45,7 @@ enum DeviceStatus : int {
     DEV_TIMEOUT_CONVERT = 106,    // converter gave up waiting for a landed stage
     DEV_TIMEOUT_DRAIN = 107,      // teardown gave up waiting for outstanding MMAs
     DEV_TIMEOUT_PARTIAL = 109,    // epilogue gave up waiting for another CTA pair's partial tile
+    DEV_TIMEOUT_GRID = 110,       // a block of a generation step gave up waiting at a grid barrier
     DEV_TIMEOUT_SELFTEST = 108,   // the self-test's wait on a barrier that nothing signals ran out, as intended
 };
 

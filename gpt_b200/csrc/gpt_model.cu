@@ -17,6 +17,7 @@
 
 #include "backend_interface.h"
 #include "b200_backend.h"
+#include "gpt_step.h"
 #include "../../include/gptb200.h"
 
 namespace {
@@ -266,7 +267,10 @@ public:
         const size_t L = c_.layers, D = c_.d_model, F = c_.d_ffn, Vp = c_.vocab_padded;
         if (!set_size(batch, prompt_len)) return GPTB200_ERR_CUDA;
         const size_t cache_floats = L * size_t(batch) * max_len * 2 * D;
-        const size_t step_floats = size_t(batch) * (D * 7 + 3 * D + 2 * F + 6) + 8;
+        gptb200::GptStep one = one_launch_step(batch, max_len);
+        size_t one_floats = 0;
+        const bool one_launch = gptb200::plan_gpt_step(ctx, one, &one_floats);
+        const size_t step_floats = operator_step_floats(batch) + (one_launch ? one_floats : 0) + 8;
         if (cache_floats + step_floats > gen_capacity_) {
             void *p = nullptr;
             be_->device_malloc(&p, (cache_floats + step_floats) * sizeof(float));
@@ -278,6 +282,8 @@ public:
         gen_batch_ = batch;
         gen_max_len_ = max_len;
         gen_pos_ = prompt_len;
+        gen_step_ = one;
+        gen_one_launch_ = one_launch;
         forward(prompt);
         const size_t M = size_t(batch) * prompt_len;
         for (size_t l = 0; l < L; ++l) {
@@ -286,9 +292,27 @@ public:
             if (rc) return rc;
         }
         gen_pos_off_ = cache_floats + step_floats - 8;
-        be_->device_memcpy_h2d(gen_ + gen_pos_off_, &gen_pos_, sizeof(int));
+        const int words[8] = {gen_pos_};   // the position, and from word 4 on the counters of the one-launch step
+        be_->device_memcpy_h2d(gen_ + gen_pos_off_, words, sizeof(words));
         (void)Vp;
         return GPTB200_OK;
+    }
+
+    size_t operator_step_floats(int batch) const { return pad4(size_t(batch) * (size_t(c_.d_model) * 10 + 2 * size_t(c_.d_ffn) + 6)); }
+
+    // The parts of a one-launch step that its plan needs.
+    gptb200::GptStep one_launch_step(int batch, int max_len) const
+    {
+        gptb200::GptStep s{};
+        s.batch = batch;
+        s.layers = c_.layers;
+        s.d = c_.d_model;
+        s.ffn = c_.d_ffn;
+        s.heads = c_.heads;
+        s.vocab_p = c_.vocab_padded;
+        s.max_len = max_len;
+        s.max_pos = c_.max_seq_len;
+        return s;
     }
 
     // One new position for every sequence: the forward pass of one row per sequence, attention against the cache.
@@ -305,6 +329,23 @@ public:
         (void)x2;
         int *pos_dev = reinterpret_cast<int *>(gen_ + gen_pos_off_);
         float *w = weights();
+        if (gen_one_launch_ && gptb200::gpt_step_enabled(ctx)) {
+            gptb200::GptStep one = gen_step_;
+            one.wte = w + lay_.wte; one.wpe = w + lay_.wpe;
+            one.ln1_w = w + lay_.ln1_w; one.ln1_b = w + lay_.ln1_b; one.qkv_w = w + lay_.qkv_w; one.qkv_b = w + lay_.qkv_b;
+            one.proj_w = w + lay_.proj_w; one.proj_b = w + lay_.proj_b; one.ln2_w = w + lay_.ln2_w; one.ln2_b = w + lay_.ln2_b;
+            one.up_w = w + lay_.up_w; one.up_b = w + lay_.up_b; one.down_w = w + lay_.down_w; one.down_b = w + lay_.down_b;
+            one.lnf_w = w + lay_.lnf_w; one.lnf_b = w + lay_.lnf_b;
+            one.scale = 1.0f / sqrtf(static_cast<float>(c_.d_model / c_.heads));
+            one.tokens = tokens;
+            one.pos = pos_dev;
+            one.logits = logits;
+            one.cache = gen_;
+            one.sync = reinterpret_cast<unsigned *>(pos_dev) + 4;
+            const int rc = gptb200::run_gpt_step(ctx, one, gen_ + cache_floats + operator_step_floats(b));
+            if (rc == 0) ++gen_pos_;
+            return rc;
+        }
         int rc = gptb200_embedding_decode(ctx, x, w + lay_.wte, w + lay_.wpe, tokens, pos_dev, b, c_.d_model);
         if (rc) return rc;
         // same operator sequence as forward() with one row per sequence; the residual stream alternates between x / proj / down
@@ -437,6 +478,8 @@ private:
     bool fused_ce_ = false, fused_ce_active_ = false, row_loss_valid_ = false;
     bool fused_gelu_ = false;
     float *gen_ = nullptr;        // KV cache of every layer, then the step's activations, then the device copy of the position
+    gptb200::GptStep gen_step_{};   // the one-launch step as planned for the cache
+    bool gen_one_launch_ = false;
     size_t gen_capacity_ = 0, gen_pos_off_ = 0;
     int gen_batch_ = 0, gen_max_len_ = 0, gen_pos_ = 0;
 };

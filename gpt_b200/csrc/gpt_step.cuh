@@ -1,0 +1,494 @@
+// Kernels of a GPT-2 generation step in one launch.
+//
+// As one launch per operator a step of 12 layers is a chain of 89 launches of 3 - 16 us for 0.5 GB of weights (75 us of HBM
+// time): bound by launches, not by memory.  Here one block per SM stays for the whole step.  Phases meet at grid barriers
+// (arrivals counted in device memory, a cooperative launch keeps all blocks resident), and while a block waits at one its weights of the
+// next phase are already on their way: they depend on nothing.  All arithmetic is fp32 FMAs; sums have a fixed order.
+#pragma once
+
+#include <cfloat>
+#include <cuda_runtime.h>
+
+#include "gemm_sm100.cuh"  // gelu_tanh
+#include "gpt_step.h"
+
+namespace gptb200 {
+namespace step {
+
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr int kCols = 64;                    // output columns per item
+constexpr int kBody = 8;                     // 16-byte weight loads in flight per thread: 256 k-rows of an item
+constexpr unsigned kPollLimit = 1u << 22;    // some seconds; reached only if a block of the grid never ran
+
+// Grid barrier in two halves, so that loads can be issued between them.  The counter only grows: `target` is what it reads once all
+// blocks have arrived at this barrier.
+__device__ __forceinline__ void arrive(const GptStep &s, unsigned &target)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(s.sync) : "memory");
+    }
+    target += gridDim.x;
+}
+
+__device__ __forceinline__ void await(const GptStep &s, unsigned target)
+{
+    if (threadIdx.x == 0) {
+        unsigned seen = 0, tries = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(s.sync) : "memory");
+            if (++tries == kPollLimit) {
+                atomicCAS(s.status, 0, DEV_TIMEOUT_GRID);
+                break;
+            }
+        } while (static_cast<int>(seen - target) < 0);
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float dot4(float4 a, float4 b, float s) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s)))); }
+
+// Sum of the slices' partial sums at one position, slice order; `stride` floats between slices.  Written by other blocks of this launch: read from L2.
+__device__ __forceinline__ float4 sum_parts4(const float *p, int splits, int stride)
+{
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (; splits > 0; splits -= 12) {   // twelve loads in flight: one L2 round trip for what the plan makes of GPT-2
+        float4 v[12];
+#pragma unroll
+        for (int i = 0; i < 12; ++i, p += stride)
+            v[i] = i < splits ? __ldcg(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 12; ++i) sum = add4(sum, v[i]);
+    }
+    return sum;
+}
+
+__device__ __forceinline__ float sum_parts(const float *p, int splits, int stride)
+{
+    float sum = 0.0f;
+    for (; splits > 0; splits -= 4) {
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i, p += stride)
+            if (i < splits) v[i] = __ldcg(p);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < splits) sum += v[i];
+    }
+    return sum;
+}
+
+// ---- one or two rows --------------------------------------------------------------------------------------------------------
+// Weights go straight to registers: thread (krow, lane16) of an item reads 16 bytes of k-rows krow, krow + 32, ... (a half-warp 256
+// contiguous bytes), all of a slice of up to 256 rows at once, before the barrier in front of the phase.  GPT-2 124M on 148 SMs: 144 items
+// in every phase.  Every block keeps the whole residual stream in shared memory and norms it itself (bitwise the same everywhere), and the
+// blocks of one head compute its attention once each: four barriers per layer instead of seven.  A phase lasts one to two
+// microseconds, so what 16 warps issue counts as much as what they wait for: addresses are worked out once per launch (Share), and
+// warps without data skip (with both left out a step of GPT-2 124M took 270 us).  One row at position 64 - 96: 236 us per step, against 445 us as
+// 89 launches (a prompt of 64 tokens and 32 steps: 9.3 ms, was 15.7).  What is left is the length of the chain: at a barrier 1.1 us
+// between the last arrival and the first use of its data, then up to 1.5 us for 148 blocks that read the same 36 KB of partial sums.
+// Tried: the next phase's weights towards L2 while a phase computes (9.4 ms: their traffic delays the partial sums).
+
+// A thread's part of an item.
+struct Share {
+    int offset;     // of its first weight
+    int count;      // its k-rows, 32 apart
+    int k0, rows;   // the item's slice
+    int split, col;   // col: of the item
+};
+
+__device__ __forceinline__ Share share_of(const StepPhase &ph, int item)
+{
+    Share r;
+    r.split = item / ph.groups;
+    r.col = (item - r.split * ph.groups) * kCols;
+    r.k0 = r.split * ph.slice;
+    r.rows = item < ph.groups * ph.splits ? min(ph.K - r.k0, ph.slice) : 0;
+    const int krow = threadIdx.x >> 4, col = r.col + (threadIdx.x & 15) * 4;
+    r.offset = (r.k0 + krow) * ph.N + col;
+    r.count = col < ph.N ? max(0, (r.rows - krow + 31) >> 5) : 0;
+    return r;
+}
+
+__device__ __forceinline__ void fetch(float4 (&wv)[kBody], const float *w, const StepPhase &ph, const Share &r, int done = 0)
+{
+    const float *p = w + r.offset + static_cast<size_t>(done * 32) * ph.N;
+    const int stride = 32 * ph.N;
+#pragma unroll
+    for (int j = 0; j < kBody; ++j, p += stride)
+        wv[j] = done + j < r.count ? __ldcs(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// part[split][m][col ..] = xs[m][.] . w over the item's slice.  wv holds the first weights; red: [kWarps][MR][kCols].
+template <int MR>
+__device__ __forceinline__ void item_product(float4 (&wv)[kBody], const float *w, const StepPhase &ph, const Share &r, const float *xs, int pitch, float *red, float *part, int batch)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float *x = xs + (threadIdx.x >> 4);
+    float acc[MR][4] = {};
+    for (int done = 0; done * 32 < r.rows; done += kBody, x += 32 * kBody) {
+        if (done > 0) fetch(wv, w, ph, r, done);
+#pragma unroll
+        for (int j = 0; j < kBody; ++j)
+            if (done + j < r.count) {
+#pragma unroll
+                for (int m = 0; m < MR; ++m) {
+                    const float v = x[m * pitch + 32 * j];
+                    acc[m][0] = fmaf(v, wv[j].x, acc[m][0]);
+                    acc[m][1] = fmaf(v, wv[j].y, acc[m][1]);
+                    acc[m][2] = fmaf(v, wv[j].z, acc[m][2]);
+                    acc[m][3] = fmaf(v, wv[j].w, acc[m][3]);
+                }
+            }
+    }
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[m][c] += __shfl_xor_sync(0xffffffffu, acc[m][c], 16);
+        if (lane < 16) *reinterpret_cast<float4 *>(red + (warp * MR + m) * kCols + lane * 4) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+    }
+    __syncthreads();
+    if (threadIdx.x < MR * kCols) {
+        const int m = threadIdx.x / kCols, col = r.col + threadIdx.x % kCols;
+        float v = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) v += red[i * MR * kCols + threadIdx.x];
+        if (m < batch && col < ph.N) part[(r.split * batch + m) * ph.N + col] = v;
+    }
+}
+
+// Count, mean and sum of squared distances from it of the values that a warp's threads hold, for each warp with any.
+// The threads of one row are kThreads / MR consecutive ones.
+template <int MR>
+__device__ __forceinline__ void warp_moments(const float *row, int d, float4 *part)
+{
+    constexpr int kPer = kThreads / MR;
+    const int at = (threadIdx.x % kPer) * 4, lane = threadIdx.x & 31;
+    if (at - lane * 4 >= d) return;
+    float sum = 0.0f, n = 0.0f, var = 0.0f;
+    for (int i = at; i < d; i += kPer * 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(row + i);
+        sum += (v.x + v.y) + (v.z + v.w);
+    }
+    for (int i = at - lane * 4; i < d; i += kPer * 4) n += static_cast<float>(min(d - i, 128));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float mean = sum / n;
+    for (int i = at; i < d; i += kPer * 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(row + i);
+        const float a = v.x - mean, b = v.y - mean, c = v.z - mean, e = v.w - mean;
+        var += (a * a + b * b) + (c * c + e * e);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) var += __shfl_xor_sync(0xffffffffu, var, o);
+    if (lane == 0) part[threadIdx.x >> 5] = make_float4(n, mean, var, 0.0f);
+}
+
+// Mean and standard deviation of every row from the warps' moments: mean of the means, distances of the means added to the squares.
+template <int MR>
+__device__ __forceinline__ void row_statistics(const float4 *part, int d, float (&mean)[MR], float (&sd)[MR])
+{
+    constexpr int kPer = kWarps / MR;
+    const int warps = min((d + 127) >> 7, kPer);
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+        float sum = 0.0f, var = 0.0f;
+        for (int w = 0; w < warps; ++w) sum = fmaf(part[m * kPer + w].x, part[m * kPer + w].y, sum);
+        mean[m] = sum / d;
+        for (int w = 0; w < warps; ++w) {
+            const float4 v = part[m * kPer + w];
+            var += fmaf(v.x * (v.y - mean[m]), v.y - mean[m], v.z);
+        }
+        sd[m] = sqrtf(var / d + 1e-5f);
+    }
+}
+
+// The largest shared memory of the kernel below, in floats.
+inline size_t small_shared_floats(int mr, int d, int hd, int max_len, int widest)
+{
+    return size_t(mr) * d + size_t(mr) * widest + size_t(kWarps) * mr * kCols + size_t(mr) * 3 * hd + size_t(kWarps) * (hd + 4) + size_t(mr) * max_len;
+}
+
+template <int MR>
+__global__ void __launch_bounds__(kThreads, 1)
+gpt_step_kernel(const GptStep s, int widest)
+{
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float4 moments[kWarps];
+    float *res = sm;                                 // [MR][d] residual stream
+    float *xs = res + MR * s.d;                      // [MR][widest] activations of an item
+    float *red = xs + MR * widest;                   // [kWarps][MR][kCols]
+    float *fresh = red + kWarps * MR * kCols;        // [MR][3][hd] new q, k, v of a head
+    float *out = fresh + MR * 3 * s.hd;              // [kWarps][hd + 4] parts of a head's output, and of its weights' sum
+    float *prob = out + kWarps * (s.hd + 4);         // [MR][max_len]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = s.d;
+    const int p = *s.pos;
+    if (p < 0 || p >= s.max_len || p >= s.max_pos) return;   // all blocks alike
+    unsigned target = s.sync[1];
+    const int first = blockIdx.x;                    // this block's first item of every phase
+    const Share of_qkv = share_of(s.qkv, first), of_proj = share_of(s.proj, first), of_up = share_of(s.up, first), of_down = share_of(s.down, first);
+    float4 wv[kBody];
+    fetch(wv, s.qkv_w, s.qkv, of_qkv);
+
+    constexpr int kPer = kThreads / MR;   // threads of a row
+    const int mine = tid / kPer, at4 = (tid % kPer) * 4;
+    for (int c = at4; c < d; c += kPer * 4)
+        *reinterpret_cast<float4 *>(res + mine * d + c) = mine < s.batch ? add4(__ldg(reinterpret_cast<const float4 *>(s.wte + static_cast<size_t>(s.tokens[mine]) * d + c)),
+                                                                               __ldg(reinterpret_cast<const float4 *>(s.wpe + static_cast<size_t>(p) * d + c)))
+                                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+    warp_moments<MR>(res + mine * d, d, moments);
+    __syncthreads();
+
+    // res += the finished product, with the moments of the new rows
+    auto add_result = [&](const float *part, const StepPhase &ph, const float *bias) {
+        if (mine < s.batch)
+            for (int c = at4; c < d; c += kPer * 4) {
+                const float4 be = __ldg(reinterpret_cast<const float4 *>(bias + c));
+                const float4 v = add4(sum_parts4(part + mine * d + c, ph.splits, s.batch * d), be);
+                *reinterpret_cast<float4 *>(res + mine * d + c) = add4(*reinterpret_cast<const float4 *>(res + mine * d + c), v);
+            }
+        warp_moments<MR>(res + mine * d, d, moments);
+        __syncthreads();
+    };
+    // a product behind a norm of the residual stream
+    // (gain0, bias0: the norm's parameters of the first item's k-row `tid`, loaded like its weights before the barrier)
+    float gain0 = 0.0f, bias0 = 0.0f;
+    auto fetch_norm = [&](const Share &r, const float *gain, const float *bias) {
+        if (tid < r.rows) {
+            gain0 = __ldg(gain + r.k0 + tid);
+            bias0 = __ldg(bias + r.k0 + tid);
+        }
+    };
+    auto normed_product = [&](const float *w, const StepPhase &ph, const Share &one, const float *gain, const float *bias, float *part) {
+        float mean[MR], sd[MR];
+        Share r = one;
+        for (int item = first; item < ph.groups * ph.splits; item += gridDim.x) {
+            if (item != first) {
+                r = share_of(ph, item);
+                fetch(wv, w, ph, r);
+                fetch_norm(r, gain, bias);
+                __syncthreads();
+            }
+            if (warp * 32 < r.rows) {
+                row_statistics<MR>(moments, d, mean, sd);
+                for (int k = tid; k < r.rows; k += kThreads) {
+                    const float ga = k == tid ? gain0 : __ldg(gain + r.k0 + k), be = k == tid ? bias0 : __ldg(bias + r.k0 + k);
+#pragma unroll
+                    for (int m = 0; m < MR; ++m) xs[m * widest + k] = (res[m * d + r.k0 + k] - mean[m]) / sd[m] * ga + be;
+                }
+            }
+            __syncthreads();
+            item_product<MR>(wv, w, ph, r, xs, widest, red, part, s.batch);
+        }
+    };
+
+    fetch_norm(of_qkv, s.ln1_w, s.ln1_b);
+    // a head's size is a power of two: lanes of a cached row, rows at a time
+    const int head_log = 31 - __clz(s.hd), per_pos = s.hd >> 2, groups = kThreads / per_pos;
+    const int g = tid >> (head_log - 2), c4 = (tid & (per_pos - 1)) * 4, row_stride = 2 * d * groups;
+    for (int l = 0; l < s.layers; ++l) {
+        const float *proj_w = s.proj_w + static_cast<size_t>(l) * d * d;
+        if (l > 0) add_result(s.down_part, s.down, s.down_b + (l - 1) * d);
+        normed_product(s.qkv_w + static_cast<size_t>(l) * d * 3 * d, s.qkv, of_qkv, s.ln1_w + l * d, s.ln1_b + l * d, s.qkv_part);
+        arrive(s, target);
+        float *cache = s.cache + static_cast<size_t>(l) * s.batch * s.max_len * 2 * d;
+        fetch(wv, proj_w, s.proj, of_proj);
+        // and the first cached rows of this block's first head
+        float4 k_first[4], v_first[4];
+        {
+            const float *row = cache + static_cast<size_t>(g) * 2 * d + of_proj.k0 + c4;
+#pragma unroll
+            for (int j = 0; j < 4; ++j, row += row_stride) {
+                const bool live = of_proj.rows > 0 && g + j * groups < p;
+                k_first[j] = live ? *reinterpret_cast<const float4 *>(row) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v_first[j] = live ? *reinterpret_cast<const float4 *>(row + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        await(s, target);
+
+        const float *up_w = s.up_w + static_cast<size_t>(l) * d * s.ffn, *down_w = s.down_w + static_cast<size_t>(l) * s.ffn * d;
+        // attention of the heads in the item's slice of k, then the slice's share of the projection
+        Share r = of_proj;
+        for (int item = first; item < s.proj.groups * s.proj.splits; item += gridDim.x) {
+            if (item != first) {
+                r = share_of(s.proj, item);
+                fetch(wv, proj_w, s.proj, r);
+            }
+            for (int at = 0; at < r.rows; at += s.hd) {   // head by head
+                const bool fetched = item == first && at == 0;   // k_first, v_first are this head's, row 0
+                if (!fetched) __syncthreads();
+                for (int i = tid; i < s.batch * 3 * s.hd; i += kThreads) {
+                    const int row = i >> head_log, m = MR == 1 ? 0 : row / 3, which = row - 3 * m, e = i & (s.hd - 1), col = which * d + r.k0 + at + e;
+                    const float be = __ldg(s.qkv_b + l * 3 * d + col);
+                    const float v = sum_parts(s.qkv_part + m * 3 * d + col, s.qkv.splits, s.batch * 3 * d) + be;
+                    fresh[i] = v;
+                    if (which > 0 && r.col == 0) cache[(static_cast<size_t>(m) * s.max_len + p) * 2 * d + (col - d)] = v;
+                }
+                __syncthreads();
+                for (int m = 0; m < s.batch; ++m) {
+                    const float *q = fresh + m * 3 * s.hd + c4, *row = cache + (static_cast<size_t>(m) * s.max_len + g) * 2 * d + r.k0 + at + c4;
+                    const float4 q4 = *reinterpret_cast<const float4 *>(q);
+                    float *probs = prob + m * s.max_len;
+                    for (int t0 = 0; t0 <= p; t0 += 4 * groups, row += 4 * row_stride) {   // four rows in flight per thread
+                        float4 kv[4];
+                        float v[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int t = t0 + g + j * groups;
+                            kv[j] = fetched && m == 0 && t0 == 0 ? k_first[j] : t < p ? *reinterpret_cast<const float4 *>(row + j * row_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (t == p) kv[j] = *reinterpret_cast<const float4 *>(q + s.hd);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[j] = dot4(q4, kv[j], 0.0f);
+                        for (int o = per_pos >> 1; o > 0; o >>= 1)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+                        if (c4 == 0)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (t0 + g + j * groups <= p) probs[t0 + g + j * groups] = v[j] * s.scale;
+                    }
+                }
+                __syncthreads();
+                for (int m = 0; m < s.batch; ++m) {
+                    const float *q = fresh + m * 3 * s.hd + c4, *row = cache + (static_cast<size_t>(m) * s.max_len + g) * 2 * d + d + r.k0 + at + c4;
+                    float *probs = prob + m * s.max_len;
+                    float mx = -FLT_MAX, weights = 0.0f;
+                    for (int t = lane; t <= p; t += 32) mx = fmaxf(mx, probs[t]);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int t0 = 0; t0 + g <= p; t0 += 4 * groups, row += 4 * row_stride) {
+                        float4 kv[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int t = t0 + g + j * groups;
+                            kv[j] = fetched && m == 0 && t0 == 0 ? v_first[j] : t < p ? *reinterpret_cast<const float4 *>(row + j * row_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (t == p) kv[j] = *reinterpret_cast<const float4 *>(q + 2 * s.hd);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (t0 + g + j * groups <= p) {
+                                const float e = expf(probs[t0 + g + j * groups] - mx);
+                                weights += e;
+                                acc.x = fmaf(e, kv[j].x, acc.x);
+                                acc.y = fmaf(e, kv[j].y, acc.y);
+                                acc.z = fmaf(e, kv[j].z, acc.z);
+                                acc.w = fmaf(e, kv[j].w, acc.w);
+                            }
+                    }
+                    for (int o = per_pos; o < 32; o <<= 1) {
+                        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+                        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+                        acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+                        weights += __shfl_xor_sync(0xffffffffu, weights, o);
+                    }
+                    if (m > 0) __syncthreads();   // the previous row's parts have been added up
+                    if (lane < per_pos) *reinterpret_cast<float4 *>(out + warp * (s.hd + 4) + c4) = acc;
+                    if (lane == 0) out[warp * (s.hd + 4) + s.hd] = weights;
+                    __syncthreads();
+                    if (tid < s.hd) {   // heads are at most 128 wide
+                        float v = 0.0f, sum = 0.0f;
+#pragma unroll
+                        for (int j = 0; j < kWarps; ++j) {
+                            v += out[j * (s.hd + 4) + tid];
+                            sum += out[j * (s.hd + 4) + s.hd];
+                        }
+                        xs[m * widest + at + tid] = v / sum;
+                    }
+                }
+            }
+            if (MR > 1 && s.batch < MR)
+                for (int i = tid; i < r.rows; i += kThreads) xs[widest + i] = 0.0f;
+            __syncthreads();
+            item_product<MR>(wv, proj_w, s.proj, r, xs, widest, red, s.proj_part, s.batch);
+        }
+        arrive(s, target);
+        fetch(wv, up_w, s.up, of_up);
+        fetch_norm(of_up, s.ln2_w + l * d, s.ln2_b + l * d);
+        await(s, target);
+
+        add_result(s.proj_part, s.proj, s.proj_b + l * d);
+        normed_product(up_w, s.up, of_up, s.ln2_w + l * d, s.ln2_b + l * d, s.up_part);
+        arrive(s, target);
+        fetch(wv, down_w, s.down, of_down);
+        await(s, target);
+
+        r = of_down;
+        for (int item = first; item < s.down.groups * s.down.splits; item += gridDim.x) {
+            if (item != first) {
+                r = share_of(s.down, item);
+                fetch(wv, down_w, s.down, r);
+                __syncthreads();
+            }
+            for (int m = 0; m < MR; ++m)
+                for (int k = tid; k < r.rows; k += kThreads) {
+                    const float be = __ldg(s.up_b + l * s.ffn + r.k0 + k);
+                    xs[m * widest + k] = m < s.batch ? gelu_tanh(sum_parts(s.up_part + m * s.ffn + r.k0 + k, s.up.splits, s.batch * s.ffn) + be) : 0.0f;
+                }
+            __syncthreads();
+            item_product<MR>(wv, down_w, s.down, r, xs, widest, red, s.down_part, s.batch);
+        }
+        arrive(s, target);
+        if (l + 1 < s.layers) {
+            fetch(wv, s.qkv_w + static_cast<size_t>(l + 1) * d * 3 * d, s.qkv, of_qkv);
+            fetch_norm(of_qkv, s.ln1_w + (l + 1) * d, s.ln1_b + (l + 1) * d);
+        }
+        await(s, target);
+    }
+
+    // final norm; logits: a warp per pair of embedding rows
+    add_result(s.down_part, s.down, s.down_b + (s.layers - 1) * d);
+    {
+        float mean[MR], sd[MR];
+        row_statistics<MR>(moments, d, mean, sd);
+        for (int k = tid; k < d; k += kThreads)
+#pragma unroll
+            for (int m = 0; m < MR; ++m) xs[m * widest + k] = (res[m * d + k] - mean[m]) / sd[m] * __ldg(s.lnf_w + k) + __ldg(s.lnf_b + k);
+    }
+    __syncthreads();
+    for (int n = 2 * (blockIdx.x * kWarps + warp); n < s.vocab_p; n += 2 * kWarps * gridDim.x) {
+        const float *wa = s.wte + static_cast<size_t>(n) * d, *wb = n + 1 < s.vocab_p ? wa + d : wa;
+        float sa[MR] = {}, sb[MR] = {};
+        for (int k0 = lane * 4; k0 < d; k0 += 6 * 128) {
+            float4 a[6], b[6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const bool live = k0 + j * 128 < d;
+                a[j] = live ? __ldcs(reinterpret_cast<const float4 *>(wa + k0 + j * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                b[j] = live ? __ldcs(reinterpret_cast<const float4 *>(wb + k0 + j * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                if (k0 + j * 128 >= d) break;
+#pragma unroll
+                for (int m = 0; m < MR; ++m) {
+                    const float4 x = *reinterpret_cast<const float4 *>(xs + m * widest + k0 + j * 128);
+                    sa[m] = dot4(a[j], x, sa[m]);
+                    sb[m] = dot4(b[j], x, sb[m]);
+                }
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < MR; ++m) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sa[m] += __shfl_xor_sync(0xffffffffu, sa[m], o);
+                sb[m] += __shfl_xor_sync(0xffffffffu, sb[m], o);
+            }
+            if (lane == 0 && m < s.batch) {
+                s.logits[static_cast<size_t>(m) * s.vocab_p + n] = sa[m];
+                if (n + 1 < s.vocab_p) s.logits[static_cast<size_t>(m) * s.vocab_p + n + 1] = sb[m];
+            }
+        }
+    }
+    if (blockIdx.x == 0 && tid == 0) {   // every block has passed a barrier since it read them
+        *s.pos = p + 1;
+        s.sync[1] = target;
+    }
+}
+
+}  // namespace step
+}  // namespace gptb200

@@ -1,0 +1,42 @@
+// One generation step of a GPT-2 model (one new token per sequence against the KV cache) as ONE persistent launch: what the
+// launcher (gpt_step.cu) and the model driver (gpt_model.cu) share.
+#pragma once
+
+#include <cstddef>
+
+struct gptb200_ctx;
+
+namespace gptb200 {
+
+// A product of the step: output columns in groups of 64, k in `splits` slices of `slice` rows.  The slices' sums meet in the
+// prologue of the next phase, in slice order.
+struct StepPhase {
+    int K, N, groups, splits, slice;
+};
+
+struct GptStep {
+    int batch, layers, d, ffn, heads, hd, vocab_p, max_len, max_pos;
+    float scale;
+    // weights, fp32; layers of a kind one after another
+    const float *wte, *wpe, *ln1_w, *ln1_b, *qkv_w, *qkv_b, *proj_w, *proj_b, *ln2_w, *ln2_b, *up_w, *up_b, *down_w, *down_b, *lnf_w, *lnf_b;
+    const int *tokens;      // [batch]
+    int *pos;               // position of the new tokens; the step advances it
+    float *logits;          // [batch][vocab_p]
+    float *cache;           // [layers][batch][max_len][2 d]
+    // scratch: partial sums [split][batch][N]; beyond two rows also residual stream, normed rows and attention output [batch][d]
+    float *qkv_part, *proj_part, *up_part, *down_part, *res, *normed, *attn;
+    StepPhase qkv, proj, up, down;
+    unsigned *sync;         // arrivals at the grid barriers so far, arrivals before this launch
+    int *status;
+};
+
+constexpr int kStepMaxBatch = 64;
+
+// Whether the step of this model and batch runs as one launch, with its phases and scratch (floats) filled in.
+bool plan_gpt_step(gptb200_ctx *ctx, GptStep &s, size_t *scratch_floats);
+// The context's options still ask for the kernels of few rows.
+bool gpt_step_enabled(const gptb200_ctx *ctx);
+// Launches it; `scratch` as planned, `sync` two words that were zero when the cache was filled.
+int run_gpt_step(gptb200_ctx *ctx, GptStep s, float *scratch);
+
+}  // namespace gptb200

@@ -1,0 +1,71 @@
+"""Generation steps of the GPT-2 model as one launch: against a float64 forward pass over the whole text."""
+import math
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _shapes(c):
+    L, D, H = c["num_layers"], c["d_model"], c["d_ffn"]
+    return [("wte", (c["vocab_size_padded"], D)), ("wpe", (c["max_seq_len"], D)), ("ln1_w", (L, D)), ("ln1_b", (L, D)), ("qkv_w", (L, D, 3 * D)), ("qkv_b", (L, 3 * D)),
+            ("proj_w", (L, D, D)), ("proj_b", (L, D)), ("ln2_w", (L, D)), ("ln2_b", (L, D)), ("up_w", (L, D, H)), ("up_b", (L, H)), ("down_w", (L, H, D)), ("down_b", (L, D)),
+            ("lnf_w", (D,)), ("lnf_b", (D,))]
+
+
+def _forward(torch, c, flat, tokens):
+    w, at = {}, 0
+    for name, shape in _shapes(c):
+        n = math.prod(shape)
+        w[name] = flat[at:at + n].view(shape)
+        at += n
+    B, T = tokens.shape
+    D, H = c["d_model"], c["num_heads"]
+    norm = lambda x, g, b: torch.nn.functional.layer_norm(x, (D,), g, b, 1e-5)
+    x = w["wte"][tokens.long()] + w["wpe"][:T]
+    mask = torch.ones(T, T, device="cuda", dtype=torch.bool).tril()
+    for i in range(c["num_layers"]):
+        q, k, v = (norm(x, w["ln1_w"][i], w["ln1_b"][i]) @ w["qkv_w"][i] + w["qkv_b"][i]).view(B, T, 3, H, D // H).permute(2, 0, 3, 1, 4)
+        p = torch.softmax((q @ k.transpose(-1, -2) * (D // H) ** -0.5).masked_fill(~mask, -math.inf), -1)
+        x = x + (p @ v).transpose(1, 2).reshape(B, T, D) @ w["proj_w"][i] + w["proj_b"][i]
+        u = norm(x, w["ln2_w"][i], w["ln2_b"][i]) @ w["up_w"][i] + w["up_b"][i]
+        x = x + torch.nn.functional.gelu(u, approximate="tanh") @ w["down_w"][i] + w["down_b"][i]
+    return norm(x, w["lnf_w"], w["lnf_b"]) @ w["wte"].t()
+
+
+GPT2 = dict(d_model=768, num_heads=12, d_ffn=3072, vocab_size_padded=1000)
+SIZES = {
+    "gpt2": GPT2,
+    "head8": dict(d_model=64, num_heads=8, d_ffn=308, vocab_size_padded=332),           # ragged column groups and slices
+    "head128": dict(d_model=384, num_heads=3, d_ffn=1284, vocab_size_padded=64),
+    "wide": dict(d_model=1600, num_heads=25, d_ffn=6400, vocab_size_padded=260),         # several items per block
+}
+
+
+@pytest.mark.parametrize("size,batch,layers,prompt,steps", [
+    ("gpt2", 1, 2, 60, 12), ("gpt2", 2, 2, 125, 8), ("gpt2", 1, 12, 1, 6), ("head8", 1, 3, 7, 40), ("head8", 2, 1, 31, 3), ("head128", 2, 2, 5, 70),
+    ("wide", 1, 2, 130, 4), ("wide", 2, 1, 9, 3), ("head128", 1, 1, 1, 1)])
+def test_generation_step_matches_the_whole_forward_pass(size, batch, layers, prompt, steps):
+    """Logits of every step within 1e-5 of their scale (fp32 sums of up to 6400 terms, layer after layer; the same bound as for the
+    operator-by-operator step)."""
+    import torch
+    import gpt_b200
+    c = dict(max_seq_len=prompt + steps + 1, num_layers=layers, **SIZES[size])
+    c["vocab_size"] = c["vocab_size_padded"] - 3
+    gen = torch.Generator(device="cuda").manual_seed(batch + prompt)
+    model = gpt_b200.Model(c, 0, torch.cuda.current_stream().cuda_stream, gpt_b200.MODE_3XTF32, use_grad=False)
+    flat = torch.cat([(torch.randn(*shape, device="cuda", generator=gen) * 0.05 + (1.0 if name in ("ln1_w", "ln2_w", "lnf_w") else 0.0)).reshape(-1) for name, shape in _shapes(c)])
+    assert flat.numel() == model.num_params
+    model.load_weights(flat.cpu().numpy())
+    text = torch.randint(0, c["vocab_size"], (batch, prompt + steps), device="cuda", dtype=torch.int32, generator=gen)
+    want = _forward(torch, c, flat.double(), text)[:, prompt:]
+    for _ in range(2):      # a second text in the same buffers
+        model.generate_begin(text[:, :prompt].contiguous(), batch, prompt, prompt + steps)
+        out = torch.full((steps, batch, c["vocab_size_padded"]), float("nan"), device="cuda")
+        for i in range(steps):
+            model.generate_step(text[:, prompt + i].contiguous(), out[i])
+        torch.cuda.synchronize()
+        got = out.transpose(0, 1).double()
+        assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+    assert model.generate_position == prompt + steps
+    model.close()
