@@ -375,7 +375,7 @@ public:
             const int rc = kernels(parts, n, n);
             generating_ = false;
             RC_TRY(rc);
-            RC_TRY(launch(sample_advance_kernel, dim3(n), dim3(512), 0, tokens_, history_, gen_control_, logits_, c_.vocab, vocab_pitch_, entries_));
+            RC_TRY(launch(sample_advance_kernel, dim3(kSampleCluster, n), dim3(kSampleThreads), 0, tokens_, history_, gen_control_, logits_, c_.vocab, vocab_pitch_, entries_));
             return launch(advance_step_kernel, dim3(1), dim3(1), 0, gen_control_);
         };
         const bool reuse = graph_ && graph_n_ == n && graph_len_ == longest && graph_history_ == history_;
