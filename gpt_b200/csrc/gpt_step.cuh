@@ -50,16 +50,17 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(
 __device__ __forceinline__ float dot4(float4 a, float4 b, float s) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s)))); }
 
 // Sum of the slices' partial sums at one position, slice order; `stride` floats between slices.  Written by other blocks of this launch: read from L2.
+template <int FLIGHT = 12>
 __device__ __forceinline__ float4 sum_parts4(const float *p, int splits, int stride)
 {
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (; splits > 0; splits -= 12) {   // twelve loads in flight: one L2 round trip for what the plan makes of GPT-2
-        float4 v[12];
+    for (; splits > 0; splits -= FLIGHT) {   // loads in flight: one L2 round trip for what the plan makes of GPT-2
+        float4 v[FLIGHT];
 #pragma unroll
-        for (int i = 0; i < 12; ++i, p += stride)
+        for (int i = 0; i < FLIGHT; ++i, p += stride)
             v[i] = i < splits ? __ldcg(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int i = 0; i < 12; ++i) sum = add4(sum, v[i]);
+        for (int i = 0; i < FLIGHT; ++i) sum = add4(sum, v[i]);
     }
     return sum;
 }
@@ -74,6 +75,21 @@ __device__ __forceinline__ float sum_parts(const float *p, int splits, int strid
             if (i < splits) v[i] = __ldcg(p);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
+            if (i < splits) sum += v[i];
+    }
+    return sum;
+}
+
+__device__ __forceinline__ float sum_parts8(const float *p, int splits, int stride)
+{
+    float sum = 0.0f;
+    for (; splits > 0; splits -= 8) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i, p += stride)
+            if (i < splits) v[i] = __ldcg(p);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
             if (i < splits) sum += v[i];
     }
     return sum;
@@ -484,6 +500,335 @@ gpt_step_kernel(const GptStep s, int widest)
             }
         }
     }
+    if (blockIdx.x == 0 && tid == 0) {   // every block has passed a barrier since it read them
+        *s.pos = p + 1;
+        s.sync[1] = target;
+    }
+}
+
+// ---- three to 64 rows --------------------------------------------------------------------------------------------------------
+// Here the fp32 FMAs weigh as much as the weights (64 rows: 10.9 GFLOP for the layers of GPT-2 124M, 0.15 ms of all FMA lanes), so an item's
+// weights and activations sit in shared memory and a thread computes ROWS / 8 rows x 8 columns; the four quarters of the block take a
+// quarter of the slice's k each.  An item is 128 columns x up to 128 k-rows (64 KB of weights): wide enough that the activations, which every column
+// group loads (and puts through the GELU) again, stay cheaper than the FMAs.  Its weights are requested as soon as the previous item's
+// main loop is over.  The norms and the attention are phases of their own: seven barriers per layer.
+constexpr int kWideCols = 128, kWideSlice = 128;
+constexpr int kQuarter = kThreads / 4;
+
+// Two fp32 FMAs of one instruction: d = a * b + d, element by element.
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long twice(float v)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+
+// x * sigmoid(2 u) = 0.5 x (1 + tanh u) without the cancellation at negative x.
+__device__ __forceinline__ float gelu_step(float x)
+{
+    const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
+    return __fdividef(x, 1.0f + expf(-2.0f * u));
+}
+
+__device__ __forceinline__ void quarter_sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + static_cast<int>(threadIdx.x) / kQuarter), "n"(kQuarter) : "memory"); }
+
+constexpr size_t wide_shared_floats(int rows) { return size_t(kWideSlice) * kWideCols + size_t(kWideSlice) * (rows + 4) + size_t(3) * rows * kWideCols; }
+// of which attention uses what is not weights: four quarters with a head's new q, k, v, parts of its output and the scores
+inline bool wide_attention_fits(int rows, int hd, int max_len)
+{
+    return 4 * (size_t(3) * hd + size_t(4) * (hd + 4) + ((max_len + 3) & ~3)) <= wide_shared_floats(rows) - size_t(kWideSlice) * kWideCols;
+}
+
+template <int ROWS>
+__global__ void __launch_bounds__(kThreads, 1)
+gpt_step_rows_kernel(const GptStep s)
+{
+    constexpr int RT = ROWS / 8, P = ROWS + 4;   // rows per thread; pitch of the activations
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float4 moments[kWarps];
+    float *ws = sm;                               // [kWideSlice][kWideCols]
+    float *xs = ws + kWideSlice * kWideCols;      // [kWideSlice][P]
+    float *sums = xs + kWideSlice * P;            // [3][ROWS][kWideCols]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = s.d, batch = s.batch, first = blockIdx.x;
+    const int p = *s.pos;
+    if (p < 0 || p >= s.max_len || p >= s.max_pos) return;   // all blocks alike
+    unsigned target = s.sync[1];
+
+    auto fetch = [&](const float *w, const StepPhase &ph, int item) {   // an item's weights, asynchronously; zeros beyond its rows and columns
+        const int split = item / ph.groups, col = (item - split * ph.groups) * kWideCols + lane * 4;
+        const int k0 = split * ph.slice, rows = item < ph.groups * ph.splits ? min(ph.K - k0, ph.slice) : 0;
+        const float *src = w + static_cast<size_t>(k0 + warp) * ph.N + col;
+        const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(ws + warp * kWideCols + lane * 4));
+        const bool in = col < ph.N;
+        for (int k = 0; k + warp < rows; k += kWarps)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + k * kWideCols * 4), "l"(in ? src + static_cast<size_t>(k) * ph.N : w), "r"(in ? 16 : 0) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    // The activations of an item, [k][row]: a warp takes pieces of eight rows x sixteen k.  load(row, k): four values from k on of a row < batch.
+    auto stage = [&](int k0, int rows, auto load) {
+        const int pieces = (ROWS / 8) * ((rows + 15) >> 4);
+        for (int t0 = warp; t0 < pieces; t0 += 2 * kWarps) {
+            float4 v[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = t0 + i * kWarps, row = (t % (ROWS / 8)) * 8 + (lane & 7), k = (t / (ROWS / 8)) * 16 + (lane >> 3) * 4;
+                v[i] = t < pieces && row < batch && k < rows ? load(row, k0 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = t0 + i * kWarps, row = (t % (ROWS / 8)) * 8 + (lane & 7), k = (t / (ROWS / 8)) * 16 + (lane >> 3) * 4;
+                if (t < pieces && k < rows) {
+                    xs[k * P + row] = v[i].x;
+                    xs[(k + 1) * P + row] = v[i].y;
+                    xs[(k + 2) * P + row] = v[i].z;
+                    xs[(k + 3) * P + row] = v[i].w;
+                }
+            }
+        }
+    };
+
+    // One phase of products; `next`: requests the weights of this block's first item of the next product.
+    const int quarter = tid / kQuarter, cg = tid & 15, rg = (tid >> 4) & 7;
+    auto product = [&](const float *w, const StepPhase &ph, float *part, auto load, auto next) {
+        const int items = ph.groups * ph.splits;
+        if (first >= items) next();
+        for (int item = first; item < items; item += gridDim.x) {
+            const int split = item / ph.groups, col0 = (item - split * ph.groups) * kWideCols, k0 = split * ph.slice, rows = min(ph.K - k0, ph.slice);
+            if (item != first) __syncthreads();   // the sums of the item before have been read
+            stage(k0, rows, load);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            unsigned long long acc[RT][4];   // columns (4 cg, + 1), (4 cg + 2, + 3), and the same 64 further on
+#pragma unroll
+            for (int r = 0; r < RT; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = 0ull;
+            const int per = (rows + 3) >> 2, kb = quarter * per, ke = min(rows, kb + per);
+            const float *wp = ws + kb * kWideCols + cg * 4, *xp = xs + kb * P + rg * RT;
+#pragma unroll 4
+            for (int k = kb; k < ke; ++k, wp += kWideCols, xp += P) {
+                const ulonglong2 wa = *reinterpret_cast<const ulonglong2 *>(wp), wb = *reinterpret_cast<const ulonglong2 *>(wp + 64);
+                float x[RT];
+                if constexpr (RT >= 4) {
+#pragma unroll
+                    for (int r = 0; r < RT; r += 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(xp + r);
+                        x[r] = v.x; x[r + 1] = v.y; x[r + 2] = v.z; x[r + 3] = v.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < RT; ++r) x[r] = xp[r];
+                }
+#pragma unroll
+                for (int r = 0; r < RT; ++r) {
+                    const unsigned long long xx = twice(x[r]);
+                    fma2(acc[r][0], wa.x, xx);
+                    fma2(acc[r][1], wa.y, xx);
+                    fma2(acc[r][2], wb.x, xx);
+                    fma2(acc[r][3], wb.y, xx);
+                }
+            }
+            __syncthreads();   // the weights and activations have been read
+            if (item + static_cast<int>(gridDim.x) < items)
+                fetch(w, ph, item + gridDim.x);
+            else
+                next();
+            if (quarter > 0) {
+#pragma unroll
+                for (int r = 0; r < RT; ++r) {
+                    float *dst = sums + ((quarter - 1) * ROWS + rg * RT + r) * kWideCols + cg * 4;
+                    *reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(acc[r][0], acc[r][1]);
+                    *reinterpret_cast<ulonglong2 *>(dst + 64) = make_ulonglong2(acc[r][2], acc[r][3]);
+                }
+            }
+            // the first quarter's sums go where the activations were
+            if (quarter == 0) {
+#pragma unroll
+                for (int r = 0; r < RT; ++r) {
+                    float *dst = xs + (rg * RT + r) * kWideCols + cg * 4;
+                    *reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(acc[r][0], acc[r][1]);
+                    *reinterpret_cast<ulonglong2 *>(dst + 64) = make_ulonglong2(acc[r][2], acc[r][3]);
+                }
+            }
+            __syncthreads();
+            for (int i = tid; i < batch * (kWideCols / 4); i += kThreads) {
+                const int row = i >> 5, c = (i & 31) * 4;
+                if (col0 + c >= ph.N) continue;
+                float4 v = *reinterpret_cast<const float4 *>(xs + row * kWideCols + c);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) v = add4(v, *reinterpret_cast<const float4 *>(sums + (q * ROWS + row) * kWideCols + c));
+                *reinterpret_cast<float4 *>(part + (static_cast<size_t>(split) * batch + row) * ph.N + col0 + c) = v;
+            }
+        }
+    };
+
+    // res += a finished product (none: the embedding), normed = its norm; a block per row
+    auto norm_phase = [&](const float *part, const StepPhase &ph, const float *bias, const float *gain, const float *shift) {
+        float *row_sm = xs, *half_sm = xs + d;   // both fit: see the plan
+        constexpr int kHalf = kThreads / 2;
+        const int half = tid / kHalf, at = (tid % kHalf) * 4, cut = (ph.splits + 1) / 2;
+        for (int row = first; row < batch; row += gridDim.x) {
+            __syncthreads();
+            if (part) {   // each half of the block adds up half of the slices
+                for (int c = at; c < d; c += kHalf * 4) {
+                    const float4 v = sum_parts4(part + static_cast<size_t>(half ? cut : 0) * batch * d + row * d + c, half ? ph.splits - cut : cut, batch * d);
+                    if (half) *reinterpret_cast<float4 *>(half_sm + c) = v; else *reinterpret_cast<float4 *>(row_sm + c) = v;
+                }
+                __syncthreads();
+            }
+            for (int c = tid * 4; c < d; c += kThreads * 4) {
+                float4 v;
+                if (part) {
+                    v = add4(add4(*reinterpret_cast<const float4 *>(row_sm + c), *reinterpret_cast<const float4 *>(half_sm + c)), __ldg(reinterpret_cast<const float4 *>(bias + c)));
+                    v = add4(__ldcg(reinterpret_cast<const float4 *>(s.res + row * d + c)), v);
+                } else {
+                    v = add4(__ldg(reinterpret_cast<const float4 *>(s.wte + static_cast<size_t>(s.tokens[row]) * d + c)),
+                             __ldg(reinterpret_cast<const float4 *>(s.wpe + static_cast<size_t>(p) * d + c)));
+                }
+                *reinterpret_cast<float4 *>(row_sm + c) = v;
+                __stcg(reinterpret_cast<float4 *>(s.res + row * d + c), v);
+            }
+            warp_moments<1>(row_sm, d, moments);   // a thread reads what it wrote
+            __syncthreads();
+            float mean[1], sd[1];
+            row_statistics<1>(moments, d, mean, sd);
+            for (int c = tid * 4; c < d; c += kThreads * 4) {
+                const float4 v = *reinterpret_cast<const float4 *>(row_sm + c), ga = __ldg(reinterpret_cast<const float4 *>(gain + c)), be = __ldg(reinterpret_cast<const float4 *>(shift + c));
+                *reinterpret_cast<float4 *>(s.normed + row * d + c) = make_float4((v.x - mean[0]) / sd[0] * ga.x + be.x, (v.y - mean[0]) / sd[0] * ga.y + be.y,
+                                                                                  (v.z - mean[0]) / sd[0] * ga.z + be.z, (v.w - mean[0]) / sd[0] * ga.w + be.w);
+            }
+        }
+    };
+
+    const int head_log = 31 - __clz(s.hd), per_pos = s.hd >> 2, groups = kQuarter / per_pos;
+    const int qt = tid & (kQuarter - 1), g = qt >> (head_log - 2), c4 = (qt & (per_pos - 1)) * 4, row_stride = 2 * d * groups;
+    float *fresh = xs + quarter * (3 * s.hd + 4 * (s.hd + 4) + ((s.max_len + 3) & ~3));   // [3][hd]
+    float *out = fresh + 3 * s.hd, *prob = out + 4 * (s.hd + 4);                            // [4][hd + 4], [max_len]
+    // a quarter of a block per (sequence, head)
+    auto attention = [&](float *cache, const float *qkv_b) {
+        for (int item = first * 4 + quarter; item < batch * s.heads; item += gridDim.x * 4) {
+            const int m = item / s.heads, at = (item - m * s.heads) << head_log;
+            float *keys = cache + static_cast<size_t>(m) * s.max_len * 2 * d + at;
+            for (int i = qt; i < 3 * s.hd; i += kQuarter) {
+                const int which = i >> head_log, e = i & (s.hd - 1), col = which * d + at + e;
+                const float be = __ldg(qkv_b + col);
+                const float v = sum_parts8(s.qkv_part + static_cast<size_t>(m) * 3 * d + col, s.qkv.splits, batch * 3 * d) + be;
+                fresh[i] = v;
+                if (which > 0) keys[static_cast<size_t>(p) * 2 * d + (which - 1) * d + e] = v;
+            }
+            quarter_sync();
+            const float *q = fresh + c4, *row = keys + static_cast<size_t>(g) * 2 * d + c4;
+            const float4 q4 = *reinterpret_cast<const float4 *>(q);
+            for (int t0 = 0; t0 <= p; t0 += 4 * groups, row += 4 * row_stride) {   // four rows in flight per thread
+                float4 kv[4];
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int t = t0 + g + j * groups;
+                    kv[j] = t < p ? *reinterpret_cast<const float4 *>(row + j * row_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (t == p) kv[j] = *reinterpret_cast<const float4 *>(q + s.hd);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = dot4(q4, kv[j], 0.0f);
+                for (int o = per_pos >> 1; o > 0; o >>= 1)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+                if (c4 == 0)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (t0 + g + j * groups <= p) prob[t0 + g + j * groups] = v[j] * s.scale;
+            }
+            quarter_sync();
+            float mx = -FLT_MAX, weights = 0.0f;
+            for (int t = lane; t <= p; t += 32) mx = fmaxf(mx, prob[t]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            row = keys + d + static_cast<size_t>(g) * 2 * d + c4;
+            for (int t0 = 0; t0 + g <= p; t0 += 4 * groups, row += 4 * row_stride) {
+                float4 kv[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int t = t0 + g + j * groups;
+                    kv[j] = t < p ? *reinterpret_cast<const float4 *>(row + j * row_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (t == p) kv[j] = *reinterpret_cast<const float4 *>(q + 2 * s.hd);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (t0 + g + j * groups <= p) {
+                        const float e = expf(prob[t0 + g + j * groups] - mx);
+                        weights += e;
+                        acc.x = fmaf(e, kv[j].x, acc.x);
+                        acc.y = fmaf(e, kv[j].y, acc.y);
+                        acc.z = fmaf(e, kv[j].z, acc.z);
+                        acc.w = fmaf(e, kv[j].w, acc.w);
+                    }
+            }
+            for (int o = per_pos; o < 32; o <<= 1) {
+                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+                acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+                acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+                weights += __shfl_xor_sync(0xffffffffu, weights, o);
+            }
+            float *mine = out + (warp & 3) * (s.hd + 4);
+            if (lane < per_pos) *reinterpret_cast<float4 *>(mine + c4) = acc;
+            if (lane == 0) mine[s.hd] = weights;
+            quarter_sync();
+            if (qt < s.hd) {   // heads are at most 128 wide
+                float v = 0.0f, sum = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v += out[j * (s.hd + 4) + qt];
+                    sum += out[j * (s.hd + 4) + s.hd];
+                }
+                s.attn[static_cast<size_t>(m) * d + at + qt] = v / sum;
+            }
+            quarter_sync();   // the next item writes fresh
+        }
+    };
+
+    fetch(s.qkv_w, s.qkv, first);
+    auto from = [&](const float *x, int K) { return [=](int row, int k) { return __ldcg(reinterpret_cast<const float4 *>(x + static_cast<size_t>(row) * K + k)); }; };
+    for (int l = 0; l < s.layers; ++l) {
+        const float *qkv_w = s.qkv_w + static_cast<size_t>(l) * d * 3 * d, *proj_w = s.proj_w + static_cast<size_t>(l) * d * d;
+        const float *up_w = s.up_w + static_cast<size_t>(l) * d * s.ffn, *down_w = s.down_w + static_cast<size_t>(l) * s.ffn * d;
+        float *cache = s.cache + static_cast<size_t>(l) * batch * s.max_len * 2 * d;
+        norm_phase(l > 0 ? s.down_part : nullptr, s.down, s.down_b + (l - 1) * d, s.ln1_w + l * d, s.ln1_b + l * d);
+        arrive(s, target);
+        await(s, target);
+        product(qkv_w, s.qkv, s.qkv_part, from(s.normed, d), [&] { fetch(proj_w, s.proj, first); });
+        arrive(s, target);
+        await(s, target);
+        attention(cache, s.qkv_b + l * 3 * d);
+        arrive(s, target);
+        await(s, target);
+        product(proj_w, s.proj, s.proj_part, from(s.attn, d), [&] { fetch(up_w, s.up, first); });
+        arrive(s, target);
+        await(s, target);
+        norm_phase(s.proj_part, s.proj, s.proj_b + l * d, s.ln2_w + l * d, s.ln2_b + l * d);
+        arrive(s, target);
+        await(s, target);
+        product(up_w, s.up, s.up_part, from(s.normed, d), [&] { fetch(down_w, s.down, first); });
+        arrive(s, target);
+        await(s, target);
+        const float *up_b = s.up_b + l * s.ffn;
+        product(down_w, s.down, s.down_part,
+                [&](int row, int k) {
+                    const float4 be = __ldg(reinterpret_cast<const float4 *>(up_b + k));
+                    const float4 v = add4(sum_parts4<6>(s.up_part + static_cast<size_t>(row) * s.ffn + k, s.up.splits, batch * s.ffn), be);
+                    return make_float4(gelu_step(v.x), gelu_step(v.y), gelu_step(v.z), gelu_step(v.w));
+                },
+                [&] { if (l + 1 < s.layers) fetch(qkv_w + static_cast<size_t>(d) * 3 * d, s.qkv, first); });
+        arrive(s, target);
+        await(s, target);
+    }
+    norm_phase(s.down_part, s.down, s.down_b + (s.layers - 1) * d, s.lnf_w, s.lnf_b);   // the product with the embedding is another launch
     if (blockIdx.x == 0 && tid == 0) {   // every block has passed a barrier since it read them
         *s.pos = p + 1;
         s.sync[1] = target;

@@ -15,6 +15,7 @@ struct StepPhase {
 };
 
 struct GptStep {
+    int rows;               // 0: the kernel of one or two rows; else the padded row count of the other
     int batch, layers, d, ffn, heads, hd, vocab_p, max_len, max_pos;
     float scale;
     // weights, fp32; layers of a kind one after another

@@ -44,7 +44,9 @@ SIZES = {
 
 @pytest.mark.parametrize("size,batch,layers,prompt,steps", [
     ("gpt2", 1, 2, 60, 12), ("gpt2", 2, 2, 125, 8), ("gpt2", 1, 12, 1, 6), ("head8", 1, 3, 7, 40), ("head8", 2, 1, 31, 3), ("head128", 2, 2, 5, 70),
-    ("wide", 1, 2, 130, 4), ("wide", 2, 1, 9, 3), ("head128", 1, 1, 1, 1)])
+    ("wide", 1, 2, 130, 4), ("wide", 2, 1, 9, 3), ("head128", 1, 1, 1, 1),
+    ("gpt2", 3, 2, 61, 6), ("gpt2", 8, 3, 9, 4), ("gpt2", 9, 1, 33, 3), ("gpt2", 16, 1, 5, 3), ("gpt2", 17, 2, 130, 4), ("gpt2", 32, 1, 3, 3), ("gpt2", 33, 1, 64, 3), ("gpt2", 64, 2, 70, 5),
+    ("head8", 5, 2, 3, 30), ("head8", 40, 1, 17, 3), ("head128", 12, 2, 6, 5), ("wide", 4, 1, 20, 3), ("wide", 50, 1, 8, 3), ("gpt2", 65, 1, 5, 2)])
 def test_generation_step_matches_the_whole_forward_pass(size, batch, layers, prompt, steps):
     """Logits of every step within 1e-5 of their scale (fp32 sums of up to 6400 terms, layer after layer; the same bound as for the
     operator-by-operator step)."""
