@@ -88,8 +88,8 @@ bool plan_rows(GptStep &s, int blocks)
     s.proj = plan_phase(s.d, s.d, blocks, 8, step::kWideCols, step::kWideSlice, 32);
     s.up = plan_phase(s.d, s.ffn, blocks, 8, step::kWideCols, step::kWideSlice, 32);
     s.down = plan_phase(s.ffn, s.d, blocks, 8, step::kWideCols, step::kWideSlice, 32);
-    // the norms keep a row and half of its sum where the products have activations and sums
-    return 2 * size_t(s.d) <= step::wide_shared_floats(s.rows) - size_t(step::kWideSlice) * step::kWideCols && step::wide_attention_fits(s.rows, s.hd, s.max_len);
+    // the norms keep a row and half of its sum there
+    return 2 * size_t(s.d) <= step::wide_scratch_floats(s.rows) && step::wide_attention_fits(s.rows, s.hd, s.max_len);
 }
 
 }  // namespace

@@ -54,6 +54,7 @@ template <int FLIGHT = 12>
 __device__ __forceinline__ float4 sum_parts4(const float *p, int splits, int stride)
 {
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
     for (; splits > 0; splits -= FLIGHT) {   // loads in flight: one L2 round trip for what the plan makes of GPT-2
         float4 v[FLIGHT];
 #pragma unroll
@@ -68,6 +69,7 @@ __device__ __forceinline__ float4 sum_parts4(const float *p, int splits, int str
 __device__ __forceinline__ float sum_parts(const float *p, int splits, int stride)
 {
     float sum = 0.0f;
+#pragma unroll 1
     for (; splits > 0; splits -= 4) {
         float v[4];
 #pragma unroll
@@ -75,21 +77,6 @@ __device__ __forceinline__ float sum_parts(const float *p, int splits, int strid
             if (i < splits) v[i] = __ldcg(p);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            if (i < splits) sum += v[i];
-    }
-    return sum;
-}
-
-__device__ __forceinline__ float sum_parts8(const float *p, int splits, int stride)
-{
-    float sum = 0.0f;
-    for (; splits > 0; splits -= 8) {
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i, p += stride)
-            if (i < splits) v[i] = __ldcg(p);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
             if (i < splits) sum += v[i];
     }
     return sum;
@@ -143,6 +130,7 @@ __device__ __forceinline__ void item_product(float4 (&wv)[kBody], const float *w
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float *x = xs + (threadIdx.x >> 4);
     float acc[MR][4] = {};
+#pragma unroll 1
     for (int done = 0; done * 32 < r.rows; done += kBody, x += 32 * kBody) {
         if (done > 0) fetch(wv, w, ph, r, done);
 #pragma unroll
@@ -183,14 +171,17 @@ __device__ __forceinline__ void warp_moments(const float *row, int d, float4 *pa
     const int at = (threadIdx.x % kPer) * 4, lane = threadIdx.x & 31;
     if (at - lane * 4 >= d) return;
     float sum = 0.0f, n = 0.0f, var = 0.0f;
+#pragma unroll 1
     for (int i = at; i < d; i += kPer * 4) {
         const float4 v = *reinterpret_cast<const float4 *>(row + i);
         sum += (v.x + v.y) + (v.z + v.w);
     }
+#pragma unroll 1
     for (int i = at - lane * 4; i < d; i += kPer * 4) n += static_cast<float>(min(d - i, 128));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float mean = sum / n;
+#pragma unroll 1
     for (int i = at; i < d; i += kPer * 4) {
         const float4 v = *reinterpret_cast<const float4 *>(row + i);
         const float a = v.x - mean, b = v.y - mean, c = v.z - mean, e = v.w - mean;
@@ -249,6 +240,7 @@ gpt_step_kernel(const GptStep s, int widest)
 
     constexpr int kPer = kThreads / MR;   // threads of a row
     const int mine = tid / kPer, at4 = (tid % kPer) * 4;
+#pragma unroll 1
     for (int c = at4; c < d; c += kPer * 4)
         *reinterpret_cast<float4 *>(res + mine * d + c) = mine < s.batch ? add4(__ldg(reinterpret_cast<const float4 *>(s.wte + static_cast<size_t>(s.tokens[mine]) * d + c)),
                                                                                __ldg(reinterpret_cast<const float4 *>(s.wpe + static_cast<size_t>(p) * d + c)))
@@ -259,6 +251,7 @@ gpt_step_kernel(const GptStep s, int widest)
     // res += the finished product, with the moments of the new rows
     auto add_result = [&](const float *part, const StepPhase &ph, const float *bias) {
         if (mine < s.batch)
+#pragma unroll 1
             for (int c = at4; c < d; c += kPer * 4) {
                 const float4 be = __ldg(reinterpret_cast<const float4 *>(bias + c));
                 const float4 v = add4(sum_parts4(part + mine * d + c, ph.splits, s.batch * d), be);
@@ -279,6 +272,7 @@ gpt_step_kernel(const GptStep s, int widest)
     auto normed_product = [&](const float *w, const StepPhase &ph, const Share &one, const float *gain, const float *bias, float *part) {
         float mean[MR], sd[MR];
         Share r = one;
+#pragma unroll 1
         for (int item = first; item < ph.groups * ph.splits; item += gridDim.x) {
             if (item != first) {
                 r = share_of(ph, item);
@@ -288,6 +282,7 @@ gpt_step_kernel(const GptStep s, int widest)
             }
             if (warp * 32 < r.rows) {
                 row_statistics<MR>(moments, d, mean, sd);
+#pragma unroll 1
                 for (int k = tid; k < r.rows; k += kThreads) {
                     const float ga = k == tid ? gain0 : __ldg(gain + r.k0 + k), be = k == tid ? bias0 : __ldg(bias + r.k0 + k);
 #pragma unroll
@@ -303,37 +298,59 @@ gpt_step_kernel(const GptStep s, int widest)
     // a head's size is a power of two: lanes of a cached row, rows at a time
     const int head_log = 31 - __clz(s.hd), per_pos = s.hd >> 2, groups = kThreads / per_pos;
     const int g = tid >> (head_log - 2), c4 = (tid & (per_pos - 1)) * 4, row_stride = 2 * d * groups;
-    for (int l = 0; l < s.layers; ++l) {
-        const float *proj_w = s.proj_w + static_cast<size_t>(l) * d * d;
-        if (l > 0) add_result(s.down_part, s.down, s.down_b + (l - 1) * d);
-        normed_product(s.qkv_w + static_cast<size_t>(l) * d * 3 * d, s.qkv, of_qkv, s.ln1_w + l * d, s.ln1_b + l * d, s.qkv_part);
+    const size_t dd = static_cast<size_t>(d) * d, df = static_cast<size_t>(d) * s.ffn;
+    // half layers: qkv, attention, projection; up, GELU, down.  Their common parts are in the code once: inlined per use the kernel had 150 KB of code,
+    // more than the instruction caches hold.
+#pragma unroll 1
+    for (int n = 0;; ++n) {
+        const int l = n >> 1;
+        const bool half = n & 1;
+        if (n > 0) add_result(half ? s.proj_part : s.down_part, half ? s.proj : s.down, half ? s.proj_b + l * d : s.down_b + (l - 1) * d);
+        if (n == 2 * s.layers) break;
+        normed_product(half ? s.up_w + df * l : s.qkv_w + 3 * dd * l, half ? s.up : s.qkv, half ? of_up : of_qkv, (half ? s.ln2_w : s.ln1_w) + l * d, (half ? s.ln2_b : s.ln1_b) + l * d,
+                       half ? s.up_part : s.qkv_part);
         arrive(s, target);
+        const float *w = half ? s.down_w + df * l : s.proj_w + dd * l;
+        const StepPhase ph = half ? s.down : s.proj;
+        const Share mine_of = half ? of_down : of_proj;
+        fetch(wv, w, ph, mine_of);
         float *cache = s.cache + static_cast<size_t>(l) * s.batch * s.max_len * 2 * d;
-        fetch(wv, proj_w, s.proj, of_proj);
         // and the first cached rows of this block's first head
         float4 k_first[4], v_first[4];
         {
             const float *row = cache + static_cast<size_t>(g) * 2 * d + of_proj.k0 + c4;
 #pragma unroll
             for (int j = 0; j < 4; ++j, row += row_stride) {
-                const bool live = of_proj.rows > 0 && g + j * groups < p;
+                const bool live = !half && of_proj.rows > 0 && g + j * groups < p;
                 k_first[j] = live ? *reinterpret_cast<const float4 *>(row) : make_float4(0.f, 0.f, 0.f, 0.f);
                 v_first[j] = live ? *reinterpret_cast<const float4 *>(row + d) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
         await(s, target);
 
-        const float *up_w = s.up_w + static_cast<size_t>(l) * d * s.ffn, *down_w = s.down_w + static_cast<size_t>(l) * s.ffn * d;
-        // attention of the heads in the item's slice of k, then the slice's share of the projection
-        Share r = of_proj;
-        for (int item = first; item < s.proj.groups * s.proj.splits; item += gridDim.x) {
+        Share r = mine_of;
+#pragma unroll 1
+        for (int item = first; item < ph.groups * ph.splits; item += gridDim.x) {
             if (item != first) {
-                r = share_of(s.proj, item);
-                fetch(wv, proj_w, s.proj, r);
+                r = share_of(ph, item);
+                fetch(wv, w, ph, r);
             }
-            for (int at = 0; at < r.rows; at += s.hd) {   // head by head
+            if (half) {   // the finished up product through the GELU
+                if (item != first) __syncthreads();
+#pragma unroll 1
+                for (int m = 0; m < MR; ++m)
+#pragma unroll 1
+                    for (int k = tid; k < r.rows; k += kThreads) {
+                        const float be = __ldg(s.up_b + l * s.ffn + r.k0 + k);
+                        xs[m * widest + k] = m < s.batch ? gelu_tanh(sum_parts(s.up_part + m * s.ffn + r.k0 + k, s.up.splits, s.batch * s.ffn) + be) : 0.0f;
+                    }
+            }
+            // or the attention of the heads in the item's slice of k
+#pragma unroll 1
+            for (int at = half ? r.rows : 0; at < r.rows; at += s.hd) {
                 const bool fetched = item == first && at == 0;   // k_first, v_first are this head's, row 0
                 if (!fetched) __syncthreads();
+#pragma unroll 1
                 for (int i = tid; i < s.batch * 3 * s.hd; i += kThreads) {
                     const int row = i >> head_log, m = MR == 1 ? 0 : row / 3, which = row - 3 * m, e = i & (s.hd - 1), col = which * d + r.k0 + at + e;
                     const float be = __ldg(s.qkv_b + l * 3 * d + col);
@@ -342,10 +359,12 @@ gpt_step_kernel(const GptStep s, int widest)
                     if (which > 0 && r.col == 0) cache[(static_cast<size_t>(m) * s.max_len + p) * 2 * d + (col - d)] = v;
                 }
                 __syncthreads();
+#pragma unroll 1
                 for (int m = 0; m < s.batch; ++m) {
                     const float *q = fresh + m * 3 * s.hd + c4, *row = cache + (static_cast<size_t>(m) * s.max_len + g) * 2 * d + r.k0 + at + c4;
                     const float4 q4 = *reinterpret_cast<const float4 *>(q);
                     float *probs = prob + m * s.max_len;
+#pragma unroll 1
                     for (int t0 = 0; t0 <= p; t0 += 4 * groups, row += 4 * row_stride) {   // four rows in flight per thread
                         float4 kv[4];
                         float v[4];
@@ -357,6 +376,7 @@ gpt_step_kernel(const GptStep s, int widest)
                         }
 #pragma unroll
                         for (int j = 0; j < 4; ++j) v[j] = dot4(q4, kv[j], 0.0f);
+#pragma unroll 1
                         for (int o = per_pos >> 1; o > 0; o >>= 1)
 #pragma unroll
                             for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
@@ -367,14 +387,17 @@ gpt_step_kernel(const GptStep s, int widest)
                     }
                 }
                 __syncthreads();
+#pragma unroll 1
                 for (int m = 0; m < s.batch; ++m) {
                     const float *q = fresh + m * 3 * s.hd + c4, *row = cache + (static_cast<size_t>(m) * s.max_len + g) * 2 * d + d + r.k0 + at + c4;
                     float *probs = prob + m * s.max_len;
                     float mx = -FLT_MAX, weights = 0.0f;
+#pragma unroll 1
                     for (int t = lane; t <= p; t += 32) mx = fmaxf(mx, probs[t]);
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
                     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
                     for (int t0 = 0; t0 + g <= p; t0 += 4 * groups, row += 4 * row_stride) {
                         float4 kv[4];
 #pragma unroll
@@ -394,6 +417,7 @@ gpt_step_kernel(const GptStep s, int widest)
                                 acc.w = fmaf(e, kv[j].w, acc.w);
                             }
                     }
+#pragma unroll 1
                     for (int o = per_pos; o < 32; o <<= 1) {
                         acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
                         acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
@@ -416,58 +440,36 @@ gpt_step_kernel(const GptStep s, int widest)
                     }
                 }
             }
-            if (MR > 1 && s.batch < MR)
+            if (MR > 1 && s.batch < MR && !half)
+#pragma unroll 1
                 for (int i = tid; i < r.rows; i += kThreads) xs[widest + i] = 0.0f;
             __syncthreads();
-            item_product<MR>(wv, proj_w, s.proj, r, xs, widest, red, s.proj_part, s.batch);
+            item_product<MR>(wv, w, ph, r, xs, widest, red, half ? s.down_part : s.proj_part, s.batch);
         }
         arrive(s, target);
-        fetch(wv, up_w, s.up, of_up);
-        fetch_norm(of_up, s.ln2_w + l * d, s.ln2_b + l * d);
-        await(s, target);
-
-        add_result(s.proj_part, s.proj, s.proj_b + l * d);
-        normed_product(up_w, s.up, of_up, s.ln2_w + l * d, s.ln2_b + l * d, s.up_part);
-        arrive(s, target);
-        fetch(wv, down_w, s.down, of_down);
-        await(s, target);
-
-        r = of_down;
-        for (int item = first; item < s.down.groups * s.down.splits; item += gridDim.x) {
-            if (item != first) {
-                r = share_of(s.down, item);
-                fetch(wv, down_w, s.down, r);
-                __syncthreads();
-            }
-            for (int m = 0; m < MR; ++m)
-                for (int k = tid; k < r.rows; k += kThreads) {
-                    const float be = __ldg(s.up_b + l * s.ffn + r.k0 + k);
-                    xs[m * widest + k] = m < s.batch ? gelu_tanh(sum_parts(s.up_part + m * s.ffn + r.k0 + k, s.up.splits, s.batch * s.ffn) + be) : 0.0f;
-                }
-            __syncthreads();
-            item_product<MR>(wv, down_w, s.down, r, xs, widest, red, s.down_part, s.batch);
-        }
-        arrive(s, target);
-        if (l + 1 < s.layers) {
-            fetch(wv, s.qkv_w + static_cast<size_t>(l + 1) * d * 3 * d, s.qkv, of_qkv);
-            fetch_norm(of_qkv, s.ln1_w + (l + 1) * d, s.ln1_b + (l + 1) * d);
+        if (n + 1 < 2 * s.layers) {
+            const int next = (n + 1) >> 1;
+            fetch(wv, half ? s.qkv_w + 3 * dd * next : s.up_w + df * next, half ? s.qkv : s.up, half ? of_qkv : of_up);
+            fetch_norm(half ? of_qkv : of_up, (half ? s.ln1_w : s.ln2_w) + next * d, (half ? s.ln1_b : s.ln2_b) + next * d);
         }
         await(s, target);
     }
 
     // final norm; logits: a warp per pair of embedding rows
-    add_result(s.down_part, s.down, s.down_b + (s.layers - 1) * d);
     {
         float mean[MR], sd[MR];
         row_statistics<MR>(moments, d, mean, sd);
+#pragma unroll 1
         for (int k = tid; k < d; k += kThreads)
 #pragma unroll
             for (int m = 0; m < MR; ++m) xs[m * widest + k] = (res[m * d + k] - mean[m]) / sd[m] * __ldg(s.lnf_w + k) + __ldg(s.lnf_b + k);
     }
     __syncthreads();
+#pragma unroll 1
     for (int n = 2 * (blockIdx.x * kWarps + warp); n < s.vocab_p; n += 2 * kWarps * gridDim.x) {
         const float *wa = s.wte + static_cast<size_t>(n) * d, *wb = n + 1 < s.vocab_p ? wa + d : wa;
         float sa[MR] = {}, sb[MR] = {};
+#pragma unroll 1
         for (int k0 = lane * 4; k0 < d; k0 += 6 * 128) {
             float4 a[6], b[6];
 #pragma unroll
@@ -508,12 +510,14 @@ gpt_step_kernel(const GptStep s, int widest)
 
 // ---- three to 64 rows --------------------------------------------------------------------------------------------------------
 // Here the fp32 FMAs weigh as much as the weights (64 rows: 10.9 GFLOP for the layers of GPT-2 124M, 0.15 ms of all FMA lanes), so an item's
-// weights and activations sit in shared memory and a thread computes ROWS / 8 rows x 8 columns; the four quarters of the block take a
-// quarter of the slice's k each.  An item is 128 columns x up to 128 k-rows (64 KB of weights): wide enough that the activations, which every column
-// group loads (and puts through the GELU) again, stay cheaper than the FMAs.  Its weights are requested as soon as the previous item's
-// main loop is over.  The norms and the attention are phases of their own: seven barriers per layer.
+// weights and activations sit in shared memory and a thread computes ROWS / 8 rows x 8 columns, each quarter of the block a quarter of the
+// slice's k (reads of 16 bytes bound the loop: 4 x 4 values per thread over all of k took 13200 cycles for an item of 128 x 128, 8 x 4 with
+// the activations stored twice 17300, 8 x 8 10700; the FMAs alone 8200).  An item is 128 columns x up to 128 k-rows (64 KB of weights).  The
+// next item's weights are requested a piece at a time inside the main loop, into the other buffer: all at once the threads wait for HBM to
+// take them (3000 cycles), and as bulk copies one warp needs 6000 cycles to issue 128 rows.  The norms, the attention and the GELU are
+// phases of their own: eight barriers per layer.  Every kind of phase is in the code once: inlined per use the kernel had 184 KB of code, more than
+// the instruction caches hold, and all of it took twice as long.
 constexpr int kWideCols = 128, kWideSlice = 128;
-constexpr int kQuarter = kThreads / 4;
 
 // Two fp32 FMAs of one instruction: d = a * b + d, element by element.
 __device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b)
@@ -534,13 +538,19 @@ __device__ __forceinline__ float gelu_step(float x)
     return __fdividef(x, 1.0f + expf(-2.0f * u));
 }
 
-__device__ __forceinline__ void quarter_sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + static_cast<int>(threadIdx.x) / kQuarter), "n"(kQuarter) : "memory"); }
+template <int THREADS>
+__device__ __forceinline__ void group_sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + static_cast<int>(threadIdx.x) / THREADS), "n"(THREADS) : "memory"); }
 
-constexpr size_t wide_shared_floats(int rows) { return size_t(kWideSlice) * kWideCols + size_t(kWideSlice) * (rows + 4) + size_t(3) * rows * kWideCols; }
-// of which attention uses what is not weights: four quarters with a head's new q, k, v, parts of its output and the scores
+__host__ __device__ constexpr size_t wide_shared_floats(int rows) { return size_t(2) * kWideSlice * kWideCols + size_t(kWideSlice) * (rows + 4); }
+__host__ __device__ constexpr int wide_attention_threads(int rows) { return rows >= 32 ? 64 : 128; }   // per (sequence, head)
+// one of the buffers of weights with the activations beside it: what the sums, the norms and the attention use between products
+__host__ __device__ constexpr size_t wide_scratch_floats(int rows) { return size_t(kWideSlice) * kWideCols + size_t(kWideSlice) * (rows + 4); }
+// attention: for every item at work a head's new q, k, v, parts of its output and the scores
+__host__ __device__ constexpr int wide_attention_floats(int threads, int hd, int max_len) { return 3 * hd + threads / 32 * (hd + 4) + ((max_len + 3) & ~3); }
 inline bool wide_attention_fits(int rows, int hd, int max_len)
 {
-    return 4 * (size_t(3) * hd + size_t(4) * (hd + 4) + ((max_len + 3) & ~3)) <= wide_shared_floats(rows) - size_t(kWideSlice) * kWideCols;
+    const int threads = wide_attention_threads(rows);
+    return size_t(kThreads / threads) * wide_attention_floats(threads, hd, max_len) <= wide_scratch_floats(rows);
 }
 
 template <int ROWS>
@@ -550,37 +560,55 @@ gpt_step_rows_kernel(const GptStep s)
     constexpr int RT = ROWS / 8, P = ROWS + 4;   // rows per thread; pitch of the activations
     extern __shared__ __align__(16) float sm[];
     __shared__ float4 moments[kWarps];
-    float *ws = sm;                               // [kWideSlice][kWideCols]
-    float *xs = ws + kWideSlice * kWideCols;      // [kWideSlice][P]
-    float *sums = xs + kWideSlice * P;            // [3][ROWS][kWideCols]
+    float *xs = sm + kWideSlice * kWideCols;      // [kWideSlice][P] activations, between two buffers of weights [kWideSlice][kWideCols]
+    float *ws = sm, *ws_next = xs + kWideSlice * P;
+    auto scratch = [&] { return ws < xs ? ws : xs; };   // the current buffer of weights and the activations: neighbours, whichever buffer it is
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = s.d, batch = s.batch, first = blockIdx.x;
     const int p = *s.pos;
     if (p < 0 || p >= s.max_len || p >= s.max_pos) return;   // all blocks alike
     unsigned target = s.sync[1];
 
-    auto fetch = [&](const float *w, const StepPhase &ph, int item) {   // an item's weights, asynchronously; zeros beyond its rows and columns
-        const int split = item / ph.groups, col = (item - split * ph.groups) * kWideCols + lane * 4;
-        const int k0 = split * ph.slice, rows = item < ph.groups * ph.splits ? min(ph.K - k0, ph.slice) : 0;
-        const float *src = w + static_cast<size_t>(k0 + warp) * ph.N + col;
-        const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(ws + warp * kWideCols + lane * 4));
-        const bool in = col < ph.N;
-        for (int k = 0; k + warp < rows; k += kWarps)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + k * kWideCols * 4), "l"(in ? src + static_cast<size_t>(k) * ph.N : w), "r"(in ? 16 : 0) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    // Piece i of eight of an item's weights into the other buffer: 16 of its k-rows, one per warp; columns beyond the matrix are zeros.
+    struct Source {
+        const float *at;
+        unsigned dst, bytes;
+        int rows, stride;
+    };
+    auto source = [&](const float *w, const StepPhase &ph, int item) {
+        const int split = item / ph.groups, col = (item - split * ph.groups) * kWideCols + lane * 4, k0 = split * ph.slice;
+        Source r;
+        r.rows = item < ph.groups * ph.splits ? min(ph.K - k0, ph.slice) - warp : 0;
+        r.bytes = col < ph.N ? 16 : 0;
+        r.at = r.bytes ? w + static_cast<size_t>(k0 + warp) * ph.N + col : w;
+        r.stride = r.bytes ? kWarps * ph.N : 0;
+        r.dst = static_cast<unsigned>(__cvta_generic_to_shared(ws_next + warp * kWideCols + lane * 4));
+        return r;
+    };
+    auto fetch = [&](Source &r) {
+        if (r.rows > 0) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(r.dst), "l"(r.at), "r"(r.bytes) : "memory");
+        r.at += r.stride;
+        r.dst += kWarps * kWideCols * 4;
+        r.rows -= kWarps;
+    };
+    auto fetch_all = [&](const float *w, const StepPhase &ph, int item) {
+        Source r = source(w, ph, item);
+#pragma unroll 1
+        while (r.rows > 0) fetch(r);
     };
 
-    // The activations of an item, [k][row]: a warp takes pieces of eight rows x sixteen k.  load(row, k): four values from k on of a row < batch.
-    auto stage = [&](int k0, int rows, auto load) {
+    // The activations of an item, [k][row]: a warp takes pieces of eight rows x sixteen k.
+    auto stage = [&](int k0, int rows, const float *x, int pitch) {
         const int pieces = (ROWS / 8) * ((rows + 15) >> 4);
-        for (int t0 = warp; t0 < pieces; t0 += 2 * kWarps) {
-            float4 v[2];
+#pragma unroll 1
+        for (int t0 = warp; t0 < pieces; t0 += 4 * kWarps) {
+            float4 v[4];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 const int t = t0 + i * kWarps, row = (t % (ROWS / 8)) * 8 + (lane & 7), k = (t / (ROWS / 8)) * 16 + (lane >> 3) * 4;
-                v[i] = t < pieces && row < batch && k < rows ? load(row, k0 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[i] = t < pieces && row < batch && k < rows ? __ldcg(reinterpret_cast<const float4 *>(x + static_cast<size_t>(row) * pitch + k0 + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 const int t = t0 + i * kWarps, row = (t % (ROWS / 8)) * 8 + (lane & 7), k = (t / (ROWS / 8)) * 16 + (lane >> 3) * 4;
                 if (t < pieces && k < rows) {
                     xs[k * P + row] = v[i].x;
@@ -592,17 +620,25 @@ gpt_step_rows_kernel(const GptStep s)
         }
     };
 
-    // One phase of products; `next`: requests the weights of this block's first item of the next product.
-    const int quarter = tid / kQuarter, cg = tid & 15, rg = (tid >> 4) & 7;
-    auto product = [&](const float *w, const StepPhase &ph, float *part, auto load, auto next) {
+    // One phase of products; `next`: where the weights of this block's first item of the next product are.
+    const int quarter = warp >> 2, cg = tid & 15, rg = (tid >> 4) & 7;
+    constexpr int HT = RT < 4 ? RT : 4, kHalf = HT * 8;   // rows per thread and block in one pass over the sums
+    auto product = [&](const float *w, const StepPhase &ph, float *part, const float *x, const float *w_next, const StepPhase &ph_next, int item_next) {
         const int items = ph.groups * ph.splits;
-        if (first >= items) next();
+        if (first >= items) fetch_all(w_next, ph_next, item_next);
+#pragma unroll 1
         for (int item = first; item < items; item += gridDim.x) {
             const int split = item / ph.groups, col0 = (item - split * ph.groups) * kWideCols, k0 = split * ph.slice, rows = min(ph.K - k0, ph.slice);
-            if (item != first) __syncthreads();   // the sums of the item before have been read
-            stage(k0, rows, load);
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            {   // the weights of this item become current
+                float *t = ws;
+                ws = ws_next;
+                ws_next = t;
+            }
+            stage(k0, rows, x, ph.K);
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
+            const bool last = item + static_cast<int>(gridDim.x) >= items;
+            Source coming = source(last ? w_next : w, last ? ph_next : ph, last ? item_next : item + static_cast<int>(gridDim.x));
             unsigned long long acc[RT][4];   // columns (4 cg, + 1), (4 cg + 2, + 3), and the same 64 further on
 #pragma unroll
             for (int r = 0; r < RT; ++r)
@@ -610,165 +646,216 @@ gpt_step_rows_kernel(const GptStep s)
                 for (int c = 0; c < 4; ++c) acc[r][c] = 0ull;
             const int per = (rows + 3) >> 2, kb = quarter * per, ke = min(rows, kb + per);
             const float *wp = ws + kb * kWideCols + cg * 4, *xp = xs + kb * P + rg * RT;
-#pragma unroll 4
-            for (int k = kb; k < ke; ++k, wp += kWideCols, xp += P) {
-                const ulonglong2 wa = *reinterpret_cast<const ulonglong2 *>(wp), wb = *reinterpret_cast<const ulonglong2 *>(wp + 64);
-                float x[RT];
-                if constexpr (RT >= 4) {
+#pragma unroll 1
+            for (int k = kb; k < ke; k += 4) {
+                fetch(coming);
 #pragma unroll
-                    for (int r = 0; r < RT; r += 4) {
-                        const float4 v = *reinterpret_cast<const float4 *>(xp + r);
-                        x[r] = v.x; x[r + 1] = v.y; x[r + 2] = v.z; x[r + 3] = v.w;
+                for (int i = 0; i < 4; ++i, wp += kWideCols, xp += P) {
+                    if (k + i >= ke) break;
+                    const ulonglong2 wa = *reinterpret_cast<const ulonglong2 *>(wp), wb = *reinterpret_cast<const ulonglong2 *>(wp + 64);
+                    float x[RT];
+                    if constexpr (RT >= 4) {
+#pragma unroll
+                        for (int r = 0; r < RT; r += 4) {
+                            const float4 v = *reinterpret_cast<const float4 *>(xp + r);
+                            x[r] = v.x; x[r + 1] = v.y; x[r + 2] = v.z; x[r + 3] = v.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < RT; ++r) x[r] = xp[r];
                     }
-                } else {
 #pragma unroll
-                    for (int r = 0; r < RT; ++r) x[r] = xp[r];
-                }
-#pragma unroll
-                for (int r = 0; r < RT; ++r) {
-                    const unsigned long long xx = twice(x[r]);
-                    fma2(acc[r][0], wa.x, xx);
-                    fma2(acc[r][1], wa.y, xx);
-                    fma2(acc[r][2], wb.x, xx);
-                    fma2(acc[r][3], wb.y, xx);
+                    for (int r = 0; r < RT; ++r) {
+                        const unsigned long long xx = twice(x[r]);
+                        fma2(acc[r][0], wa.x, xx);
+                        fma2(acc[r][1], wa.y, xx);
+                        fma2(acc[r][2], wb.x, xx);
+                        fma2(acc[r][3], wb.y, xx);
+                    }
                 }
             }
-            __syncthreads();   // the weights and activations have been read
-            if (item + static_cast<int>(gridDim.x) < items)
-                fetch(w, ph, item + gridDim.x);
-            else
-                next();
-            if (quarter > 0) {
+#pragma unroll 1
+            while (coming.rows > 0) fetch(coming);
+            // the quarters' sums meet where this item's weights and activations were
+            float *sums = scratch();
 #pragma unroll
-                for (int r = 0; r < RT; ++r) {
-                    float *dst = sums + ((quarter - 1) * ROWS + rg * RT + r) * kWideCols + cg * 4;
-                    *reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(acc[r][0], acc[r][1]);
-                    *reinterpret_cast<ulonglong2 *>(dst + 64) = make_ulonglong2(acc[r][2], acc[r][3]);
+            for (int h = 0; h < RT; h += HT) {
+                __syncthreads();   // the weights and activations, or the sums of the pass before, have been read
+#pragma unroll
+                for (int r = 0; r < HT; ++r) {
+                    float *dst = sums + (quarter * kHalf + rg * HT + r) * kWideCols + cg * 4;
+                    *reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(acc[h + r][0], acc[h + r][1]);
+                    *reinterpret_cast<ulonglong2 *>(dst + 64) = make_ulonglong2(acc[h + r][2], acc[h + r][3]);
+                }
+                __syncthreads();
+#pragma unroll
+                for (int i = tid; i < kHalf * (kWideCols / 4); i += kThreads) {
+                    const int at = i >> 5, row = at / HT * RT + h + at % HT, c = (i & 31) * 4;
+                    if (row >= batch || col0 + c >= ph.N) continue;
+                    float4 v = *reinterpret_cast<const float4 *>(sums + at * kWideCols + c);
+#pragma unroll
+                    for (int q = 1; q < 4; ++q) v = add4(v, *reinterpret_cast<const float4 *>(sums + (q * kHalf + at) * kWideCols + c));
+                    *reinterpret_cast<float4 *>(part + (static_cast<size_t>(split) * batch + row) * ph.N + col0 + c) = v;
                 }
             }
-            // the first quarter's sums go where the activations were
-            if (quarter == 0) {
-#pragma unroll
-                for (int r = 0; r < RT; ++r) {
-                    float *dst = xs + (rg * RT + r) * kWideCols + cg * 4;
-                    *reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(acc[r][0], acc[r][1]);
-                    *reinterpret_cast<ulonglong2 *>(dst + 64) = make_ulonglong2(acc[r][2], acc[r][3]);
-                }
-            }
-            __syncthreads();
-            for (int i = tid; i < batch * (kWideCols / 4); i += kThreads) {
-                const int row = i >> 5, c = (i & 31) * 4;
-                if (col0 + c >= ph.N) continue;
-                float4 v = *reinterpret_cast<const float4 *>(xs + row * kWideCols + c);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) v = add4(v, *reinterpret_cast<const float4 *>(sums + (q * ROWS + row) * kWideCols + c));
-                *reinterpret_cast<float4 *>(part + (static_cast<size_t>(split) * batch + row) * ph.N + col0 + c) = v;
-            }
+            if (!last) __syncthreads();   // the next item's activations go where the sums are
+        }
+    };
+
+    // act = gelu(finished up product), written over the first slice's sums
+    auto gelu_phase = [&](const float *bias) {
+        const int quads = s.ffn >> 2;
+#pragma unroll 1
+        for (int i = first * kThreads + tid; i < batch * quads; i += gridDim.x * kThreads) {
+            const int row = i / quads, c = (i - row * quads) * 4;
+            const float4 be = __ldg(reinterpret_cast<const float4 *>(bias + c));
+            float *at = s.up_part + static_cast<size_t>(row) * s.ffn + c;
+            const float4 v = add4(sum_parts4<6>(at, s.up.splits, batch * s.ffn), be);
+            *reinterpret_cast<float4 *>(at) = make_float4(gelu_step(v.x), gelu_step(v.y), gelu_step(v.z), gelu_step(v.w));
         }
     };
 
     // res += a finished product (none: the embedding), normed = its norm; a block per row
     auto norm_phase = [&](const float *part, const StepPhase &ph, const float *bias, const float *gain, const float *shift) {
-        float *row_sm = xs, *half_sm = xs + d;   // both fit: see the plan
-        constexpr int kHalf = kThreads / 2;
-        const int half = tid / kHalf, at = (tid % kHalf) * 4, cut = (ph.splits + 1) / 2;
+        float *row_sm = scratch(), *half_sm = row_sm + d;   // both fit: see the plan
+        constexpr int kSide = kThreads / 2;
+        const int half = tid / kSide, at = (tid % kSide) * 4, cut = (ph.splits + 1) / 2;
+        const auto at4 = [](const float *q) { return *reinterpret_cast<const float4 *>(q); };
+#pragma unroll 1
         for (int row = first; row < batch; row += gridDim.x) {
             __syncthreads();
+            // what does not depend on the sums is on its way before them
+            float4 before = make_float4(0.f, 0.f, 0.f, 0.f), more = before, ga = before, be = before;
+            if (tid * 4 < d) {
+                before = part ? __ldcg(reinterpret_cast<const float4 *>(s.res + row * d + tid * 4)) : at4(s.wte + static_cast<size_t>(s.tokens[row]) * d + tid * 4);
+                more = part ? at4(bias + tid * 4) : at4(s.wpe + static_cast<size_t>(p) * d + tid * 4);
+                ga = at4(gain + tid * 4);
+                be = at4(shift + tid * 4);
+            }
             if (part) {   // each half of the block adds up half of the slices
-                for (int c = at; c < d; c += kHalf * 4) {
-                    const float4 v = sum_parts4(part + static_cast<size_t>(half ? cut : 0) * batch * d + row * d + c, half ? ph.splits - cut : cut, batch * d);
-                    if (half) *reinterpret_cast<float4 *>(half_sm + c) = v; else *reinterpret_cast<float4 *>(row_sm + c) = v;
-                }
+#pragma unroll 1
+                for (int c = at; c < d; c += kSide * 4)
+                    *reinterpret_cast<float4 *>((half ? half_sm : row_sm) + c) = sum_parts4(part + static_cast<size_t>(half ? cut : 0) * batch * d + row * d + c, half ? ph.splits - cut : cut, batch * d);
                 __syncthreads();
             }
+#pragma unroll 1
             for (int c = tid * 4; c < d; c += kThreads * 4) {
-                float4 v;
-                if (part) {
-                    v = add4(add4(*reinterpret_cast<const float4 *>(row_sm + c), *reinterpret_cast<const float4 *>(half_sm + c)), __ldg(reinterpret_cast<const float4 *>(bias + c)));
-                    v = add4(__ldcg(reinterpret_cast<const float4 *>(s.res + row * d + c)), v);
-                } else {
-                    v = add4(__ldg(reinterpret_cast<const float4 *>(s.wte + static_cast<size_t>(s.tokens[row]) * d + c)),
-                             __ldg(reinterpret_cast<const float4 *>(s.wpe + static_cast<size_t>(p) * d + c)));
+                if (c != tid * 4) {
+                    before = part ? __ldcg(reinterpret_cast<const float4 *>(s.res + row * d + c)) : at4(s.wte + static_cast<size_t>(s.tokens[row]) * d + c);
+                    more = part ? at4(bias + c) : at4(s.wpe + static_cast<size_t>(p) * d + c);
                 }
+                const float4 v = add4(before, part ? add4(add4(at4(row_sm + c), at4(half_sm + c)), more) : more);
                 *reinterpret_cast<float4 *>(row_sm + c) = v;
                 __stcg(reinterpret_cast<float4 *>(s.res + row * d + c), v);
             }
             warp_moments<1>(row_sm, d, moments);   // a thread reads what it wrote
             __syncthreads();
+            if (warp * 128 >= d) continue;
             float mean[1], sd[1];
             row_statistics<1>(moments, d, mean, sd);
+#pragma unroll 1
             for (int c = tid * 4; c < d; c += kThreads * 4) {
-                const float4 v = *reinterpret_cast<const float4 *>(row_sm + c), ga = __ldg(reinterpret_cast<const float4 *>(gain + c)), be = __ldg(reinterpret_cast<const float4 *>(shift + c));
+                if (c != tid * 4) {
+                    ga = at4(gain + c);
+                    be = at4(shift + c);
+                }
+                const float4 v = at4(row_sm + c);
                 *reinterpret_cast<float4 *>(s.normed + row * d + c) = make_float4((v.x - mean[0]) / sd[0] * ga.x + be.x, (v.y - mean[0]) / sd[0] * ga.y + be.y,
                                                                                   (v.z - mean[0]) / sd[0] * ga.z + be.z, (v.w - mean[0]) / sd[0] * ga.w + be.w);
             }
         }
     };
 
-    const int head_log = 31 - __clz(s.hd), per_pos = s.hd >> 2, groups = kQuarter / per_pos;
-    const int qt = tid & (kQuarter - 1), g = qt >> (head_log - 2), c4 = (qt & (per_pos - 1)) * 4, row_stride = 2 * d * groups;
-    float *fresh = xs + quarter * (3 * s.hd + 4 * (s.hd + 4) + ((s.max_len + 3) & ~3));   // [3][hd]
-    float *out = fresh + 3 * s.hd, *prob = out + 4 * (s.hd + 4);                            // [4][hd + 4], [max_len]
-    // a quarter of a block per (sequence, head)
+    constexpr int kAtt = wide_attention_threads(ROWS), kAttItems = kThreads / kAtt, kAttWarps = kAtt / 32;
+    const int head_log = 31 - __clz(s.hd), per_pos = s.hd >> 2, groups = kAtt / per_pos;
+    const int worker = tid / kAtt, qt = tid & (kAtt - 1), g = qt >> (head_log - 2), c4 = (qt & (per_pos - 1)) * 4, row_stride = 2 * d * groups;
+    // The cached rows of this block's items towards L2 while the FMAs of the product before keep HBM idle: 37 MB per layer at 64 sequences of 96.
+    auto prefetch_cache = [&](const float *cache) {
+        const int lines = (s.hd * 4 + 127) >> 7, per_row = 2 * lines;
+#pragma unroll 1
+        for (int item = first * kAttItems + worker; item < batch * s.heads; item += gridDim.x * kAttItems) {
+            const int m = item / s.heads, at = (item - m * s.heads) << head_log;
+            const float *keys = cache + static_cast<size_t>(m) * s.max_len * 2 * d + at;
+#pragma unroll 2
+            for (int i = qt; i < p * per_row; i += kAtt) {
+                const int t = i / per_row, j = i - t * per_row;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(keys + static_cast<size_t>(t) * 2 * d + (j >= lines ? d + (j - lines) * 32 : j * 32)));
+            }
+        }
+    };
+    // kAtt threads per (sequence, head); sixteen cached rows in flight per thread, the first keys before the new q, k, v are known, the first
+    // values before the softmax
     auto attention = [&](float *cache, const float *qkv_b) {
-        for (int item = first * 4 + quarter; item < batch * s.heads; item += gridDim.x * 4) {
+        constexpr int kFlight = 16;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        float *fresh = scratch() + worker * wide_attention_floats(kAtt, s.hd, s.max_len);      // [3][hd]
+        float *out = fresh + 3 * s.hd, *prob = out + kAttWarps * (s.hd + 4);                    // [kAttWarps][hd + 4], [max_len]
+#pragma unroll 1
+        for (int item = first * kAttItems + worker; item < batch * s.heads; item += gridDim.x * kAttItems) {
             const int m = item / s.heads, at = (item - m * s.heads) << head_log;
             float *keys = cache + static_cast<size_t>(m) * s.max_len * 2 * d + at;
-            for (int i = qt; i < 3 * s.hd; i += kQuarter) {
+            const float *row = keys + static_cast<size_t>(g) * 2 * d + c4;
+            float4 kv[kFlight];
+            auto load = [&](int t0, const float *src) {
+#pragma unroll
+                for (int j = 0; j < kFlight; ++j, src += row_stride) kv[j] = t0 + g + j * groups < p ? *reinterpret_cast<const float4 *>(src) : zero;
+            };
+            load(0, row);
+#pragma unroll 1
+            for (int i = qt * 4; i < 3 * s.hd; i += kAtt * 4) {
                 const int which = i >> head_log, e = i & (s.hd - 1), col = which * d + at + e;
-                const float be = __ldg(qkv_b + col);
-                const float v = sum_parts8(s.qkv_part + static_cast<size_t>(m) * 3 * d + col, s.qkv.splits, batch * 3 * d) + be;
-                fresh[i] = v;
-                if (which > 0) keys[static_cast<size_t>(p) * 2 * d + (which - 1) * d + e] = v;
+                const float4 be = __ldg(reinterpret_cast<const float4 *>(qkv_b + col));
+                const float4 v = add4(sum_parts4<8>(s.qkv_part + static_cast<size_t>(m) * 3 * d + col, s.qkv.splits, batch * 3 * d), be);
+                *reinterpret_cast<float4 *>(fresh + i) = v;
+                if (which > 0) *reinterpret_cast<float4 *>(keys + static_cast<size_t>(p) * 2 * d + (which - 1) * d + e) = v;
             }
-            quarter_sync();
-            const float *q = fresh + c4, *row = keys + static_cast<size_t>(g) * 2 * d + c4;
+            group_sync<kAtt>();
+            const float *q = fresh + c4;
             const float4 q4 = *reinterpret_cast<const float4 *>(q);
-            for (int t0 = 0; t0 <= p; t0 += 4 * groups, row += 4 * row_stride) {   // four rows in flight per thread
-                float4 kv[4];
-                float v[4];
+#pragma unroll 1
+            for (int t0 = 0; t0 <= p; t0 += kFlight * groups) {
+                if (t0 > 0) load(t0, row + static_cast<size_t>(t0) * 2 * d);
+                float v[kFlight];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int t = t0 + g + j * groups;
-                    kv[j] = t < p ? *reinterpret_cast<const float4 *>(row + j * row_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (t == p) kv[j] = *reinterpret_cast<const float4 *>(q + s.hd);
+                for (int j = 0; j < kFlight; ++j) {
+                    if (t0 + g + j * groups == p) kv[j] = *reinterpret_cast<const float4 *>(q + s.hd);
+                    v[j] = dot4(q4, kv[j], 0.0f);
                 }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = dot4(q4, kv[j], 0.0f);
+#pragma unroll 1
                 for (int o = per_pos >> 1; o > 0; o >>= 1)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+                    for (int j = 0; j < kFlight; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
                 if (c4 == 0)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < kFlight; ++j)
                         if (t0 + g + j * groups <= p) prob[t0 + g + j * groups] = v[j] * s.scale;
             }
-            quarter_sync();
+            load(0, row + d);
+            group_sync<kAtt>();
             float mx = -FLT_MAX, weights = 0.0f;
+#pragma unroll 2
             for (int t = lane; t <= p; t += 32) mx = fmaxf(mx, prob[t]);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            row = keys + d + static_cast<size_t>(g) * 2 * d + c4;
-            for (int t0 = 0; t0 + g <= p; t0 += 4 * groups, row += 4 * row_stride) {
-                float4 kv[4];
+            float4 acc = zero;
+#pragma unroll 1
+            for (int t0 = 0; t0 <= p; t0 += kFlight * groups) {
+                if (t0 > 0) load(t0, row + d + static_cast<size_t>(t0) * 2 * d);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < kFlight; ++j) {
                     const int t = t0 + g + j * groups;
-                    kv[j] = t < p ? *reinterpret_cast<const float4 *>(row + j * row_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
                     if (t == p) kv[j] = *reinterpret_cast<const float4 *>(q + 2 * s.hd);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (t0 + g + j * groups <= p) {
-                        const float e = expf(prob[t0 + g + j * groups] - mx);
+                    if (t <= p) {
+                        const float e = expf(prob[t] - mx);
                         weights += e;
                         acc.x = fmaf(e, kv[j].x, acc.x);
                         acc.y = fmaf(e, kv[j].y, acc.y);
                         acc.z = fmaf(e, kv[j].z, acc.z);
                         acc.w = fmaf(e, kv[j].w, acc.w);
                     }
+                }
             }
+#pragma unroll 1
             for (int o = per_pos; o < 32; o <<= 1) {
                 acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
                 acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
@@ -776,59 +863,53 @@ gpt_step_rows_kernel(const GptStep s)
                 acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
                 weights += __shfl_xor_sync(0xffffffffu, weights, o);
             }
-            float *mine = out + (warp & 3) * (s.hd + 4);
+            float *mine = out + (warp & (kAttWarps - 1)) * (s.hd + 4);
             if (lane < per_pos) *reinterpret_cast<float4 *>(mine + c4) = acc;
             if (lane == 0) mine[s.hd] = weights;
-            quarter_sync();
-            if (qt < s.hd) {   // heads are at most 128 wide
+            group_sync<kAtt>();
+#pragma unroll 1
+            for (int i = qt; i < s.hd; i += kAtt) {
                 float v = 0.0f, sum = 0.0f;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    v += out[j * (s.hd + 4) + qt];
+                for (int j = 0; j < kAttWarps; ++j) {
+                    v += out[j * (s.hd + 4) + i];
                     sum += out[j * (s.hd + 4) + s.hd];
                 }
-                s.attn[static_cast<size_t>(m) * d + at + qt] = v / sum;
+                s.attn[static_cast<size_t>(m) * d + at + i] = v / sum;
             }
-            quarter_sync();   // the next item writes fresh
+            group_sync<kAtt>();   // the next item writes fresh
         }
     };
 
-    fetch(s.qkv_w, s.qkv, first);
-    auto from = [&](const float *x, int K) { return [=](int row, int k) { return __ldcg(reinterpret_cast<const float4 *>(x + static_cast<size_t>(row) * K + k)); }; };
-    for (int l = 0; l < s.layers; ++l) {
-        const float *qkv_w = s.qkv_w + static_cast<size_t>(l) * d * 3 * d, *proj_w = s.proj_w + static_cast<size_t>(l) * d * d;
-        const float *up_w = s.up_w + static_cast<size_t>(l) * d * s.ffn, *down_w = s.down_w + static_cast<size_t>(l) * s.ffn * d;
+    // Four products per layer (qkv, projection, up, down), each behind a phase that makes its input; after the last layer the final norm, and
+    // the product with the embedding is another launch.
+    fetch_all(s.qkv_w, s.qkv, first);
+    const size_t dd = static_cast<size_t>(d) * d, df = static_cast<size_t>(d) * s.ffn;
+#pragma unroll 1
+    for (int n = 0;; ++n) {
+        const int l = n >> 2, kind = n & 3;
         float *cache = s.cache + static_cast<size_t>(l) * batch * s.max_len * 2 * d;
-        norm_phase(l > 0 ? s.down_part : nullptr, s.down, s.down_b + (l - 1) * d, s.ln1_w + l * d, s.ln1_b + l * d);
+        if ((kind & 1) == 0) {
+            const bool attended = kind == 2, end = l == s.layers;
+            norm_phase(attended ? s.proj_part : l > 0 ? s.down_part : nullptr, attended ? s.proj : s.down, attended ? s.proj_b + l * d : s.down_b + (l - 1) * d,
+                       end ? s.lnf_w : (attended ? s.ln2_w : s.ln1_w) + l * d, end ? s.lnf_b : (attended ? s.ln2_b : s.ln1_b) + l * d);
+            if (end) break;
+        } else if (kind == 1) {
+            attention(cache, s.qkv_b + l * 3 * d);
+        } else {
+            gelu_phase(s.up_b + l * s.ffn);
+        }
         arrive(s, target);
         await(s, target);
-        product(qkv_w, s.qkv, s.qkv_part, from(s.normed, d), [&] { fetch(proj_w, s.proj, first); });
-        arrive(s, target);
-        await(s, target);
-        attention(cache, s.qkv_b + l * 3 * d);
-        arrive(s, target);
-        await(s, target);
-        product(proj_w, s.proj, s.proj_part, from(s.attn, d), [&] { fetch(up_w, s.up, first); });
-        arrive(s, target);
-        await(s, target);
-        norm_phase(s.proj_part, s.proj, s.proj_b + l * d, s.ln2_w + l * d, s.ln2_b + l * d);
-        arrive(s, target);
-        await(s, target);
-        product(up_w, s.up, s.up_part, from(s.normed, d), [&] { fetch(down_w, s.down, first); });
-        arrive(s, target);
-        await(s, target);
-        const float *up_b = s.up_b + l * s.ffn;
-        product(down_w, s.down, s.down_part,
-                [&](int row, int k) {
-                    const float4 be = __ldg(reinterpret_cast<const float4 *>(up_b + k));
-                    const float4 v = add4(sum_parts4<6>(s.up_part + static_cast<size_t>(row) * s.ffn + k, s.up.splits, batch * s.ffn), be);
-                    return make_float4(gelu_step(v.x), gelu_step(v.y), gelu_step(v.z), gelu_step(v.w));
-                },
-                [&] { if (l + 1 < s.layers) fetch(qkv_w + static_cast<size_t>(d) * 3 * d, s.qkv, first); });
+        if (kind == 0) prefetch_cache(cache);
+        const StepPhase ph = kind == 0 ? s.qkv : kind == 1 ? s.proj : kind == 2 ? s.up : s.down, ph_next = kind == 0 ? s.proj : kind == 1 ? s.up : kind == 2 ? s.down : s.qkv;
+        const float *w = kind == 0 ? s.qkv_w + 3 * dd * l : kind == 1 ? s.proj_w + dd * l : kind == 2 ? s.up_w + df * l : s.down_w + df * l;
+        const float *w_next = kind == 0 ? s.proj_w + dd * l : kind == 1 ? s.up_w + df * l : kind == 2 ? s.down_w + df * l : s.qkv_w + 3 * dd * (l + 1);
+        product(w, ph, kind == 0 ? s.qkv_part : kind == 1 ? s.proj_part : kind == 2 ? s.up_part : s.down_part, kind == 1 ? s.attn : kind == 3 ? s.up_part : s.normed,
+                w_next, ph_next, kind == 3 && l + 1 == s.layers ? ph_next.groups * ph_next.splits : first);
         arrive(s, target);
         await(s, target);
     }
-    norm_phase(s.down_part, s.down, s.down_b + (s.layers - 1) * d, s.lnf_w, s.lnf_b);   // the product with the embedding is another launch
     if (blockIdx.x == 0 && tid == 0) {   // every block has passed a barrier since it read them
         *s.pos = p + 1;
         s.sync[1] = target;
