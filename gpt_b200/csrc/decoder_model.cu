@@ -19,6 +19,7 @@
 #include "ctx_internal.h"
 #include "decoder_config.h"
 #include "decoder_rows.cuh"
+#include "decoder_step_rows.cuh"
 #include "grouped_attention.cuh"
 #include "latent_attention.cuh"
 #include "latent_decode.cuh"
@@ -815,6 +816,20 @@ private:
     // threads per row of the stream: with few rows a row is spread wider
     int row_threads(int rows) const { return std::min(rows <= 2 * ctx_->num_sms ? 1024 : 256, std::max(32, pad_to(pitch_ / 4, 32))); }
 
+    // The row kernels of decoder_step_rows.cuh: steps of one token per sequence with no more rows than run at once.  The fp32 products let
+    // their successor start before their own wait, so what the row kernels read early would not be complete.
+    bool single_rows(int rows) const { return !kF32 && single_tokens_ && rows <= ctx_->num_sms && pitch_ <= 4096; }
+
+    int sublayer_end(int rows, float *x, const Norm &after, const Norm &before)
+    {
+        const float eps = static_cast<float>(c_.eps);
+        const auto run = [&](auto kernel, int threads, size_t smem) {
+            return launch(kernel, dim3(rows), dim3(threads), smem, x, static_cast<const float *>(y_), static_cast<const float *>(after.w), static_cast<const float *>(after.b),
+                          static_cast<const float *>(before.w), static_cast<const float *>(before.b), h_, c_.width, pitch_, eps);
+        };
+        return single_rows(rows) ? run(&sublayer_end_row_kernel<T>, pad_to(pitch_ / 4, 32), 0) : run(&sublayer_end_kernel<T>, row_threads(rows), size_t(pitch_) * sizeof(float));
+    }
+
     int layer_begin(int rows, int layer, const T *h, const int *row_list)
     {
         // layer: the layer that begins; layers_.size(): the final norm over the wanted rows
@@ -840,6 +855,7 @@ private:
         }
         b.h = const_cast<T *>(h);
         b.entries = entries_; b.row_entry = row_entry_; b.row_list = row_list;
+        if (b.side_y && single_rows(rows)) return launch(layer_begin_row_kernel<T>, dim3(rows), dim3(pad_to(pitch_ / 4, 32)), 0, b);
         b.tile = rows <= 512 || !b.shift ? 1 : rows <= 2048 ? 4 : 8;
         return launch(layer_begin_kernel<T>, dim3((rows + b.tile - 1) / b.tile), dim3(row_threads(rows)), 2 * size_t(pitch_) * sizeof(float), b);
     }
@@ -1349,6 +1365,7 @@ private:
         }
         b.h = h;
         b.entries = entries_; b.row_entry = row_entry_; b.row_list = row_list;
+        if (y && single_rows(rows)) return launch(residual_norm_row_kernel<T>, dim3(rows), dim3(pad_to(pitch_ / 4, 32)), 0, b);
         b.tile = rows <= 512 || !b.mixes ? 1 : rows <= 2048 ? 4 : 8;
         return launch(residual_norm_kernel<T>, dim3((rows + b.tile - 1) / b.tile), dim3(row_threads(rows)), 2 * size_t(pitch_) * sizeof(float), b);
     }
@@ -1390,8 +1407,8 @@ private:
     // All kernels of one step; everything that changes from step to step is read from device memory.
     int kernels(const std::vector<Part> &parts, int rows, int n_want)
     {
+        single_tokens_ = std::all_of(parts.begin(), parts.end(), [](const Part &p) { return p.count == 1; });
         if (!norms_around()) return kernels_norms_before(parts, rows, n_want);
-        const float eps = static_cast<float>(c_.eps);
         RC_TRY(launch(embed_rows_kernel<T>, dim3(rows), dim3(row_threads(rows)), 0, states_, static_cast<const T *>(embed_), static_cast<const int *>(tokens_), pitch_));
         RC_TRY(rotary_tables(rows));
         for (size_t i = 0; i < layers_.size(); ++i) {
@@ -1400,13 +1417,10 @@ private:
             RC_TRY(layer_begin(rows, static_cast<int>(i), h_, nullptr));
             RC_TRY(mixer(static_cast<int>(i), parts, rows));
             RC_TRY(linear_f32(y_, act_, d.w_o, rows, pitch_, d.mix_out));
-            const size_t smem = size_t(pitch_) * sizeof(float);
-            RC_TRY(launch(sublayer_end_kernel<T>, dim3(rows), dim3(row_threads(rows)), smem, x, static_cast<const float *>(y_), static_cast<const float *>(d.norm1b.w),
-                          static_cast<const float *>(d.norm1b.b), static_cast<const float *>(d.norm2.w), static_cast<const float *>(d.norm2.b), h_, c_.width, pitch_, eps));
+            RC_TRY(sublayer_end(rows, x, d.norm1b, d.norm2));
             if (d.ff) {
                 RC_TRY(feed_forward(d, rows));
-                RC_TRY(launch(sublayer_end_kernel<T>, dim3(rows), dim3(row_threads(rows)), smem, x, static_cast<const float *>(y_), static_cast<const float *>(d.norm2b.w),
-                              static_cast<const float *>(d.norm2b.b), static_cast<const float *>(nullptr), static_cast<const float *>(nullptr), h_, c_.width, pitch_, eps));
+                RC_TRY(sublayer_end(rows, x, d.norm2b, Norm{}));
             }
             if (d.side_gate) {
                 if constexpr (kF32) {
@@ -1428,6 +1442,7 @@ private:
         return GPTB200_OK;
     }
 
+    bool single_tokens_ = false;   // the step at hand has one token per sequence
     std::vector<Layer> layers_;
     std::vector<Rotary> rotaries_;
     T *embed_ = nullptr, *head_ = nullptr, *pairs_ = nullptr;
