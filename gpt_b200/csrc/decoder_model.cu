@@ -904,7 +904,7 @@ private:
             RC_TRY(k == 2 ? recurrent_chunks(s, {xbc_, ld_xbc, dt_, decay_, s.heads, d.d_skip}, parts, entry0, n) : mamba_tokens(d, entry0, n, ld_xbc));
         }
         const int part = s.inner / s.norm_groups;
-        return launch(mamba_gated_norm_kernel<T>, dim3(rows, s.norm_groups), dim3(std::min(256, pad_to((part + 3) / 4, 32))), size_t(part) * sizeof(float), act_, d.mix_out,
+        return launch(mamba_gated_norm_kernel<T>, dim3(rows, s.norm_groups), dim3(std::min(rows <= 2 * ctx_->num_sms ? 1024 : 256, pad_to((part + 3) / 4, 32))), size_t(part) * sizeof(float), act_, d.mix_out,
                       static_cast<const float *>(ssm_y_), static_cast<const T *>(proj_), ld, static_cast<const float *>(d.mix_norm), s, static_cast<float>(c_.eps));
     }
 

@@ -8,6 +8,7 @@
 
 #include <cfloat>
 #include <cooperative_groups.h>
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -365,12 +366,26 @@ __global__ void normed_sigmoid_gate_kernel(T *__restrict__ out, int ld_out, cons
 {
     extern __shared__ float sm[];   // [width], every thread its own columns
     __shared__ float red[32];
-    grid_dependency_wait();
-    grid_dependency_launch();
     const long long row = blockIdx.x;
     y += row * width;
     gate += row * ld_gate;
     out += row * ld_out;
+    if (!std::is_same<T, float>::value && width % 4 == 0 && width <= 4 * static_cast<int>(blockDim.x)) {
+        // the row in registers; gate and weights are older than the predecessor (see decoder_step_rows.cuh)
+        const int i = 4 * threadIdx.x;
+        const bool live = i < width;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 z = live ? load4(gate + i) : zero, w = live ? load4(weight + i) : zero;
+        const float4 g = make_float4(sigmoid_f(z.x), sigmoid_f(z.y), sigmoid_f(z.z), sigmoid_f(z.w));
+        grid_dependency_wait();
+        grid_dependency_launch();
+        const float4 v = live ? load4(y + i) : zero;
+        const float inv = rsqrtf(block_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w, red) / width + eps);
+        if (live) store4(out + i, make_float4(v.x * inv * w.x * g.x, v.y * inv * w.y * g.y, v.z * inv * w.z * g.z, v.w * inv * w.w * g.w));
+        return;
+    }
+    grid_dependency_wait();
+    grid_dependency_launch();
     float ss = 0.0f;
     if (width % 4 == 0) {
         for (int i = 4 * threadIdx.x; i < width; i += 4 * blockDim.x) {

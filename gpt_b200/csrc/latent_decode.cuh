@@ -283,9 +283,23 @@ latent_combine_kernel(__nv_bfloat16 *__restrict__ out, int ld_out, const float *
     const int slices = (s.vdim + kCombineRows - 1) / kCombineRows;
     const int h = blockIdx.x / slices, v0 = (blockIdx.x % slices) * kCombineRows, row = row0 + blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the weights of this warp's four value rows (up to 512 columns) and its gates are older than the predecessor: loaded before the wait
+    constexpr int kRowsPerWarp = kCombineRows / 8, kHeldPieces = 2;
+    uint4 held[kRowsPerWarp][kHeldPieces];
+    float gate[kRowsPerWarp];
+#pragma unroll
+    for (int i = 0; i < kRowsPerWarp; ++i) {
+        const int v = v0 + warp + 8 * i;
+        const bool live = v < min(v0 + kCombineRows, s.vdim);
+#pragma unroll
+        for (int c = 0; c < kHeldPieces; ++c)
+            held[i][c] = live && lane * 8 + 256 * c < s.rank_pitch ? __ldg(reinterpret_cast<const uint4 *>(w_uv + (static_cast<long long>(h) * s.v_pad + v) * s.rank_pitch + lane * 8 + 256 * c))
+                                                                 : make_uint4(0u, 0u, 0u, 0u);
+        gate[i] = live ? to_f(proj[row * ld + s.off_g + h * s.vdim + v]) : 0.0f;
+    }
+    const StepEntry e = entries[row_entry[row]];
     grid_dependency_wait();
     grid_dependency_launch();
-    const StepEntry e = entries[row_entry[row]];
     const int n = e.pos0 + row - e.row0 + 1;
     const int used = (n + split_length(n, splits) - 1) / split_length(n, splits);
     const float *ml = part_ml + (static_cast<long long>(blockIdx.y) * s.heads + h) * splits * 2;
@@ -312,18 +326,24 @@ latent_combine_kernel(__nv_bfloat16 *__restrict__ out, int ld_out, const float *
         latent[j] = v / total;
     }
     __syncthreads();
-    for (int v = v0 + warp; v < min(v0 + kCombineRows, s.vdim); v += 8) {
-        const __nv_bfloat16 *w = w_uv + (static_cast<long long>(h) * s.v_pad + v) * s.rank_pitch;
+#pragma unroll
+    for (int i = 0; i < kRowsPerWarp; ++i) {
+        const int v = v0 + warp + 8 * i;
+        if (v >= min(v0 + kCombineRows, s.vdim)) break;
         float acc = 0.0f;
-        for (int j = lane * 8; j < s.rank_pitch; j += 256) {
-            const uint4 x = __ldg(reinterpret_cast<const uint4 *>(w + j));
+        auto add = [&](const uint4 &x, int j) {
             const uint32_t u[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc = fmaf(bf16_lo(u[i]), latent[j + 2 * i], fmaf(bf16_hi(u[i]), latent[j + 2 * i + 1], acc));
-        }
+            for (int k = 0; k < 4; ++k) acc = fmaf(bf16_lo(u[k]), latent[j + 2 * k], fmaf(bf16_hi(u[k]), latent[j + 2 * k + 1], acc));
+        };
+#pragma unroll
+        for (int c = 0; c < kHeldPieces; ++c)
+            if (lane * 8 + 256 * c < s.rank_pitch) add(held[i][c], lane * 8 + 256 * c);
+        const __nv_bfloat16 *w = w_uv + (static_cast<long long>(h) * s.v_pad + v) * s.rank_pitch;
+        for (int j = lane * 8 + 256 * kHeldPieces; j < s.rank_pitch; j += 256) add(__ldg(reinterpret_cast<const uint4 *>(w + j)), j);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) out[static_cast<long long>(row) * ld_out + h * s.vdim + v] = __float2bfloat16_rn(acc * sigmoid_f(to_f(proj[row * ld + s.off_g + h * s.vdim + v])));
+        if (lane == 0) out[static_cast<long long>(row) * ld_out + h * s.vdim + v] = __float2bfloat16_rn(acc * sigmoid_f(gate[i]));
     }
 }
 

@@ -5,6 +5,8 @@
 // each, see StepEntry::parity).  Steps, decays, exponentials, states and their sums are fp32.
 #pragma once
 
+#include <type_traits>
+
 #include "decoder_rows.cuh"
 
 namespace gptb200 {
@@ -244,8 +246,13 @@ mamba_step_kernel(float *__restrict__ y, const T *__restrict__ proj, long long l
     const int per_group = s.heads / s.groups, g = h / per_group;
     float *x = sm + 2 * N, *part = x + kStepCols;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    grid_dependency_wait();
-    grid_dependency_launch();
+    // In a bf16 step everything but the projection is older than this kernel's predecessor (see decoder_step_rows.cuh): the convolution's
+    // past and parameters and the state's first rows are on their way before the wait.
+    constexpr bool kEarly = !std::is_same<T, float>::value;
+    if (!kEarly) {
+        grid_dependency_wait();
+        grid_dependency_launch();
+    }
     const StepEntry e = entries[blockIdx.y];
     const long long row = e.row0;
     const int back = s.taps - 1;
@@ -253,28 +260,65 @@ mamba_step_kernel(float *__restrict__ y, const T *__restrict__ proj, long long l
     const T *old = conv + static_cast<long long>(e.parity) * back * s.channels;
     T *next = conv + static_cast<long long>(e.parity ^ 1) * back * s.channels;
     const bool owns_bc = p0 == 0 && h == g * per_group;
-    for (int i = threadIdx.x; i < 2 * N + kStepCols; i += blockDim.x) {
-        const bool is_x = i >= 2 * N;
-        if (is_x && p0 + i - 2 * N >= P) {
-            x[i - 2 * N] = 0.0f;
+    const int values = 2 * N + kStepCols;
+    const auto channel = [&](int i) { return i >= 2 * N ? h * P + p0 + i - 2 * N : i < N ? s.inner + g * N + i : s.inner + s.groups * N + g * N + i - N; };
+    const auto beyond = [&](int i) { return i >= 2 * N && p0 + i - 2 * N >= P; };
+    constexpr int kTaps = 3;   // past values held for this thread's first channel
+    float past[kTaps], tap[kTaps + 1], bias = 0.0f;
+    const int i0 = threadIdx.x;
+    const bool held = kEarly && back <= kTaps && i0 < values && !beyond(i0);
+    if (held) {
+        const int c = channel(i0);
+        bias = conv_b[c];
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) {
+            past[k] = k < back ? to_f(old[static_cast<long long>(k) * s.channels + c]) : 0.0f;
+            tap[k] = k < back ? taps[c * s.taps + k] : 0.0f;
+        }
+        tap[kTaps] = taps[c * s.taps + back];
+    }
+    const float *old_rows = reinterpret_cast<const float *>(e.slot + s.ssm_state) + static_cast<long long>(h) * N * P + p0 + lane + static_cast<long long>(e.parity) * s.heads * N * P;
+    float first[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) first[i] = p0 + lane < P && warp + 8 * i < N ? old_rows[static_cast<long long>(warp + 8 * i) * P] : 0.0f;
+    const float step_bias = dt_bias[h], rate = expf(a_log[h]);
+    if (kEarly) {
+        grid_dependency_wait();
+        grid_dependency_launch();
+    }
+    for (int i = threadIdx.x; i < values; i += blockDim.x) {
+        if (beyond(i)) {
+            sm[i] = 0.0f;
             continue;
         }
-        const int c = is_x ? h * P + p0 + i - 2 * N : i < N ? s.inner + g * N + i : s.inner + s.groups * N + g * N + i - N;
+        const bool keeps = i >= 2 * N || owns_bc;
+        const int c = channel(i);
         const T now = proj[row * ld_proj + s.inner + c];
-        float acc = conv_b[c];
-        for (int k = 0; k < back; ++k) {
-            const T v = old[static_cast<long long>(k) * s.channels + c];
-            acc = fmaf(taps[c * s.taps + k], to_f(v), acc);
-            if ((is_x || owns_bc) && k > 0) next[static_cast<long long>(k - 1) * s.channels + c] = v;
+        float acc;
+        if (held && i == i0) {
+            acc = bias;
+#pragma unroll
+            for (int k = 0; k < kTaps; ++k)
+                if (k < back) {
+                    acc = fmaf(tap[k], past[k], acc);
+                    if (keeps && k > 0) next[static_cast<long long>(k - 1) * s.channels + c] = from_f<T>(past[k]);
+                }
+            acc = fmaf(tap[kTaps], to_f(now), acc);
+        } else {
+            acc = conv_b[c];
+            for (int k = 0; k < back; ++k) {
+                const T v = old[static_cast<long long>(k) * s.channels + c];
+                acc = fmaf(taps[c * s.taps + k], to_f(v), acc);
+                if (keeps && k > 0) next[static_cast<long long>(k - 1) * s.channels + c] = v;
+            }
+            acc = fmaf(taps[c * s.taps + back], to_f(now), acc);
         }
-        if ((is_x || owns_bc) && back > 0) next[static_cast<long long>(back - 1) * s.channels + c] = now;
-        acc = fmaf(taps[c * s.taps + back], to_f(now), acc);
+        if (keeps && back > 0) next[static_cast<long long>(back - 1) * s.channels + c] = now;
         sm[i] = to_f(from_f<T>(silu_t<T>(acc)));   // rounded as the convolution of longer portions leaves it
     }
-    const float step = softplus_f(dt_raw[row * ld_dt + h] + dt_bias[h]), keep = expf(-expf(a_log[h]) * step);
+    const float step = softplus_f(dt_raw[row * ld_dt + h] + step_bias), keep = expf(-rate * step);
     __syncthreads();
     float *state = reinterpret_cast<float *>(e.slot + s.ssm_state) + static_cast<long long>(h) * N * P + p0 + lane;
-    const float *old_state = state + static_cast<long long>(e.parity) * s.heads * N * P;
     state += static_cast<long long>(e.parity ^ 1) * s.heads * N * P;
     float acc = 0.0f;
     if (p0 + lane < P) {
@@ -282,7 +326,7 @@ mamba_step_kernel(float *__restrict__ y, const T *__restrict__ proj, long long l
         for (int n0 = warp; n0 < N; n0 += 64) {   // eight rows in flight
             float v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = n0 + 8 * i < N ? old_state[static_cast<long long>(n0 + 8 * i) * P] : 0.0f;
+            for (int i = 0; i < 8; ++i) v[i] = n0 == warp ? first[i] : n0 + 8 * i < N ? old_rows[static_cast<long long>(n0 + 8 * i) * P] : 0.0f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int n = n0 + 8 * i;
@@ -311,10 +355,25 @@ __global__ void mamba_gated_norm_kernel(T *__restrict__ out, int ld_out, const f
 {
     extern __shared__ float sm[];   // [part]
     __shared__ float red[32];
-    grid_dependency_wait();
-    grid_dependency_launch();
     const long long row = blockIdx.x;
     const int part = s.inner / s.norm_groups, c0 = blockIdx.y * part;
+    if (!std::is_same<T, float>::value && part % 4 == 0 && part <= 4 * static_cast<int>(blockDim.x)) {
+        // a part in registers; z and the weights are older than the predecessor (see decoder_step_rows.cuh)
+        const int i = 4 * threadIdx.x;
+        const bool live = i < part;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 z = live ? load4(proj + row * ld_proj + c0 + i) : zero, w = live ? load4(weight + c0 + i) : zero;
+        const float4 g = make_float4(silu_t<T>(z.x), silu_t<T>(z.y), silu_t<T>(z.z), silu_t<T>(z.w));
+        grid_dependency_wait();
+        grid_dependency_launch();
+        const float4 a = live ? load4(y + row * s.inner + c0 + i) : zero;
+        const float4 v = make_float4(a.x * g.x, a.y * g.y, a.z * g.z, a.w * g.w);
+        const float inv = rsqrtf(block_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w, red) / part + eps);
+        if (live) store4(out + row * ld_out + c0 + i, make_float4(v.x * inv * w.x, v.y * inv * w.y, v.z * inv * w.z, v.w * inv * w.w));
+        return;
+    }
+    grid_dependency_wait();
+    grid_dependency_launch();
     float ss = 0.0f;
     if (part % 4 == 0) {   // y, z and the output are then aligned to four values
         for (int i = 4 * threadIdx.x; i < part; i += 4 * blockDim.x) {
