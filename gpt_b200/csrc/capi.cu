@@ -708,7 +708,7 @@ int make_word_tmap(gptb200_ctx *ctx, CUtensorMap *map, const void *base, long lo
 }
 
 // Launch of a weight-streaming kernel, early when the context allows it (see the kernels' header).
-int launch_gemv(gptb200_ctx *ctx, void (*kernel)(GemvParams), const GemvParams &g, int ctas, int groups, size_t smem)
+int launch_gemv(gptb200_ctx *ctx, void (*kernel)(GemvParams), const GemvParams &g, int ctas, int groups, size_t smem, int cluster = 1)
 {
     const void *key = reinterpret_cast<const void *>(kernel);
     if (smem > 48 * 1024 && !ctx->configured.count(key)) {
@@ -716,15 +716,24 @@ int launch_gemv(gptb200_ctx *ctx, void (*kernel)(GemvParams), const GemvParams &
         ctx->configured.insert(key);
     }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(ctas, groups);
+    cfg.gridDim = dim3(ctas, groups, cluster);
     cfg.blockDim = dim3(kGemvThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = ctx->decode_early_launch ? 1 : 0;
+    cudaLaunchAttribute attrs[2]{};
+    int n = 0;
+    if (cluster > 1) {
+        attrs[n].id = cudaLaunchAttributeClusterDimension;
+        attrs[n].val.clusterDim = {1, 1, static_cast<unsigned>(cluster)};
+        ++n;
+    }
+    if (ctx->decode_early_launch) {
+        attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attrs[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = attrs;
+    cfg.numAttrs = n;
     ctx->launches++;
     CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, g));
     return GPTB200_OK;
@@ -748,9 +757,12 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
             return g.k_warps > 1 ? launch_gemv(ctx, gemv_bf16_kernel<true>, g, need, groups, size_t(c.K) * 2)
                                  : launch_gemv(ctx, gemv_bf16_kernel<false>, g, std::max(1, std::min(need, ctx->num_sms * 4 / groups)), groups, size_t(c.K) * 2);
         }
-        const int tiles = is_glu(c.out_kind) || c.N >= 48 * ctx->num_sms ? 2 : 1;
+        const int tiles = is_glu(c.out_kind) ? 2 : 1;   // a gate tile and its up tile
         const int ctas = (widest + tiles * 16 - 1) / (tiles * 16);
-        return tiles == 2 ? launch_gemv(ctx, gemv_bf16_mma_kernel<2>, g, ctas, groups, 0) : launch_gemv(ctx, gemv_bf16_mma_kernel<1>, g, ctas, groups, 0);
+        // fewer CTAs than two per SM: a cluster shares a tile's k, each CTA at least 512 of it
+        int cluster = 1;
+        while (cluster < kGemvMaxCluster && ctas * groups * cluster < 2 * ctx->num_sms && c.K / (cluster * 2) >= 512) cluster *= 2;
+        return tiles == 2 ? launch_gemv(ctx, gemv_bf16_mma_kernel<2>, g, ctas, groups, 0, cluster) : launch_gemv(ctx, gemv_bf16_mma_kernel<1>, g, ctas, groups, 0, cluster);
     }
     const bool f32 = c.out_kind == OUT_F32;
     const long long out_words = f32 ? c.N : is_glu(c.out_kind) ? c.N / 4 : (std::min(c.N, c.tail_col) + 1) / 2;

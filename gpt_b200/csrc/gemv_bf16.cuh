@@ -8,6 +8,8 @@
 // by a kernel of a step).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "gemm_sm100.cuh"
 
 namespace gptb200 {
@@ -179,8 +181,11 @@ gemv_bf16_kernel(const GemvParams p)
 // block takes TILES x 16 weight rows (gated kinds: 16 gate rows and their 16 up rows) and its eight warps share k, so no value of x is read
 // twice by a block and x comes straight from L2.  The order of k inside a block
 // of 32 is permuted alike on both sides so that a lane loads 16 contiguous bytes of a row: piece c of a block (8 values) feeds
-// two products, values 0-3 the first and 4-7 the second.
-constexpr int kGemvMmaUnroll = 4;   // blocks of 32 k in flight per warp
+// two products, values 0-3 the first and 4-7 the second.  While a warp multiplies, its next blocks' weights are on their way.
+// Layers with few weight rows: the CTAs of a cluster (blockIdx.z) share a tile's k, so that all SMs have loads in flight; their sums meet
+// in the first CTA's shared memory in rank order.  Eight rows of the 2048-wide models, the products of a step: 415 -> 395 us for 1.8 GB.
+constexpr int kGemvMmaUnroll = 4;   // blocks of 32 k and tiles per buffer of weights and warp: two buffers of 32 registers leave two CTAs per SM
+constexpr int kGemvMaxCluster = 4;
 
 __device__ __forceinline__ void gemv_mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
 {
@@ -193,70 +198,100 @@ template <int TILES>
 __global__ void __launch_bounds__(kGemvThreads)
 gemv_bf16_mma_kernel(const GemvParams p)
 {
-    __shared__ float sums[8 * TILES * 16 * 8];   // [warp][weight row][row of x]
+    namespace cg = cooperative_groups;
+    constexpr int kSums = TILES * 16 * 8, kUnroll = kGemvMmaUnroll / TILES;
+    __shared__ float sums[8 * kSums];                 // [warp][weight row][row of x]
+    __shared__ float from_others[(kGemvMaxCluster - 1) * kSums];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;
     const int n0 = blockIdx.y * p.group_cols, N = min(p.N - n0, p.group_cols);   // this group's columns
+    const int S = gridDim.z, rank = blockIdx.z;
     const uint16_t *w = p.w + static_cast<long long>(n0) * p.K;
     // weight rows of the block's tiles
     int row[TILES];
 #pragma unroll
     for (int t = 0; t < TILES; ++t)
         row[t] = is_glu(p.out_kind) ? (blockIdx.x >> 1) * 64 + (blockIdx.x & 1) * 16 + t * 32 : (blockIdx.x * TILES + t) * 16;
-    const int blocks = (p.K + 31) / 32, per_warp = (blocks + 7) / 8;
-    const int first = warp * per_warp, end = min(blocks, first + per_warp);
-    uint4 wv[kGemvMmaUnroll][TILES][2];
-    auto fetch = [&](int blk) {
+    const int blocks = (p.K + 31) / 32, per_warp = (blocks + 8 * S - 1) / (8 * S);
+    const int first = min(blocks, (rank * 8 + warp) * per_warp), end = min(blocks, first + per_warp);
+    uint4 wv[2][kUnroll][TILES][2];
+    auto fetch = [&](uint4 (&v)[kUnroll][TILES][2], int blk) {
 #pragma unroll
-        for (int u = 0; u < kGemvMmaUnroll; ++u) {
+        for (int u = 0; u < kUnroll; ++u) {
             const int k = (blk + u) * 32 + c * 8;
 #pragma unroll
             for (int t = 0; t < TILES; ++t)
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     const int r = row[t] + g + 8 * half;
-                    wv[u][t][half] = blk + u < end && k < p.K && r < N ? __ldg(reinterpret_cast<const uint4 *>(w + static_cast<long long>(r) * p.K + k)) : make_uint4(0u, 0u, 0u, 0u);
+                    v[u][t][half] = blk + u < end && k < p.K && r < N ? __ldg(reinterpret_cast<const uint4 *>(w + static_cast<long long>(r) * p.K + k)) : make_uint4(0u, 0u, 0u, 0u);
                 }
         }
     };
-    fetch(first);
-    grid_dependency_wait();
-    grid_dependency_launch();
     float acc[TILES][4] = {};
     const bool live = g < p.M;   // this lane's row of x
     const uint16_t *xs = p.x + blockIdx.y * p.group_x + (live ? g : 0) * p.ldx + c * 8;
-    for (int blk = first; blk < end; blk += kGemvMmaUnroll) {
-        if (blk > first) fetch(blk);
-        uint4 xv[kGemvMmaUnroll];
+    auto multiply = [&](const uint4 (&v)[kUnroll][TILES][2], int blk) {
+        uint4 xv[kUnroll];
 #pragma unroll
-        for (int u = 0; u < kGemvMmaUnroll; ++u)
+        for (int u = 0; u < kUnroll; ++u)
             xv[u] = live && blk + u < end && (blk + u) * 32 + c * 8 < p.K ? *reinterpret_cast<const uint4 *>(xs + (blk + u) * 32) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-        for (int u = 0; u < kGemvMmaUnroll; ++u) {
+        for (int u = 0; u < kUnroll; ++u) {
             const uint4 x = xv[u];
 #pragma unroll
             for (int t = 0; t < TILES; ++t) {
-                const uint4 a = wv[u][t][0], b = wv[u][t][1];
+                const uint4 a = v[u][t][0], b = v[u][t][1];
                 gemv_mma_bf16(acc[t], a.x, b.x, a.y, b.y, x.x, x.y);
                 gemv_mma_bf16(acc[t], a.z, b.z, a.w, b.w, x.z, x.w);
             }
         }
+    };
+    fetch(wv[0], first);
+    if (first + kUnroll < end) fetch(wv[1], first + kUnroll);
+    grid_dependency_wait();
+    grid_dependency_launch();
+    for (int blk = first; blk < end; blk += 2 * kUnroll) {
+        multiply(wv[0], blk);
+        if (blk + 2 * kUnroll < end) fetch(wv[0], blk + 2 * kUnroll);
+        if (blk + kUnroll < end) {
+            multiply(wv[1], blk + kUnroll);
+            if (blk + 3 * kUnroll < end) fetch(wv[1], blk + 3 * kUnroll);
+        }
     }
+    if (S > 1) cg::this_cluster().barrier_arrive();   // this CTA runs: its shared memory may be written once all have arrived
 #pragma unroll
     for (int t = 0; t < TILES; ++t)
 #pragma unroll
         for (int i = 0; i < 4; ++i) sums[(warp * TILES * 16 + t * 16 + g + (i >> 1) * 8) * 8 + 2 * c + (i & 1)] = acc[t][i];
     __syncthreads();
-    const int outputs = is_glu(p.out_kind) ? 128 : TILES * 128;
+    if (S > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.barrier_wait();
+        if (rank > 0) {
+            float *there = cluster.map_shared_rank(from_others, 0) + (rank - 1) * kSums;
+            for (int i = threadIdx.x; i < kSums; i += kGemvThreads) {
+                float v = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v += sums[q * kSums + i];
+                there[i] = v;
+            }
+        }
+        cluster.sync();   // nothing remote is touched after this
+        if (rank > 0) return;
+    }
+    const int outputs = is_glu(p.out_kind) ? 128 : kSums;
     for (int i = threadIdx.x; i < outputs; i += kGemvThreads) {
         const int r = i >> 3, m = i & 7;
         if (m >= p.M) continue;
-        float v = 0.0f, up = 0.0f;
+        auto total = [&](int at) {
+            float v = 0.0f;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            v += sums[(w * TILES * 16 + r) * 8 + m];
-            if (TILES == 2 && is_glu(p.out_kind)) up += sums[(w * TILES * 16 + 16 + r) * 8 + m];
-        }
+            for (int q = 0; q < 8; ++q) v += sums[q * kSums + at];
+            for (int q = 1; q < S; ++q) v += from_others[(q - 1) * kSums + at];
+            return v;
+        };
+        const float v = total(i), up = TILES == 2 && is_glu(p.out_kind) ? total(128 + i) : 0.0f;
         const int n = is_glu(p.out_kind) ? row[0] + r : blockIdx.x * TILES * 16 + r;
         if (n < N) gemv_emit(p, m, n0 + n, v, up);
     }
