@@ -343,8 +343,20 @@ constexpr int kTileK = 32;
 //   (16-byte reads of 32 consecutive rows then touch every bank once) and a thread owns columns lane, lane + 32, + 64, + 96.
 constexpr int kTileNkPitch = 36;
 
+__device__ __forceinline__ void fma_pair(unsigned long long &d, unsigned long long a, unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ ulonglong2 pairs_of(const float4 &v)
+{
+    ulonglong2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.x) : "f"(v.x), "f"(v.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.y) : "f"(v.z), "f"(v.w));
+    return r;
+}
+
 template <int TM, bool W_NK>
-__global__ void __launch_bounds__(kDecodeThreads)
+__global__ void __launch_bounds__(kDecodeThreads, 2)
 decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const float *__restrict__ x, const float *__restrict__ w,
                            const float *__restrict__ bias, int M, int N, int K, int early_launch)
 {
@@ -410,10 +422,14 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };   // one group per chunk, empty past the end
 
     float acc[RT][4];
+    unsigned long long acc2[W_NK ? RT : 1][4];   // sums over even and odd k
 #pragma unroll
     for (int j = 0; j < RT; ++j)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[j][c] = 0.0f;
+        for (int c = 0; c < 4; ++c) {
+            acc[j][c] = 0.0f;
+            if (W_NK) acc2[j][c] = 0ull;
+        }
 
     // Early launch: the first stages' weights are requested before the predecessor on the stream is known to have finished,
     // x only after (the first group then holds all of those weights and the first x chunk: still in chunk order).
@@ -440,10 +456,17 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
                 float4 wc[4];   // four k-values of each of this thread's four columns
 #pragma unroll
                 for (int c = 0; c < 4; ++c) wc[c] = *reinterpret_cast<const float4 *>(ws + (lane + 32 * c) * kTileNkPitch + kk);
+                // packed FMAs: even and odd k side by side, as x and w lie in the stage: half the instructions (64 rows, k 768, n 50304: 155 -> 136 us, 36 TFLOP/s)
 #pragma unroll
-                for (int j = 0; j < RT; ++j)
+                for (int j = 0; j < RT; ++j) {
+                    const ulonglong2 xp = pairs_of(xv[j]);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[j][c] += xv[j].x * wc[c].x + xv[j].y * wc[c].y + xv[j].z * wc[c].z + xv[j].w * wc[c].w;
+                    for (int c = 0; c < 4; ++c) {
+                        const ulonglong2 wp = pairs_of(wc[c]);
+                        fma_pair(acc2[j][c], xp.x, wp.x);
+                        fma_pair(acc2[j][c], xp.y, wp.y);
+                    }
+                }
                 continue;
             }
             const float4 w0 = *reinterpret_cast<const float4 *>(ws + (kk + 0) * 128 + lane * 4);
@@ -467,7 +490,7 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
     for (int j = 0; j < RT; ++j) {
         if (W_NK) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) tile_smem[(warp * RT + j) * 128 + lane + 32 * c] = acc[j][c];
+            for (int c = 0; c < 4; ++c) tile_smem[(warp * RT + j) * 128 + lane + 32 * c] = __uint_as_float(static_cast<unsigned>(acc2[j][c])) + __uint_as_float(static_cast<unsigned>(acc2[j][c] >> 32));
         } else {
             *reinterpret_cast<float4 *>(tile_smem + (warp * RT + j) * 128 + lane * 4) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
         }
