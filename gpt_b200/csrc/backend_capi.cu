@@ -323,7 +323,7 @@ int gptb200_layernorm_backward(gptb200_ctx *ctx, float *grad_x, float *grad_gamm
             case 7: layernorm_backward_warp<7>(ctx, blocks, grad_x, wg, wb, grad_y, grad_residual, x, means, vars, gamma, rows); break;
             default: layernorm_backward_warp<8>(ctx, blocks, grad_x, wg, wb, grad_y, grad_residual, x, means, vars, gamma, rows); break;
         }
-        ops::layernorm_backward_params_final_kernel<<<(d + 31) / 32, dim3(32, 8), 0, ctx->stream>>>(grad_gamma, grad_beta, wg, wb, d, blocks);
+        ops::layernorm_backward_params_final_kernel<<<(d + 31) / 32, dim3(32, ops::kParamRows), 0, ctx->stream>>>(grad_gamma, grad_beta, wg, wb, d, blocks);
         return launched(ctx, 2);
     }
     const int threads = std::min(1024, std::max(32, ((d + 31) / 32) * 32));
@@ -337,7 +337,7 @@ int gptb200_layernorm_backward(gptb200_ctx *ctx, float *grad_x, float *grad_gamm
     float *wg = ctx->ws, *wb = ctx->ws + size_t(chunks) * d;
     ops::layernorm_backward_params_partial_kernel<<<dim3(col_groups, chunks), dim3(32, 8), 0, ctx->stream>>>(wg, wb, grad_y, x, means, vars,
                                                                                                              rows, d, rows_per_chunk);
-    ops::layernorm_backward_params_final_kernel<<<(d + 31) / 32, dim3(32, 8), 0, ctx->stream>>>(grad_gamma, grad_beta, wg, wb, d, chunks);
+    ops::layernorm_backward_params_final_kernel<<<(d + 31) / 32, dim3(32, ops::kParamRows), 0, ctx->stream>>>(grad_gamma, grad_beta, wg, wb, d, chunks);
     return launched(ctx, 3);
 }
 
