@@ -30,6 +30,10 @@ __global__ void kv_fill_kernel(float *__restrict__ cache, const float *__restric
     const int t = blockIdx.x, b = blockIdx.y;
     const float *src = qkv + (size_t(b) * seq_len + t) * 3 * d + d;
     float *dst = cache + (size_t(b) * max_len + t) * 2 * d;
+    if (d % 4 == 0 && ((reinterpret_cast<size_t>(src) | reinterpret_cast<size_t>(dst)) & 15) == 0) {
+        for (int i = 4 * threadIdx.x; i < 2 * d; i += 4 * blockDim.x) *reinterpret_cast<float4 *>(dst + i) = __ldcs(reinterpret_cast<const float4 *>(src + i));
+        return;
+    }
     for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) dst[i] = src[i];
 }
 

@@ -9,6 +9,7 @@
 // What is added for data-parallel training: the backward pass can report, layer by layer, that the weight
 // gradients of a layer are complete (a host callback fired right after that layer's operators were enqueued),
 // so that the caller can start all-reducing finished slices on another stream while the remaining layers run.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -286,9 +287,11 @@ public:
         gen_one_launch_ = one_launch;
         forward(prompt);
         const size_t M = size_t(batch) * prompt_len;
-        for (size_t l = 0; l < L; ++l) {
-            const int rc = gptb200_kv_cache_fill(ctx, gen_ + l * size_t(batch) * max_len * 2 * D, acts_ + a_.qkv + l * M * 3 * D, batch, prompt_len, max_len,
-                                                 c_.d_model);
+        // layers follow one another in the cache and in the activations as sequences do: as many per launch as a grid has room for
+        const size_t per = std::max<size_t>(1, 32768 / batch);
+        for (size_t l = 0; l < L; l += per) {
+            const int rc = gptb200_kv_cache_fill(ctx, gen_ + l * size_t(batch) * max_len * 2 * D, acts_ + a_.qkv + l * M * 3 * D, static_cast<int>(std::min(per, L - l)) * batch,
+                                                 prompt_len, max_len, c_.d_model);
             if (rc) return rc;
         }
         gen_pos_off_ = cache_floats + step_floats - 8;
