@@ -40,6 +40,16 @@ struct PrefillParams {
     int *status;
 };
 
+// The requests of one launch (blockIdx.z): several prompts of a step side by side, each with its own rows, keys and values.  One prompt of 870 tokens and
+// 12 heads is 48 blocks, a third of the machine.
+constexpr int kPrefillRequests = 8;
+
+template <int REQUESTS>
+struct alignas(64) PrefillBatch {
+    CUtensorMap q[REQUESTS], kv[REQUESTS], shared[REQUESTS];
+    PrefillParams p[REQUESTS];
+};
+
 constexpr int kPrefillThreads = 384;
 constexpr int kPrefillBlock = 128 * 128;   // bytes of one [128 rows x 64 bf16] block
 constexpr int kPrefillMaxStages = 3;
@@ -149,13 +159,18 @@ __device__ __forceinline__ float capped(float x, float cap) { return fmaf(-2.0f 
 
 }  // namespace ptx_attn
 
-// grid: (heads, blocks of 256 rows).  map_kv: rows of [keys of all heads | values of all heads]; map_shared: rows with the key part that all heads share.
+// grid: (heads, blocks of 256 rows of the longest request, requests).  map_kv: rows of [keys of all heads | values of all heads]; map_shared: rows with the key part that all heads share.
 // CAPPED: scores become cap * tanh(score / cap).  Special-function instructions (exponential, reciprocal) are what this kernel runs out of
 // first, so where all scores of a warp's rows lie within the cap tanh is a polynomial; else 1 - 2 / (1 + exp(2 score / cap)).
-template <bool CAPPED>
+template <bool CAPPED, int REQUESTS>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
-attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_shared, const PrefillParams p)
+attention_prefill_kernel(const __grid_constant__ PrefillBatch<REQUESTS> batch)
 {
+    const int request = REQUESTS > 1 ? blockIdx.z : 0;
+    const CUtensorMap &map_q = batch.q[request], &map_kv = batch.kv[request], &map_shared = batch.shared[request];
+    const PrefillParams &p = batch.p[request];
+    const int row_blocks = (p.rows + 255) / 256;
+    if (static_cast<int>(blockIdx.y) >= row_blocks) return;   // a shorter request's
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *gen = smem_raw + (base - ptx::smem_u32(smem_raw));
@@ -178,7 +193,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int head = blockIdx.x, kv_head = head / p.kv_share;
-    const int row_base = (gridDim.y - 1 - blockIdx.y) * 256;   // the longest rows of all heads first
+    const int row_base = (row_blocks - 1 - static_cast<int>(blockIdx.y)) * 256;   // the longest rows of all heads first
     // key blocks of the two tiles
     int n_blocks[2];
 #pragma unroll

@@ -279,6 +279,7 @@ public:
         if (!strcmp(key, "segment_tokens")) {   // Mamba-2 and lightning prompts: tokens per segment (a multiple of 64)
             if (value < kChunk || value % kChunk) return fail(ctx_, GPTB200_ERR_INVALID_ARG, "segment_tokens must be a multiple of %d", kChunk);
             segment_tokens_ = value;
+            segment_auto_ = false;
             return GPTB200_OK;
         }
         if (!strcmp(key, "wkv_segment_tokens")) {   // wkv prompts: tokens per segment (a multiple of 16; 0: automatic)
@@ -926,7 +927,14 @@ private:
             int longest = 0;
             for (int i = 0; i < n; ++i) longest = std::max(longest, parts[entry0 + i].count);
             const int blocks = s.heads * ((s.vdim + kChunkCols - 1) / kChunkCols);
-            const int tokens = longest > segment_tokens_ + segment_tokens_ / 2 ? segment_tokens_ : pad_to(longest, kChunk);
+            // of the option's tokens, or shorter where the heads and requests of a step leave blocks of the machine (two per SM) idle: a chunk after the
+            // other takes 5 us, the pass for the states in front of the segments half of what it saves (three prompts of 870 tokens, 12 heads of 64)
+            int segment = segment_tokens_;
+            if (segment_auto_) {
+                const int side_by_side = std::max(1, 2 * ctx_->num_sms / (blocks * n));
+                segment = std::min(segment, std::max(kShortestSegment, pad_to((longest + side_by_side - 1) / side_by_side, kChunk)));
+            }
+            const int tokens = longest > segment + segment / 2 ? segment : pad_to(longest, kChunk);
             const int segments = (longest + tokens - 1) / tokens;
             const size_t smem = size_t(chunk_smem_bytes(s.state));
             float *seg_state = nullptr, *seg_decay = nullptr;
@@ -1045,12 +1053,12 @@ private:
             Bf16Linear c{};
             c.M = positions; c.N = cols; c.K = s.rank_pitch; c.a = cache; c.lda = s.row_pitch; c.w = d.w_uk; c.out_kind = OUT_BF16; c.out = expanded_; c.ldo = cols;
             RC_TRY(run_linear_bf16(ctx_, c));
-            CUtensorMap mq, mkv, mc;
+            PrefillBatch<1> batch{};
             const T *q = proj_ + size_t(part.row0) * d.proj_cols;
-            RC_TRY(bf16_operand_map(ctx_, &mq, q, part.count, d.proj_cols, d.proj_cols, 128));
-            RC_TRY(bf16_operand_map(ctx_, &mkv, expanded_, positions, cols, cols, 128));
-            RC_TRY(bf16_operand_map(ctx_, &mc, cache, positions, s.row_pitch, s.row_pitch, 128));
-            PrefillParams p{};
+            RC_TRY(bf16_operand_map(ctx_, &batch.q[0], q, part.count, d.proj_cols, d.proj_cols, 128));
+            RC_TRY(bf16_operand_map(ctx_, &batch.kv[0], expanded_, positions, cols, cols, 128));
+            RC_TRY(bf16_operand_map(ctx_, &batch.shared[0], cache, positions, s.row_pitch, s.row_pitch, 128));
+            PrefillParams &p = batch.p[0];
             p.rows = part.count; p.pos0 = slot.length;
             p.heads = s.heads; p.vdim = s.vdim; p.v_pad = s.v_pad;
             p.kv_share = 1;
@@ -1064,8 +1072,8 @@ private:
             p.out = act_ + size_t(part.row0) * d.mix_out; p.ld_out = d.mix_out;
             p.gate = q + s.off_g; p.ld_gate = d.proj_cols;
             p.status = ctx_->d_status;
-            return launch(attention_prefill_kernel<false>, dim3(s.heads, (part.count + 255) / 256), dim3(kPrefillThreads),
-                          size_t(prefill_smem_bytes(p.u_blocks, p.r_blocks, p.v_blocks, p.k_stages, p.v_stages)), mq, mkv, mc, p);
+            return launch(attention_prefill_kernel<false, 1>, dim3(s.heads, (part.count + 255) / 256), dim3(kPrefillThreads),
+                          size_t(prefill_smem_bytes(p.u_blocks, p.r_blocks, p.v_blocks, p.k_stages, p.v_stages)), batch);
         }
     }
 
@@ -1132,14 +1140,15 @@ private:
             if (widest <= 256) return run(grouped_rows_kernel<T, 8>);
             return run(grouped_rows_kernel<T, 24>);
         } else {
-            // long portions one by one on the tensor cores, runs of short ones together over ranges of positions
+            // runs of long portions together on the tensor cores, runs of short ones over ranges of positions
             int v_stages = 0;
             const int k_stages = prefill_stages(s.dim_pad, 0, s.v_pad, &v_stages);
             const auto is_long = [&](const Part &p) { return k_stages > 0 && p.count >= expand_rows_; };
             for (size_t i = 0, j; i < parts.size(); i = j) {
                 j = i + 1;
                 if (is_long(parts[i])) {
-                    RC_TRY(grouped_prompt(d, parts[i], k_stages, v_stages));
+                    while (j < parts.size() && j - i < kPrefillRequests && is_long(parts[j])) ++j;
+                    RC_TRY(j - i == 1 ? grouped_prompts<1>(d, &parts[i], 1, k_stages, v_stages) : grouped_prompts<kPrefillRequests>(d, &parts[i], static_cast<int>(j - i), k_stages, v_stages));
                     continue;
                 }
                 int positions = 0;
@@ -1179,39 +1188,48 @@ private:
         }
     }
 
-    int grouped_prompt(const Layer &d, const Part &part, int k_stages, int v_stages)
+    // Prompts of neighbouring requests, one launch.
+    template <int REQUESTS>
+    int grouped_prompts(const Layer &d, const Part *parts, int n, int k_stages, int v_stages)
     {
         if constexpr (kF32) {
             return GPTB200_OK;
         } else {
             const GroupedShape &s = d.grouped;
-            const Slot &slot = slots_[part.slot];
-            const T *cache = reinterpret_cast<const T *>(slot.base + s.cache_base + s.cache_per_position * slot.capacity), *q = proj_ + size_t(part.row0) * d.proj_cols;
-            CUtensorMap mq, mkv;
-            RC_TRY(bf16_operand_map(ctx_, &mq, q, part.count, d.proj_cols, d.proj_cols, 128));
-            RC_TRY(bf16_operand_map(ctx_, &mkv, cache, slot.length + part.count, s.row_pitch, s.row_pitch, 128));
-            PrefillParams p{};
-            p.rows = part.count; p.pos0 = slot.length;
-            p.heads = s.heads; p.vdim = s.vdim; p.v_pad = s.v_pad;
-            p.kv_share = s.heads / s.kv_heads;
-            p.q_stride = s.dim_pad; p.q_rot = s.dim_pad;
-            p.dim_pad = s.dim_pad; p.rot_pad = 0;
-            p.u_blocks = (s.dim_pad + 63) / 64; p.r_blocks = 0; p.v_blocks = (s.v_pad + 63) / 64;
-            p.k_stages = k_stages; p.v_stages = v_stages;
-            p.v_col0 = s.kv_heads * s.dim_pad;
-            constexpr double kLog2e = 1.4426950408889634;
-            p.scale_log2 = static_cast<float>(s.scale * kLog2e);
-            if (s.softcap > 0.0f) {
-                p.cap_log2 = static_cast<float>(s.softcap * kLog2e);
-                p.cap_arg = s.scale / s.softcap;
+            PrefillBatch<REQUESTS> batch{};
+            int longest = 0;
+            for (int i = 0; i < n; ++i) {
+                const Part &part = parts[i];
+                const Slot &slot = slots_[part.slot];
+                const T *cache = reinterpret_cast<const T *>(slot.base + s.cache_base + s.cache_per_position * slot.capacity), *q = proj_ + size_t(part.row0) * d.proj_cols;
+                RC_TRY(bf16_operand_map(ctx_, &batch.q[i], q, part.count, d.proj_cols, d.proj_cols, 128));
+                RC_TRY(bf16_operand_map(ctx_, &batch.kv[i], cache, slot.length + part.count, s.row_pitch, s.row_pitch, 128));
+                batch.shared[i] = batch.kv[i];
+                PrefillParams &p = batch.p[i];
+                p.rows = part.count; p.pos0 = slot.length;
+                p.heads = s.heads; p.vdim = s.vdim; p.v_pad = s.v_pad;
+                p.kv_share = s.heads / s.kv_heads;
+                p.q_stride = s.dim_pad; p.q_rot = s.dim_pad;
+                p.dim_pad = s.dim_pad; p.rot_pad = 0;
+                p.u_blocks = (s.dim_pad + 63) / 64; p.r_blocks = 0; p.v_blocks = (s.v_pad + 63) / 64;
+                p.k_stages = k_stages; p.v_stages = v_stages;
+                p.v_col0 = s.kv_heads * s.dim_pad;
+                constexpr double kLog2e = 1.4426950408889634;
+                p.scale_log2 = static_cast<float>(s.scale * kLog2e);
+                if (s.softcap > 0.0f) {
+                    p.cap_log2 = static_cast<float>(s.softcap * kLog2e);
+                    p.cap_arg = s.scale / s.softcap;
+                }
+                p.out = act_ + size_t(part.row0) * d.mix_out; p.ld_out = d.mix_out;
+                p.gate = q + s.off_g; p.ld_gate = d.proj_cols;
+                p.status = ctx_->d_status;
+                longest = std::max(longest, part.count);
             }
-            p.out = act_ + size_t(part.row0) * d.mix_out; p.ld_out = d.mix_out;
-            p.gate = q + s.off_g; p.ld_gate = d.proj_cols;
-            p.status = ctx_->d_status;
+            const PrefillParams &p = batch.p[0];
             const size_t smem = size_t(prefill_smem_bytes(p.u_blocks, 0, p.v_blocks, k_stages, v_stages));
-            const dim3 grid(s.heads, (part.count + 255) / 256);
-            return s.softcap > 0.0f ? launch(attention_prefill_kernel<true>, grid, dim3(kPrefillThreads), smem, mq, mkv, mkv, p)
-                                    : launch(attention_prefill_kernel<false>, grid, dim3(kPrefillThreads), smem, mq, mkv, mkv, p);
+            const dim3 grid(s.heads, (longest + 255) / 256, n);
+            return s.softcap > 0.0f ? launch(attention_prefill_kernel<true, REQUESTS>, grid, dim3(kPrefillThreads), smem, batch)
+                                    : launch(attention_prefill_kernel<false, REQUESTS>, grid, dim3(kPrefillThreads), smem, batch);
         }
     }
 
@@ -1454,6 +1472,8 @@ private:
     std::vector<void *> weights_, work_;
     std::vector<Slot> slots_;
     int pass_rows_ = 4096, expand_rows_ = 32, chunk_rows_ = 8, segment_tokens_ = 1024, wkv_segment_tokens_ = 0;
+    bool segment_auto_ = true;   // segment_tokens_ was not set: shorter segments where they fill the machine
+    static constexpr int kShortestSegment = 256;
     T *expanded_ = nullptr;
     size_t expanded_count_ = 0;
     float *scratch_ = nullptr;

@@ -357,7 +357,7 @@ int gptb200_model_step_count(gptb200_model *m);
  *                   in the tensor-core form for prompts, default 32; shorter ones split the positions, latent attention then uses the
  *                   latents as they are), "chunk_rows" (recurrent layers in bf16: shortest portion that runs in chunks on the tensor
  *                   cores, default 8; shorter ones token by token), "segment_tokens" (Mamba-2 and lightning prompts: tokens per segment of the
- *                   segments that run side by side, default 1024), "wkv_segment_tokens" (the same for wkv, a multiple of 16, default 0:
+ *                   segments that run side by side; unless set 1024, or fewer where a step would leave the GPU idle), "wkv_segment_tokens" (the same for wkv, a multiple of 16, default 0:
  *                   automatic) and those of gptb200_ctx_set_option */
 typedef enum gptb200_dtype { GPTB200_DTYPE_BF16 = 0, GPTB200_DTYPE_F32 = 1 } gptb200_dtype;
 typedef struct gptb200_decoder gptb200_decoder;
