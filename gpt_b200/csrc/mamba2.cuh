@@ -247,7 +247,8 @@ mamba_step_kernel(float *__restrict__ y, const T *__restrict__ proj, long long l
     float *x = sm + 2 * N, *part = x + kStepCols;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // In a bf16 step everything but the projection is older than this kernel's predecessor (see decoder_step_rows.cuh): the convolution's
-    // past and parameters and the state's first rows are on their way before the wait.
+    // past and parameters and the state's first rows are on their way before the wait (with the gated norm and the latent combination done alike a step
+    // of the 768-wide model of 12 layers: 402 -> 378 us).
     constexpr bool kEarly = !std::is_same<T, float>::value;
     if (!kEarly) {
         grid_dependency_wait();
