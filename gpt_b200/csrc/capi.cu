@@ -256,7 +256,7 @@ bool cluster16_allowed(gptb200_ctx *ctx)
 {
     if (ctx->cluster16 < 0) {
         auto kernel = decode_tile_cluster_kernel<64, false>;
-        const size_t smem = size_t(kTileStages) * (kTileK * 128 + 64 * kTileK) * sizeof(float);
+        const size_t smem = tile_smem_floats(64, false) * sizeof(float);
         int clusters = 0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1, 16, 1);
@@ -316,7 +316,7 @@ template <int TM, bool W_NK>
 int launch_decode_tile(gptb200_ctx *ctx, const GemmCall &c, int cluster)
 {
     auto kernel = decode_tile_cluster_kernel<TM, W_NK>;
-    const size_t smem = size_t(kTileStages) * ((W_NK ? 128 * kTileNkPitch : kTileK * 128) + TM * kTileK) * sizeof(float);
+    const size_t smem = tile_smem_floats(TM, W_NK) * sizeof(float);
     const void *key = reinterpret_cast<const void *>(kernel);
     if (!ctx->configured.count(key)) {
         CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));

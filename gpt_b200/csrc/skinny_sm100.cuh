@@ -335,24 +335,16 @@ decode_gemm_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
 // zero-padded), a thread TM/8 rows x 4 columns.  k is split over the S CTAs of a thread-block cluster (cluster shape
 // (1, S, 1)); the partial tiles meet through distributed shared memory in rank order, each CTA finishing 1/S of the rows
 // (bias, GELU).  No scratch, no second launch; results do not depend on timing.
-//   grid (ceil(n / 128), S, ceil(m / TM)); dynamic shared memory kTileStages * (32 * 128 + TM * 32) floats.
-constexpr int kTileStages = 4;
-constexpr int kTileK = 32;
-
 //   W_NK: W stored [n][k] instead (the tied un-embedding, grad_x): the stage holds w[128 n][32 k] with rows padded to 36 floats
 //   (16-byte reads of 32 consecutive rows then touch every bank once) and a thread owns columns lane, lane + 32, + 64, + 96.
+//   grid (ceil(n / 128), S, ceil(m / TM)); dynamic shared memory tile_smem_floats().
+constexpr int kTileK = 32;
 constexpr int kTileNkPitch = 36;
-
-__device__ __forceinline__ void fma_pair(unsigned long long &d, unsigned long long a, unsigned long long b)
+constexpr int kTileRun = 8;   // W_NK: stages that a running sum goes through
+__host__ __device__ constexpr int tile_stages(int tm, bool w_nk) { return w_nk && tm == 64 ? 3 : 4; }   // two CTAs fit an SM
+__host__ __device__ constexpr size_t tile_smem_floats(int tm, bool w_nk)
 {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ ulonglong2 pairs_of(const float4 &v)
-{
-    ulonglong2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.x) : "f"(v.x), "f"(v.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.y) : "f"(v.z), "f"(v.w));
-    return r;
+    return size_t(tile_stages(tm, w_nk)) * ((w_nk ? 128 * kTileNkPitch : kTileK * 128) + tm * kTileK) + (w_nk ? tm * 128 : 0);
 }
 
 template <int TM, bool W_NK>
@@ -364,7 +356,7 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
     cg::cluster_group cluster = cg::this_cluster();
     constexpr int RT = TM / 8;                                   // rows per thread
     constexpr int kWFloats = W_NK ? 128 * kTileNkPitch : kTileK * 128;
-    constexpr int kStageFloats = kWFloats + TM * kTileK;         // w[32][128] (or w[128][36]) then x[TM][32]
+    constexpr int kStageFloats = kWFloats + TM * kTileK, kStages = tile_stages(TM, W_NK);   // w[32][128] (or w[128][36]) then x[TM][32]
     extern __shared__ __align__(16) float tile_smem[];
     const int S = gridDim.y, rank = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -382,7 +374,7 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
 
     auto load_w = [&](int chunk) {   // weights: 32 rows of 32 16-byte pieces
         if (chunk >= chunks) return;
-        float *ws = tile_smem + (chunk % kTileStages) * kStageFloats;
+        float *ws = tile_smem + (chunk % kStages) * kStageFloats;
         const int k0 = k_begin + chunk * kTileK;
 #pragma unroll
         for (int i = 0; i < (kTileK * 32) / kDecodeThreads; ++i) {
@@ -406,7 +398,7 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
     };
     auto load_x = [&](int chunk) {   // x: TM rows of 8 pieces
         if (chunk >= chunks) return;
-        float *xs = tile_smem + (chunk % kTileStages) * kStageFloats + kWFloats;
+        float *xs = tile_smem + (chunk % kStages) * kStageFloats + kWFloats;
         const int k0 = k_begin + chunk * kTileK;
 #pragma unroll
         for (int i = 0; i < (TM * 8 + kDecodeThreads - 1) / kDecodeThreads; ++i) {
@@ -421,79 +413,85 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };   // one group per chunk, empty past the end
 
-    float acc[RT][4];
-    unsigned long long acc2[W_NK ? RT : 1][4];   // sums over even and odd k
+    float acc[W_NK ? 1 : RT][4] = {};
+    unsigned long long run[W_NK ? RT : 1][4] = {};   // W_NK: running sums over even and odd k, side by side as x and w lie in the stage,
+    float *tile = tile_smem + (W_NK ? kStages * kStageFloats : 0);   // this CTA's partial tile [TM][128]
+    bool first_run = true;
+    auto end_run = [&] {   // added to the tile (each thread has its own places)
 #pragma unroll
-    for (int j = 0; j < RT; ++j)
+        for (int j = 0; j < (W_NK ? RT : 0); ++j)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            acc[j][c] = 0.0f;
-            if (W_NK) acc2[j][c] = 0ull;
-        }
+            for (int c = 0; c < 4; ++c) {
+                float *at = tile + (warp * RT + j) * 128 + lane + 32 * c;
+                const float v = __uint_as_float(static_cast<unsigned>(run[j][c])) + __uint_as_float(static_cast<unsigned>(run[j][c] >> 32));
+                *at = first_run ? v : *at + v;
+                run[j][c] = 0ull;
+            }
+        first_run = false;
+    };
 
     // Early launch: the first stages' weights are requested before the predecessor on the stream is known to have finished,
     // x only after (the first group then holds all of those weights and the first x chunk: still in chunk order).
-    for (int sidx = 0; sidx < kTileStages - 1; ++sidx) load_w(sidx);
+    for (int sidx = 0; sidx < kStages - 1; ++sidx) load_w(sidx);
     if (early_launch) asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int sidx = 0; sidx < kTileStages - 1; ++sidx) {
+    for (int sidx = 0; sidx < kStages - 1; ++sidx) {
         load_x(sidx);
         commit();
     }
     for (int chunk = 0; chunk < chunks; ++chunk) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kTileStages - 2) : "memory");   // this chunk has landed (own copies)
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");   // this chunk has landed (own copies)
         __syncthreads();                                                              // ... everyone's; and the slot refilled below is free
-        load_w(chunk + kTileStages - 1);
-        load_x(chunk + kTileStages - 1);
+        load_w(chunk + kStages - 1);
+        load_x(chunk + kStages - 1);
         commit();
-        const float *ws = tile_smem + (chunk % kTileStages) * kStageFloats;
+        const float *ws = tile_smem + (chunk % kStages) * kStageFloats;
         const float *xs = ws + kWFloats + warp * RT * kTileK;
+        if constexpr (W_NK) {
+            // Packed FMAs, bound by their number: 64 rows, k 768, n 50304 take 142 us, 154 as scalar FMAs that add up four products before the running
+            // sum.  One running sum over all of k takes 138 us, but its chain of roundings is twice as long as the scalar form's and the error 3.5e-7 of the
+            // result instead of 2.5e-7; in runs of kTileRun stages it is 2.1e-7 (four stages: 144 us, 1.6e-7).
 #pragma unroll
-        for (int kk = 0; kk < kTileK; kk += 4) {
-            float4 xv[RT];
+            for (int kk = 0; kk < kTileK; kk += 4) {
+                ulonglong2 wc[4];   // four k-values of each of this thread's four columns
 #pragma unroll
-            for (int j = 0; j < RT; ++j) xv[j] = *reinterpret_cast<const float4 *>(xs + j * kTileK + kk);   // warp-uniform: broadcast
-            if (W_NK) {
-                float4 wc[4];   // four k-values of each of this thread's four columns
-#pragma unroll
-                for (int c = 0; c < 4; ++c) wc[c] = *reinterpret_cast<const float4 *>(ws + (lane + 32 * c) * kTileNkPitch + kk);
-                // packed FMAs: even and odd k side by side, as x and w lie in the stage: half the instructions (64 rows, k 768, n 50304: 155 -> 136 us, 36 TFLOP/s)
+                for (int c = 0; c < 4; ++c) wc[c] = *reinterpret_cast<const ulonglong2 *>(ws + (lane + 32 * c) * kTileNkPitch + kk);
 #pragma unroll
                 for (int j = 0; j < RT; ++j) {
-                    const ulonglong2 xp = pairs_of(xv[j]);
+                    const ulonglong2 xp = *reinterpret_cast<const ulonglong2 *>(xs + j * kTileK + kk);   // warp-uniform: broadcast
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const ulonglong2 wp = pairs_of(wc[c]);
-                        fma_pair(acc2[j][c], xp.x, wp.x);
-                        fma_pair(acc2[j][c], xp.y, wp.y);
-                    }
+                    for (int c = 0; c < 4; ++c) run[j][c] = ptx::fma2(xp.y, wc[c].y, ptx::fma2(xp.x, wc[c].x, run[j][c]));
                 }
-                continue;
             }
-            const float4 w0 = *reinterpret_cast<const float4 *>(ws + (kk + 0) * 128 + lane * 4);
-            const float4 w1 = *reinterpret_cast<const float4 *>(ws + (kk + 1) * 128 + lane * 4);
-            const float4 w2 = *reinterpret_cast<const float4 *>(ws + (kk + 2) * 128 + lane * 4);
-            const float4 w3 = *reinterpret_cast<const float4 *>(ws + (kk + 3) * 128 + lane * 4);
+            if (chunk % kTileRun == kTileRun - 1) end_run();
+        } else {
 #pragma unroll
-            for (int j = 0; j < RT; ++j) {
-                acc[j][0] += xv[j].x * w0.x + xv[j].y * w1.x + xv[j].z * w2.x + xv[j].w * w3.x;
-                acc[j][1] += xv[j].x * w0.y + xv[j].y * w1.y + xv[j].z * w2.y + xv[j].w * w3.y;
-                acc[j][2] += xv[j].x * w0.z + xv[j].y * w1.z + xv[j].z * w2.z + xv[j].w * w3.z;
-                acc[j][3] += xv[j].x * w0.w + xv[j].y * w1.w + xv[j].z * w2.w + xv[j].w * w3.w;
+            for (int kk = 0; kk < kTileK; kk += 4) {
+                float4 xv[RT];
+#pragma unroll
+                for (int j = 0; j < RT; ++j) xv[j] = *reinterpret_cast<const float4 *>(xs + j * kTileK + kk);   // warp-uniform: broadcast
+                const float4 w0 = *reinterpret_cast<const float4 *>(ws + (kk + 0) * 128 + lane * 4);
+                const float4 w1 = *reinterpret_cast<const float4 *>(ws + (kk + 1) * 128 + lane * 4);
+                const float4 w2 = *reinterpret_cast<const float4 *>(ws + (kk + 2) * 128 + lane * 4);
+                const float4 w3 = *reinterpret_cast<const float4 *>(ws + (kk + 3) * 128 + lane * 4);
+#pragma unroll
+                for (int j = 0; j < RT; ++j) {
+                    acc[j][0] += xv[j].x * w0.x + xv[j].y * w1.x + xv[j].z * w2.x + xv[j].w * w3.x;
+                    acc[j][1] += xv[j].x * w0.y + xv[j].y * w1.y + xv[j].z * w2.y + xv[j].w * w3.y;
+                    acc[j][2] += xv[j].x * w0.z + xv[j].y * w1.z + xv[j].z * w2.z + xv[j].w * w3.z;
+                    acc[j][3] += xv[j].x * w0.w + xv[j].y * w1.w + xv[j].z * w2.w + xv[j].w * w3.w;
+                }
             }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     // the successor may start now (its CTAs hold shared memory while they wait: not before this kernel's main loop is over)
     if (early_launch) asm volatile("griddepcontrol.launch_dependents;");
-    __syncthreads();   // all reads of the ring are done: it becomes this CTA's partial tile [TM][128]
+    if constexpr (W_NK) {
+        end_run();
+    } else {
+        __syncthreads();   // all reads of the ring are done: it becomes this CTA's partial tile
 #pragma unroll
-    for (int j = 0; j < RT; ++j) {
-        if (W_NK) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) tile_smem[(warp * RT + j) * 128 + lane + 32 * c] = __uint_as_float(static_cast<unsigned>(acc2[j][c])) + __uint_as_float(static_cast<unsigned>(acc2[j][c] >> 32));
-        } else {
-            *reinterpret_cast<float4 *>(tile_smem + (warp * RT + j) * 128 + lane * 4) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
-        }
+        for (int j = 0; j < RT; ++j) *reinterpret_cast<float4 *>(tile + (warp * RT + j) * 128 + lane * 4) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
     }
     cluster.sync();
     // rank order; this CTA finishes every S-th group of 256 four-column pieces
@@ -505,7 +503,7 @@ decode_tile_cluster_kernel(float *__restrict__ y, float *__restrict__ act, const
             float4 v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                v[j] = q0 + j < S ? reinterpret_cast<const float4 *>(cluster.map_shared_rank(tile_smem, q0 + j))[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[j] = q0 + j < S ? reinterpret_cast<const float4 *>(cluster.map_shared_rank(tile, q0 + j))[e] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int j = 0; j < 8; ++j)
                 if (q0 + j < S) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
