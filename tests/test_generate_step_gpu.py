@@ -71,3 +71,36 @@ def test_generation_step_matches_the_whole_forward_pass(size, batch, layers, pro
         assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
     assert model.generate_position == prompt + steps
     model.close()
+
+
+@pytest.mark.parametrize("batch,prompt,steps", [(1, 8, 40), (2, 8, 24), (5, 8, 16), (12, 5, 12), (64, 2, 6)])
+def test_one_launch_is_as_exact_as_the_operators(batch, prompt, steps):
+    """GPT-2 124M's layers: the logits' error against 64 bits is no larger than that of the step that runs operator by operator (option
+    skinny_rows) on the same cache, texts and weights; both are fixed, so there is nothing to allow for."""
+    import torch
+    import gpt_b200
+    c = dict(max_seq_len=64, num_layers=12, vocab_size=2000, **dict(GPT2, vocab_size_padded=2000))
+    gen = torch.Generator(device="cuda").manual_seed(batch)
+    parts = []
+    for name, shape in _shapes(c):
+        t = torch.randn(*shape, device="cuda", generator=gen) * (0.004 if name in ("proj_w", "down_w") else 0.02)
+        parts.append((t + (1.0 if name in ("ln1_w", "ln2_w", "lnf_w") else 0.0)).reshape(-1))
+    flat = torch.cat(parts)
+    text = torch.randint(0, c["vocab_size"], (batch, prompt + steps), device="cuda", dtype=torch.int32, generator=gen)
+    want = _forward(torch, c, flat.double(), text)[:, prompt:].transpose(0, 1)
+    errors = []
+    for operators in (False, True):
+        model = gpt_b200.Model(c, 0, torch.cuda.current_stream().cuda_stream, gpt_b200.MODE_3XTF32, use_grad=False)
+        model.load_weights(flat.cpu().numpy())
+        if operators:
+            model.set_option("skinny_rows", 64)
+        model.generate_begin(text[:, :prompt].contiguous(), batch, prompt, prompt + steps)
+        out = torch.empty(steps, batch, c["vocab_size_padded"], device="cuda")
+        before = model.launch_count()
+        for i in range(steps):
+            model.generate_step(text[:, prompt + i].contiguous(), out[i])
+        assert (model.launch_count() - before > 2 * steps) == operators
+        torch.cuda.synchronize()
+        errors.append(float((out.double() - want).norm() / want.norm()))
+        model.close()
+    assert errors[0] <= errors[1], errors
