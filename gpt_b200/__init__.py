@@ -26,7 +26,7 @@ MODE_TF32 = 1
 EXPORTED_SYMBOLS = [
     "gptb200_ctx_create", "gptb200_ctx_destroy", "gptb200_ctx_set_mode", "gptb200_ctx_get_mode",
     "gptb200_ctx_set_stream", "gptb200_ctx_set_option", "gptb200_ctx_synchronize", "gptb200_ctx_launch_count", "gptb200_ctx_tensor_map_encodes", "gptb200_ctx_read_trace",
-    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_decode", "gptb200_selftest_wait_timeout",
+    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_decode", "gptb200_selftest_wait_timeout", "gptb200_selftest_grid_barrier",
     "gptb200_linear_forward", "gptb200_linear_backward", "gptb200_linear_backward_weights", "gptb200_linear_backward_input",
     "gptb200_linear_backward_input_gelu", "gptb200_gemm_batched",
     "gptb200_gelu_backward",
@@ -77,6 +77,7 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         "gptb200_ctx_launch_count": (ctypes.c_longlong, [vp]),
         "gptb200_ctx_tensor_map_encodes": (ctypes.c_longlong, [vp]),
         "gptb200_selftest_wait_timeout": (i, [vp, i]),
+        "gptb200_selftest_grid_barrier": (i, [vp, i]),
         "gptb200_plan_gemm": (i, [i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_plan_decode": (i, [i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_status_string": (ctypes.c_char_p, [i]),

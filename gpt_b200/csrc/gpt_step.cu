@@ -127,3 +127,19 @@ int run_gpt_step(gptb200_ctx *ctx, GptStep s, float *scratch)
 }
 
 }  // namespace gptb200
+
+int gptb200_selftest_grid_barrier(gptb200_ctx *ctx, int polls)
+{
+    using namespace gptb200;
+    if (!ctx || polls <= 0 || polls > 100000) return GPTB200_ERR_INVALID_ARG;
+    const int rc = ensure_workspace(ctx, 64);
+    if (rc) return rc;
+    GptStep s{};
+    s.sync = reinterpret_cast<unsigned *>(ctx->ws);
+    s.status = ctx->d_status;
+    CUDA_TRY(ctx, cudaMemsetAsync(s.sync, 0, 3 * sizeof(unsigned), ctx->stream));
+    step::barrier_selftest_kernel<<<1, 64, 0, ctx->stream>>>(s, static_cast<unsigned>(polls));
+    ctx->launches++;
+    CUDA_TRY(ctx, cudaGetLastError());
+    return GPTB200_OK;
+}

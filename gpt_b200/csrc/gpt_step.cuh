@@ -31,19 +31,45 @@ __device__ __forceinline__ void arrive(const GptStep &s, unsigned &target)
     target += gridDim.x;
 }
 
-__device__ __forceinline__ void await(const GptStep &s, unsigned target)
+// A wait that runs out sets `gave_up` (thread 0's).  The block waits at no later barrier then, and goes on to the end of the step with whatever sums it
+// finds: it writes neither logits nor position, and the keys and values that it writes lie behind the last valid position.  (Leaving at once, by a
+// __syncthreads_or in every barrier, made a step of one sequence 4 us longer and one of 32 14 us.)
+__device__ __forceinline__ void await(const GptStep &s, unsigned target, bool &gave_up, unsigned limit = kPollLimit)
 {
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && !gave_up) {
         unsigned seen = 0, tries = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(s.sync) : "memory");
-            if (++tries == kPollLimit) {
+            if (tries++ == limit) {
+                gave_up = true;
+                atomicExch(s.sync + 2, 1u);
                 atomicCAS(s.status, 0, DEV_TIMEOUT_GRID);
                 break;
             }
         } while (static_cast<int>(seen - target) < 0);
     }
     __syncthreads();
+}
+
+// Whether a barrier of this generation ran out in an earlier launch: the counter is short of arrivals then, and no launch can wait on it until the
+// cache is filled anew.  For thread 0 of a block.
+__device__ __forceinline__ bool lost(const GptStep &s)
+{
+    const bool is = *reinterpret_cast<volatile unsigned *>(s.sync + 2) != 0;
+    if (is) atomicCAS(s.status, 0, DEV_TIMEOUT_GRID);
+    return is;
+}
+
+// Self-test: a barrier that all blocks of a grid of one reach, one that nothing reaches, and what that leaves behind.
+static __global__ void barrier_selftest_kernel(const GptStep s, unsigned limit)
+{
+    unsigned target = 0;
+    bool gave_up = false;
+    arrive(s, target);
+    await(s, target, gave_up, limit);
+    const bool early = gave_up;
+    await(s, target + 1, gave_up, limit);
+    if (threadIdx.x == 0 && (early || !gave_up || !lost(s))) atomicExch(s.status, DEV_TIMEOUT_SELFTEST);
 }
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
@@ -250,6 +276,7 @@ gpt_step_kernel(const GptStep s, int widest)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = s.d;
     const int p = *s.pos;
     if (p < 0 || p >= s.max_len || p >= s.max_pos) return;   // all blocks alike
+    bool gave_up = tid == 0 && lost(s);
     unsigned target = s.sync[1];
     const int first = blockIdx.x;                    // this block's first item of every phase
     const Share of_qkv = share_of(s.qkv, first), of_proj = share_of(s.proj, first), of_up = share_of(s.up, first), of_down = share_of(s.down, first);
@@ -264,7 +291,7 @@ gpt_step_kernel(const GptStep s, int widest)
                                                                                __ldg(reinterpret_cast<const float4 *>(s.wpe + static_cast<size_t>(p) * d + c)))
                                                                         : make_float4(0.f, 0.f, 0.f, 0.f);
     warp_moments<MR>(res + mine * d, d, moments);
-    __syncthreads();
+    if (__syncthreads_or(gave_up)) return;
 
     // res += the finished product, with the moments of the new rows
     auto add_result = [&](const float *part, const StepPhase &ph, const float *bias) {
@@ -344,7 +371,7 @@ gpt_step_kernel(const GptStep s, int widest)
                 v_first[j] = live ? *reinterpret_cast<const float4 *>(row + d) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
-        await(s, target);
+        await(s, target, gave_up);
 
         Share r = mine_of;
 #pragma unroll 1
@@ -470,7 +497,7 @@ gpt_step_kernel(const GptStep s, int widest)
             fetch(wv, half ? s.qkv_w + 3 * dd * next : s.up_w + df * next, half ? s.qkv : s.up, half ? of_qkv : of_up);
             fetch_norm(half ? of_qkv : of_up, (half ? s.ln1_w : s.ln2_w) + next * d, (half ? s.ln1_b : s.ln2_b) + next * d);
         }
-        await(s, target);
+        await(s, target, gave_up);
     }
 
     // final norm; logits: a warp per pair of embedding rows
@@ -482,7 +509,7 @@ gpt_step_kernel(const GptStep s, int widest)
 #pragma unroll
             for (int m = 0; m < MR; ++m) xs[m * widest + k] = (res[m * d + k] - mean[m]) / sd[m] * __ldg(s.lnf_w + k) + __ldg(s.lnf_b + k);
     }
-    __syncthreads();
+    if (__syncthreads_or(gave_up)) return;
 #pragma unroll 1
     for (int n = 2 * (blockIdx.x * kWarps + warp); n < s.vocab_p; n += 2 * kWarps * gridDim.x) {
         const float *wa = s.wte + static_cast<size_t>(n) * d, *wb = n + 1 < s.vocab_p ? wa + d : wa;
@@ -574,6 +601,8 @@ gpt_step_rows_kernel(const GptStep s)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = s.d, batch = s.batch, first = blockIdx.x;
     const int p = *s.pos;
     if (p < 0 || p >= s.max_len || p >= s.max_pos) return;   // all blocks alike
+    __shared__ bool gave_up;   // thread 0's; no register is free for it, nor for leaving here
+    if (tid == 0) gave_up = lost(s);
     unsigned target = s.sync[1];
 
     // Piece i of eight of an item's weights into the other buffer: 16 of its k-rows, one per warp; columns beyond the matrix are zeros.
@@ -915,7 +944,7 @@ gpt_step_rows_kernel(const GptStep s)
             gelu_phase(s.up_b + l * s.ffn);
         }
         arrive(s, target);
-        await(s, target);
+        await(s, target, gave_up);
         if (kind == 0) prefetch_cache(cache);
         const StepPhase ph = kind == 0 ? s.qkv : kind == 1 ? s.proj : kind == 2 ? s.up : s.down, ph_next = kind == 0 ? s.proj : kind == 1 ? s.up : kind == 2 ? s.down : s.qkv;
         const float *w = kind == 0 ? s.qkv_w + 3 * dd * l : kind == 1 ? s.proj_w + dd * l : kind == 2 ? s.up_w + df * l : s.down_w + df * l;
@@ -923,9 +952,9 @@ gpt_step_rows_kernel(const GptStep s)
         product(w, ph, kind == 0 ? s.qkv_part : kind == 1 ? s.proj_part : kind == 2 ? s.up_part : s.down_part, kind == 1 ? s.attn : kind == 3 ? s.up_part : s.normed,
                 w_next, ph_next, kind == 3 && l + 1 == s.layers ? ph_next.groups * ph_next.splits : first);
         arrive(s, target);
-        await(s, target);
+        await(s, target, gave_up);
     }
-    if (blockIdx.x == 0 && tid == 0) {   // every block has passed a barrier since it read them
+    if (blockIdx.x == 0 && tid == 0 && !gave_up) {   // every block has passed a barrier since it read them
         *s.pos = p + 1;
         s.sync[1] = target;
     }

@@ -27,7 +27,7 @@ struct GptStep {
     // scratch: partial sums [split][batch][N]; beyond two rows also residual stream, normed rows and attention output [batch][d]
     float *qkv_part, *proj_part, *up_part, *down_part, *res, *normed, *attn;
     StepPhase qkv, proj, up, down;
-    unsigned *sync;         // arrivals at the grid barriers so far, arrivals before this launch
+    unsigned *sync;         // arrivals at the grid barriers so far, arrivals before this launch, whether a wait for them ran out
     int *status;
 };
 
@@ -37,7 +37,7 @@ constexpr int kStepMaxBatch = 64;
 bool plan_gpt_step(gptb200_ctx *ctx, GptStep &s, size_t *scratch_floats);
 // The context's options still ask for the kernels of few rows.
 bool gpt_step_enabled(const gptb200_ctx *ctx);
-// Launches it; `scratch` as planned, `sync` two words that were zero when the cache was filled.
+// Launches it; `scratch` as planned, `sync` three words that were zero when the cache was filled.
 int run_gpt_step(gptb200_ctx *ctx, GptStep s, float *scratch);
 
 }  // namespace gptb200

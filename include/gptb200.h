@@ -119,6 +119,9 @@ long long gptb200_ctx_tensor_map_encodes(const gptb200_ctx *ctx);
  * barrier that nothing signals.  The wait runs out, the kernel returns normally, and the next gptb200_ctx_synchronize reports
  * GPTB200_ERR_DEVICE_TIMEOUT (and clears the device status); the context stays usable. */
 int gptb200_selftest_wait_timeout(gptb200_ctx *ctx, int limit_us);
+/* The same for the barrier between the blocks of a one-launch generation step (gptb200_model_generate_step): one block waits `polls` times (at most
+ * 100000) at a barrier that nothing reaches, reports device status 110 and returns; 108 if anything went another way. */
+int gptb200_selftest_grid_barrier(gptb200_ctx *ctx, int polls);
 /* The launch plan for D[m x n] = A[m x k] . B[k x n] on a GPU with num_sms SMs, without touching a GPU (host logic only,
  * default options).  plan8 = {kernel (0 none, 1 CTA-pair tcgen05, 2 one-CTA tcgen05, 3 weight streaming, 4 SIMT), tile_n,
  * tiles_m, tiles_n, split_k, k-blocks (or k elements for kernel 3) per split, CTAs, scratch KiB}.  For kernel 1 split_k is the

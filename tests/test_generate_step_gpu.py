@@ -104,3 +104,18 @@ def test_one_launch_is_as_exact_as_the_operators(batch, prompt, steps):
         errors.append(float((out.double() - want).norm() / want.norm()))
         model.close()
     assert errors[0] <= errors[1], errors
+
+
+def test_a_grid_barrier_that_nothing_reaches_ends_and_is_reported():
+    """The wait gives up after its limit, for the whole block and in every later launch; the context stays usable."""
+    import torch
+    import gpt_b200
+    b = gpt_b200.Backend(0)
+    assert b.lib.gptb200_selftest_grid_barrier(b.handle, 0) == 1 and b.lib.gptb200_selftest_grid_barrier(None, 10) == 1
+    for polls in (1, 1000):
+        assert b.lib.gptb200_selftest_grid_barrier(b.handle, polls) == 0
+        with pytest.raises(gpt_b200.GptB200Error) as e:
+            b.synchronize()
+        assert e.value.status == 4 and "device status 110" in str(e.value)
+    b.synchronize()
+    b.close()
