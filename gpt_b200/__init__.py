@@ -26,7 +26,7 @@ MODE_TF32 = 1
 EXPORTED_SYMBOLS = [
     "gptb200_ctx_create", "gptb200_ctx_destroy", "gptb200_ctx_set_mode", "gptb200_ctx_get_mode",
     "gptb200_ctx_set_stream", "gptb200_ctx_set_option", "gptb200_ctx_synchronize", "gptb200_ctx_launch_count", "gptb200_ctx_tensor_map_encodes", "gptb200_ctx_read_trace",
-    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_decode", "gptb200_selftest_wait_timeout", "gptb200_selftest_grid_barrier",
+    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_decode", "gptb200_selftest_wait_timeout", "gptb200_selftest_grid_barrier", "gptb200_plan_generate_step",
     "gptb200_linear_forward", "gptb200_linear_backward", "gptb200_linear_backward_weights", "gptb200_linear_backward_input",
     "gptb200_linear_backward_input_gelu", "gptb200_gemm_batched",
     "gptb200_gelu_backward",
@@ -80,6 +80,7 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         "gptb200_selftest_grid_barrier": (i, [vp, i]),
         "gptb200_plan_gemm": (i, [i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_plan_decode": (i, [i, i, i, i, i, i, ctypes.POINTER(i)]),
+        "gptb200_plan_generate_step": (i, [i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_status_string": (ctypes.c_char_p, [i]),
         "gptb200_last_error": (ctypes.c_char_p, [vp]),
         "gptb200_linear_forward": (i, [vp, fp, fp, fp, fp, fp, i, i, i, i]),
@@ -173,6 +174,20 @@ def plan_decode(num_sms: int, m: int, n: int, k: int, w_kn: bool, has_epilogue: 
     d = dict(zip(["kernel", "rows", "groups", "cluster"], list(out)))
     d["kernel"] = DECODE_KERNELS[d["kernel"]]
     return d
+
+
+STEP_KERNELS = {0: "operators", 1: "few", 2: "rows"}
+
+
+def plan_generate_step(num_sms: int, batch: int, d_model: int, d_ffn: int, heads: int, max_len: int, position: int, replayed: bool = False) -> dict:
+    """How Model.generate_step runs a step (host logic only); see gptb200_plan_generate_step in include/gptb200.h.  Products: (slices of k, k-rows each)."""
+    lib = load_library()
+    out = (ctypes.c_int * 10)()
+    rc = lib.gptb200_plan_generate_step(num_sms, batch, d_model, d_ffn, heads, max_len, position, int(replayed), out)
+    if rc != 0:
+        raise GptB200Error(rc, "gptb200_plan_generate_step")
+    pairs = {name: (out[2 + 2 * i], out[3 + 2 * i]) for i, name in enumerate(["qkv", "proj", "up", "down"])}
+    return dict(kernel=STEP_KERNELS[out[0]], rows=out[1], **pairs)
 
 
 def _ptr(t: Any) -> int | None:

@@ -268,10 +268,10 @@ public:
         const size_t L = c_.layers, D = c_.d_model, F = c_.d_ffn, Vp = c_.vocab_padded;
         if (!set_size(batch, prompt_len)) return GPTB200_ERR_CUDA;
         const size_t cache_floats = L * size_t(batch) * max_len * 2 * D;
-        gptb200::GptStep one = one_launch_step(batch, max_len);
+        gptb200::GptStepForms forms;
         size_t one_floats = 0;
-        const bool one_launch = gptb200::plan_gpt_step(ctx, one, &one_floats);
-        const size_t step_floats = operator_step_floats(batch) + (one_launch ? one_floats : 0) + 8;
+        gptb200::plan_gpt_step(ctx, one_launch_step(batch, max_len), forms, &one_floats);
+        const size_t step_floats = operator_step_floats(batch) + one_floats + 8;
         if (cache_floats + step_floats > gen_capacity_) {
             void *p = nullptr;
             be_->device_malloc(&p, (cache_floats + step_floats) * sizeof(float));
@@ -283,8 +283,7 @@ public:
         gen_batch_ = batch;
         gen_max_len_ = max_len;
         gen_pos_ = prompt_len;
-        gen_step_ = one;
-        gen_one_launch_ = one_launch;
+        gen_forms_ = forms;
         forward(prompt);
         const size_t M = size_t(batch) * prompt_len;
         // layers follow one another in the cache and in the activations as sequences do: as many per launch as a grid has room for
@@ -332,8 +331,9 @@ public:
         (void)x2;
         int *pos_dev = reinterpret_cast<int *>(gen_ + gen_pos_off_);
         float *w = weights();
-        if (gen_one_launch_ && gptb200::gpt_step_enabled(ctx)) {
-            gptb200::GptStep one = gen_step_;
+        const gptb200::GptStep *form = gptb200::gpt_step_enabled(ctx) ? gptb200::gpt_step_form(gen_forms_, gen_pos_, gptb200::gpt_step_replayed(ctx)) : nullptr;
+        if (form) {
+            gptb200::GptStep one = *form;
             one.wte = w + lay_.wte; one.wpe = w + lay_.wpe;
             one.ln1_w = w + lay_.ln1_w; one.ln1_b = w + lay_.ln1_b; one.qkv_w = w + lay_.qkv_w; one.qkv_b = w + lay_.qkv_b;
             one.proj_w = w + lay_.proj_w; one.proj_b = w + lay_.proj_b; one.ln2_w = w + lay_.ln2_w; one.ln2_b = w + lay_.ln2_b;
@@ -481,8 +481,7 @@ private:
     bool fused_ce_ = false, fused_ce_active_ = false, row_loss_valid_ = false;
     bool fused_gelu_ = false;
     float *gen_ = nullptr;        // KV cache of every layer, then the step's activations, then the device copy of the position
-    gptb200::GptStep gen_step_{};   // the one-launch step as planned for the cache
-    bool gen_one_launch_ = false;
+    gptb200::GptStepForms gen_forms_{};   // the one-launch steps as planned for the cache
     size_t gen_capacity_ = 0, gen_pos_off_ = 0;
     int gen_batch_ = 0, gen_max_len_ = 0, gen_pos_ = 0;
 };

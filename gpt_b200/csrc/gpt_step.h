@@ -33,8 +33,18 @@ struct GptStep {
 
 constexpr int kStepMaxBatch = 64;
 
-// Whether the step of this model and batch runs as one launch, with its phases and scratch (floats) filled in.
-bool plan_gpt_step(gptb200_ctx *ctx, GptStep &s, size_t *scratch_floats);
+// A step in both its forms, as far as they fit the model and batch: the kernel of one or two rows, and that of up to 64.
+struct GptStepForms {
+    GptStep few, many;
+    bool few_fits, many_fits;
+};
+
+// Plans the forms of a model and batch (whose sizes `shape` holds), and the scratch (floats) that either needs; false: neither fits.
+bool plan_gpt_step(gptb200_ctx *ctx, const GptStep &shape, GptStepForms &forms, size_t *scratch_floats);
+// The faster one at a position of the text, or over the positions that a captured step is replayed at; null: operator by operator.
+const GptStep *gpt_step_form(const GptStepForms &forms, int position, bool replayed);
+// Whether the context's stream is being captured into a graph.
+bool gpt_step_replayed(const gptb200_ctx *ctx);
 // The context's options still ask for the kernels of few rows.
 bool gpt_step_enabled(const gptb200_ctx *ctx);
 // Launches it; `scratch` as planned, `sync` three words that were zero when the cache was filled.

@@ -133,6 +133,12 @@ int gptb200_plan_gemm(int num_sms, int m, int n, int k, int a_mn_major, int b_mn
  * grad_x).  plan4 = {kernel (0 k-split with scratch, 1 per-warp cluster kernel, 2 register-tiled cluster kernel, 3 warp per
  * weight-row pair), rows of x per CTA, row groups, CTAs per cluster}; clusters of 16 are assumed to be schedulable. */
 int gptb200_plan_decode(int num_sms, int m, int n, int k, int w_kn_major, int has_epilogue, int *plan4);
+/* How gptb200_model_generate_step runs a step at a position, called or (replayed != 0) captured into a CUDA graph, with default options (host logic
+ * only).  plan10 = {0 operator by operator, 1 one launch of
+ * the kernel of one or two rows, 2 one launch of the kernel of padded rows and the un-embedding; its padded rows; slices of k and k-rows per slice of
+ * the qkv, attention output, up and down products}. */
+int gptb200_plan_generate_step(int num_sms, int batch, int d_model, int d_ffn, int heads, int max_len, int position, int replayed,
+                               int *plan10);
 const char *gptb200_status_string(int status);
 const char *gptb200_last_error(const gptb200_ctx *ctx);
 

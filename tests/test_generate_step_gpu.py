@@ -38,7 +38,9 @@ SIZES = {
     "gpt2": GPT2,
     "head8": dict(d_model=64, num_heads=8, d_ffn=308, vocab_size_padded=332),           # ragged column groups and slices
     "head128": dict(d_model=384, num_heads=3, d_ffn=1284, vocab_size_padded=64),
-    "wide": dict(d_model=1600, num_heads=25, d_ffn=6400, vocab_size_padded=260),         # several items per block
+    "wide": dict(d_model=1600, num_heads=25, d_ffn=6400, vocab_size_padded=260),         # up to three items per block, five heads per slice
+    "medium": dict(d_model=1024, num_heads=16, d_ffn=4096, vocab_size_padded=516),       # two heads per slice, slices of more than 256 rows
+    "large": dict(d_model=1280, num_heads=20, d_ffn=5120, vocab_size_padded=516),        # two items per block, three heads per slice
 }
 
 
@@ -119,3 +121,69 @@ def test_a_grid_barrier_that_nothing_reaches_ends_and_is_reported():
         assert e.value.status == 4 and "device status 110" in str(e.value)
     b.synchronize()
     b.close()
+
+
+def _generated(torch, c, batch, text, prompt, prepare=lambda model: None, between=lambda model, i: None, graph=False):
+    """(logits of the steps, launches of each) of a text in a new model, and the float64 logits."""
+    import gpt_b200
+    steps = text.shape[1] - prompt
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    flat = torch.cat([(torch.randn(*shape, device="cuda", generator=gen) * 0.05 + (1.0 if name in ("ln1_w", "ln2_w", "lnf_w") else 0.0)).reshape(-1) for name, shape in _shapes(c)])
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        model = gpt_b200.Model(c, 0, stream.cuda_stream, gpt_b200.MODE_3XTF32, use_grad=False)
+        model.load_weights(flat.cpu().numpy())
+        prepare(model)
+        model.generate_begin(text[:, :prompt].contiguous(), batch, prompt, prompt + steps)
+        out, launches = torch.full((steps, batch, c["vocab_size_padded"]), float("nan"), device="cuda"), []
+        token, logits, captured = torch.empty(batch, device="cuda", dtype=torch.int32), torch.empty(batch, c["vocab_size_padded"], device="cuda"), None
+        for i in range(steps):
+            between(model, i)
+            token.copy_(text[:, prompt + i])
+            before = model.launch_count()
+            if captured:
+                captured.replay()
+            else:
+                model.generate_step(token, logits)
+                if graph and i == 0:     # the steps after the first are replays of the second's capture
+                    captured = torch.cuda.CUDAGraph()
+                    before = model.launch_count()
+                    with torch.cuda.graph(captured, stream=stream):
+                        model.generate_step(token, logits)
+            launches.append(model.launch_count() - before)
+            out[i].copy_(logits)
+        stream.synchronize()
+        model.synchronize()
+        del captured
+        model.close()
+    return out.transpose(0, 1).double(), launches, _forward(torch, c, flat.double(), text)[:, prompt:]
+
+
+def _case(torch, size, batch, layers, prompt, steps):
+    c = dict(max_seq_len=prompt + steps + 1, num_layers=layers, **SIZES[size])
+    c["vocab_size"] = c["vocab_size_padded"] - 3
+    return c, torch.randint(0, c["vocab_size"], (batch, prompt + steps), device="cuda", dtype=torch.int32, generator=torch.Generator(device="cuda").manual_seed(batch + prompt))
+
+
+FEW, ROWS = 1, 2     # launches of a step: the kernel of one or two rows; the other with the un-embedding
+
+
+@pytest.mark.parametrize("size,batch,prompt,steps,kernel", [
+    ("medium", 1, 70, 3, FEW), ("medium", 2, 130, 3, FEW), ("large", 1, 33, 3, FEW), ("large", 2, 150, 2, FEW), ("wide", 1, 60, 3, FEW),
+    ("medium", 2, 401, 2, ROWS), ("large", 2, 256, 2, ROWS), ("medium", 12, 9, 3, ROWS), ("large", 64, 5, 2, ROWS)])
+def test_widths_beyond_768(size, batch, prompt, steps, kernel):
+    """Several items per block, several heads per slice, slices of more than one body of weights: 1e-5 of the logits' scale, as above."""
+    import torch
+    c, text = _case(torch, size, batch, 2, prompt, steps)
+    got, launches, want = _generated(torch, c, batch, text, prompt)
+    assert launches == [kernel] * steps
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+def test_the_kernel_changes_with_the_position():
+    """From the kernel of one or two rows to the operators and on to the other kernel, over one cache."""
+    import torch
+    c, text = _case(torch, "large", 2, 1, 198, 61)
+    got, launches, want = _generated(torch, c, 2, text, 198)
+    assert launches[:3] == [FEW] * 3 and all(n > ROWS for n in launches[3:58]) and launches[58:] == [ROWS] * 3
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())

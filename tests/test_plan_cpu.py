@@ -153,3 +153,39 @@ def test_decode_kernel_choice_for_gpt2_124m():
             assert k // p["cluster"] >= 32 or p["cluster"] == 1
         if p["kernel"] == "rowwise":
             assert p["rows"] * k <= 12288
+
+
+def test_generation_step_plans(built_library):
+    """Which kernel runs a generation step.  Blocks take few rounds of items (a partial sum per slice is read back), the kernel of one or two rows ends
+    where its repeated attention costs more than the other kernel's padding, and sizes that no kernel takes go operator by operator."""
+    from gpt_b200 import plan_generate_step as step
+
+    def of(batch, d, heads, position, max_len=1024, replayed=False):
+        return step(SMS, batch, d, 4 * d, heads, max_len, position, replayed)["kernel"]
+    # GPT-2's widths: one round of items for 768 and 1024, at most three beyond
+    small = step(SMS, 1, 768, 3072, 12, 256, 64)
+    assert small == dict(kernel="few", rows=0, qkv=(4, 192), proj=(12, 64), up=(3, 256), down=(12, 256))
+    for d, heads, most in ((768, 12, 1), (1024, 16, 1), (1280, 20, 2), (1600, 25, 3)):
+        p = step(SMS, 1, d, 4 * d, heads, 256, 64)
+        assert p["kernel"] == "few"
+        for name, k, n in (("qkv", d, 3 * d), ("proj", d, d), ("up", d, 4 * d), ("down", 4 * d, d)):
+            splits, rows = p[name]
+            assert (splits - 1) * rows < k <= splits * rows and -(-(-(-n // 64) * splits) // SMS) <= most, (d, name)
+        assert p["proj"][1] % (d // heads) == 0
+    # both sides of each line
+    assert all(of(b, 768, 12, p) == "few" for b in (1, 2) for p in (1, 1000))
+    assert of(2, 1024, 16, 400) == "few" and of(2, 1024, 16, 401) == "rows"
+    assert of(2, 1280, 20, 200) == "few" and of(2, 1280, 20, 201) == "operators" and of(2, 1280, 20, 256) == "rows"
+    assert of(1, 1600, 25, 533) == "few" and of(1, 1600, 25, 534) == "rows"
+    assert of(2, 1600, 25, 5) == "operators" and of(2, 1600, 25, 319) == "operators" and of(2, 1600, 25, 320) == "rows"
+    assert of(3, 1024, 16, 79) == "operators" and of(4, 1024, 16, 80) == "rows" and of(5, 1024, 16, 5) == "rows" and of(3, 768, 12, 5) == "rows"
+    assert of(3, 768, 12, 64, 255, True) == "operators" and of(3, 768, 12, 64, 256, True) == "rows" and of(5, 768, 12, 64, 255, True) == "rows"
+    assert of(4, 512, 8, 256, 446, True) == "operators" and of(4, 512, 8, 256, 448, True) == "rows"
+    for batch, line in ((1, 640), (2, 640), (4, 480), (8, 256)):
+        assert of(batch, 2048, 32, line - 1) == "operators" and of(batch, 2048, 32, line) == "rows"
+    assert of(9, 2048, 32, 5) == "rows"
+    assert step(SMS, 17, 768, 3072, 12, 256, 64)["rows"] == 32 and step(SMS, 64, 768, 3072, 12, 256, 64)["rows"] == 64
+    # sizes that neither takes: more rows, other head sizes, odd widths, offsets within a layer's matrix beyond an int, scores beyond shared memory
+    for args in ((65, 768, 3072, 12, 256), (1, 768, 3072, 8, 256), (1, 768, 3072, 768 // 4, 256), (1, 770, 3072, 77, 256), (1, 768, 3070, 12, 256),
+                 (1, 4096, 2 ** 19, 32, 256), (64, 16384, 2 ** 17, 128, 256), (1, 768, 3072, 12, 200000), (0, 768, 3072, 12, 256)):
+        assert step(SMS, *args, 10)["kernel"] == "operators", args
