@@ -187,3 +187,38 @@ def test_the_kernel_changes_with_the_position():
     got, launches, want = _generated(torch, c, 2, text, 198)
     assert launches[:3] == [FEW] * 3 and all(n > ROWS for n in launches[3:58]) and launches[58:] == [ROWS] * 3
     assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("size,batch,prompt,steps,kernel", [("gpt2", 1, 20, 8, FEW), ("medium", 2, 20, 5, FEW), ("gpt2", 8, 20, 6, ROWS), ("gpt2", 64, 3, 5, ROWS), ("gpt2", 3, 20, 6, 0)])
+def test_a_captured_step_is_replayed_at_every_position(size, batch, prompt, steps, kernel):
+    """The position and the barriers' counters live on the device: one capture serves all steps after the first.  Three rows over a short cache are
+    captured operator by operator."""
+    import torch
+    c, text = _case(torch, size, batch, 2, prompt, steps)
+    got, launches, want = _generated(torch, c, batch, text, prompt, graph=True)
+    assert (launches[0] == kernel or (kernel == 0 and launches[0] > ROWS)) and launches[1:] == [0] * (steps - 1)
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("size,batch,sms,kernel", [("gpt2", 1, 100, FEW), ("head128", 2, 89, FEW), ("gpt2", 20, 90, ROWS), ("gpt2", 1, 60, 0), ("gpt2", 9, 16, 0)])
+def test_steps_on_part_of_the_sms(size, batch, sms, kernel):
+    """Option max_sms: more items per block on fewer blocks, operators where too few are left."""
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines are drawn for 148 SMs")
+    c, text = _case(torch, size, batch, 2, 11, 4)
+    got, launches, want = _generated(torch, c, batch, text, 11, prepare=lambda model: model.set_option("max_sms", sms))
+    assert launches == [kernel] * 4 if kernel else min(launches) > ROWS
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("batch", [1, 8])
+def test_the_form_may_change_between_steps(batch):
+    """Options are read at every step: one launch, operators, one launch over the same cache, and fewer SMs than planned for."""
+    import torch
+    c, text = _case(torch, "gpt2", batch, 2, 15, 7)
+    changes = {2: ("skinny", 0), 4: ("skinny", 1), 5: ("max_sms", 120)}
+    got, launches, want = _generated(torch, c, batch, text, 15, between=lambda model, i: i in changes and model.set_option(*changes[i]))
+    one = FEW if batch <= 2 else ROWS
+    assert launches[:2] == [one] * 2 and min(launches[2:4]) > ROWS and launches[4:] == [one] * 3
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
