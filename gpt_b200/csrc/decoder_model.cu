@@ -817,9 +817,9 @@ private:
     // threads per row of the stream: with few rows a row is spread wider
     int row_threads(int rows) const { return std::min(rows <= 2 * ctx_->num_sms ? 1024 : 256, std::max(32, pad_to(pitch_ / 4, 32))); }
 
-    // The row kernels of decoder_step_rows.cuh: steps of one token per sequence with no more rows than run at once.  The fp32 products let
+    // The row kernels of decoder_step_rows.cuh (bf16): steps of one token per sequence with no more rows than run at once.  The fp32 products let
     // their successor start before their own wait, so what the row kernels read early would not be complete.
-    bool single_rows(int rows) const { return !kF32 && single_tokens_ && rows <= ctx_->num_sms && pitch_ <= 4096; }
+    bool single_rows(int rows) const { return single_tokens_ && rows <= ctx_->num_sms && pitch_ <= 4096; }
 
     int sublayer_end(int rows, float *x, const Norm &after, const Norm &before)
     {
@@ -828,7 +828,9 @@ private:
             return launch(kernel, dim3(rows), dim3(threads), smem, x, static_cast<const float *>(y_), static_cast<const float *>(after.w), static_cast<const float *>(after.b),
                           static_cast<const float *>(before.w), static_cast<const float *>(before.b), h_, c_.width, pitch_, eps);
         };
-        return single_rows(rows) ? run(&sublayer_end_row_kernel<T>, pad_to(pitch_ / 4, 32), 0) : run(&sublayer_end_kernel<T>, row_threads(rows), size_t(pitch_) * sizeof(float));
+        if constexpr (!kF32)
+            if (single_rows(rows)) return run(&sublayer_end_row_kernel<T>, pad_to(pitch_ / 4, 32), 0);
+        return run(&sublayer_end_kernel<T>, row_threads(rows), size_t(pitch_) * sizeof(float));
     }
 
     int layer_begin(int rows, int layer, const T *h, const int *row_list)
@@ -856,7 +858,8 @@ private:
         }
         b.h = const_cast<T *>(h);
         b.entries = entries_; b.row_entry = row_entry_; b.row_list = row_list;
-        if (b.side_y && single_rows(rows)) return launch(layer_begin_row_kernel<T>, dim3(rows), dim3(pad_to(pitch_ / 4, 32)), 0, b);
+        if constexpr (!kF32)
+            if (b.side_y && single_rows(rows)) return launch(layer_begin_row_kernel<T>, dim3(rows), dim3(pad_to(pitch_ / 4, 32)), 0, b);
         b.tile = rows <= 512 || !b.shift ? 1 : rows <= 2048 ? 4 : 8;
         return launch(layer_begin_kernel<T>, dim3((rows + b.tile - 1) / b.tile), dim3(row_threads(rows)), 2 * size_t(pitch_) * sizeof(float), b);
     }
@@ -929,6 +932,7 @@ private:
             const int blocks = s.heads * ((s.vdim + kChunkCols - 1) / kChunkCols);
             // of the option's tokens, or shorter where the heads and requests of a step leave blocks of the machine (two per SM) idle: a chunk after the
             // other takes 5 us, the pass for the states in front of the segments half of what it saves (three prompts of 870 tokens, 12 heads of 64)
+            constexpr int kShortestSegment = 256;
             int segment = segment_tokens_;
             if (segment_auto_) {
                 const int side_by_side = std::max(1, 2 * ctx_->num_sms / (blocks * n));
@@ -1383,7 +1387,8 @@ private:
         }
         b.h = h;
         b.entries = entries_; b.row_entry = row_entry_; b.row_list = row_list;
-        if (y && single_rows(rows)) return launch(residual_norm_row_kernel<T>, dim3(rows), dim3(pad_to(pitch_ / 4, 32)), 0, b);
+        if constexpr (!kF32)
+            if (y && single_rows(rows)) return launch(residual_norm_row_kernel<T>, dim3(rows), dim3(pad_to(pitch_ / 4, 32)), 0, b);
         b.tile = rows <= 512 || !b.mixes ? 1 : rows <= 2048 ? 4 : 8;
         return launch(residual_norm_kernel<T>, dim3((rows + b.tile - 1) / b.tile), dim3(row_threads(rows)), 2 * size_t(pitch_) * sizeof(float), b);
     }
@@ -1473,7 +1478,6 @@ private:
     std::vector<Slot> slots_;
     int pass_rows_ = 4096, expand_rows_ = 32, chunk_rows_ = 8, segment_tokens_ = 1024, wkv_segment_tokens_ = 0;
     bool segment_auto_ = true;   // segment_tokens_ was not set: shorter segments where they fill the machine
-    static constexpr int kShortestSegment = 256;
     T *expanded_ = nullptr;
     size_t expanded_count_ = 0;
     float *scratch_ = nullptr;

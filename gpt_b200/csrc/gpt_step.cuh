@@ -169,7 +169,7 @@ __device__ __forceinline__ void fetch(float4 (&wv)[kBody], const float *w, const
 
 // part[split][m][col ..] = xs[m][.] . w over the item's slice.  wv holds the first weights; red: [kWarps][MR][kCols].
 template <int MR>
-__device__ __forceinline__ void item_product(float4 (&wv)[kBody], const float *w, const StepPhase &ph, const Share &r, const float *xs, int pitch, float *red, float *part, int batch)
+__device__ __forceinline__ void item_product(float4 (&wv)[kBody], const float *w, const StepPhase &ph, const Share &r, const float *xs, int pitch, float *red, float *part)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float *x = xs + (threadIdx.x >> 4);
@@ -202,7 +202,7 @@ __device__ __forceinline__ void item_product(float4 (&wv)[kBody], const float *w
         float v[kWarps];
 #pragma unroll
         for (int i = 0; i < kWarps; ++i) v[i] = red[i * MR * kCols + threadIdx.x];
-        if (col < ph.N) part[(r.split * batch + m) * ph.N + col] = pairwise(v);
+        if (col < ph.N) part[(r.split * MR + m) * ph.N + col] = pairwise(v);
     }
 }
 
@@ -261,6 +261,7 @@ inline size_t small_shared_floats(int mr, int d, int hd, int max_len, int widest
     return size_t(mr) * d + size_t(mr) * widest + size_t(kWarps) * mr * kCols + size_t(mr) * 3 * hd + size_t(kWarps) * (hd + 4) + size_t(mr) * max_len;
 }
 
+// MR: the sequences.
 template <int MR>
 __global__ void __launch_bounds__(kThreads, 1)
 gpt_step_kernel(const GptStep s, int widest)
@@ -287,21 +288,19 @@ gpt_step_kernel(const GptStep s, int widest)
     const int mine = tid / kPer, at4 = (tid % kPer) * 4;
 #pragma unroll 1
     for (int c = at4; c < d; c += kPer * 4)
-        *reinterpret_cast<float4 *>(res + mine * d + c) = mine < s.batch ? add4(__ldg(reinterpret_cast<const float4 *>(s.wte + static_cast<size_t>(s.tokens[mine]) * d + c)),
-                                                                               __ldg(reinterpret_cast<const float4 *>(s.wpe + static_cast<size_t>(p) * d + c)))
-                                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4 *>(res + mine * d + c) = add4(__ldg(reinterpret_cast<const float4 *>(s.wte + static_cast<size_t>(s.tokens[mine]) * d + c)),
+                                                               __ldg(reinterpret_cast<const float4 *>(s.wpe + static_cast<size_t>(p) * d + c)));
     warp_moments<MR>(res + mine * d, d, moments);
     if (__syncthreads_or(gave_up)) return;
 
     // res += the finished product, with the moments of the new rows
     auto add_result = [&](const float *part, const StepPhase &ph, const float *bias) {
-        if (mine < s.batch)
 #pragma unroll 1
-            for (int c = at4; c < d; c += kPer * 4) {
-                const float4 be = __ldg(reinterpret_cast<const float4 *>(bias + c));
-                const float4 v = add4(sum_parts4(part + mine * d + c, ph.splits, s.batch * d), be);
-                *reinterpret_cast<float4 *>(res + mine * d + c) = add4(*reinterpret_cast<const float4 *>(res + mine * d + c), v);
-            }
+        for (int c = at4; c < d; c += kPer * 4) {
+            const float4 be = __ldg(reinterpret_cast<const float4 *>(bias + c));
+            const float4 v = add4(sum_parts4(part + mine * d + c, ph.splits, MR * d), be);
+            *reinterpret_cast<float4 *>(res + mine * d + c) = add4(*reinterpret_cast<const float4 *>(res + mine * d + c), v);
+        }
         warp_moments<MR>(res + mine * d, d, moments);
         __syncthreads();
     };
@@ -335,7 +334,7 @@ gpt_step_kernel(const GptStep s, int widest)
                 }
             }
             __syncthreads();
-            item_product<MR>(wv, w, ph, r, xs, widest, red, part, s.batch);
+            item_product<MR>(wv, w, ph, r, xs, widest, red, part);
         }
     };
 
@@ -359,7 +358,7 @@ gpt_step_kernel(const GptStep s, int widest)
         const StepPhase ph = half ? s.down : s.proj;
         const Share mine_of = half ? of_down : of_proj;
         fetch(wv, w, ph, mine_of);
-        float *cache = s.cache + static_cast<size_t>(l) * s.batch * s.max_len * 2 * d;
+        float *cache = s.cache + static_cast<size_t>(l) * MR * s.max_len * 2 * d;
         // and the first cached rows of this block's first head
         float4 k_first[4], v_first[4];
         {
@@ -387,7 +386,7 @@ gpt_step_kernel(const GptStep s, int widest)
 #pragma unroll 1
                     for (int k = tid; k < r.rows; k += kThreads) {
                         const float be = __ldg(s.up_b + l * s.ffn + r.k0 + k);
-                        xs[m * widest + k] = m < s.batch ? gelu_tanh(sum_parts(s.up_part + m * s.ffn + r.k0 + k, s.up.splits, s.batch * s.ffn) + be) : 0.0f;
+                        xs[m * widest + k] = gelu_tanh(sum_parts(s.up_part + m * s.ffn + r.k0 + k, s.up.splits, MR * s.ffn) + be);
                     }
             }
             // or the attention of the heads in the item's slice of k
@@ -396,16 +395,16 @@ gpt_step_kernel(const GptStep s, int widest)
                 const bool fetched = item == first && at == 0;   // k_first, v_first are this head's, row 0
                 if (!fetched) __syncthreads();
 #pragma unroll 1
-                for (int i = tid; i < s.batch * 3 * s.hd; i += kThreads) {
+                for (int i = tid; i < MR * 3 * s.hd; i += kThreads) {
                     const int row = i >> head_log, m = MR == 1 ? 0 : row / 3, which = row - 3 * m, e = i & (s.hd - 1), col = which * d + r.k0 + at + e;
                     const float be = __ldg(s.qkv_b + l * 3 * d + col);
-                    const float v = sum_parts(s.qkv_part + m * 3 * d + col, s.qkv.splits, s.batch * 3 * d) + be;
+                    const float v = sum_parts(s.qkv_part + m * 3 * d + col, s.qkv.splits, MR * 3 * d) + be;
                     fresh[i] = v;
                     if (which > 0 && r.col == 0) cache[(static_cast<size_t>(m) * s.max_len + p) * 2 * d + (col - d)] = v;
                 }
                 __syncthreads();
 #pragma unroll 1
-                for (int m = 0; m < s.batch; ++m) {
+                for (int m = 0; m < MR; ++m) {
                     const float *q = fresh + m * 3 * s.hd + c4, *row = cache + (static_cast<size_t>(m) * s.max_len + g) * 2 * d + r.k0 + at + c4;
                     const float4 q4 = *reinterpret_cast<const float4 *>(q);
                     float *probs = prob + m * s.max_len;
@@ -433,7 +432,7 @@ gpt_step_kernel(const GptStep s, int widest)
                 }
                 __syncthreads();
 #pragma unroll 1
-                for (int m = 0; m < s.batch; ++m) {
+                for (int m = 0; m < MR; ++m) {
                     const float *q = fresh + m * 3 * s.hd + c4, *row = cache + (static_cast<size_t>(m) * s.max_len + g) * 2 * d + d + r.k0 + at + c4;
                     float *probs = prob + m * s.max_len;
                     float mx = -FLT_MAX, weights = 0.0f;
@@ -485,11 +484,8 @@ gpt_step_kernel(const GptStep s, int widest)
                     }
                 }
             }
-            if (MR > 1 && s.batch < MR && !half)
-#pragma unroll 1
-                for (int i = tid; i < r.rows; i += kThreads) xs[widest + i] = 0.0f;
             __syncthreads();
-            item_product<MR>(wv, w, ph, r, xs, widest, red, half ? s.down_part : s.proj_part, s.batch);
+            item_product<MR>(wv, w, ph, r, xs, widest, red, half ? s.down_part : s.proj_part);
         }
         arrive(s, target);
         if (n + 1 < 2 * s.layers) {
@@ -541,7 +537,7 @@ gpt_step_kernel(const GptStep s, int widest)
                 sa[m] += __shfl_xor_sync(0xffffffffu, sa[m], o);
                 sb[m] += __shfl_xor_sync(0xffffffffu, sb[m], o);
             }
-            if (lane == 0 && m < s.batch) {
+            if (lane == 0) {
                 s.logits[static_cast<size_t>(m) * s.vocab_p + n] = sa[m];
                 if (n + 1 < s.vocab_p) s.logits[static_cast<size_t>(m) * s.vocab_p + n + 1] = sb[m];
             }
