@@ -178,12 +178,14 @@ gemv_bf16_kernel(const GemvParams p)
 }
 
 // Two to eight rows: the same stream of weights as the A operand of m16n8k16 products (16 weight rows, up to eight rows of x).  A
-// block takes 16 weight rows (GATED: 16 gate rows and their 16 up rows) and its eight warps share k, so no value of x is read
+// block takes TILES x 16 weight rows (gated kinds: 16 gate rows and their 16 up rows) and its eight warps share k, so no value of x is read
 // twice by a block and x comes straight from L2.  The order of k inside a block
 // of 32 is permuted alike on both sides so that a lane loads 16 contiguous bytes of a row: piece c of a block (8 values) feeds
 // two products, values 0-3 the first and 4-7 the second.  While a warp multiplies, its next blocks' weights are on their way.
 // Layers with few weight rows: the CTAs of a cluster (blockIdx.z) share a tile's k, so that all SMs have loads in flight; their sums meet
 // in the first CTA's shared memory in rank order.  Eight rows of the 2048-wide models, the products of a step: 415 -> 395 us for 1.8 GB.
+// (TILES = 2 is for the gated kinds, 1 for the others.  With the kind known at compile time the gated form needs 12 registers less and a step of eight
+// sequences of the 2048-wide linear-attention model took 2 % longer.)
 constexpr int kGemvMmaUnroll = 4;   // blocks of 32 k and tiles per buffer of weights and warp: two buffers of 32 registers leave two CTAs per SM
 constexpr int kGemvMaxCluster = 4;
 
@@ -194,12 +196,12 @@ __device__ __forceinline__ void gemv_mma_bf16(float (&d)[4], uint32_t a0, uint32
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <bool GATED>
+template <int TILES>
 __global__ void __launch_bounds__(kGemvThreads)
 gemv_bf16_mma_kernel(const GemvParams p)
 {
     namespace cg = cooperative_groups;
-    constexpr int TILES = GATED ? 2 : 1, kSums = TILES * 16 * 8, kUnroll = kGemvMmaUnroll / TILES;
+    constexpr int kSums = TILES * 16 * 8, kUnroll = kGemvMmaUnroll / TILES;
     __shared__ float sums[8 * kSums];                 // [warp][weight row][row of x]
     __shared__ float from_others[(kGemvMaxCluster - 1) * kSums];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -211,7 +213,7 @@ gemv_bf16_mma_kernel(const GemvParams p)
     int row[TILES];
 #pragma unroll
     for (int t = 0; t < TILES; ++t)
-        row[t] = GATED ? (blockIdx.x >> 1) * 64 + (blockIdx.x & 1) * 16 + t * 32 : blockIdx.x * 16;
+        row[t] = is_glu(p.out_kind) ? (blockIdx.x >> 1) * 64 + (blockIdx.x & 1) * 16 + t * 32 : (blockIdx.x * TILES + t) * 16;
     const int blocks = (p.K + 31) / 32, per_warp = (blocks + 8 * S - 1) / (8 * S);
     const int first = min(blocks, (rank * 8 + warp) * per_warp), end = min(blocks, first + per_warp);
     uint4 wv[2][kUnroll][TILES][2];
@@ -280,7 +282,8 @@ gemv_bf16_mma_kernel(const GemvParams p)
         cluster.sync();   // nothing remote is touched after this
         if (rank > 0) return;
     }
-    for (int i = threadIdx.x; i < 128; i += kGemvThreads) {
+    const int outputs = is_glu(p.out_kind) ? 128 : kSums;
+    for (int i = threadIdx.x; i < outputs; i += kGemvThreads) {
         const int r = i >> 3, m = i & 7;
         if (m >= p.M) continue;
         auto total = [&](int at) {
@@ -290,8 +293,8 @@ gemv_bf16_mma_kernel(const GemvParams p)
             for (int q = 1; q < S; ++q) v += from_others[(q - 1) * kSums + at];
             return v;
         };
-        const float v = total(i), up = GATED ? total(128 + i) : 0.0f;
-        const int n = row[0] + r;
+        const float v = total(i), up = TILES == 2 && is_glu(p.out_kind) ? total(128 + i) : 0.0f;
+        const int n = is_glu(p.out_kind) ? row[0] + r : blockIdx.x * TILES * 16 + r;
         if (n < N) gemv_emit(p, m, n0 + n, v, up);
     }
 }
