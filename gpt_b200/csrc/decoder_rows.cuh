@@ -518,7 +518,7 @@ __global__ void sample_rows_kernel(int *__restrict__ tokens, const float *__rest
 
 // The same inside a generation step: the token goes to the next step's input and to history [step][sequence], and the sequence's
 // entry moves on by one position.  The step waits for it, and one block alone is bound by the latency of its loads: a cluster
-// shares a row (blockIdx.y), its blocks' bests meet in the first one's shared memory.  50304 logits, inside a step: 30 us by one block, 7 by
+// shares a row (blockIdx.y), its blocks' bests meet in the first one's shared memory.  50304 logits, inside a step, from the predecessor's end: 30 us by one block, 4.4 by
 // a cluster of eight (a step of a 768-wide model of 12 layers 505 -> 482 us).
 constexpr int kSampleCluster = 8, kSampleThreads = 512;
 

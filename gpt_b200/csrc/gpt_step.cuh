@@ -131,8 +131,8 @@ __device__ __forceinline__ float sum_parts(const float *p, int splits, int strid
 // in every phase.  Every block keeps the whole residual stream in shared memory and norms it itself (bitwise the same everywhere), and the
 // blocks of one head compute its attention once each: four barriers per layer instead of seven.  A phase lasts one to two
 // microseconds, so what 16 warps issue counts as much as what they wait for: addresses are worked out once per launch (Share), and
-// warps without data skip (with both left out a step of GPT-2 124M took 270 us).  One row at position 64 - 96: 236 us per step, against 445 us as
-// 89 launches (a prompt of 64 tokens and 32 steps: 8.9 - 9.0 ms, was 15.7 - 16.2).  What is left is the length of the chain: at a barrier 1.1 us
+// warps without data skip (with both left out a step of GPT-2 124M took 270 us).  One row at position 64 - 96: 223 us per step, against 435 us as
+// 89 launches (a prompt of 64 tokens and 32 steps: 8.6 ms, was 15.7 - 16.2).  What is left is the length of the chain: at a barrier 1.1 us
 // between the last arrival and the first use of its data, then up to 1.5 us for 148 blocks that read the same 36 KB of partial sums.
 // Tried: the next phase's weights towards L2 while a phase computes (0.15 ms slower: their traffic delays the partial sums); clusters of two blocks that
 // each read half of the partial sums (no faster).
@@ -558,7 +558,7 @@ gpt_step_kernel(const GptStep s, int widest)
 // take them (3000 cycles), and as bulk copies one warp needs 6000 cycles to issue 128 rows.  The norms, the attention and the GELU are
 // phases of their own: eight barriers per layer.  Every kind of phase is in the code once: inlined per use the kernel had 184 KB of code, more than
 // the instruction caches hold, and its norms and staging took twice as long.
-// 64 rows at position 64 - 96: 775 us per step and 136 for the un-embedding, against 1450 as 89 launches.  An item of 128 x 128 takes 3400 cycles to stage,
+// 64 rows at position 64 - 96: 777 us per step and 143 for the un-embedding, against 1450 as 89 launches (of 128 registers, with 132 bytes spilled).  An item of 128 x 128 takes 3400 cycles to stage,
 // 12000 to multiply and 2800 to add up and store; a barrier 2400, the attention of 768 heads 24000.
 constexpr int kWideCols = 128, kWideSlice = 128;
 

@@ -8,8 +8,8 @@ struct gptb200_ctx;
 
 namespace gptb200 {
 
-// A product of the step: output columns in groups of 64, k in `splits` slices of `slice` rows.  The slices' sums meet in the
-// prologue of the next phase, in slice order.
+// A product of the step: `groups` of output columns (64 wide in the kernel of one or two rows, 128 in the other) x `splits` slices of k of `slice`
+// rows.  The slices' sums meet, neighbours first, where the next phase reads them.
 struct StepPhase {
     int K, N, groups, splits, slice;
 };

@@ -84,8 +84,8 @@ int gptb200_ctx_set_stream(gptb200_ctx *ctx, void *cuda_stream);
  * "fuse_dbias" (weight-gradient launches of the CTA-pair kernel also produce the bias gradient: 1 = on (default), 0 = the
  * separate column-sum kernels; results differ only in summation order),
  * "gemv_rows" (gptb200_linear_bf16: most rows the weight-streaming kernel takes, 0 .. 8, default 8),
- * "max_sms" (0 = all SMs; otherwise the GEMM kernels occupy at most this many, which leaves SMs to a collective that runs
- * at the same time on another stream),
+ * "max_sms" (0 = all SMs; otherwise the GEMM kernels and a one-launch generation step occupy at most this many, which leaves SMs to a
+ * collective that runs at the same time on another stream),
  * "trace" (record a kernel-phase trace of each CTA-pair GEMM launch: 1 = on, 0 = off (default)),
  * "exact3x" (3xTF32 mode, CTA-pair kernel: form of the correction terms a_lo.b + a.b_lo -- 0 = one bf16 chain (error about 2^-20
  * per term, 8 tensor-core instructions per k-block), 1 = TF32 products of fp32 low-part tiles (2^-22, 12 instructions: 8 % slower
@@ -326,6 +326,12 @@ int gptb200_model_loss(gptb200_model *m, const int *labels_dev, float *loss_out)
  *   generate_step   one new position: tokens_dev [batch] are the tokens AT that position (sampled from the previous logits);
  *                   logits_dev [batch x vocab_size_padded] receives the logits that predict the next one; every linear layer
  *                   runs with m = batch rows.  The position advances by one; GPTB200_ERR_INVALID_ARG beyond max_len.
+ *                   Up to 64 sequences (head size a power of two from 8 to 128, d_model and d_ffn multiples of 4, "skinny" on, "skinny_rows" 0)
+ *                   most steps are one cooperative launch of a block per SM (gptb200_plan_generate_step says which): it starts when that many SMs are
+ *                   free at once, so it waits for a kernel of another stream that holds some, and two models on two streams take turns.  Option
+ *                   "max_sms" bounds it; below three fifths of the SMs, or with "skinny" off, the step runs operator by operator, which takes
+ *                   whatever SMs are free.  A block that waits for the others in vain (seconds) is reported by the next synchronize as
+ *                   GPTB200_ERR_DEVICE_TIMEOUT, device status 110; no later step advances until generate_begin.
  *   generate_position  the position the next generate_step will fill (prompt_len after generate_begin). */
 int gptb200_model_generate_begin(gptb200_model *m, const int *prompt_dev, int batch, int prompt_len, int max_len);
 int gptb200_model_generate_step(gptb200_model *m, const int *tokens_dev, float *logits_dev);
@@ -366,7 +372,8 @@ int gptb200_model_step_count(gptb200_model *m);
  *                   in the tensor-core form for prompts, default 32; shorter ones split the positions, latent attention then uses the
  *                   latents as they are), "chunk_rows" (recurrent layers in bf16: shortest portion that runs in chunks on the tensor
  *                   cores, default 8; shorter ones token by token), "segment_tokens" (Mamba-2 and lightning prompts: tokens per segment of the
- *                   segments that run side by side; unless set 1024, or fewer where a step would leave the GPU idle), "wkv_segment_tokens" (the same for wkv, a multiple of 16, default 0:
+ *                   segments that run side by side; unless set 1024, or down to 256 where the requests of a step would leave the GPU idle: the last bits of a long
+ *                   prompt then depend on how many requests share its step and on the longest of them; set, on the longest only), "wkv_segment_tokens" (the same for wkv, a multiple of 16, default 0:
  *                   automatic) and those of gptb200_ctx_set_option */
 typedef enum gptb200_dtype { GPTB200_DTYPE_BF16 = 0, GPTB200_DTYPE_F32 = 1 } gptb200_dtype;
 typedef struct gptb200_decoder gptb200_decoder;
