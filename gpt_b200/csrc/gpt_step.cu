@@ -148,8 +148,9 @@ bool gpt_step_replayed(const gptb200_ctx *ctx)
 //   1024, 2 (4)                 850 / 1212 / 1037, 1137                   1614 / 1596 / 2252, 2365       2532 / 2085 / 3583, 3687
 //   1280, 1 (3)                 1249 / 2224 / 1844, 2063                  2113 / 2811 / 3388, 3604       3126 / 3541 / 5342, 5552
 //   1280, 2 (6)                 1925 / 2260 / 2019, 2214                  3540 / 2866 / 3474, 3666       5589 / 3606 / 5402, 5609
-//   1600, 1 (5)                 2722 / 4090 / 3297, 3541                  4445 / 4870 / 5247, 5498       6735 / 5915 / 7825, 8079
-//   1600, 2 (10)                4019 / 4170 / 3480, 3715                  7468 / 4966 / 5330, 5558       -    / 6000 / 7804, 8028
+//   1600, 1 (5)                 2722 / 4219 / 3297, 3541                  4445 / 4991 / 5247, 5498       6735 / 5915 / 7825, 8079
+//   1600, 2 (10)                4019 / 4286 / 3480, 3715                  7468 / 4966 / 5330, 5558       -    / 6000 / 7804, 8028
+// (The other kernel's figures at 768, and at 1024 at position 96, are those of three rows; 1600 at position 96, and one row at 480, with slightly other slices.)
 // The other kernel pads up to four rows to eight, and the operators have kernels for four; their attention is the slower one:
 //   768, 3    position 64: 461 / 428, 507    128: 504 / 469, 556    256: 569 / 568, 634    480: 664 / 1065, 1122
 //   768, 4                 469 / 434, 507         513 / 478, 556         570 / 711, 763         660 / 1065, 1129
