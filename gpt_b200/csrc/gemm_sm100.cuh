@@ -344,7 +344,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * (3 * STAGES + 5));
     volatile uint32_t *abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = ptx::warp_uniform(threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -371,7 +371,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = ptx::warp_uniform(*tmem_slot);
 
     const long long num_items = 1LL * p.tiles_m * p.tiles_n * p.splits;
 
@@ -422,84 +422,79 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
             }
         } else if (warp == 1) {
-            // ------------------------------------------------------------ MMA issuer
-            if (lane == 0) {
-                uint32_t it = 0;
-                uint32_t g = 0;  // accumulator hand-offs so far
-                bool ok = true;
-                for (long long w = blockIdx.x; ok && w < num_items; w += gridDim.x) {
-                    int tm, tn, kb0, kb1, split;
-                    decode(w, tm, tn, kb0, kb1, split);
-                    int kb = kb0;
-                    while (ok && kb < kb1) {
-                        const int kend = C::kChunked ? min(kb + kChunkKB, kb1) : kb1;
-                        const uint32_t buf = g & 1u;
-                        const uint32_t use = (g >> 1) & 1u;
-                        if (!bounded_wait(tmem_empty_bar(buf), use ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM)) {
+            // ------------------------------------------------------------ MMA issuer: the warp walks, one lane issues
+            const bool issuer = ptx::elect_one();
+            uint32_t s = 0, ph = 0;   // stage and the parity of its barriers
+            uint32_t g = 0;  // accumulator hand-offs so far
+            bool ok = true;
+            // K-major tile: rows of 128 B (32 k), 16-byte-chunk swizzle over 8-row atoms of 1024 B;
+            //   a k-step (8 floats) is 32 bytes along the row, 8-row groups are 1024 B apart (SBO).
+            // MN-major tile: boxes of [32 k-rows x 32 floats], 32-byte-chunk swizzle over 4-row atoms
+            //   of 512 B; a k-step is 8 rows = 1024 B, 4-row groups are 512 B apart (SBO) and the
+            //   32-float column groups are one 4 KiB box apart (LBO).
+            constexpr uint32_t a_step = A_MN ? 1024 : 32, b_step = B_MN ? 1024 : 32;
+            const ptx::SmemDesc desc_a = ptx::smem_desc_words(smem_base, A_MN ? kBoxBytesMN : 16, A_MN ? 512 : 1024, A_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128);
+            const ptx::SmemDesc desc_b = ptx::smem_desc_words(smem_base + kATileBytes, B_MN ? kBoxBytesMN : 16, B_MN ? 512 : 1024, B_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128);
+            for (long long w = blockIdx.x; ok && w < num_items; w += gridDim.x) {
+                int tm, tn, kb0, kb1, split;
+                decode(w, tm, tn, kb0, kb1, split);
+                int kb = kb0;
+                while (ok && kb < kb1) {
+                    const int kend = C::kChunked ? min(kb + kChunkKB, kb1) : kb1;
+                    const uint32_t buf = g & 1u;
+                    const uint32_t use = (g >> 1) & 1u;
+                    if (!bounded_wait(tmem_empty_bar(buf), use ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM)) {
+                        ok = false;
+                        break;
+                    }
+                    ptx::tc_fence_after();
+                    const uint32_t d_tmem = tmem_base + buf * BN;
+                    uint32_t accumulate = 0;
+                    for (; kb < kend; ++kb) {
+                        if (!bounded_wait(full_bar(s), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
                             ok = false;
                             break;
                         }
-                        ptx::tc_fence_after();
-                        const uint32_t d_tmem = tmem_base + buf * BN;
-                        uint32_t accumulate = 0;
-                        for (; kb < kend; ++kb, ++it) {
-                            const int s = it % STAGES;
-                            const uint32_t ph = (it / STAGES) & 1u;
-                            if (!bounded_wait(full_bar(s), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                        if (X3) {
+                            if (!bounded_wait(conv_bar(s), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) {
                                 ok = false;
                                 break;
                             }
-                            if (X3) {
-                                if (!bounded_wait(conv_bar(s), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) {
-                                    ok = false;
-                                    break;
-                                }
-                            }
-                            ptx::tc_fence_after();
-                            const uint32_t a_hi = smem_base + s * C::kStageBytes;
-                            const uint32_t b_hi = a_hi + kATileBytes;
-                            const uint32_t a_lo = a_hi + C::kHiBytes;
-                            const uint32_t b_lo = b_hi + C::kHiBytes;
+                        }
+                        ptx::tc_fence_after();
+                        const uint32_t hi = s * C::kStageBytes, lo = hi + C::kHiBytes;
+                        if (issuer) {
+                            if (!A_MN && !B_MN && !X3 && p.bf16) {
 #pragma unroll
-                            for (int k = 0; k < kBK / kUmmaK; ++k) {
-                                // K-major tile: rows of 128 B (32 k), 16-byte-chunk swizzle over 8-row atoms of 1024 B;
-                                //   a k-step (8 floats) is 32 bytes along the row, 8-row groups are 1024 B apart (SBO).
-                                // MN-major tile: boxes of [32 k-rows x 32 floats], 32-byte-chunk swizzle over 4-row atoms
-                                //   of 512 B; a k-step is 8 rows = 1024 B, 4-row groups are 512 B apart (SBO) and the
-                                //   32-float column groups are one 4 KiB box apart (LBO).
-                                const uint32_t a_off = A_MN ? k * 1024 : k * 32;
-                                const uint32_t b_off = B_MN ? k * 1024 : k * 32;
-                                constexpr uint32_t a_lbo = A_MN ? kBoxBytesMN : 16, a_sbo = A_MN ? 512 : 1024;
-                                constexpr uint32_t b_lbo = B_MN ? kBoxBytesMN : 16, b_sbo = B_MN ? 512 : 1024;
-                                constexpr uint32_t a_lay = A_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128;
-                                constexpr uint32_t b_lay = B_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128;
-                                const uint64_t da_hi = ptx::make_smem_desc(a_hi + a_off, a_lbo, a_sbo, a_lay);
-                                const uint64_t db_hi = ptx::make_smem_desc(b_hi + b_off, b_lbo, b_sbo, b_lay);
-                                if (X3) {
-                                    const uint64_t da_lo = ptx::make_smem_desc(a_lo + a_off, a_lbo, a_sbo, a_lay);
-                                    const uint64_t db_lo = ptx::make_smem_desc(b_lo + b_off, b_lbo, b_sbo, b_lay);
-                                    ptx::mma_tf32_ss(d_tmem, da_lo, db_hi, kIdesc, accumulate);
-                                    ptx::mma_tf32_ss(d_tmem, da_hi, db_lo, kIdesc, 1u);
-                                    ptx::mma_tf32_ss(d_tmem, da_hi, db_hi, kIdesc, 1u);
-                                } else if (!A_MN && !B_MN && p.bf16) {
-                                    ptx::mma_f16_ss(d_tmem, da_hi, db_hi, ptx::make_idesc_bf16(kBM, BN, false, false), accumulate);
-                                } else {
-                                    ptx::mma_tf32_ss(d_tmem, da_hi, db_hi, kIdesc, accumulate);
+                                for (int k = 0; k < kBK / kUmmaK; ++k)
+                                    ptx::mma_f16_ss(d_tmem, desc_a.at(hi + k * a_step), desc_b.at(hi + k * b_step), ptx::make_idesc_bf16(kBM, BN, false, false), k ? 1u : accumulate);
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < kBK / kUmmaK; ++k) {
+                                    if (X3) {
+                                        ptx::mma_tf32_ss(d_tmem, desc_a.at(lo + k * a_step), desc_b.at(hi + k * b_step), kIdesc, k ? 1u : accumulate);
+                                        ptx::mma_tf32_ss(d_tmem, desc_a.at(hi + k * a_step), desc_b.at(lo + k * b_step), kIdesc, 1u);
+                                    }
+                                    ptx::mma_tf32_ss(d_tmem, desc_a.at(hi + k * a_step), desc_b.at(hi + k * b_step), kIdesc, X3 || k ? 1u : accumulate);
                                 }
-                                accumulate = 1u;
                             }
                             ptx::mma_commit(empty_bar(s));  // frees the stage once these MMAs have read it
                         }
-                        if (ok) {
-                            ptx::mma_commit(tmem_full_bar(buf));
-                            ++g;
+                        accumulate = 1u;
+                        if (++s == STAGES) {
+                            s = 0;
+                            ph ^= 1u;
                         }
                     }
+                    if (ok) {
+                        if (issuer) ptx::mma_commit(tmem_full_bar(buf));
+                        ++g;
+                    }
                 }
-                // Do not leave with MMAs still running: they write TMEM that is about to be released.
-                ptx::mma_commit(drain_bar);
-                bounded_wait(drain_bar, 0u, abort_flag, p.status, DEV_TIMEOUT_DRAIN);
             }
+            // Do not leave with MMAs still running: they write TMEM that is about to be released.
+            if (issuer) ptx::mma_commit(drain_bar);
+            bounded_wait(drain_bar, 0u, abort_flag, p.status, DEV_TIMEOUT_DRAIN);
             __syncwarp();
         }
     } else if (warp < kFirstConvWarp) {

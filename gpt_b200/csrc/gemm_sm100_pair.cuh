@@ -105,24 +105,6 @@ struct PairCfg {
     static_assert(kSmemBytes <= 232448, "exceeds 227 KiB of shared memory");
 };
 
-__device__ __forceinline__ bool bounded_wait_cluster(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag, int *status, int code)
-{
-    if (ptx::mbar_try_wait_cluster(bar, parity)) return true;
-    const long long t0 = clock64();
-    uint32_t spins = 0;
-    while (true) {
-        if (ptx::mbar_try_wait_cluster(bar, parity)) return true;
-        if ((++spins & 31u) == 0) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > kWaitTimeoutCycles) {
-                *abort_flag = 1u;
-                atomicCAS(status, 0, code);
-                return false;
-            }
-        }
-    }
-}
-
 // 3xTF32 on CTA pairs computes a.b as  a_hi.b_hi (tf32 MMAs on the raw fp32 tiles: the tensor core drops the low 13
 // mantissa bits)  +  a_lo.b + a.b_lo (bf16 MMAs), with a_lo = a - a_hi.  The converter warps write, per operand tile, a
 // bf16 tile with 64 k-positions per 32 k of the raw tile:  A: [a_lo | a]   B: [b | b_lo]  (groups of 8 values of each kind
@@ -411,7 +393,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * C::kNumBarriers);
     volatile uint32_t *abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = ptx::warp_uniform(threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_ctarank();   // 0 = leader
     const bool leader = rank == 0;
@@ -447,7 +429,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     __syncthreads();
     ptx::cluster_sync();   // the peer's barriers exist before anything is signalled across CTAs
     ptx::tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = ptx::warp_uniform(*tmem_slot);
 
     const int tiles_m2 = (p.tiles_m + 1) / 2;   // pairs of 128-row tiles
     // narrow batched form: only the first mma_n / 2 columns of this CTA's B tile are loaded, split and read (K-major: that many
@@ -494,7 +476,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 const int j = it % NL;
                 const uint32_t lph = (it / NL) & 1u;
                 // the low-part buffer must have been read by the MMAs of its previous use, the raw tile must have landed
-                if (!bounded_wait_cluster(lo_empty_bar(j), lph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT) ||
+                if (!bounded_wait(lo_empty_bar(j), lph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT) ||
                     !bounded_wait(full_bar(s), ph, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
                     ok = false;
                     break;
@@ -549,7 +531,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1u;
-                    if (!bounded_wait_cluster(empty_bar(s), ph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
+                    if (!bounded_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
                         ok = false;
                         break;
                     }
@@ -595,7 +577,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         //   MN-major: [64 k-positions x 64 rows-of-the-operand] atoms: one box per half of the CTA's 128 rows.
                         const int j = it % NL;
                         const uint32_t lph = (it / NL) & 1u;
-                        if (!bounded_wait_cluster(lo_empty_bar(j), lph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
+                        if (!bounded_wait(lo_empty_bar(j), lph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
                             ok = false;
                             break;
                         }
@@ -616,21 +598,33 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 }
             }
         } else if (warp == 1) {
-            // ------------------------------------------------------------ MMA issuer (leader CTA, one thread)
-            if (leader && lane == 0) {
+            // ------------------------------------------------------------ MMA issuer (leader CTA): the warp walks, one lane issues
+            if (leader) {
+                const bool issuer = ptx::elect_one();
                 uint32_t it = 0, g = 0;
+                uint32_t s = 0, ph = 0, j = 0, lph = 0;   // raw stage and correction buffer, with the parities of their barriers
                 bool ok = true;
                 PairWork work = my_work();
                 int tm2, tn, kb0, kb1;
                 const uint32_t idesc = p.mma_n ? ptx::make_idesc_tf32(2 * kBM, p.mma_n, A_MN, B_MN) : kIdesc;
                 const uint32_t idesc_corr = p.mma_n ? ptx::make_idesc_bf16(2 * kBM, p.mma_n, A_MN, B_MN) : kIdescCorr;
+                // Raw tiles and fp32 low-part tiles.  K-major: a k-step is 32 bytes along the row; MN-major: 8 rows of a box.
+                constexpr uint32_t a_step = A_MN ? 1024 : 32, b_step = B_MN ? 1024 : 32;
+                const ptx::SmemDesc desc_a = ptx::smem_desc_words(smem_base, A_MN ? kBoxBytesMN : 16, A_MN ? 512 : 1024, A_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128);
+                const ptx::SmemDesc desc_b = ptx::smem_desc_words(smem_base + kATileBytes, B_MN ? kBoxBytesMN : 16, B_MN ? 512 : 1024, B_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128);
+                // bf16 correction tiles with 64 k-positions (low parts and whole values side by side), 16 of them per instruction.  K-major: 128-byte
+                // rows, +32 bytes per step; MN-major: [8 k x 64 m] atoms, 1 KiB per group of 8 k, 8 KiB to the next 64 rows.
+                constexpr uint32_t a_corr_step = A_MN ? 2048 : 32, b_corr_step = B_MN ? 2048 : 32;
+                const ptx::SmemDesc corr_a = ptx::smem_desc_words(lo_base, A_MN ? 8192 : 16, 1024, ptx::kLayoutSw128);
+                const ptx::SmemDesc corr_b = ptx::smem_desc_words(lo_base + kATileBytes, B_MN ? 8192 : 16, 1024, ptx::kLayoutSw128);
+                constexpr uint32_t lo_offset = STAGES * C::kHiBytes;   // of the correction ring behind the raw ring
                 while (ok && work.next(tm2, tn, kb0, kb1)) {
                     int kb = kb0;
                     while (ok && kb < kb1) {
                         const int kend = C::kChunked ? min(kb + (p.chunk_kb ? p.chunk_kb : pair_chunk_kb(kb == kb0)), kb1) : kb1;
                         const uint32_t buf = g & 1u;
                         const uint32_t use = (g >> 1) & 1u;
-                        if (!bounded_wait_cluster(tmem_empty_bar(buf), use ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM)) {
+                        if (!bounded_wait(tmem_empty_bar(buf), use ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM)) {
                             ok = false;
                             break;
                         }
@@ -638,75 +632,51 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         const uint32_t d_tmem = tmem_base + buf * BN;
                         uint32_t accumulate = 0;
                         for (; kb < kend; ++kb, ++it) {
-                            const int s = it % STAGES;
-                            const uint32_t ph = (it / STAGES) & 1u;
                             // 3xTF32: the converters of both CTAs report to one barrier of the leader; they have seen their raw
                             // tiles land, so that barrier stands for the loads as well
-                            if (!X3 && !bounded_wait_cluster(full_bar(s), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) { ok = false; break; }
-                            trace(TRACE_MMA_FULL, it);
-                            const int j = it % NL;
-                            const uint32_t lph = (it / NL) & 1u;
-                            if (X3 && !bounded_wait_cluster(conv_bar(j), lph, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) { ok = false; break; }
+                            if (!X3 && !bounded_wait(full_bar(s), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) { ok = false; break; }
+                            if (issuer) trace(TRACE_MMA_FULL, it);
+                            if (X3 && !bounded_wait(conv_bar(j), lph, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) { ok = false; break; }
                             ptx::tc_fence_after();
-                            trace(TRACE_MMA_READY, it);
-                            const uint32_t a_hi = smem_base + s * C::kHiBytes;
-                            const uint32_t b_hi = a_hi + kATileBytes;
-                            const uint32_t a_lo = lo_base + j * C::kHiBytes;
-                            const uint32_t b_lo = a_lo + kATileBytes;
-                            constexpr uint32_t a_lbo = A_MN ? kBoxBytesMN : 16, a_sbo = A_MN ? 512 : 1024;
-                            constexpr uint32_t b_lbo = B_MN ? kBoxBytesMN : 16, b_sbo = B_MN ? 512 : 1024;
-                            constexpr uint32_t a_lay = A_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128;
-                            constexpr uint32_t b_lay = B_MN ? ptx::kLayoutSw128Base32B : ptx::kLayoutSw128;
-                            if (X3 && p.exact3x) {
-                                // correction terms in TF32 as well: a_lo.b + a.b_lo with fp32 low-part tiles laid out like the raw ones
+                            if (issuer) {
+                                trace(TRACE_MMA_READY, it);
+                                const uint32_t raw = s * C::kHiBytes, cor = j * C::kHiBytes;
+                                if (X3 && p.exact3x) {
+                                    // correction terms in TF32 as well: a_lo.b + a.b_lo with fp32 low-part tiles laid out like the raw ones
 #pragma unroll
-                                for (int k = 0; k < kBK / kUmmaK; ++k) {
-                                    const uint32_t a_off = A_MN ? k * 1024 : k * 32;
-                                    const uint32_t b_off = B_MN ? k * 1024 : k * 32;
-                                    const uint64_t da_hi = ptx::make_smem_desc(a_hi + a_off, a_lbo, a_sbo, a_lay);
-                                    const uint64_t db_hi = ptx::make_smem_desc(b_hi + b_off, b_lbo, b_sbo, b_lay);
-                                    const uint64_t da_lo = ptx::make_smem_desc(a_lo + a_off, a_lbo, a_sbo, a_lay);
-                                    const uint64_t db_lo = ptx::make_smem_desc(b_lo + b_off, b_lbo, b_sbo, b_lay);
-                                    ptx::mma_tf32_ss_pair(d_tmem, da_lo, db_hi, idesc, accumulate);
-                                    ptx::mma_tf32_ss_pair(d_tmem, da_hi, db_lo, idesc, 1u);
-                                    accumulate = 1u;
+                                    for (int k = 0; k < kBK / kUmmaK; ++k) {
+                                        ptx::mma_tf32_ss_pair(d_tmem, desc_a.at(lo_offset + cor + k * a_step), desc_b.at(raw + k * b_step), idesc, k ? 1u : accumulate);
+                                        ptx::mma_tf32_ss_pair(d_tmem, desc_a.at(raw + k * a_step), desc_b.at(lo_offset + cor + k * b_step), idesc, 1u);
+                                    }
+                                } else if (X3) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k)
+                                        ptx::mma_f16_ss_pair(d_tmem, corr_a.at(cor + k * a_corr_step), corr_b.at(cor + k * b_corr_step), idesc_corr, k ? 1u : accumulate);
                                 }
-                            } else if (X3) {
-                                // correction terms a_lo.b + a.b_lo: bf16 tiles with 64 k-positions (low parts and whole values
-                                // side by side), 16 of them per instruction.  K-major: 128-byte rows, +32 bytes per step;
-                                // MN-major: [8 k x 64 m] atoms, 1 KiB per group of 8 k, 8 KiB to the next 64 rows.
+                                if (!A_MN && !B_MN && !X3 && p.bf16) {
 #pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    const uint64_t da = ptx::make_smem_desc(a_lo + (A_MN ? k * 2048 : k * 32), A_MN ? 8192 : 16, 1024, ptx::kLayoutSw128);
-                                    const uint64_t db = ptx::make_smem_desc(b_lo + (B_MN ? k * 2048 : k * 32), B_MN ? 8192 : 16, 1024, ptx::kLayoutSw128);
-                                    ptx::mma_f16_ss_pair(d_tmem, da, db, idesc_corr, accumulate);
-                                    accumulate = 1u;
+                                    for (int k = 0; k < 4; ++k) ptx::mma_f16_ss_pair(d_tmem, desc_a.at(raw + k * 32), desc_b.at(raw + k * 32), idesc_corr, k ? 1u : accumulate);
+                                } else {
+#pragma unroll
+                                    for (int k = 0; k < kBK / kUmmaK; ++k)
+                                        ptx::mma_tf32_ss_pair(d_tmem, desc_a.at(raw + k * a_step), desc_b.at(raw + k * b_step), idesc, X3 || k ? 1u : accumulate);
                                 }
+                                // the stage is free in both CTAs once these MMAs have read it
+                                ptx::mma_commit_pair_both(empty_bar(s), 3);
+                                if (X3) ptx::mma_commit_pair_both(lo_empty_bar(j), 3);
+                                trace(TRACE_MMA_ISSUED, it);
                             }
-#pragma unroll
-                            for (int k = 0; k < kBK / kUmmaK; ++k) {
-                                const uint32_t a_off = A_MN ? k * 1024 : k * 32;
-                                const uint32_t b_off = B_MN ? k * 1024 : k * 32;
-                                const uint64_t da_hi = ptx::make_smem_desc(a_hi + a_off, a_lbo, a_sbo, a_lay);
-                                const uint64_t db_hi = ptx::make_smem_desc(b_hi + b_off, b_lbo, b_sbo, b_lay);
-                                if (!A_MN && !B_MN && !X3 && p.bf16)
-                                    ptx::mma_f16_ss_pair(d_tmem, da_hi, db_hi, idesc_corr, accumulate);
-                                else
-                                    ptx::mma_tf32_ss_pair(d_tmem, da_hi, db_hi, idesc, accumulate);
-                                accumulate = 1u;
-                            }
-                            // the stage is free in both CTAs once these MMAs have read it
-                            ptx::mma_commit_pair_both(empty_bar(s), 3);
-                            if (X3) ptx::mma_commit_pair_both(lo_empty_bar(j), 3);
-                            trace(TRACE_MMA_ISSUED, it);
+                            accumulate = 1u;
+                            if (++s == STAGES) { s = 0; ph ^= 1u; }
+                            if (++j == NL) { j = 0; lph ^= 1u; }
                         }
                         if (ok) {
-                            ptx::mma_commit_pair_both(tmem_full_bar(buf), 3);
+                            if (issuer) ptx::mma_commit_pair_both(tmem_full_bar(buf), 3);
                             ++g;
                         }
                     }
                 }
-                ptx::mma_commit_pair(drain_bar);
+                if (issuer) ptx::mma_commit_pair(drain_bar);
                 bounded_wait(drain_bar, 0u, abort_flag, p.status, DEV_TIMEOUT_DRAIN);
             }
             __syncwarp();
@@ -892,7 +862,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 for (int kb = kb0; ok && kb < kb1; kb += (p.chunk_kb ? p.chunk_kb : pair_chunk_kb(kb == kb0)), ++g) {
                     const uint32_t buf = g & 1u;
                     const uint32_t use = (g >> 1) & 1u;
-                    if (!bounded_wait_cluster(tmem_full_bar(buf), use, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
+                    if (!bounded_wait(tmem_full_bar(buf), use, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
                         ok = false;
                         break;
                     }
@@ -908,7 +878,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                     }
                     ptx::tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive_cluster(leader_tmem_empty[buf]);
+                    if (lane == 0) ptx::mbar_arrive_remote(leader_tmem_empty[buf]);
                     // this tile's share of the k-blocks of the chunk just drained (fetched by the operand loads a moment ago)
                     if (duty) {
                         const int first = kb + (tm2 - kb % db_rows + db_rows) % db_rows;
@@ -958,7 +928,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                     column_sums_16<16>(bsum, p.dbias_src, p.N, db_first, db_rows, kb1, p.K, bcol, bcol < p.N, lane);
                     column_sums_finish(bsum);
                 }
-                if (!bounded_wait_cluster(tmem_full_bar(buf), use, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
+                if (!bounded_wait(tmem_full_bar(buf), use, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
                     ok = false;
                     break;
                 }
@@ -980,7 +950,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                     if (c == C::kColsPerEpiWarp / 32 - 1) {
                         ptx::tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive_cluster(leader_tmem_empty[buf]);
+                        if (lane == 0) ptx::mbar_arrive_remote(leader_tmem_empty[buf]);
                     }
                     float v[32];
 #pragma unroll

@@ -27,6 +27,12 @@ __device__ __forceinline__ bool elect_one()
     return pred != 0;
 }
 
+// A value that all lanes of the warp hold alike, in a form that the compiler knows to be alike.  The tensor-core instructions take their operands from uniform
+// registers: with a warp that walks its loop as a
+// whole and issues from one elected lane, a k-block of four 256 x 128 x 16 instructions and a commit takes 225 ns; with one lane that walks alone 320 ns,
+// whatever the width of the instruction.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // ---------------------------------------------------------------- two fp32 values per register pair
 
 __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
@@ -100,19 +106,6 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity)
     asm volatile(
         "{\n\t.reg .pred P;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, P;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ bool mbar_test_wait_cluster(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred P;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, P;\n\t}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
@@ -325,32 +318,13 @@ __device__ __forceinline__ void cluster_sync()
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Arrive on an mbarrier that lives in another CTA of the cluster (address from map_to_cta).
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar)
-{
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-
-// The same with the default semantics (release at CTA scope): enough where the arrival only hands over shared memory of the
-// arriving CTA that was written before a proxy fence and is read next by the tensor cores, and much cheaper than the
-// cluster-scope release, which was measured to hold the arriving warp for more than a thousand cycles.
+// Arrive on an mbarrier that lives in another CTA of the cluster (address from map_to_cta), with the default semantics (release at CTA scope): enough where the
+// arrival only hands over TMEM that was read behind a tcgen05 fence, or shared memory of the arriving CTA that was written before a proxy fence and is read
+// next by the tensor cores.  The waits on such barriers are the plain ones as well.  Cluster scope costs: a release was measured to hold the arriving warp for
+// more than a thousand cycles, an acquire to add 1.5 us to a launch of 15 us (2611 x 3072 x 768 in bf16).
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar)
 {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-
-// try_wait with cluster-scope acquire: for barriers that other CTAs of the cluster arrive on.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred P;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, P;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
 }
 
 // ---- CTA-pair (cta_group::2) forms of the tcgen05 instructions: issued in both CTAs (alloc / dealloc) or by
@@ -430,6 +404,19 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
     d |= static_cast<uint64_t>(1) << 46;
     d |= static_cast<uint64_t>(layout_type) << 61;
     return d;
+}
+
+// The same as two words, for loops that move along a ring: only the start address changes and stays inside its 14 bits (shared memory is smaller than
+// 256 KB), so a step is one 32-bit add.  Building the whole descriptor for every instruction is a chain of 64-bit shifts in the one thread that issues them.
+struct SmemDesc {
+    uint32_t lo, hi;
+    __device__ __forceinline__ uint64_t at(uint32_t byte_offset) const { return (static_cast<uint64_t>(hi) << 32) | (lo + (byte_offset >> 4)); }
+};
+
+__device__ __forceinline__ SmemDesc smem_desc_words(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout_type)
+{
+    const uint64_t d = make_smem_desc(smem_addr, lbo_bytes, sbo_bytes, layout_type);
+    return {static_cast<uint32_t>(d), static_cast<uint32_t>(d >> 32)};
 }
 
 // Instruction descriptor for kind::tf32, fp32 accumulate, dense, no negate.
