@@ -73,6 +73,29 @@ int make_tmap(gptb200_ctx *ctx, CUtensorMap *map, const float *base, long long r
     return GPTB200_OK;
 }
 
+// MN-major operand [rows = k][cols] whose columns are a multiple of 32: (32 columns, rows, groups of 32 columns), so that one load brings `groups` boxes of
+// [32 rows x 32 columns] one behind the other.  With other widths the last group would reach into the next row: make_tmap and a load per box.
+int make_grouped_tmap(gptb200_ctx *ctx, CUtensorMap *map, const float *base, long long rows, long long cols, int groups)
+{
+    const TmapKey key{reinterpret_cast<uintptr_t>(base), cols, rows, 0, 32, groups, 8};
+    const auto hit = ctx->tmaps.find(key);
+    if (hit != ctx->tmaps.end()) {
+        *map = hit->second;
+        return GPTB200_OK;
+    }
+    cuuint64_t dims[3] = {32, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 32)};
+    cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * sizeof(float), 32 * sizeof(float)};
+    cuuint32_t box[3] = {32, kBK, static_cast<cuuint32_t>(groups)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = ctx->encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    ctx->tmap_encodes++;
+    if (r != CUDA_SUCCESS) return fail(ctx, GPTB200_ERR_CUDA, "cuTensorMapEncodeTiled (grouped) failed (%d) rows=%lld cols=%lld groups=%d", int(r), rows, cols, groups);
+    if (ctx->tmaps.size() >= kTmapCacheMax) ctx->tmaps.clear();
+    ctx->tmaps.emplace(key, *map);
+    return GPTB200_OK;
+}
+
 // Tensor map of an operand's expanded bf16 correction matrix (split_operand_kernel), described in 4-byte words:
 //   K-major: [rows][k8 words], box 32 words x 128 rows (like the raw operand);  MN-major: [2 k8 rows][cols / 2 words], box 32 words x 64 rows.
 int make_pre_tmap(gptb200_ctx *ctx, CUtensorMap *map, const void *base, long long rows, long long words, int box_rows)
@@ -121,6 +144,31 @@ int make_batched_tmap(gptb200_ctx *ctx, CUtensorMap *map, const float *base, lon
     if (r != CUDA_SUCCESS)
         return fail(ctx, GPTB200_ERR_CUDA, "cuTensorMapEncodeTiled (batched) failed (%d) cols=%lld rows=%lld batches=%lldx%lld strides=%lld,%lld,%lld", int(r), cols,
                     rows, inner, outer, stride_inner, ld, stride_outer);
+    if (ctx->tmaps.size() >= kTmapCacheMax) ctx->tmaps.clear();
+    ctx->tmaps.emplace(key, *map);
+    return GPTB200_OK;
+}
+
+// The batched form of make_grouped_tmap: (32 columns, rows, groups, inner batch, outer batch); cols a multiple of 32.
+int make_batched_grouped_tmap(gptb200_ctx *ctx, CUtensorMap *map, const float *base, long long cols, long long rows, long long inner, long long outer, long long ld,
+                              long long stride_inner, long long stride_outer, int groups)
+{
+    if (inner == 1) stride_inner = ld;   // the coordinate is always 0
+    if (outer == 1) stride_outer = ld * rows;
+    const TmapKey key{reinterpret_cast<uintptr_t>(base), cols, rows, ld, 32, groups, 9, inner, outer, stride_inner, stride_outer};
+    const auto hit = ctx->tmaps.find(key);
+    if (hit != ctx->tmaps.end()) {
+        *map = hit->second;
+        return GPTB200_OK;
+    }
+    cuuint64_t dims[5] = {32, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 32), static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
+    cuuint64_t strides[4] = {static_cast<cuuint64_t>(ld) * 4, 32 * sizeof(float), static_cast<cuuint64_t>(stride_inner) * 4, static_cast<cuuint64_t>(stride_outer) * 4};
+    cuuint32_t box[5] = {32, kBK, static_cast<cuuint32_t>(groups), 1, 1};
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = ctx->encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    ctx->tmap_encodes++;
+    if (r != CUDA_SUCCESS) return fail(ctx, GPTB200_ERR_CUDA, "cuTensorMapEncodeTiled (batched, grouped) failed (%d) cols=%lld rows=%lld batches=%lldx%lld", int(r), cols, rows, inner, outer);
     if (ctx->tmaps.size() >= kTmapCacheMax) ctx->tmaps.clear();
     ctx->tmaps.emplace(key, *map);
     return GPTB200_OK;
@@ -564,12 +612,18 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
     } else {
         tact = to;
     }
-    if (c.a_mn)
+    p.a_one_load = c.a_mn && c.M % 32 == 0;
+    p.b_one_load = c.b_mn && c.N % 32 == 0;
+    if (p.a_one_load)
+        rc = make_grouped_tmap(ctx, &ta, c.a, c.K, c.M, kBM / 32);
+    else if (c.a_mn)
         rc = make_tmap(ctx, &ta, c.a, c.K, c.M, 32, kBK, true);
     else
         rc = make_tmap(ctx, &ta, c.a, c.M, c.K, kBK, kBM, false);
     if (rc != GPTB200_OK) return rc;
-    if (c.b_mn)
+    if (p.b_one_load)
+        rc = make_grouped_tmap(ctx, &tb, c.b, c.K, c.N, (pair ? bn / 2 : bn) / 32);
+    else if (c.b_mn)
         rc = make_tmap(ctx, &tb, c.b, c.K, c.N, 32, kBK, true);
     else
         rc = make_tmap(ctx, &tb, c.b, c.N, c.K, kBK, pair ? bn / 2 : bn, false);
@@ -668,11 +722,16 @@ int run_gemm_batched_impl(gptb200_ctx *ctx, float *out, long long out_ld, long l
     const int sms = ctx->max_sms > 0 ? std::min(ctx->max_sms, ctx->num_sms) : ctx->num_sms;   // option "max_sms" bounds these launches too
     const int pairs = static_cast<int>(std::min<long long>(std::max(1, sms / 2), tiles));
     CUtensorMap ta, tb, to;
-    int rc = a.mn ? make_batched_tmap(ctx, &ta, a.base, M, K, inner, outer, a.ld, a.stride_inner, a.stride_outer, 32, kBK, 1)
-                  : make_batched_tmap(ctx, &ta, a.base, K, M, inner, outer, a.ld, a.stride_inner, a.stride_outer, kBK, kBM, 0);
+    const int b_cols = p.mma_n ? p.mma_n / 2 : 128;   // of one CTA
+    p.a_one_load = a.mn && M % 32 == 0;
+    p.b_one_load = b.mn && N % 32 == 0 && b_cols % 32 == 0;
+    int rc = p.a_one_load ? make_batched_grouped_tmap(ctx, &ta, a.base, M, K, inner, outer, a.ld, a.stride_inner, a.stride_outer, kBM / 32)
+             : a.mn       ? make_batched_tmap(ctx, &ta, a.base, M, K, inner, outer, a.ld, a.stride_inner, a.stride_outer, 32, kBK, 1)
+                          : make_batched_tmap(ctx, &ta, a.base, K, M, inner, outer, a.ld, a.stride_inner, a.stride_outer, kBK, kBM, 0);
     if (rc) return rc;
-    rc = b.mn ? make_batched_tmap(ctx, &tb, b.base, N, K, inner, outer, b.ld, b.stride_inner, b.stride_outer, 32, kBK, 1)
-              : make_batched_tmap(ctx, &tb, b.base, K, N, inner, outer, b.ld, b.stride_inner, b.stride_outer, kBK, N <= 128 ? (N + 31) / 32 * 16 : 128, 0);
+    rc = p.b_one_load ? make_batched_grouped_tmap(ctx, &tb, b.base, N, K, inner, outer, b.ld, b.stride_inner, b.stride_outer, b_cols / 32)
+         : b.mn       ? make_batched_tmap(ctx, &tb, b.base, N, K, inner, outer, b.ld, b.stride_inner, b.stride_outer, 32, kBK, 1)
+                      : make_batched_tmap(ctx, &tb, b.base, K, N, inner, outer, b.ld, b.stride_inner, b.stride_outer, kBK, N <= 128 ? (N + 31) / 32 * 16 : 128, 0);
     if (rc) return rc;
     rc = make_batched_tmap(ctx, &to, out, N, M, inner, outer, out_ld, out_si, out_so, PairCfg<false>::kStageCols, 32, 0);
     if (rc) return rc;

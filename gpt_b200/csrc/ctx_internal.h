@@ -22,7 +22,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
 struct TmapKey {
     uintptr_t base;
     long long d0, d1, d2;   // extents (innermost first; d2 = 0 for 2-D maps)
-    int box0, box1, kind;   // kind: 0 K-major operand, 1 MN-major operand, 2 output, 3 pre-split operand, 4 / 5 batched (4-D) with either swizzle
+    int box0, box1, kind;   // kind: 0 K-major operand, 1 MN-major operand, 2 output, 3 pre-split operand, 4 / 5 batched (4-D) with either swizzle,
+                            // 6 / 7 16-bit operand / output, 8 / 9 MN-major operand in groups of 32 columns, one or batched
     long long b0 = 0, b1 = 0, b2 = 0, b3 = 0;   // batched maps: inner and outer batch counts (d2 = row pitch), inner and outer batch strides
     bool operator==(const TmapKey &o) const
     {

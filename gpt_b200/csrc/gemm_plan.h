@@ -314,4 +314,43 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
     return p;
 }
 
+// ---- bf16 products of more than a few rows ----------------------------------------------------------------------------------------
+// Whole tiles of 256 rows on CTA pairs (gemm_bf16_pair_kernel).  A k-block of 64 takes 385 ns at 256 columns (the tensor pipe at the power limit), 225 at 128
+// and 180 at 64 (loads and the issue of instructions), so narrower tiles pay only where wider ones leave pairs idle: 2611 x 768 x 3072 in 33 tiles of 256
+// columns 22.8 us, 66 of 128 16.7, 132 of 64 23.2; 2611 x 3072 x 768 in two waves of 256 16.5, four of 128 18.7.
+// With few tiles and a long k, split-K over one-CTA tiles (8 us with its reduction + 485 ns per k-block of a split) beats the one chain of k-blocks (6 us + the
+// above) where the output can be added up at all, contiguous fp32 without a bias: 16 x 2048 x 8192 15.5 us against 26.9, 300 x 768 x 3072 12.6 against 14.6;
+// the other way 512 x 2048 x 8192 30.9 against 27.0, 300 x 768 x 1536 12.2 against 10.5.
+struct Bf16Plan {
+    int columns;       // per tile, or
+    bool split_k;      // the one-CTA kernel (plan_gemm without pairs)
+};
+
+inline Bf16Plan plan_bf16(int M, int N, int K, int num_sms, bool gated, bool plain_f32, size_t ws_limit)
+{
+    const long long pairs = std::max(1, num_sms / 2), rows = (M + 255) / 256;
+    Bf16Plan p{256, false};
+    long long least = 0;
+    for (const int bn : {256, 128, 64}) {
+        if (gated && bn == 64) break;   // a gate column and its up column lie 32 apart and belong to one warp, which has half of a tile's columns
+        const long long tiles = rows * ((N + bn - 1) / bn), cost = (tiles + pairs - 1) / pairs * (bn == 256 ? 385 : bn == 128 ? 225 : 180);
+        if (bn == 256 || cost < least) {
+            least = cost;
+            p.columns = bn;
+        }
+    }
+    if (plain_f32 && N % 4 == 0) {
+        GemmPlanInput in{};
+        in.M = M; in.N = N; in.K = K / 2;      // in 4-byte words: a k-block of 32 words is 64 bf16
+        in.aligned = true;
+        in.num_sms = num_sms;
+        in.opt_pair = -1;
+        in.ws_limit = ws_limit;
+        const GemmPlan s = plan_gemm(in);
+        const long long waves = (1LL * s.tiles_m * s.tiles_n * s.splits + num_sms - 1) / num_sms;
+        p.split_k = s.kernel == KERNEL_SINGLE && s.splits > 1 && 8000 + waves * s.kb_per_split * 485 < 6000 + least * ((K + 63) / 64);
+    }
+    return p;
+}
+
 }  // namespace gptb200

@@ -128,6 +128,8 @@ struct GemmParams {
     const int *factor_rows;     // row of the table per output row
     int factor_pitch;
     int silu_cols;              // OUT_BF16: silu is applied to the columns before this one (a multiple of 32)
+    // MN-major operands: the tensor map has a dimension for the columns of 32-float boxes, so that a tile is one load instead of four (or eight).
+    int a_one_load, b_one_load;
     // bf16 form: columns [g * a_group_cols, (g + 1) * a_group_cols) of the output multiply rows from g * a_group_rows on of A -- several
     // products of differently mixed rows with one weight matrix in one launch.  a_group_cols is a multiple of 256; 0: one group.
     int a_group_cols, a_group_rows;
@@ -387,38 +389,46 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (warp < 4) {
         if (C::kChunked) ptx::reg_dec<56>();
         if (warp == 0) {
-            // ------------------------------------------------------------ TMA producer
-            uint32_t it = 0;
+            // ------------------------------------------------------------ TMA producer: one elected lane issues
+            const bool issuer = ptx::elect_one();
+            uint32_t s = 0, ph = 0;
             bool ok = true;
             for (long long w = blockIdx.x; ok && w < num_items; w += gridDim.x) {
                 int tm, tn, kb0, kb1, split;
                 decode(w, tm, tn, kb0, kb1, split);
                 const int n0 = tn * BN, m0 = tm * kBM + (p.a_group_cols ? n0 / p.a_group_cols * p.a_group_rows : 0);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!bounded_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
                         ok = false;
                         break;
                     }
-                    if (lane == 0) ptx::mbar_arrive_expect_tx(full_bar(s), C::kHiBytes);
-                    __syncwarp();
-                    const uint32_t a_dst = smem_base + s * C::kStageBytes;
-                    const uint32_t b_dst = a_dst + kATileBytes;
-                    const int k0 = kb * kBK;
-                    if (lane < kBoxesA) {
-                        if (A_MN)
-                            ptx::tma_load_2d(a_dst + lane * kBoxBytesMN, &tmap_a, m0 + 32 * lane, k0, full_bar(s));
-                        else
+                    if (issuer) {
+                        ptx::mbar_arrive_expect_tx(full_bar(s), C::kHiBytes);
+                        const uint32_t a_dst = smem_base + s * C::kStageBytes;
+                        const uint32_t b_dst = a_dst + kATileBytes;
+                        const int k0 = kb * kBK;
+                        if (!A_MN) {
                             ptx::tma_load_2d(a_dst, &tmap_a, k0, m0, full_bar(s));
-                    } else if (lane < kBoxesA + kBoxesB) {
-                        const int j = lane - kBoxesA;
-                        if (B_MN)
-                            ptx::tma_load_2d(b_dst + j * kBoxBytesMN, &tmap_b, n0 + 32 * j, k0, full_bar(s));
-                        else
+                        } else if (p.a_one_load) {
+                            ptx::tma_load_3d(a_dst, &tmap_a, 0, k0, m0 / 32, full_bar(s));
+                        } else {
+#pragma unroll 1
+                            for (int j = 0; j < kBoxesA; ++j) ptx::tma_load_2d(a_dst + j * kBoxBytesMN, &tmap_a, m0 + 32 * j, k0, full_bar(s));
+                        }
+                        if (!B_MN) {
                             ptx::tma_load_2d(b_dst, &tmap_b, k0, n0, full_bar(s));
+                        } else if (p.b_one_load) {
+                            ptx::tma_load_3d(b_dst, &tmap_b, 0, k0, n0 / 32, full_bar(s));
+                        } else {
+#pragma unroll 1
+                            for (int j = 0; j < kBoxesB; ++j) ptx::tma_load_2d(b_dst + j * kBoxBytesMN, &tmap_b, n0 + 32 * j, k0, full_bar(s));
+                        }
                     }
                     __syncwarp();
+                    if (++s == STAGES) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
             }
         } else if (warp == 1) {
@@ -597,12 +607,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     ptx::mbar_arrive(tmem_empty_bar(buf));
                 }
                 if (ok) {
-#pragma unroll
+                    // one copy of the code, the sums move down: unrolled, a launch's first tile waited for the instruction caches
+#pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
                         float v[32];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = acc[c * 32 + j];
+                        for (int j = 0; j < 32; ++j) v[j] = acc[j];
                         emit(v, row0, n0 + c * 32, split);
+#pragma unroll
+                        for (int j = 0; j < 96; ++j) acc[j] = acc[j + 32];
                     }
                 }
             } else {

@@ -516,8 +516,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     if (warp < 4) {
         if (C::kChunked) ptx::reg_dec<64>();
         if (warp == 0) {
-            // ------------------------------------------------------------ TMA producer (both CTAs)
+            // ------------------------------------------------------------ TMA producer (both CTAs): one elected lane issues
+            const bool issuer = ptx::elect_one();
             uint32_t it = 0;
+            uint32_t s = 0, ph = 0, j = 0, lph = 0;
             bool ok = true;
             PairWork work = my_work();
             int tm2, tn, kb0, kb1;
@@ -529,45 +531,50 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                                + (p.a_group_cols ? tn * BN / p.a_group_cols * p.a_group_rows : 0);
                 const int n0 = tn * BN + static_cast<int>(rank) * (p.mma_n ? p.mma_n / 2 : C::kBRows);   // the half of B this CTA loads
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
                     if (!bounded_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
                         ok = false;
                         break;
                     }
-                    if (lane == 0) trace(TRACE_LOAD_ISSUE, it);
-                    // TF32: every load of the pair reports to the leader's barrier, armed by the leader for both CTAs.
-                    // 3xTF32: each CTA's loads report to its own barrier (its converter warps wait on it).
-                    const uint32_t bar = X3 ? full_bar(s) : ptx::map_to_cta(full_bar(s), 0u);
-                    if (lane == 0 && (X3 || leader)) ptx::mbar_arrive_expect_tx(full_bar(s), (X3 ? 1u : 2u) * (kATileBytes + b_used));
-                    __syncwarp();
-                    const uint32_t a_dst = smem_base + s * C::kHiBytes;
-                    const uint32_t b_dst = a_dst + kATileBytes;
                     const int k0 = kb * kBK;
-                    if (p.batches > 0) {
-                        if (lane < kBoxesA) {
-                            if (A_MN)
-                                ptx::tma_load_4d_pair(a_dst + lane * kBoxBytesMN, &tmap_a, m0 + 32 * lane, zi, k0, zo, bar);
-                            else
+                    if (issuer) {
+                        trace(TRACE_LOAD_ISSUE, it);
+                        // TF32: every load of the pair reports to the leader's barrier, armed by the leader for both CTAs.
+                        // 3xTF32: each CTA's loads report to its own barrier (its converter warps wait on it).
+                        const uint32_t bar = X3 ? full_bar(s) : ptx::map_to_cta(full_bar(s), 0u);
+                        if (X3 || leader) ptx::mbar_arrive_expect_tx(full_bar(s), (X3 ? 1u : 2u) * (kATileBytes + b_used));
+                        const uint32_t a_dst = smem_base + s * C::kHiBytes;
+                        const uint32_t b_dst = a_dst + kATileBytes;
+                        if (p.batches > 0) {
+                            if (!A_MN)
                                 ptx::tma_load_4d_pair(a_dst, &tmap_a, k0, zi, m0, zo, bar);
-                        } else if (lane < kBoxesA + (B_MN ? static_cast<int>(b_boxes) : 1)) {
-                            const int j = lane - kBoxesA;
-                            if (B_MN)
-                                ptx::tma_load_4d_pair(b_dst + j * kBoxBytesMN, &tmap_b, n0 + 32 * j, zi, k0, zo, bar);
+                            else if (p.a_one_load)
+                                ptx::tma_load_5d_pair(a_dst, &tmap_a, 0, k0, m0 / 32, zi, zo, bar);
                             else
+#pragma unroll 1
+                                for (int i = 0; i < kBoxesA; ++i) ptx::tma_load_4d_pair(a_dst + i * kBoxBytesMN, &tmap_a, m0 + 32 * i, zi, k0, zo, bar);
+                            if (!B_MN)
                                 ptx::tma_load_4d_pair(b_dst, &tmap_b, k0, zi, n0, zo, bar);
+                            else if (p.b_one_load)
+                                ptx::tma_load_5d_pair(b_dst, &tmap_b, 0, k0, n0 / 32, zi, zo, bar);
+                            else
+#pragma unroll 1
+                                for (uint32_t i = 0; i < b_boxes; ++i) ptx::tma_load_4d_pair(b_dst + i * kBoxBytesMN, &tmap_b, n0 + 32 * i, zi, k0, zo, bar);
+                        } else {
+                            if (!A_MN)
+                                ptx::tma_load_2d_pair(a_dst, &tmap_a, k0, m0, bar);
+                            else if (p.a_one_load)
+                                ptx::tma_load_3d_pair(a_dst, &tmap_a, 0, k0, m0 / 32, bar);
+                            else
+#pragma unroll 1
+                                for (int i = 0; i < kBoxesA; ++i) ptx::tma_load_2d_pair(a_dst + i * kBoxBytesMN, &tmap_a, m0 + 32 * i, k0, bar);
+                            if (!B_MN)
+                                ptx::tma_load_2d_pair(b_dst, &tmap_b, k0, n0, bar);
+                            else if (p.b_one_load)
+                                ptx::tma_load_3d_pair(b_dst, &tmap_b, 0, k0, n0 / 32, bar);
+                            else
+#pragma unroll 1
+                                for (int i = 0; i < kBoxesB; ++i) ptx::tma_load_2d_pair(b_dst + i * kBoxBytesMN, &tmap_b, n0 + 32 * i, k0, bar);
                         }
-                    } else if (lane < kBoxesA) {
-                        if (A_MN)
-                            ptx::tma_load_2d_pair(a_dst + lane * kBoxBytesMN, &tmap_a, m0 + 32 * lane, k0, bar);
-                        else
-                            ptx::tma_load_2d_pair(a_dst, &tmap_a, k0, m0, bar);
-                    } else if (lane < kBoxesA + kBoxesB) {
-                        const int j = lane - kBoxesA;
-                        if (B_MN)
-                            ptx::tma_load_2d_pair(b_dst + j * kBoxBytesMN, &tmap_b, n0 + 32 * j, k0, bar);
-                        else
-                            ptx::tma_load_2d_pair(b_dst, &tmap_b, k0, n0, bar);
                     }
                     __syncwarp();
                     if (X3 && p.pre_operand) {
@@ -575,26 +582,28 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         // bf16 matrix (64 k-positions per 32 k) into correction buffer j, bytes reported to the leader's conv[j].
                         //   K-major:  rows of the operand, 32 four-byte words (64 bf16) per k-block, 128-byte swizzle: one box;
                         //   MN-major: [64 k-positions x 64 rows-of-the-operand] atoms: one box per half of the CTA's 128 rows.
-                        const int j = it % NL;
-                        const uint32_t lph = (it / NL) & 1u;
                         if (!bounded_wait(lo_empty_bar(j), lph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
                             ok = false;
                             break;
                         }
-                        const bool pre_a = p.pre_operand == 1;
-                        const bool pre_mn = pre_a ? A_MN : B_MN;
-                        const int r0 = pre_a ? m0 : n0;   // first of this CTA's 128 rows (A) / columns (B)
-                        const uint32_t dst = lo_base + j * C::kHiBytes + (pre_a ? 0 : kATileBytes);
-                        const uint32_t cbar = ptx::map_to_cta(conv_bar(j), 0u);
-                        if (leader && lane == 0) ptx::mbar_arrive_expect_tx(conv_bar(j), 2 * kATileBytes);
-                        __syncwarp();
-                        if (pre_mn) {
-                            if (lane < 2) ptx::tma_load_2d_pair(dst + lane * 8192, &tmap_pre, (r0 + 64 * lane) / 2, 2 * k0, cbar);
-                        } else {
-                            if (lane == 0) ptx::tma_load_2d_pair(dst, &tmap_pre, k0, r0, cbar);
+                        if (issuer) {
+                            const bool pre_a = p.pre_operand == 1;
+                            const bool pre_mn = pre_a ? A_MN : B_MN;
+                            const int r0 = pre_a ? m0 : n0;   // first of this CTA's 128 rows (A) / columns (B)
+                            const uint32_t dst = lo_base + j * C::kHiBytes + (pre_a ? 0 : kATileBytes);
+                            const uint32_t cbar = ptx::map_to_cta(conv_bar(j), 0u);
+                            if (leader) ptx::mbar_arrive_expect_tx(conv_bar(j), 2 * kATileBytes);
+                            if (pre_mn) {
+                                ptx::tma_load_2d_pair(dst, &tmap_pre, r0 / 2, 2 * k0, cbar);
+                                ptx::tma_load_2d_pair(dst + 8192, &tmap_pre, (r0 + 64) / 2, 2 * k0, cbar);
+                            } else {
+                                ptx::tma_load_2d_pair(dst, &tmap_pre, k0, r0, cbar);
+                            }
                         }
                         __syncwarp();
                     }
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
+                    if (++j == NL) { j = 0; lph ^= 1u; }
                 }
             }
         } else if (warp == 1) {
@@ -908,12 +917,18 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                     if (ok) {
                         dbias_write();
                         if (e == 0 && lane == 0) trace(TRACE_EPI_BEGIN, tile_count);
-#pragma unroll
+                        // One copy of the code, the sums (and the bias) move down.  Unrolled, a launch's first tile took 36 000 cycles, the later ones
+                        // 12 000: the straight-line code of four pieces comes through the instruction caches of all SMs at the same time.
+#pragma unroll 1
                         for (int c = 0; c < 4; ++c) {
                             float v[32];
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = acc[c * 32 + j];
-                            emit(v, row0, n0 + c * 32, bias_pre[c]);
+                            for (int j = 0; j < 32; ++j) v[j] = acc[j];
+                            emit(v, row0, n0 + c * 32, bias_pre[0]);
+#pragma unroll
+                            for (int j = 0; j < 96; ++j) acc[j] = acc[j + 32];
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) bias_pre[j] = bias_pre[j + 1];
                         }
                         if (e == 0 && lane == 0) trace(TRACE_EPI_END, tile_count);
                         ++tile_count;

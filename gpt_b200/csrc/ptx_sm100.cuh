@@ -137,6 +137,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int3
         : "memory");
 }
 
+// The same for a 3-D tensor map (x innermost).
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void *tmap, int32_t x, int32_t y, int32_t z, uint32_t bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        :
+        : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
+
 // CTA-pair form of the 2-D load: the data lands in this CTA's shared memory, the byte count is reported to
 // `cluster_bar`, which may be a barrier of the other CTA of the pair (address from map_to_cta).  No multicast.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void *tmap, int32_t x, int32_t y, uint32_t cluster_bar)
@@ -145,6 +155,25 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void *tmap,
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         :
         : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(cluster_bar)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void *tmap, int32_t x, int32_t y, int32_t z, uint32_t cluster_bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        :
+        : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(cluster_bar)
+        : "memory");
+}
+
+// 5-D: batched operands whose tile is several columns of boxes (column in the box, row, box column, inner batch index, outer batch index).
+__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const void *tmap, int32_t x, int32_t y, int32_t z, int32_t v, int32_t w, uint32_t cluster_bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+        :
+        : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(v), "r"(w), "r"(cluster_bar)
         : "memory");
 }
 
