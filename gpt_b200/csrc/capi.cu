@@ -14,6 +14,7 @@
 #include "ctx_internal.h"
 #include "gemm_plan.h"
 #include "gemm_sm100.cuh"
+#include "gemm_bf16_sm100.cuh"
 #include "gemm_sm100_pair.cuh"
 #include "skinny_sm100.cuh"
 #include "gemv_bf16.cuh"
@@ -798,6 +799,57 @@ int launch_gemv(gptb200_ctx *ctx, void (*kernel)(GemvParams), const GemvParams &
     return GPTB200_OK;
 }
 
+template <int BN, int FORM>
+int launch_bf16_pair(gptb200_ctx *ctx, const CUtensorMap &ta, const CUtensorMap &tw, const CUtensorMap &to, const Bf16GemmParams &p, int pairs)
+{
+    using C = Bf16Cfg<BN>;
+    auto kernel = gemm_bf16_pair_kernel<BN, FORM>;
+    const void *key = reinterpret_cast<const void *>(kernel);
+    if (!ctx->configured.count(key)) {
+        CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+        ctx->configured.insert(key);
+    }
+    ctx->launches++;
+    kernel<<<2 * pairs, C::kThreads, C::kSmemBytes, ctx->stream>>>(ta, tw, to, p);
+    CUDA_TRY(ctx, cudaGetLastError());
+    return GPTB200_OK;
+}
+
+template <int BN>
+int launch_bf16_form(gptb200_ctx *ctx, int form, const CUtensorMap &ta, const CUtensorMap &tw, const CUtensorMap &to, const Bf16GemmParams &p, int pairs)
+{
+    if (form == BF16_F32) return launch_bf16_pair<BN, BF16_F32>(ctx, ta, tw, to, p, pairs);
+    if (form == BF16_PLAIN) return launch_bf16_pair<BN, BF16_PLAIN>(ctx, ta, tw, to, p, pairs);
+    if (form == BF16_FACTOR) return launch_bf16_pair<BN, BF16_FACTOR>(ctx, ta, tw, to, p, pairs);
+    if constexpr (BN >= 128) return launch_bf16_pair<BN, BF16_GLU>(ctx, ta, tw, to, p, pairs);
+    return fail(ctx, GPTB200_ERR_INVALID_ARG, "bf16 product: gated columns in tiles of %d", BN);
+}
+
+int run_bf16_pairs(gptb200_ctx *ctx, const Bf16Linear &c, int bn, long long out_words, long long ldo_words)
+{
+    const int form = c.out_kind == OUT_F32 ? BF16_F32 : c.out_kind == OUT_BF16 ? BF16_PLAIN : c.out_kind == OUT_GELU_MUL ? BF16_FACTOR : BF16_GLU;
+    const int sms = ctx->max_sms > 0 ? std::min(ctx->max_sms, ctx->num_sms) : ctx->num_sms;
+    Bf16GemmParams p{};
+    p.M = c.M; p.N = c.N; p.num_kb = (c.K + 63) / 64;
+    p.tiles_m = (c.M + 255) / 256; p.tiles_n = (c.N + bn - 1) / bn;
+    p.status = ctx->d_status;
+    p.bias = c.bias;
+    p.glu = c.out_kind;
+    p.tail = c.tail; p.tail_col = c.tail_col; p.tail_pitch = c.tail_pitch;
+    p.silu_cols = c.silu_cols;
+    p.factor = static_cast<const uint16_t *>(c.factor); p.factor_rows = c.factor_rows; p.factor_pitch = c.factor_pitch;
+    p.a_group_cols = c.group_cols; p.a_group_rows = c.group_rows;
+    CUtensorMap ta, tw, to;
+    const long long a_rows = c.group_cols ? (c.N + c.group_cols - 1LL) / c.group_cols * c.group_rows : c.M;
+    int rc = make_word_tmap(ctx, &ta, c.a, a_rows, c.K / 2, c.lda / 2, kBK, kBM, false);
+    if (rc == GPTB200_OK) rc = make_word_tmap(ctx, &tw, c.w, c.N, c.K / 2, c.K / 2, kBK, bn / 2, false);
+    if (rc == GPTB200_OK) rc = make_word_tmap(ctx, &to, c.out, c.M, out_words, ldo_words, bf16_out_box(bn, form), 32, true);
+    if (rc != GPTB200_OK) return rc;
+    const int pairs = static_cast<int>(std::min<long long>(std::max(1, sms / 2), 1LL * p.tiles_m * p.tiles_n));
+    return bn == 256 ? launch_bf16_form<256>(ctx, form, ta, tw, to, p, pairs)
+         : bn == 128 ? launch_bf16_form<128>(ctx, form, ta, tw, to, p, pairs) : launch_bf16_form<64>(ctx, form, ta, tw, to, p, pairs);
+}
+
 int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
 {
     if (c.M <= 0 || c.N <= 0) return GPTB200_OK;
@@ -827,16 +879,20 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
     const long long out_words = f32 ? c.N : is_glu(c.out_kind) ? c.N / 4 : (std::min(c.N, c.tail_col) + 1) / 2;
     const long long ldo_words = f32 ? c.ldo : c.ldo / 2;
     if (ldo_words % 4 || c.ldo % 2) return fail(ctx, GPTB200_ERR_INVALID_ARG, "bf16 product: output pitch %lld", c.ldo);
+    const int sms = ctx->max_sms > 0 ? std::min(ctx->max_sms, ctx->num_sms) : ctx->num_sms;
+    const Bf16Plan plan = plan_bf16(c.M, c.N, c.K, sms, is_glu(c.out_kind), f32 && !c.bias && c.ldo == c.N && !c.group_cols, ctx->ws_limit);
+    // options that ask for the one-CTA kernel or for its sizes
+    const bool one_cta = ctx->pair < 0 || (ctx->pair == 0 && (ctx->tile_n != 0 || ctx->max_splits != 0 || plan.split_k));
+    if (!one_cta) return run_bf16_pairs(ctx, c, plan.columns, out_words, ldo_words);
     GemmPlanInput in{};
     in.M = c.M; in.N = (c.N + 3) & ~3; in.K = c.K / 2;      // in 4-byte words: a k-block of 32 words is 64 bf16
     in.has_epilogue = !f32 || c.bias || c.ldo != c.N || c.N % 4 != 0;   // split-K adds contiguous fp32 partial sums
     in.aligned = true;
-    in.num_sms = ctx->max_sms > 0 ? std::min(ctx->max_sms, ctx->num_sms) : ctx->num_sms;
-    in.opt_tile_n = ctx->tile_n; in.opt_max_splits = ctx->max_splits; in.opt_pair = ctx->pair; in.opt_stream_k = ctx->stream_k;
+    in.num_sms = sms;
+    in.opt_tile_n = ctx->tile_n; in.opt_max_splits = ctx->max_splits; in.opt_pair = -1;
     in.ws_limit = ctx->ws_limit;
     const GemmPlan pl = plan_gemm(in);
-    const bool pair = pl.kernel == KERNEL_PAIR;
-    if (!pair && pl.kernel != KERNEL_SINGLE) return fail(ctx, GPTB200_ERR_INVALID_ARG, "bf16 product: no kernel for M=%d N=%d K=%d", c.M, c.N, c.K);
+    if (pl.kernel != KERNEL_SINGLE) return fail(ctx, GPTB200_ERR_INVALID_ARG, "bf16 product: no kernel for M=%d N=%d K=%d", c.M, c.N, c.K);
     GemmParams p{};
     p.M = c.M; p.N = c.N; p.K = in.K;
     p.tiles_m = pl.tiles_m; p.tiles_n = pl.tiles_n; p.num_kb = pl.num_kb; p.kb_per_split = pl.kb_per_split; p.splits = pl.splits;
@@ -849,17 +905,7 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
     p.a_group_cols = c.group_cols; p.a_group_rows = c.group_rows;
     p.epi_mode = EPI_STORE;
     float *out_base = static_cast<float *>(c.out);
-    if (pair) {
-        p.sk_total = pl.sk_total;
-        p.sk_unit = pl.sk_unit;
-        if (pl.sk_max_share > 1) {
-            const int rc = ensure_workspace(ctx, pl.workspace_bytes);
-            if (rc != GPTB200_OK) return rc;
-            p.sk_slots = ctx->ws;
-            p.sk_flags = ctx->d_pair_flags;
-            p.sk_state = ctx->d_pair_flags + size_t(ctx->num_sms) * 8;
-        }
-    } else if (pl.splits > 1) {
+    if (pl.splits > 1) {
         const int rc = ensure_workspace(ctx, size_t(c.M) * c.N * sizeof(float) * pl.splits);
         if (rc != GPTB200_OK) return rc;
         out_base = ctx->ws;
@@ -868,14 +914,12 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
     CUtensorMap ta, tb, to;
     const long long a_rows = c.group_cols ? (c.N + c.group_cols - 1LL) / c.group_cols * c.group_rows : c.M;
     int rc = make_word_tmap(ctx, &ta, c.a, a_rows, c.K / 2, c.lda / 2, kBK, kBM, false);
-    if (rc == GPTB200_OK) rc = make_word_tmap(ctx, &tb, c.w, c.N, c.K / 2, c.K / 2, kBK, pair ? pl.tile_n / 2 : pl.tile_n, false);
+    if (rc == GPTB200_OK) rc = make_word_tmap(ctx, &tb, c.w, c.N, c.K / 2, c.K / 2, kBK, pl.tile_n, false);
     if (rc == GPTB200_OK && pl.splits > 1) rc = make_out_tmap(ctx, &to, out_base, pl.splits, c.M, c.N);
     if (rc == GPTB200_OK && pl.splits <= 1) rc = make_word_tmap(ctx, &to, c.out, c.M, out_words, ldo_words, f32 ? 32 : 16, 32, true);
     if (rc != GPTB200_OK) return rc;
     cudaError_t e;
-    if (pair)
-        e = launch_pair_instance<false, false, false>(ctx, ta, tb, to, to, to, p, pl.grid);
-    else if (pl.tile_n == 256)
+    if (pl.tile_n == 256)
         e = launch_instance<256, false, false, false>(ctx, ta, tb, to, to, p, pl.grid);
     else
         e = launch_instance<128, false, false, false>(ctx, ta, tb, to, to, p, pl.grid);

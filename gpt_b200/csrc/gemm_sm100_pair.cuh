@@ -527,8 +527,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 const int z = p.batches > 0 ? tn / p.tiles_n : 0;                     // batched form: the tile columns of all batches are numbered through
                 if (p.batches > 0) tn -= z * p.tiles_n;
                 const int zi = p.batches > 0 ? z % p.batch_inner : 0, zo = p.batches > 0 ? z / p.batch_inner : 0;
-                const int m0 = tm2 * 2 * kBM + static_cast<int>(rank) * kBM           // the rows this CTA owns
-                               + (p.a_group_cols ? tn * BN / p.a_group_cols * p.a_group_rows : 0);
+                const int m0 = tm2 * 2 * kBM + static_cast<int>(rank) * kBM;          // the rows this CTA owns
                 const int n0 = tn * BN + static_cast<int>(rank) * (p.mma_n ? p.mma_n / 2 : C::kBRows);   // the half of B this CTA loads
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     if (!bounded_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
@@ -662,14 +661,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                                     for (int k = 0; k < 4; ++k)
                                         ptx::mma_f16_ss_pair(d_tmem, corr_a.at(cor + k * a_corr_step), corr_b.at(cor + k * b_corr_step), idesc_corr, k ? 1u : accumulate);
                                 }
-                                if (!A_MN && !B_MN && !X3 && p.bf16) {
 #pragma unroll
-                                    for (int k = 0; k < 4; ++k) ptx::mma_f16_ss_pair(d_tmem, desc_a.at(raw + k * 32), desc_b.at(raw + k * 32), idesc_corr, k ? 1u : accumulate);
-                                } else {
-#pragma unroll
-                                    for (int k = 0; k < kBK / kUmmaK; ++k)
-                                        ptx::mma_tf32_ss_pair(d_tmem, desc_a.at(raw + k * a_step), desc_b.at(raw + k * b_step), idesc, X3 || k ? 1u : accumulate);
-                                }
+                                for (int k = 0; k < kBK / kUmmaK; ++k)
+                                    ptx::mma_tf32_ss_pair(d_tmem, desc_a.at(raw + k * a_step), desc_b.at(raw + k * b_step), idesc, X3 || k ? 1u : accumulate);
                                 // the stage is free in both CTAs once these MMAs have read it
                                 ptx::mma_commit_pair_both(empty_bar(s), 3);
                                 if (X3) ptx::mma_commit_pair_both(lo_empty_bar(j), 3);
@@ -710,28 +704,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         const uint32_t leader_tmem_empty[2] = {ptx::map_to_cta(tmem_empty_bar(0), 0u), ptx::map_to_cta(tmem_empty_bar(1), 0u)};
 
         int ezi = 0, ezo = 0;   // batched form: batch coordinates of the tile being written
-        float held[32];   // bf16 form: gate columns of the gated kinds
         // bias_lane: bias[col0 + lane], fetched when the tile was started
         auto emit = [&](float (&v)[32], int row0, int col0, float bias_lane) {
-            if constexpr (!A_MN && !B_MN && !X3) {
-                if (p.out_kind != OUT_F32) {
-                    uint32_t w[16];
-                    int word0;
-                    const bool some = piece_to_bf16(p, v, held, row0, col0, lane, w, word0);
-                    if (__any_sync(0xffffffffu, some)) {
-                        const uint32_t buf = ring.acquire(lane);
-                        stage_row_bf16(buf, lane, w);
-                        ptx::fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            ptx::tma_store_3d(&tmap_act, word0, row0, 0, buf);
-                            ptx::tma_store_commit();
-                        }
-                        ring.count++;
-                    }
-                    return;
-                }
-            }
             if (p.mma_n && col0 >= p.mma_n) return;   // narrow batched form: these accumulator columns were not computed
             if (p.causal_skip && col0 > row0 + 31) return;   // nobody reads these
             if (p.bias && p.epi_mode == EPI_STORE) {

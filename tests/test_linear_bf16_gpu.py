@@ -102,6 +102,45 @@ def test_forced_kernels(backend, option, value):
         backend.set_option(option, 8 if option == "gemv_rows" else 0)
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (255, 9536, 1024),     # tiles of 256 columns, the last one of 64; sums of one hand-off of the accumulator
+    (513, 9664, 1032),     # ... two waves, a k-block of 8 behind the hand-off
+    (257, 4160, 2056),     # 128 columns: three hand-offs, a last tile of 64 columns
+    (9, 4672, 2048),       # 64 columns, rows of one warp
+    (320, 2112, 72),       # ... one k-block and a piece of one
+])
+def test_pair_tiles(backend, m, n, k):
+    """Tile edges and hand-offs of the CTA-pair kernel in every form; the fp32 sums are chains of at most 64 truncating additions between round-to-nearest ones,
+    each off by at most 2^-23 of the running sum, below 1e-5 of the largest."""
+    torch.manual_seed(m + n + k)
+    x, w = torch.randn(m, k, device="cuda").bfloat16(), (torch.randn(n, k, device="cuda") / k ** 0.5).bfloat16()
+    ref = (x.double() @ w.double().T).float()
+    backend.set_option("pair", 1)
+    try:
+        out = torch.full((m + 1, n), 77.0, device="cuda")
+        run(backend, 0, out, x, w, n)
+        close(out[:m], ref, 1e-5)
+        assert (out[m] == 77).all()
+        cut = n - 96
+        out, tail = torch.full((m + 1, cut + 8), 77.0, device="cuda", dtype=torch.bfloat16), torch.full((m + 1, 96), 77.0, device="cuda")
+        run(backend, 1, out, x, w, n, tail=tail, tail_col=cut)
+        close(out[:m, :cut], ref[:, :cut], 5e-3)
+        close(tail[:m], ref[:, cut:], 1e-5)
+        assert (out[:, cut:] == 77).all() and (out[m] == 77).all() and (tail[m] == 77).all()
+        g = ref.view(m, n // 64, 2, 32)
+        out = torch.full((m + 1, n // 2), 77.0, device="cuda", dtype=torch.bfloat16)
+        run(backend, 4, out, x, w, n)
+        close(out[:m], (torch.nn.functional.silu(g[:, :, 0]) * g[:, :, 1]).reshape(m, n // 2), 5e-3)
+        assert (out[m] == 77).all()
+        factor, rows = torch.randn(5, n, device="cuda").bfloat16(), torch.randint(0, 5, (m,), device="cuda", dtype=torch.int32)
+        out = torch.full((m + 1, n), 77.0, device="cuda", dtype=torch.bfloat16)
+        run(backend, 3, out, x, w, n, factor=factor, rows=rows)
+        close(out[:m], gelu(ref) * factor[rows.long()].float(), 5e-3)
+        assert (out[m] == 77).all()
+    finally:
+        backend.set_option("pair", 0)
+
+
 def test_wrong_sizes_are_refused(backend):
     from gpt_b200 import decoder
     lib = decoder.load_library()
