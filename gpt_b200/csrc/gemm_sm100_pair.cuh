@@ -120,6 +120,8 @@ struct PairCfg {
 //   k-position), the 8 atoms of a 64-row half one after the other, 8 KiB to the other half.
 //   K-major raw tile: 128-byte rows (32 k), 16-byte chunks XOR-ed with (row & 7); piece p holds rows 8 p .. 8 p + 7.  The
 //   bf16 tile has the same geometry and swizzle.  Odd rows start with the odd chunk, which is also the logically first.
+constexpr int kPairConvWarps = 6;   // warps 2, 3 and the last four
+
 struct ConvLane {
     uint32_t src, dst_even, dst_odd;
 };
@@ -184,14 +186,14 @@ __device__ __forceinline__ void convert_store(float4 f1, float4 f2, uint32_t dst
     }
 }
 
-// The pieces first, first + 3, ... (< 16) of one operand tile.  Deliberately a rolled loop: the kernel's code is large
+// The pieces first, first + 6, ... (< 16) of one operand tile.  Deliberately a rolled loop: the kernel's code is large
 // (the unrolled epilogue above all) and the converter warps were measured to run faster with a compact body than with
 // unrolled or load-batched ones.
 template <bool MN, bool IS_B>
 __device__ __forceinline__ void convert_tile(uint32_t raw, uint32_t cor, const ConvLane &c, int first, int lane)
 {
 #pragma unroll 1
-    for (int p = first; p < 16; p += 3) {
+    for (int p = first; p < 16; p += kPairConvWarps) {
         const uint32_t src = raw + c.src + conv_src_offset<MN>(p);
         const float4 f1 = ptx::lds128(src), f2 = ptx::lds128(src ^ 16u);
         convert_store<MN, IS_B>(f1, f2, cor + ((p & 1) ? c.dst_odd : c.dst_even) + conv_dst_offset<MN>(p), lane);
@@ -404,9 +406,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             ptx::mbar_init(empty_bar(s), 1);
         }
         for (int j = 0; j < NL; ++j) {
-            // leader: one arrival per converter warp (three of each CTA) of the group that owns the buffer, plus the producer's
-            // arrival that announces the bytes of a correction tile fetched by TMA (pre_operand)
-            ptx::mbar_init(conv_bar(j), (X3 && p.pre_operand) ? 7 : 6);
+            // leader: one arrival per converter warp of either CTA, plus the producer's arrival that announces the bytes of a correction tile fetched by TMA (pre_operand)
+            ptx::mbar_init(conv_bar(j), 2 * kPairConvWarps + (X3 && p.pre_operand ? 1 : 0));
             ptx::mbar_init(lo_empty_bar(j), 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -455,13 +456,13 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         return w;
     };
 
-    // 3xTF32 converters: six warps (warps 2, 3 and the last four) in two groups of three; group g handles the
-    // k-blocks with (iteration & 1) == g, so that waking up, converting and signalling one stage overlaps with
-    // the other group's stage.
-    auto convert_loop = [&](int group, int wgrp) {
-        // A stage is 32 warp-sized pieces (32 units of 8 floats): 16 of the A tile, 16 of the B tile.  The three warps of a
-        // group take every third piece of A and, starting one warp later, every third piece of B (11, 11 and 10 pieces).
-        const int wgrp_b = (wgrp + 2) % 3;
+    // 3xTF32 converters: all six warps share every k-block.  With three raw stages what counts is how long a stage lives (loads 1 100 cycles, conversion, 1 050
+    // of instructions): two groups of three that alternate k-blocks convert as many per second, but each takes twice as long (output layer forward at
+    // 2048 rows 590 us against 505, QKV forward + backward at 8192 rows 329 against 316).  Loading the next piece ahead of the conversion was slower.
+    auto convert_loop = [&](int w) {
+        // A stage is 32 warp-sized pieces (32 units of 8 floats): 16 of the A tile, 16 of the B tile.  A warp takes every sixth piece of A and, starting two
+        // warps later, every sixth piece of B (five or six pieces in all).
+        const int w_b = (w + 2) % kPairConvWarps;
         const ConvLane lane_a = conv_lane<A_MN>(lane, 0u);
         const ConvLane lane_b = conv_lane<B_MN>(lane, kATileBytes);
         uint32_t it = 0;
@@ -470,7 +471,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         int tm2, tn, kb0, kb1;
         while (ok && work.next(tm2, tn, kb0, kb1)) {
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                if (static_cast<int>(it & 1u) != group) continue;
                 const int s = it % STAGES;
                 const uint32_t ph = (it / STAGES) & 1u;
                 const int j = it % NL;
@@ -481,13 +481,13 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                     ok = false;
                     break;
                 }
-                if (wgrp == 0 && lane == 0) trace(TRACE_CONV_BEGIN, it);
+                if (w == 0 && lane == 0) trace(TRACE_CONV_BEGIN, it);
                 const uint32_t raw = smem_base + s * C::kHiBytes;
                 const uint32_t cor = lo_base + j * C::kHiBytes;
                 if (p.exact3x) {
-                    // low parts as fp32 tiles in the raw tiles' own layout: every 16-byte piece of the stage, a third per warp
+                    // low parts as fp32 tiles in the raw tiles' own layout: every 16-byte piece of the stage, a sixth per warp
 #pragma unroll 1
-                    for (uint32_t idx = wgrp * 32 + lane; idx < (kATileBytes + b_used) / 16; idx += 96) {
+                    for (uint32_t idx = w * 32 + lane; idx < (kATileBytes + b_used) / 16; idx += 32 * kPairConvWarps) {
                         const uint32_t off = idx * 16;   // the A tile, then the part of the B tile that the instruction reads
                         float4 v = ptx::lds128(raw + off);
                         v.x -= __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u);
@@ -497,8 +497,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         ptx::sts128(cor + off, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
                     }
                 } else {
-                    if (p.pre_operand != 1) convert_tile<A_MN, false>(raw, cor, lane_a, wgrp, lane);
-                    if (p.pre_operand != 2) convert_tile<B_MN, true>(raw, cor, lane_b, p.pre_operand ? wgrp : wgrp_b, lane);
+                    if (p.pre_operand != 1) convert_tile<A_MN, false>(raw, cor, lane_a, w, lane);
+                    if (p.pre_operand != 2) convert_tile<B_MN, true>(raw, cor, lane_b, p.pre_operand ? w : w_b, lane);
                 }
                 ptx::fence_proxy_async_smem();
                 __syncwarp();
@@ -507,7 +507,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         ptx::mbar_arrive(conv_bar(j));
                     else
                         ptx::mbar_arrive_remote(ptx::map_to_cta(conv_bar(j), 0u));
-                    if (wgrp == 0) trace(TRACE_CONV_END, it);
+                    if (w == 0) trace(TRACE_CONV_END, it);
                 }
             }
         }
@@ -684,7 +684,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             }
             __syncwarp();
         } else if (X3) {
-            convert_loop(warp - 2, 0);   // warps 2 and 3: first warp of converter group 0 and 1
+            convert_loop(warp - 2);
         }
     } else if (warp < kFirstConvWarp) {
         // ------------------------------------------------------------ epilogue (both CTAs, own 128 rows)
@@ -971,8 +971,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     } else if (X3) {
         // ------------------------------------------------------------ 3xTF32 converters (last four warps)
         ptx::reg_dec<64>();
-        const int j = warp - kFirstConvWarp;
-        convert_loop(j >> 1, 1 + (j & 1));
+        convert_loop(2 + warp - kFirstConvWarp);
     }
 
     // ---------------------------------------------------------------- teardown
