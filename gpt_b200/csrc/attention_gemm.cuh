@@ -10,6 +10,8 @@
 #include <cfloat>
 #include <cuda_runtime.h>
 
+#include "ptx_sm100.cuh"
+
 namespace gptb200 {
 namespace ops {
 
@@ -21,6 +23,8 @@ template <int CHUNKS>
 __global__ void __launch_bounds__(kScoreRowsPerBlock * 32)
 attention_scores_softmax_kernel(float *__restrict__ s, float *__restrict__ logsumexp, int seq_len, int num_heads, float scale, long long rows)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     const int lane = threadIdx.x & 31;
     const long long r = 1LL * blockIdx.x * kScoreRowsPerBlock + (threadIdx.x >> 5);
     if (r >= rows) return;
@@ -74,6 +78,8 @@ __global__ void __launch_bounds__(kScoreRowsPerBlock * 32)
 attention_scores_backward_kernel(float *__restrict__ s, float *__restrict__ dp, const float *__restrict__ logsumexp, const float *__restrict__ dcache,
                                  int seq_len, int num_heads, float scale, long long rows)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     const int lane = threadIdx.x & 31;
     const long long r = 1LL * blockIdx.x * kScoreRowsPerBlock + (threadIdx.x >> 5);
     if (r >= rows) return;

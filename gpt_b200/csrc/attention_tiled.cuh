@@ -13,6 +13,8 @@
 #include <cstddef>
 #include <cuda_runtime.h>
 
+#include "ptx_sm100.cuh"
+
 namespace gptb200 {
 namespace ops {
 
@@ -190,6 +192,8 @@ attention64_forward_kernel(float *__restrict__ y, float *__restrict__ logsumexp,
 __global__ void attention64_rowsum_kernel(float *__restrict__ dcache, const float *__restrict__ grad_y, const float *__restrict__ y,
                                           long long rows, int d_model, int num_heads)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     const int lane = threadIdx.x & 31;
     const long long row = (1LL * blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= rows) return;   // whole warps leave together

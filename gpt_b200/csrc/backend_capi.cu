@@ -87,14 +87,14 @@ void layernorm_forward_warp(gptb200_ctx *ctx, float *y, float *means, float *var
                             const float *beta, int rows)
 {
     const int blocks = (rows + ops::kLnWarpsPerBlock - 1) / ops::kLnWarpsPerBlock;
-    ops::layernorm_forward_warp_kernel<VEC><<<blocks, ops::kLnWarpsPerBlock * 32, 0, ctx->stream>>>(y, means, vars, x, residual, gamma, beta, rows);
+    launch_chained(ctx, ops::layernorm_forward_warp_kernel<VEC>, dim3(blocks), dim3(ops::kLnWarpsPerBlock * 32), 0, y, means, vars, x, residual, gamma, beta, rows);
 }
 
 template <int VEC>
 void layernorm_backward_warp(gptb200_ctx *ctx, int blocks, float *gx, float *wg, float *wb, const float *gy, const float *gres, const float *x,
                              const float *means, const float *vars, const float *gamma, int rows)
 {
-    ops::layernorm_backward_warp_kernel<VEC><<<blocks, ops::kLnWarpsPerBlock * 32, 0, ctx->stream>>>(gx, wg, wb, gy, gres, x, means, vars, gamma, rows);
+    launch_chained(ctx, ops::layernorm_backward_warp_kernel<VEC>, dim3(blocks), dim3(ops::kLnWarpsPerBlock * 32), 0, gx, wg, wb, gy, gres, x, means, vars, gamma, rows);
 }
 
 // Row lengths the one-warp-per-row LayerNorm kernels cover.
@@ -106,7 +106,7 @@ int attention64_backward(gptb200_ctx *ctx, float *gqkv, float *dcache, const flo
     CUDA_TRY(ctx, allow_smem(ctx, ops::attention64_backward_dq_kernel, ops::kFaDqSmem));
     CUDA_TRY(ctx, allow_smem(ctx, ops::attention64_backward_dkv_kernel, ops::kFaDkvSmem));
     const long long rows = 1LL * batch * seq_len;
-    ops::attention64_rowsum_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, ctx->stream>>>(dcache, gy, y, rows, d, heads);
+    launch_chained(ctx, ops::attention64_rowsum_kernel, dim3(static_cast<unsigned>((rows + 7) / 8)), dim3(256), 0, dcache, gy, y, rows, d, heads);
     dim3 grid((seq_len + ops::kFaBlock - 1) / ops::kFaBlock, heads, batch);
     ops::attention64_backward_dq_kernel<<<grid, ops::kFaThreads, ops::kFaDqSmem, ctx->stream>>>(gqkv, dcache, lse, gy, qkv, seq_len, d, heads);
     ops::attention64_backward_dkv_kernel<<<grid, ops::kFaThreads, ops::kFaDkvSmem, ctx->stream>>>(gqkv, dcache, lse, gy, qkv, seq_len, d, heads);
@@ -155,11 +155,11 @@ template <typename... Args>
 void launch_scores_softmax(gptb200_ctx *ctx, int T, unsigned blocks, Args... args)
 {
     if (T <= 256)
-        ops::attention_scores_softmax_kernel<2><<<blocks, ops::kScoreRowsPerBlock * 32, 0, ctx->stream>>>(args...);
+        launch_chained(ctx, ops::attention_scores_softmax_kernel<2>, dim3(blocks), dim3(ops::kScoreRowsPerBlock * 32), 0, args...);
     else if (T <= 512)
-        ops::attention_scores_softmax_kernel<4><<<blocks, ops::kScoreRowsPerBlock * 32, 0, ctx->stream>>>(args...);
+        launch_chained(ctx, ops::attention_scores_softmax_kernel<4>, dim3(blocks), dim3(ops::kScoreRowsPerBlock * 32), 0, args...);
     else
-        ops::attention_scores_softmax_kernel<8><<<blocks, ops::kScoreRowsPerBlock * 32, 0, ctx->stream>>>(args...);
+        launch_chained(ctx, ops::attention_scores_softmax_kernel<8>, dim3(blocks), dim3(ops::kScoreRowsPerBlock * 32), 0, args...);
 }
 
 int attention_gemm_forward(gptb200_ctx *ctx, float *y, float *lse, const float *qkv, int batch, int seq_len, int d, int heads)
@@ -190,7 +190,7 @@ int attention_gemm_backward(gptb200_ctx *ctx, float *gqkv, float *dcache, const 
     const int T = seq_len, G = attention_group(ctx, batch, T, heads, 2);
     if (!attention_scratch(ctx, 2 * sizeof(float) * G * T * heads * T)) return -1;
     float *s = ctx->attn_ws, *dp = ctx->attn_ws + 1LL * G * T * heads * T;
-    ops::attention64_rowsum_kernel<<<static_cast<unsigned>((1LL * batch * T + 7) / 8), 256, 0, ctx->stream>>>(dcache, gy, y, 1LL * batch * T, d, heads);
+    launch_chained(ctx, ops::attention64_rowsum_kernel, dim3(static_cast<unsigned>((1LL * batch * T + 7) / 8)), dim3(256), 0, dcache, gy, y, 1LL * batch * T, d, heads);
     int rc = launched(ctx);
     if (rc) return rc;
     const long long sl = 1LL * heads * T, so = 1LL * T * heads * T, xo = 1LL * T * 3 * d;
@@ -204,7 +204,7 @@ int attention_gemm_backward(gptb200_ctx *ctx, float *gqkv, float *dcache, const 
         if (rc) return rc;
         const long long rows = 1LL * nb * T * heads;
         const unsigned blocks = static_cast<unsigned>((rows + ops::kScoreRowsPerBlock - 1) / ops::kScoreRowsPerBlock);
-        ops::attention_scores_backward_kernel<<<blocks, ops::kScoreRowsPerBlock * 32, 0, ctx->stream>>>(s, dp, lse + 1LL * b0 * T * heads,
+        launch_chained(ctx, ops::attention_scores_backward_kernel, dim3(blocks), dim3(ops::kScoreRowsPerBlock * 32), 0, s, dp, lse + 1LL * b0 * T * heads,
                                                                                                      dcache + 1LL * b0 * T * heads, T, heads, 0.125f, rows);
         rc = launched(ctx);
         if (rc) return rc;
@@ -323,7 +323,7 @@ int gptb200_layernorm_backward(gptb200_ctx *ctx, float *grad_x, float *grad_gamm
             case 7: layernorm_backward_warp<7>(ctx, blocks, grad_x, wg, wb, grad_y, grad_residual, x, means, vars, gamma, rows); break;
             default: layernorm_backward_warp<8>(ctx, blocks, grad_x, wg, wb, grad_y, grad_residual, x, means, vars, gamma, rows); break;
         }
-        ops::layernorm_backward_params_final_kernel<<<(d + 31) / 32, dim3(32, ops::kParamRows), 0, ctx->stream>>>(grad_gamma, grad_beta, wg, wb, d, blocks);
+        launch_chained(ctx, ops::layernorm_backward_params_final_kernel, dim3((d + 31) / 32), dim3(32, ops::kParamRows), 0, grad_gamma, grad_beta, wg, wb, d, blocks);
         return launched(ctx, 2);
     }
     const int threads = std::min(1024, std::max(32, ((d + 31) / 32) * 32));
@@ -337,7 +337,7 @@ int gptb200_layernorm_backward(gptb200_ctx *ctx, float *grad_x, float *grad_gamm
     float *wg = ctx->ws, *wb = ctx->ws + size_t(chunks) * d;
     ops::layernorm_backward_params_partial_kernel<<<dim3(col_groups, chunks), dim3(32, 8), 0, ctx->stream>>>(wg, wb, grad_y, x, means, vars,
                                                                                                              rows, d, rows_per_chunk);
-    ops::layernorm_backward_params_final_kernel<<<(d + 31) / 32, dim3(32, ops::kParamRows), 0, ctx->stream>>>(grad_gamma, grad_beta, wg, wb, d, chunks);
+    launch_chained(ctx, ops::layernorm_backward_params_final_kernel, dim3((d + 31) / 32), dim3(32, ops::kParamRows), 0, grad_gamma, grad_beta, wg, wb, d, chunks);
     return launched(ctx, 3);
 }
 

@@ -11,6 +11,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "ptx_sm100.cuh"
+
 namespace gptb200 {
 namespace ops {
 
@@ -238,6 +240,8 @@ constexpr int kParamRows = 32;
 __global__ void __launch_bounds__(32 * kParamRows)
 layernorm_backward_params_final_kernel(float *__restrict__ grad_gamma, float *__restrict__ grad_beta, const float *__restrict__ ws_gamma, const float *__restrict__ ws_beta, int d, int chunks)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     __shared__ float rg[kParamRows][33], rb[kParamRows][33];
     const int col = blockIdx.x * 32 + threadIdx.x;
     float sg = 0.0f, sb = 0.0f;

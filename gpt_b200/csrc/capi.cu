@@ -206,8 +206,7 @@ cudaError_t launch_instance(gptb200_ctx *ctx, const CUtensorMap &ta, const CUten
         if (e != cudaSuccess) return e;
         ctx->configured.insert(key);
     }
-    kernel<<<grid, C::kThreads, C::kSmemBytes, ctx->stream>>>(ta, tb, to, tact, p);
-    return cudaGetLastError();
+    return launch_chained(ctx, kernel, dim3(grid), dim3(C::kThreads), C::kSmemBytes, ta, tb, to, tact, p);
 }
 
 template <int BN, bool X3>
@@ -232,8 +231,7 @@ cudaError_t launch_pair_instance(gptb200_ctx *ctx, const CUtensorMap &ta, const 
         if (e != cudaSuccess) return e;
         ctx->configured.insert(key);
     }
-    kernel<<<grid, C::kThreads, C::kSmemBytes, ctx->stream>>>(ta, tb, to, tact, tpre, p);  // cluster shape (2,1,1) is a kernel attribute
-    return cudaGetLastError();
+    return launch_chained(ctx, kernel, dim3(grid), dim3(C::kThreads), C::kSmemBytes, ta, tb, to, tact, tpre, p);  // cluster shape (2,1,1) is a kernel attribute
 }
 
 template <bool X3>
@@ -665,9 +663,8 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
     if (splits > 1) {
         const long long n4 = (1LL * c.M * c.N) >> 2;
         const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, 1LL * ctx->num_sms * 8));
-        splitk_reduce_kernel<<<blocks, 256, 0, ctx->stream>>>(c.out, ctx->ws, n4, splits, c.accumulate ? 1 : 0);
         ctx->launches++;
-        CUDA_TRY(ctx, cudaGetLastError());
+    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, c.out, ctx->ws, n4, splits, c.accumulate ? 1 : 0));
     }
     return GPTB200_OK;
 }
@@ -682,12 +679,10 @@ int run_bias_grad(gptb200_ctx *ctx, float *gb, const float *gy, int M, int N)
     chunks = (M + rows_per_chunk - 1) / rows_per_chunk;
     const int rc = ensure_workspace(ctx, size_t(chunks) * N * sizeof(float));
     if (rc != GPTB200_OK) return rc;
-    bias_grad_partial_kernel<<<dim3(col_groups, chunks), dim3(32, 8), 0, ctx->stream>>>(ctx->ws, gy, M, N, rows_per_chunk);
     ctx->launches++;
-    CUDA_TRY(ctx, cudaGetLastError());
-    bias_grad_final_kernel<<<(N + 127) / 128, 128, 0, ctx->stream>>>(gb, ctx->ws, N, chunks);
+    CUDA_TRY(ctx, launch_chained(ctx, bias_grad_partial_kernel, dim3(col_groups, chunks), dim3(32, 8), 0, ctx->ws, gy, M, N, rows_per_chunk));
     ctx->launches++;
-    CUDA_TRY(ctx, cudaGetLastError());
+    CUDA_TRY(ctx, launch_chained(ctx, bias_grad_final_kernel, dim3((N + 127) / 128), dim3(128), 0, gb, ctx->ws, N, chunks));
     return GPTB200_OK;
 }
 
@@ -810,8 +805,7 @@ int launch_bf16_pair(gptb200_ctx *ctx, const CUtensorMap &ta, const CUtensorMap 
         ctx->configured.insert(key);
     }
     ctx->launches++;
-    kernel<<<2 * pairs, C::kThreads, C::kSmemBytes, ctx->stream>>>(ta, tw, to, p);
-    CUDA_TRY(ctx, cudaGetLastError());
+    CUDA_TRY(ctx, launch_chained(ctx, kernel, dim3(2 * pairs), dim3(C::kThreads), C::kSmemBytes, ta, tw, to, p));
     return GPTB200_OK;
 }
 
@@ -928,9 +922,8 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
     if (pl.splits > 1) {
         const long long n4 = (1LL * c.M * c.N) >> 2;
         const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, 1LL * ctx->num_sms * 8));
-        splitk_reduce_kernel<<<blocks, 256, 0, ctx->stream>>>(static_cast<float *>(c.out), ctx->ws, n4, pl.splits, 0);
         ctx->launches++;
-        CUDA_TRY(ctx, cudaGetLastError());
+    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, static_cast<float *>(c.out), ctx->ws, n4, pl.splits, 0));
     }
     return GPTB200_OK;
 }
@@ -1355,9 +1348,8 @@ int gptb200_gelu_backward(gptb200_ctx *ctx, float *grad_x, const float *grad_y, 
     if (total == 0) return GPTB200_OK;
     if (!grad_x || !grad_y || !x) return fail(ctx, GPTB200_ERR_INVALID_ARG, "null tensor pointer");
     const int blocks = static_cast<int>(std::min<long long>((total / 4 + 255) / 256 + 1, 1LL * ctx->num_sms * 16));
-    gelu_backward_kernel<<<blocks, 256, 0, ctx->stream>>>(grad_x, grad_y, x, total);
     ctx->launches++;
-    CUDA_TRY(ctx, cudaGetLastError());
+    CUDA_TRY(ctx, launch_chained(ctx, gelu_backward_kernel, dim3(blocks), dim3(256), 0, grad_x, grad_y, x, total));
     return GPTB200_OK;
 }
 

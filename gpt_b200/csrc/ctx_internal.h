@@ -112,6 +112,24 @@ inline int fail(gptb200_ctx *ctx, int code, const char *fmt, ...)
     return code;
 }
 
+// Launch of a kernel that begins with grid_dependency_wait: it may start, and set itself up, while the last blocks of its predecessor on the stream run.
+// Launch latency, barriers, TMEM and tensor maps were 4 of the 6.4 us that a product of one k-block takes.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(gptb200_ctx *ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // out[z] = a[z] . b[z] for inner * outer batches in one launch of the CTA-pair kernel (capi.cu).  Operands as stored: K-major
 // (rows = free extent, k columns) or MN-major (k rows, free extent as columns); ld = row pitch, stride_inner / stride_outer =
 // distance between consecutive inner / outer batches, all in floats.

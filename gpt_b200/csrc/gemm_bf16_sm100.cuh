@@ -106,6 +106,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     ptx::cluster_sync();   // the peer's barriers exist before anything is signalled across CTAs
     ptx::tc_fence_after();
     const uint32_t tmem_base = ptx::warp_uniform(*tmem_slot);
+    grid_dependency_wait();      // the set-up above overlaps the predecessor's last CTAs
+    if (threadIdx.x == 0) grid_dependency_launch();
 
     const int pairs = gridDim.x >> 1, pair = blockIdx.x >> 1, tiles = p.tiles_m * p.tiles_n;
 

@@ -374,6 +374,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = ptx::warp_uniform(*tmem_slot);
+    grid_dependency_wait();      // the set-up above overlaps the predecessor's last CTAs
+    if (threadIdx.x == 0) grid_dependency_launch();
 
     const long long num_items = 1LL * p.tiles_m * p.tiles_n * p.splits;
 
@@ -718,6 +720,8 @@ static __global__ void wait_timeout_selftest_kernel(int *status, long long limit
 // out[i] (+)= sum_s ws[s][i], fixed order s = 0..splits-1 (deterministic split-K reduction).
 static __global__ void splitk_reduce_kernel(float *__restrict__ out, const float *__restrict__ ws, long long n4, int splits, int accumulate)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     const long long stride = 1LL * gridDim.x * blockDim.x;
     for (long long i = 1LL * blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
         float4 acc = reinterpret_cast<const float4 *>(ws)[i];

@@ -431,6 +431,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     ptx::cluster_sync();   // the peer's barriers exist before anything is signalled across CTAs
     ptx::tc_fence_after();
     const uint32_t tmem_base = ptx::warp_uniform(*tmem_slot);
+    grid_dependency_wait();      // the set-up above overlaps the predecessor's last CTAs
+    if (threadIdx.x == 0) grid_dependency_launch();
 
     const int tiles_m2 = (p.tiles_m + 1) / 2;   // pairs of 128-row tiles
     // narrow batched form: only the first mma_n / 2 columns of this CTA's B tile are loaded, split and read (K-major: that many

@@ -14,9 +14,6 @@
 
 namespace gptb200 {
 
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 struct GemvParams {
     int M, N, K;            // K in elements, a multiple of 8
     const uint16_t *x;      // bf16 [M][ldx]

@@ -18,6 +18,8 @@ __device__ __forceinline__ float gelu_tanh_grad(float x)
 
 __global__ void gelu_backward_kernel(float *__restrict__ gx, const float *__restrict__ gy, const float *__restrict__ x, long long n)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     const long long stride = 1LL * gridDim.x * blockDim.x;
     const long long n4 = n >> 2;
     const bool vec_ok = ((reinterpret_cast<uintptr_t>(gx) | reinterpret_cast<uintptr_t>(gy) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
@@ -44,6 +46,8 @@ __global__ void gelu_backward_kernel(float *__restrict__ gx, const float *__rest
 // depend on scheduling.
 __global__ void bias_grad_partial_kernel(float *__restrict__ ws, const float *__restrict__ gy, int M, int N, int rows_per_chunk)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     __shared__ float red[8][33];
     const int col = blockIdx.x * 32 + threadIdx.x;
     const int chunk = blockIdx.y;
@@ -65,6 +69,8 @@ __global__ void bias_grad_partial_kernel(float *__restrict__ ws, const float *__
 
 __global__ void bias_grad_final_kernel(float *__restrict__ gb, const float *__restrict__ ws, int N, int chunks)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= N) return;
     float s = 0.0f;

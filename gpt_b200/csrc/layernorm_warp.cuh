@@ -9,6 +9,8 @@
 #include <cstddef>
 #include <cuda_runtime.h>
 
+#include "ptx_sm100.cuh"
+
 namespace gptb200 {
 namespace ops {
 
@@ -26,6 +28,8 @@ __global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
 layernorm_forward_warp_kernel(float *__restrict__ y, float *__restrict__ means, float *__restrict__ vars, float *__restrict__ x,
                               const float *__restrict__ residual, const float *__restrict__ gamma, const float *__restrict__ beta, int rows)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     constexpr int D = 128 * VEC;
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kLnWarpsPerBlock + (threadIdx.x >> 5);
@@ -82,6 +86,8 @@ layernorm_backward_warp_kernel(float *__restrict__ grad_x, float *__restrict__ w
                                const float *__restrict__ grad_y, const float *__restrict__ grad_residual, const float *__restrict__ x,
                                const float *__restrict__ means, const float *__restrict__ vars, const float *__restrict__ gamma, int rows)
 {
+    grid_dependency_wait();
+    grid_dependency_launch();
     constexpr int D = 128 * VEC;
     constexpr int kSlots = kLnWarpsPerBlock / 2;
     __shared__ __align__(16) float sum_g[kSlots][D], sum_b[kSlots][D];

@@ -9,6 +9,13 @@
 #include <cuda_runtime.h>
 
 namespace gptb200 {
+
+// Programmatic dependent launch: a kernel launched with the attribute may start while its predecessor on the stream still runs and waits here until that one
+// has completed and its writes are visible; the second call lets the successor start.  A kernel that makes the second call after the first one keeps the order
+// of the whole chain: its successor starts when everything before this kernel has completed.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 namespace ptx {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
