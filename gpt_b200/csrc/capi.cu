@@ -16,6 +16,7 @@
 #include "gemm_sm100.cuh"
 #include "gemm_bf16_sm100.cuh"
 #include "gemm_sm100_pair.cuh"
+#include "rows_sm100.cuh"
 #include "skinny_sm100.cuh"
 #include "gemv_bf16.cuh"
 #include "kernels_misc.cuh"
@@ -392,6 +393,106 @@ int launch_decode_tile(gptb200_ctx *ctx, const GemmCall &c, int cluster)
     return GPTB200_OK;
 }
 
+// Weights [k][n] in boxes of 32 k x 128 columns, as they are (rows_tensor_kernel).
+int make_plain_tmap(gptb200_ctx *ctx, CUtensorMap *map, const float *base, long long rows, long long cols)
+{
+    const TmapKey key{reinterpret_cast<uintptr_t>(base), cols, rows, 0, 128, 32, 10};
+    const auto hit = ctx->tmaps.find(key);
+    if (hit != ctx->tmaps.end()) {
+        *map = hit->second;
+        return GPTB200_OK;
+    }
+    cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * sizeof(float)};
+    cuuint32_t box[2] = {128, 32};
+    cuuint32_t estr[2] = {1, 1};
+    const CUresult r = ctx->encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    ctx->tmap_encodes++;
+    if (r != CUDA_SUCCESS) return fail(ctx, GPTB200_ERR_CUDA, "cuTensorMapEncodeTiled (rows) failed (%d) rows=%lld cols=%lld", int(r), rows, cols);
+    if (ctx->tmaps.size() >= kTmapCacheMax) ctx->tmaps.clear();
+    ctx->tmaps.emplace(key, *map);
+    return GPTB200_OK;
+}
+
+template <int MR, bool W_NK>
+int launch_rows_tensor(gptb200_ctx *ctx, const CUtensorMap &tw, const RowsParams &p, int ctas, int cluster)
+{
+    auto kernel = rows_tensor_kernel<MR, W_NK>;
+    constexpr int smem = rows_smem_bytes(MR);
+    const void *key = reinterpret_cast<const void *>(kernel);
+    if (!ctx->configured.count(key)) {
+        CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        ctx->configured.insert(key);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas, cluster);
+    cfg.blockDim = dim3(kRowsThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = cluster;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    ctx->launches++;
+    CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, tw, p));
+    return GPTB200_OK;
+}
+
+// How many clusters of this many blocks of the kernel above run at once: they lie within a GPC, so that it is fewer than SMs / size.  Asked once per context.
+int rows_clusters(gptb200_ctx *ctx, int size)
+{
+    if (ctx->rows_clusters[size] == 0) {
+        auto kernel = rows_tensor_kernel<64, false>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, size);
+        cfg.blockDim = dim3(kRowsThreads);
+        cfg.dynamicSmemBytes = rows_smem_bytes(64);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1;
+        attr[0].val.clusterDim.y = size;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem_bytes(64)) == cudaSuccess &&
+                        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess;
+        if (!ok) cudaGetLastError();   // a refused query must not surface as the next launch's error
+        ctx->rows_clusters[size] = ok && clusters > 0 ? clusters : -1;
+    }
+    return ctx->rows_clusters[size];
+}
+
+int run_rows_tensor(gptb200_ctx *ctx, const GemmCall &c)
+{
+    const bool nk = !c.b_mn;
+    RowsParams p{};
+    p.y = c.out; p.act = c.act; p.x = c.a; p.bias = c.bias;
+    p.M = c.M; p.N = c.N; p.K = c.K;
+    p.tiles = (c.N + 127) / 128;
+    p.status = ctx->d_status;
+    p.early = ctx->decode_early_launch ? 1 : 0;
+    // the largest cluster of which one per column tile runs at once; at least 32 of k each
+    int cluster = std::max(1, std::min({16, ctx->num_sms / p.tiles, (c.K + 31) / 32}));
+    while (cluster > 1 && rows_clusters(ctx, cluster) < p.tiles) --cluster;
+    p.slice = ((c.K + cluster - 1) / cluster + 15) / 16 * 16;
+    CUtensorMap tw;
+    const int rc = nk ? make_tmap(ctx, &tw, c.b, c.N, c.K, 32, 128, false) : make_plain_tmap(ctx, &tw, c.b, c.K, c.N);
+    if (rc != GPTB200_OK) return rc;
+    const int ctas = cluster > 1 ? p.tiles : std::min(p.tiles, ctx->num_sms);
+    if (c.M <= 16) return nk ? launch_rows_tensor<16, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<16, false>(ctx, tw, p, ctas, cluster);
+    if (c.M <= 32) return nk ? launch_rows_tensor<32, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<32, false>(ctx, tw, p, ctas, cluster);
+    return nk ? launch_rows_tensor<64, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<64, false>(ctx, tw, p, ctas, cluster);
+}
+
 // One-launch warp-per-row kernel for decode-shaped products with W stored [n][k] (see rowwise_gemv_kernel).
 template <int MR>
 int launch_rowwise(gptb200_ctx *ctx, const GemmCall &c)
@@ -426,6 +527,7 @@ int run_skinny(gptb200_ctx *ctx, const GemmCall &c, const GemmPlan &pl)
             default: return launch_decode_cluster<16>(ctx, c, d.cluster, d.groups);
         }
     }
+    if (d.kernel == DECODE_TILE_CLUSTER && ctx->skinny_tensor && ctx->skinny_rows == 0 && !c.fma_only) return run_rows_tensor(ctx, c);
     if (d.kernel == DECODE_TILE_CLUSTER) {
         if (w_kn) {
             if (d.rows == 16) return launch_decode_tile<16, false>(ctx, c, d.cluster);
@@ -1128,6 +1230,10 @@ int gptb200_ctx_set_option(gptb200_ctx *ctx, const char *key, int value)
     if (!strcmp(key, "skinny_tile_rows")) {
         if (value != 0 && value != 32 && value != 64) return fail(ctx, GPTB200_ERR_INVALID_ARG, "skinny_tile_rows must be 0, 32 or 64");
         ctx->skinny_tile_rows = value;
+        return GPTB200_OK;
+    }
+    if (!strcmp(key, "skinny_tensor")) {
+        ctx->skinny_tensor = value != 0;
         return GPTB200_OK;
     }
     if (!strcmp(key, "skinny_tile")) {

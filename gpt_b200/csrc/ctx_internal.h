@@ -59,6 +59,8 @@ struct gptb200_ctx {
     int skinny_cluster_rows = 8;   // ... for calls with at most this many rows
     int skinny_tile_rows = 0;      // that kernel's row tile beyond 32 rows: 0 or 64 = one tile of 64, 32 = row groups of 32
     bool skinny_tile = true;       // beyond that many rows: one-launch register-tiled cluster kernel (false: the k-split kernel)
+    bool skinny_tensor = true;     // those calls run on the tensor cores with three bf16 parts per operand (false: the fp32 FMA kernel)
+    int rows_clusters[17] = {};    // clusters of that kernel, by size, that run at once (0: not asked yet, -1: none)
     int gemv_rows = 8;             // bf16 products: most rows the weight-streaming kernel takes (0 .. 8)
     int decode_early_launch = 0;     // that kernel is launched with programmatic stream serialization: it prefetches weights while
                                        // its predecessor on the stream still runs (caller's promise: the predecessor does not write them)

@@ -1,0 +1,444 @@
+// Products of 9 to 64 rows of fp32 with a weight matrix stored [k][n] (linear layers) or [n][k] (un-embedding, grad_x): y[m][n] = x[m][k] . w, bias and GELU,
+// on the tensor cores and no less exact than fp32 FMAs.
+//
+// Both operands are split exactly into three bf16 values (8 + 8 + 8 bits: the first truncated, the others rounded), and the six products of 2^-16 and more
+// are added: what is left out is 2^-24 of a product and less.  The tensor core adds into its accumulator with truncation, so the accumulator is handed to fp32
+// sums in registers (round to nearest) after every kRowsChunk steps of 16 k.  Infinite inputs give NaN, as in the products of more rows.
+//
+// A block computes 128 columns for all rows over its share of k.  The weights are the M = 128 operand; split, they never go back to shared memory: the converter
+// warps write them to TMEM, where the instructions take their A operand from.
+//   warps 0-7    converters: 16 k of the landed tile (lane = column) -> three bf16 pairs of 8 TMEM columns; the two groups of four alternate
+//   warps 8-15   sums: accumulator -> registers, half of the rows each
+//   warps 16-19  x: global -> three bf16 tiles of 64 k in shared memory (B operand)
+//   warp 20      TMA producer: 32 KB of weights per 64 k, four stages
+//   warp 21      issues the instructions
+// The un-embedding has enough column tiles for all SMs (blocks walk over them); narrow layers share k in a cluster, partial tiles meet in rank order through
+// distributed shared memory.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "gemm_sm100.cuh"
+
+namespace gptb200 {
+
+#ifndef GPTB200_ROWS_CHUNK
+#define GPTB200_ROWS_CHUNK 1
+#endif
+constexpr int kRowsChunk = GPTB200_ROWS_CHUNK;
+constexpr int kRowsThreads = 22 * 32;
+constexpr int kRowsStages = 4, kRowsStageBytes = 128 * 64 * 4;
+constexpr int kRowsSlots = 8, kRowsSlotCols = 24;      // split weights of 16 k: 3 x 8 TMEM columns
+constexpr int kRowsAccCols = 64;
+constexpr int kRowsSlotBase = 2 * kRowsAccCols;
+constexpr int kRowsXBufs = 2;
+
+struct RowsParams {
+    float *y, *act;            // act: null, or gelu(y)
+    const float *x, *bias;     // bias: null for none
+    int M, N, K;
+    int slice;                 // k per block of a cluster, a multiple of 16
+    int tiles;                 // of 128 columns
+    int *status;
+    int early;                 // weights may be read before the predecessor on the stream has completed
+};
+
+constexpr int rows_smem_bytes(int mr) { return kRowsStages * kRowsStageBytes + kRowsXBufs * 3 * mr * 128 + 1024 + 512; }
+
+namespace rows {
+
+// Two neighbours in k -> their three bf16 pairs (the first value in the low half).
+__device__ __forceinline__ void split3(float a, float b, uint32_t &p0, uint32_t &p1, uint32_t &p2)
+{
+    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+    p0 = __byte_perm(ua, ub, 0x7632);
+    const float ra = a - __uint_as_float(ua & 0xFFFF0000u), rb = b - __uint_as_float(ub & 0xFFFF0000u);
+    p1 = ptx::pack_bf16x2(ra, rb);
+    p2 = ptx::pack_bf16x2(ra - bf16_lo(p1), rb - bf16_hi(p1));
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                 "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+// A from TMEM (lane = row of A, a column = two neighbours in k), B from shared memory.
+__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "setp.ne.b32 P, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, P;\n\t}"
+        :
+        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+}  // namespace rows
+
+// Walk over the steps of 16 k of a block's tiles; every role takes it alike.
+struct RowsWalk {
+    int steps, blocks;      // of 16 k, of 64 k
+    int k0;
+    __device__ __forceinline__ RowsWalk(const RowsParams &p, int rank)
+    {
+        k0 = rank * p.slice;
+        steps = max(0, (min(p.K, k0 + p.slice) - k0 + 15) / 16);
+        blocks = (steps + 3) / 4;
+    }
+    __device__ __forceinline__ int in_block(int b) const { return min(4, steps - 4 * b); }
+};
+
+// grid (column tiles, or blocks that walk over them; cluster over k)
+template <int MR, bool W_NK>
+__global__ void __launch_bounds__(kRowsThreads, 1)
+rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams p)
+{
+    namespace cg = cooperative_groups;
+    constexpr int kXBytes = 3 * MR * 128, kCols = MR / 2;
+    constexpr uint32_t kIdesc = ptx::make_idesc_bf16(128, MR, false, false);
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *smem_gen = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
+    const uint32_t x_base = smem_base + kRowsStages * kRowsStageBytes;
+    const uint32_t bar_base = x_base + kRowsXBufs * kXBytes;
+    auto w_full = [&](int s) { return bar_base + 8u * s; };
+    auto w_empty = [&](int s) { return bar_base + 8u * (kRowsStages + s); };
+    auto a_full = [&](int r) { return bar_base + 8u * (2 * kRowsStages + r); };
+    auto a_empty = [&](int r) { return bar_base + 8u * (2 * kRowsStages + kRowsSlots + r); };
+    constexpr int kX = 2 * kRowsStages + 2 * kRowsSlots;
+    auto x_full = [&](int b) { return bar_base + 8u * (kX + b); };
+    auto x_empty = [&](int b) { return bar_base + 8u * (kX + kRowsXBufs + b); };
+    auto acc_full = [&](int b) { return bar_base + 8u * (kX + 2 * kRowsXBufs + b); };
+    auto acc_empty = [&](int b) { return bar_base + 8u * (kX + 2 * kRowsXBufs + 2 + b); };
+    const uint32_t drain_bar = bar_base + 8u * (kX + 2 * kRowsXBufs + 4);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * (kX + 2 * kRowsXBufs + 5));
+    static_assert(8 * (kX + 2 * kRowsXBufs + 5) + 8 <= 512, "barriers");
+    volatile uint32_t *abort_flag = tmem_slot + 1;
+
+    const int warp = ptx::warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int S = gridDim.y, rank = blockIdx.y;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kRowsStages; ++s) {
+            ptx::mbar_init(w_full(s), 1);
+            ptx::mbar_init(w_empty(s), 8);
+        }
+        for (int r = 0; r < kRowsSlots; ++r) {
+            ptx::mbar_init(a_full(r), 4);
+            ptx::mbar_init(a_empty(r), 1);
+        }
+        for (int b = 0; b < kRowsXBufs; ++b) {
+            ptx::mbar_init(x_full(b), 4);
+            ptx::mbar_init(x_empty(b), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            ptx::mbar_init(acc_full(b), 1);
+            ptx::mbar_init(acc_empty(b), 8);
+        }
+        ptx::mbar_init(drain_bar, 1);
+        *abort_flag = 0u;
+        ptx::fence_mbar_init();
+        ptx::prefetch_tensormap(&tmap_w);
+    }
+    if (warp == 21) {
+        ptx::tmem_alloc(ptx::smem_u32(tmem_slot), 512);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem = ptx::warp_uniform(*tmem_slot);
+    const RowsWalk walk(p, rank);
+    if (!p.early) grid_dependency_wait();
+    bool ok = true;
+
+    if (warp < 8) {
+        // ------------------------------------------------------------ converters
+        const int set = warp >> 2, quarter = warp & 3, n = quarter * 32 + lane;
+        const uint32_t slots = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kRowsSlotBase;
+        uint32_t g = 0, s = 0, ph = 0;
+        for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
+            for (int b = 0; ok && b < walk.blocks; ++b) {
+                if (!bounded_wait(w_full(s), ph, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t stage = smem_base + s * kRowsStageBytes;
+                const int steps = walk.in_block(b);
+                for (int ks = 0; ks < steps; ++ks, ++g) {
+                    if (static_cast<int>(g & 1u) != set) continue;
+                    float v[16];
+                    if (W_NK) {   // boxes of 32 k: [128 columns][32 k], 16-byte pieces XOR-ed with the column mod 8
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 f = ptx::lds128(stage + (ks >> 1) * 16384 + n * 128 + ((((ks & 1) * 4 + j) ^ (n & 7)) << 4));
+                            v[4 * j] = f.x;
+                            v[4 * j + 1] = f.y;
+                            v[4 * j + 2] = f.z;
+                            v[4 * j + 3] = f.w;
+                        }
+                    } else {      // [64 k][128 columns]
+                        const float *w = reinterpret_cast<const float *>(smem_gen + s * kRowsStageBytes) + ks * 16 * 128 + n;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = w[j * 128];
+                    }
+                    uint32_t p0[8], p1[8], p2[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) rows::split3(v[2 * j], v[2 * j + 1], p0[j], p1[j], p2[j]);
+                    const uint32_t r = g % kRowsSlots;
+                    if (!bounded_wait(a_empty(r), ((g / kRowsSlots) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
+                        ok = false;
+                        break;
+                    }
+                    ptx::tc_fence_after();
+                    rows::tmem_st8(slots + r * kRowsSlotCols, p0);
+                    rows::tmem_st8(slots + r * kRowsSlotCols + 8, p1);
+                    rows::tmem_st8(slots + r * kRowsSlotCols + 16, p2);
+                    rows::tmem_st_wait();
+                    ptx::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(a_full(r));
+                }
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(w_empty(s));
+                if (++s == kRowsStages) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp < 16) {
+        // ------------------------------------------------------------ sums
+        const int half = (warp - 8) >> 2, quarter = warp & 3, n = quarter * 32 + lane;
+        const uint32_t mine = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + half * kCols;
+        uint32_t c = 0;
+        if (p.early) grid_dependency_wait();   // y may still be read by it
+        for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
+            float acc[kCols];
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
+            for (int ks = 0; ks < walk.steps; ks += kRowsChunk, ++c) {
+                const uint32_t b = c & 1u;
+                if (!bounded_wait(acc_full(b), (c >> 1) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after();
+                uint32_t v[kCols];
+#pragma unroll
+                for (int j = 0; j < kCols; j += 8) rows::tmem_ld8(mine + b * kRowsAccCols + j, v + j);
+                ptx::tmem_ld_wait();
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(acc_empty(b));
+#pragma unroll
+                for (int j = 0; j < kCols; ++j) acc[j] += __uint_as_float(v[j]);
+            }
+            if (!ok) break;
+            if (S == 1) {
+                const int col = t * 128 + n;
+                if (col < p.N) {
+                    const float bias = p.bias ? __ldg(p.bias + col) : 0.0f;
+#pragma unroll
+                    for (int j = 0; j < kCols; ++j) {
+                        const int m = half * kCols + j;
+                        if (m < p.M) {
+                            const float v = acc[j] + bias;
+                            p.y[static_cast<long long>(m) * p.N + col] = v;
+                            if (p.act) p.act[static_cast<long long>(m) * p.N + col] = gelu_tanh(v);
+                        }
+                    }
+                }
+            } else {   // the partial tile [row][column] takes the place of the weights: all of them have been converted
+                float *tile = reinterpret_cast<float *>(smem_gen);
+#pragma unroll
+                for (int j = 0; j < kCols; ++j) tile[(half * kCols + j) * 128 + n] = acc[j];
+            }
+        }
+    } else if (warp < 20) {
+        // ------------------------------------------------------------ x
+        if (p.early) grid_dependency_wait();
+        if (threadIdx.x == 16 * 32) grid_dependency_launch();
+        constexpr int kUnits = MR * 8 / 128;   // of 8 k per thread
+        const int tid = threadIdx.x - 16 * 32;
+        uint32_t xb = 0, ph = 0;
+        float4 v[kUnits][2];
+        auto fetch = [&](int b) {
+#pragma unroll
+            for (int u = 0; u < kUnits; ++u) {
+                const int i = tid + u * 128, row = i >> 3, k = walk.k0 + b * 64 + (i & 7) * 8;
+                const float4 *src = reinterpret_cast<const float4 *>(p.x + static_cast<long long>(row) * p.K + k);
+                v[u][0] = row < p.M && k < p.K ? __ldg(src) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);          // K is a multiple of 4
+                v[u][1] = row < p.M && k + 4 < p.K ? __ldg(src + 1) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        };
+        if (walk.blocks > 0) fetch(0);
+        for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
+            for (int b = 0; b < walk.blocks; ++b) {
+                if (!bounded_wait(x_empty(xb), ph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t dst = x_base + xb * kXBytes;
+#pragma unroll
+                for (int u = 0; u < kUnits; ++u) {
+                    const int i = tid + u * 128, row = i >> 3, c = i & 7;
+                    const float f[8] = {v[u][0].x, v[u][0].y, v[u][0].z, v[u][0].w, v[u][1].x, v[u][1].y, v[u][1].z, v[u][1].w};
+                    uint32_t p0[4], p1[4], p2[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) rows::split3(f[2 * j], f[2 * j + 1], p0[j], p1[j], p2[j]);
+                    const uint32_t at = dst + row * 128 + ((c ^ (row & 7)) << 4);
+                    ptx::sts128(at, p0[0], p0[1], p0[2], p0[3]);
+                    ptx::sts128(at + MR * 128, p1[0], p1[1], p1[2], p1[3]);
+                    ptx::sts128(at + 2 * MR * 128, p2[0], p2[1], p2[2], p2[3]);
+                }
+                ptx::fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(x_full(xb));
+                fetch(b + 1 < walk.blocks ? b + 1 : 0);   // the next block, or the next tile's first
+                if (++xb == kRowsXBufs) {
+                    xb = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else if (warp == 20) {
+        // ------------------------------------------------------------ TMA producer
+        const bool issuer = ptx::elect_one();
+        uint32_t s = 0, ph = 0;
+        for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
+            for (int b = 0; b < walk.blocks; ++b) {
+                if (!bounded_wait(w_empty(s), ph ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) {
+                    ok = false;
+                    break;
+                }
+                if (issuer) {
+                    const int boxes = (walk.in_block(b) + 1) / 2, k = walk.k0 + b * 64;   // of 32 k
+                    ptx::mbar_arrive_expect_tx(w_full(s), boxes * 16384);
+                    for (int i = 0; i < boxes; ++i) {
+                        const uint32_t dst = smem_base + s * kRowsStageBytes + i * 16384;
+                        if (W_NK)
+                            ptx::tma_load_2d(dst, &tmap_w, k + 32 * i, t * 128, w_full(s));
+                        else
+                            ptx::tma_load_2d(dst, &tmap_w, t * 128, k + 32 * i, w_full(s));
+                    }
+                }
+                __syncwarp();
+                if (++s == kRowsStages) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ instructions
+        const bool issuer = ptx::elect_one();
+        const ptx::SmemDesc desc_x = ptx::smem_desc_words(x_base, 16, 1024, ptx::kLayoutSw128);
+        uint32_t g = 0, c = 0, xb = 0, ph = 0;
+        for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
+            uint32_t accumulate = 0;
+            for (int b = 0; ok && b < walk.blocks; ++b) {
+                if (!bounded_wait(x_full(xb), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
+                    ok = false;
+                    break;
+                }
+                const int steps = walk.in_block(b);
+                for (int ks = 0; ks < steps; ++ks, ++g) {
+                    const int step = 4 * b + ks;
+                    const uint32_t buf = c & 1u, r = g % kRowsSlots;
+                    if (step % kRowsChunk == 0) {
+                        accumulate = 0;
+                        if (!bounded_wait(acc_empty(buf), ((c >> 1) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM)) {
+                            ok = false;
+                            break;
+                        }
+                    }
+                    if (!bounded_wait(a_full(r), (g / kRowsSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) {
+                        ok = false;
+                        break;
+                    }
+                    ptx::tc_fence_after();
+                    const uint32_t d = tmem + buf * kRowsAccCols, a = tmem + kRowsSlotBase + r * kRowsSlotCols, x = xb * kXBytes + ks * 32;
+                    const bool last = step % kRowsChunk == kRowsChunk - 1 || step + 1 == walk.steps;
+                    if (issuer) {   // the smallest products first
+                        rows::mma_ts(d, a + 16, desc_x.at(x), kIdesc, accumulate);
+                        rows::mma_ts(d, a, desc_x.at(x + 2 * MR * 128), kIdesc, 1u);
+                        rows::mma_ts(d, a + 8, desc_x.at(x + MR * 128), kIdesc, 1u);
+                        rows::mma_ts(d, a + 8, desc_x.at(x), kIdesc, 1u);
+                        rows::mma_ts(d, a, desc_x.at(x + MR * 128), kIdesc, 1u);
+                        rows::mma_ts(d, a, desc_x.at(x), kIdesc, 1u);
+                        ptx::mma_commit(a_empty(r));
+                        if (last) ptx::mma_commit(acc_full(buf));
+                        if (ks == steps - 1) ptx::mma_commit(x_empty(xb));
+                    }
+                    accumulate = 1u;
+                    if (last) ++c;
+                }
+                if (++xb == kRowsXBufs) {
+                    xb = 0;
+                    ph ^= 1u;
+                }
+            }
+        }
+        if (issuer) ptx::mma_commit(drain_bar);   // TMEM is about to be released
+        bounded_wait(drain_bar, 0u, abort_flag, p.status, DEV_TIMEOUT_DRAIN);
+        __syncwarp();
+    }
+
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {   // a wait ran out: copies still in flight get time to land
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    }
+    if (warp == 21) {
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc(tmem, 512);
+    }
+    if (S > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        // rank order; this block finishes every S-th run of four-column pieces
+        float *tile = reinterpret_cast<float *>(smem_gen);
+        for (int e = rank * kRowsThreads + threadIdx.x; e < p.M * 32; e += S * kRowsThreads) {
+            const int m = e >> 5, col = blockIdx.x * 128 + 4 * (e & 31);
+            if (col >= p.N) continue;
+            float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int q0 = 0; q0 < S; q0 += 8) {   // up to eight remote loads in flight
+                float4 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    v[j] = q0 + j < S ? reinterpret_cast<const float4 *>(cluster.map_shared_rank(tile, q0 + j))[e] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    sum.x += v[j].x;
+                    sum.y += v[j].y;
+                    sum.z += v[j].z;
+                    sum.w += v[j].w;
+                }
+            }
+            if (p.bias) {   // need not be 16-byte aligned
+                sum.x += __ldg(p.bias + col);
+                sum.y += __ldg(p.bias + col + 1);
+                sum.z += __ldg(p.bias + col + 2);
+                sum.w += __ldg(p.bias + col + 3);
+            }
+            *reinterpret_cast<float4 *>(p.y + static_cast<long long>(m) * p.N + col) = sum;
+            if (p.act) *reinterpret_cast<float4 *>(p.act + static_cast<long long>(m) * p.N + col) = make_float4(gelu_tanh(sum.x), gelu_tanh(sum.y), gelu_tanh(sum.z), gelu_tanh(sum.w));
+        }
+        cluster.sync();   // no block leaves while its tile may still be read
+    }
+}
+
+}  // namespace gptb200
