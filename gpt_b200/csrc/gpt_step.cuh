@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "gemm_sm100.cuh"  // gelu_tanh
+#include "rows_sm100.cuh"  // products in three bf16 parts
 #include "gpt_step.h"
 
 namespace gptb200 {
@@ -572,9 +573,12 @@ __device__ __forceinline__ float gelu_step(float x)
 template <int THREADS>
 __device__ __forceinline__ void group_sync() { asm volatile("bar.sync %0, %1;" ::"r"(1 + static_cast<int>(threadIdx.x) / THREADS), "n"(THREADS) : "memory"); }
 
-__host__ __device__ constexpr size_t wide_shared_floats(int rows) { return size_t(2) * kWideSlice * kWideCols + size_t(kWideSlice) * (rows + 4); }
+// activations of an item: [k][row], or on the tensor cores [half of k][part][row][64 k] in bf16, 128-byte swizzle
+__host__ __device__ constexpr bool wide_tensor(int rows) { return rows >= 16; }
+__host__ __device__ constexpr size_t wide_x_floats(int rows) { return wide_tensor(rows) ? size_t(rows) * 192 : size_t(kWideSlice) * (rows + 4); }
+__host__ __device__ constexpr size_t wide_shared_floats(int rows) { return size_t(2) * kWideSlice * kWideCols + wide_x_floats(rows) + 256; }   // 1 KB to align
 __host__ __device__ constexpr int wide_attention_threads(int rows) { return rows >= 32 ? 64 : 128; }   // per (sequence, head)
-// one of the buffers of weights with the activations beside it: what the sums, the norms and the attention use between products
+// one of the buffers of weights with the activations beside it: what the sums, the norms and the attention use between products (at least)
 __host__ __device__ constexpr size_t wide_scratch_floats(int rows) { return size_t(kWideSlice) * kWideCols + size_t(kWideSlice) * (rows + 4); }
 // attention: for every item at work a head's new q, k, v, parts of its output and the scores
 __host__ __device__ constexpr int wide_attention_floats(int threads, int hd, int max_len) { return 3 * hd + threads / 32 * (hd + 4) + ((max_len + 3) & ~3); }
@@ -589,16 +593,36 @@ __global__ void __launch_bounds__(kThreads, 1)
 gpt_step_rows_kernel(const GptStep s)
 {
     constexpr int RT = ROWS / 8, P = ROWS + 4;   // rows per thread; pitch of the activations
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) float sm_raw[];
     __shared__ float4 moments[kWarps];
-    float *xs = sm + kWideSlice * kWideCols;      // [kWideSlice][P] activations, between two buffers of weights [kWideSlice][kWideCols]
-    float *ws = sm, *ws_next = xs + kWideSlice * P;
+    float *sm = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~uintptr_t(1023));
+    float *xs = sm + kWideSlice * kWideCols;      // activations, between two buffers of weights [kWideSlice][kWideCols]
+    float *ws = sm, *ws_next = xs + wide_x_floats(ROWS);
     auto scratch = [&] { return ws < xs ? ws : xs; };   // the current buffer of weights and the activations: neighbours, whichever buffer it is
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = s.d, batch = s.batch, first = blockIdx.x;
     const int p = *s.pos;
     if (p < 0 || p >= s.max_len || p >= s.max_pos) return;   // all blocks alike
     __shared__ bool gave_up;   // thread 0's; no register is free for it, nor for leaving here
     if (tid == 0) gave_up = lost(s);
+    __shared__ __align__(8) unsigned long long step_bar;
+    __shared__ uint32_t step_tmem, step_abort;
+    uint32_t tmem = 0, bar_phase = 0;
+    const uint32_t bar = ptx::smem_u32(&step_bar);
+    if constexpr (wide_tensor(ROWS)) {
+        if (tid == 0) {
+            ptx::mbar_init(bar, 4);
+            step_abort = 0u;
+            ptx::fence_mbar_init();
+        }
+        if (warp == 0) {
+            ptx::tmem_alloc(ptx::smem_u32(&step_tmem), 512);
+            ptx::tmem_relinquish();
+        }
+        ptx::tc_fence_before();
+        __syncthreads();
+        ptx::tc_fence_after();
+        tmem = ptx::warp_uniform(step_tmem);
+    }
     unsigned target = s.sync[1];
 
     // Piece i of eight of an item's weights into the other buffer: 16 of its k-rows, one per warp; columns beyond the matrix are zeros.
@@ -739,6 +763,117 @@ gpt_step_rows_kernel(const GptStep s)
                 }
             }
             if (!last) __syncthreads();   // the next item's activations go where the sums are
+        }
+    };
+
+    // The same on the tensor cores, operands in three bf16 parts as in rows_sm100.cuh.  An item's weights go through registers to TMEM at once (lane = column, 24
+    // columns per step of 16 k), four warps issue the products of a step each into an accumulator of its own, and the sixteen warps add up a sixteenth of
+    // all accumulators each, in fp32 and in the order of k.
+    auto product_tensor = [&](const float *w, const StepPhase &ph, float *part, const float *x, const float *w_next, const StepPhase &ph_next, int item_next) {
+        constexpr int kAccs = ROWS == 64 ? 4 : 8, kAccCols = 256 / kAccs, kMine = ROWS / 4;      // accumulators, rows per warp
+        constexpr uint32_t kIdesc = ptx::make_idesc_bf16(128, ROWS, false, false), kPart = ROWS * 128;
+        const int items = ph.groups * ph.splits, set = warp >> 2, q4 = warp & 3, n = q4 * 32 + lane;
+        const uint32_t lanes = static_cast<uint32_t>(q4 * 32) << 16, x_at = ptx::smem_u32(xs);
+        const ptx::SmemDesc desc_x = ptx::smem_desc_words(x_at, 16, 1024, ptx::kLayoutSw128);
+        if (first >= items) fetch_all(w_next, ph_next, item_next);
+#pragma unroll 1
+        for (int item = first; item < items; item += gridDim.x) {
+            const int split = item / ph.groups, col0 = (item - split * ph.groups) * kWideCols, k0 = split * ph.slice, rows = min(ph.K - k0, ph.slice), steps = (rows + 15) >> 4;
+            {   // the weights of this item become current
+                float *t = ws;
+                ws = ws_next;
+                ws_next = t;
+            }
+            // x: pieces of eight k of a row
+            constexpr int kUnits = (ROWS * 16 + kThreads - 1) / kThreads;
+            float4 v[kUnits][2];
+#pragma unroll
+            for (int u = 0; u < kUnits; ++u) {
+                const int i = tid + u * kThreads, row = i >> 4, k = (i & 15) * 8;
+                const float4 *src = reinterpret_cast<const float4 *>(x + static_cast<size_t>(row) * ph.K + k0 + k);
+                v[u][0] = row < batch && k < rows ? __ldcg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[u][1] = row < batch && k + 4 < rows ? __ldcg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < kUnits; ++u) {
+                const int i = tid + u * kThreads, row = i >> 4, c = i & 15;
+                if (row >= ROWS) break;
+                const float f[8] = {v[u][0].x, v[u][0].y, v[u][0].z, v[u][0].w, v[u][1].x, v[u][1].y, v[u][1].z, v[u][1].w};
+                uint32_t p0[4], p1[4], p2[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) rows::split3(f[2 * j], f[2 * j + 1], p0[j], p1[j], p2[j]);
+                const uint32_t to = x_at + (c >> 3) * 3 * kPart + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+                ptx::sts128(to, p0[0], p0[1], p0[2], p0[3]);
+                ptx::sts128(to + kPart, p1[0], p1[1], p1[2], p1[3]);
+                ptx::sts128(to + 2 * kPart, p2[0], p2[1], p2[2], p2[3]);
+            }
+            ptx::fence_proxy_async_smem();
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            const bool last = item + static_cast<int>(gridDim.x) >= items;
+            fetch_all(last ? w_next : w, last ? ph_next : ph, last ? item_next : item + static_cast<int>(gridDim.x));
+            // weights: sixteen k of a column
+#pragma unroll 1
+            for (int ks = set; ks < steps; ks += 4) {
+                float f[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) f[j] = ks * 16 + j < rows ? ws[(ks * 16 + j) * kWideCols + n] : 0.0f;
+                uint32_t p0[8], p1[8], p2[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) rows::split3(f[2 * j], f[2 * j + 1], p0[j], p1[j], p2[j]);
+                const uint32_t slot = tmem + lanes + kRowsSlotBase + ks * kRowsSlotCols;
+                rows::tmem_st8(slot, p0);
+                rows::tmem_st8(slot + 8, p1);
+                rows::tmem_st8(slot + 16, p2);
+            }
+            rows::tmem_st_wait();
+            float acc[kMine];
+#pragma unroll
+            for (int j = 0; j < kMine; ++j) acc[j] = 0.0f;
+#pragma unroll 1
+            for (int base = 0; base < steps; base += kAccs) {
+                const int count = min(kAccs, steps - base);
+                ptx::tc_fence_before();
+                __syncthreads();      // the split weights are there; the sums of the steps before have been read
+                if (warp < 4) {
+                    ptx::tc_fence_after();
+                    if (ptx::elect_one()) {
+                        for (int a = warp; a < count; a += 4) {
+                            const int ks = base + a;
+                            rows::issue_step(tmem + a * kAccCols, tmem + kRowsSlotBase + ks * kRowsSlotCols, desc_x, (ks >> 2) * 3 * kPart + (ks & 3) * 32, kPart, kIdesc);
+                        }
+                        ptx::mma_commit(bar);
+                    }
+                    __syncwarp();
+                }
+                if (!bounded_wait(bar, bar_phase, &step_abort, s.status, DEV_TIMEOUT_EPILOGUE) && tid == 0) {   // as at a barrier that ran out
+                    gave_up = true;
+                    atomicExch(s.sync + 2, 1u);
+                }
+                bar_phase ^= 1u;
+                __syncwarp();
+                ptx::tc_fence_after();
+#pragma unroll 1
+                for (int a = 0; a < count; ++a) {
+                    uint32_t r[kMine];
+                    const uint32_t at = tmem + lanes + a * kAccCols + set * kMine;
+                    if constexpr (kMine == 4)
+                        rows::tmem_ld4(at, r);
+                    else
+#pragma unroll
+                        for (int j = 0; j < kMine; j += 8) rows::tmem_ld8(at + j, r + j);
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < kMine; ++j) acc[j] += __uint_as_float(r[j]);
+                }
+            }
+            if (col0 + n < ph.N) {
+#pragma unroll
+                for (int j = 0; j < kMine; ++j)
+                    if (set * kMine + j < batch) part[(static_cast<size_t>(split) * batch + set * kMine + j) * ph.N + col0 + n] = acc[j];
+            }
+            ptx::tc_fence_before();
+            if (!last) __syncthreads();   // every warp has read its sums: the next item's products may overwrite them
         }
     };
 
@@ -945,10 +1080,19 @@ gpt_step_rows_kernel(const GptStep s)
         const StepPhase ph = kind == 0 ? s.qkv : kind == 1 ? s.proj : kind == 2 ? s.up : s.down, ph_next = kind == 0 ? s.proj : kind == 1 ? s.up : kind == 2 ? s.down : s.qkv;
         const float *w = kind == 0 ? s.qkv_w + 3 * dd * l : kind == 1 ? s.proj_w + dd * l : kind == 2 ? s.up_w + df * l : s.down_w + df * l;
         const float *w_next = kind == 0 ? s.proj_w + dd * l : kind == 1 ? s.up_w + df * l : kind == 2 ? s.down_w + df * l : s.qkv_w + 3 * dd * (l + 1);
-        product(w, ph, kind == 0 ? s.qkv_part : kind == 1 ? s.proj_part : kind == 2 ? s.up_part : s.down_part, kind == 1 ? s.attn : kind == 3 ? s.up_part : s.normed,
-                w_next, ph_next, kind == 3 && l + 1 == s.layers ? ph_next.groups * ph_next.splits : first);
+        float *part = kind == 0 ? s.qkv_part : kind == 1 ? s.proj_part : kind == 2 ? s.up_part : s.down_part;
+        const float *x = kind == 1 ? s.attn : kind == 3 ? s.up_part : s.normed;
+        const int item_next = kind == 3 && l + 1 == s.layers ? ph_next.groups * ph_next.splits : first;
+        if constexpr (wide_tensor(ROWS))
+            product_tensor(w, ph, part, x, w_next, ph_next, item_next);
+        else
+            product(w, ph, part, x, w_next, ph_next, item_next);
         arrive(s, target);
         await(s, target, gave_up);
+    }
+    if constexpr (wide_tensor(ROWS)) {
+        __syncthreads();
+        if (warp == 0) ptx::tmem_dealloc(tmem, 512);
     }
     if (blockIdx.x == 0 && tid == 0 && !gave_up) {   // every block has passed a barrier since it read them
         *s.pos = p + 1;

@@ -3,7 +3,8 @@
 //
 // Both operands are split exactly into three bf16 values (8 + 8 + 8 bits: the first truncated, the others rounded), and the six products of 2^-16 and more
 // are added: what is left out is 2^-24 of a product and less.  The tensor core adds into its accumulator with truncation, so the accumulator is handed to fp32
-// sums in registers (round to nearest) after every kRowsChunk steps of 16 k.  Infinite inputs give NaN, as in the products of more rows.
+// sums in registers (round to nearest) after every step of 16 k: 64 rows, k 768, n 50304 are off by 1.40e-7 of the result's size, 2.2e-7 with two steps, 4.3e-7 with
+// four (fp32 FMAs: 2.1e-7).  Infinite inputs give NaN, as in the products of more rows.
 //
 // A block computes 128 columns for all rows over its share of k.  The weights are the M = 128 operand; split, they never go back to shared memory: the converter
 // warps write them to TMEM, where the instructions take their A operand from.
@@ -11,7 +12,8 @@
 //   warps 8-15   sums: accumulator -> registers, half of the rows each
 //   warps 16-19  x: global -> three bf16 tiles of 64 k in shared memory (B operand)
 //   warp 20      TMA producer: 32 KB of weights per 64 k, four stages
-//   warp 21      issues the instructions
+//   warps 21, 22 issue the instructions, every other step each: one of them took 500 cycles per step for its waits, six instructions and commits (output layer
+//                55 us at 64 rows and 40 at 9; two 47 and 33, three 47 and 32).  More converters, or the instructions of several steps in turn, were slower.
 // The un-embedding has enough column tiles for all SMs (blocks walk over them); narrow layers share k in a cluster, partial tiles meet in rank order through
 // distributed shared memory.
 #pragma once
@@ -22,15 +24,13 @@
 
 namespace gptb200 {
 
-#ifndef GPTB200_ROWS_CHUNK
-#define GPTB200_ROWS_CHUNK 1
-#endif
-constexpr int kRowsChunk = GPTB200_ROWS_CHUNK;
-constexpr int kRowsThreads = 22 * 32;
+constexpr int kRowsIssuers = 2;
+constexpr int kRowsThreads = (21 + kRowsIssuers) * 32;
 constexpr int kRowsStages = 4, kRowsStageBytes = 128 * 64 * 4;
 constexpr int kRowsSlots = 8, kRowsSlotCols = 24;      // split weights of 16 k: 3 x 8 TMEM columns
-constexpr int kRowsAccCols = 64;
-constexpr int kRowsSlotBase = 2 * kRowsAccCols;
+constexpr int kRowsAccs = 4, kRowsAccCols = 64;        // accumulators: with two of them the way to the sums and back was what a step took
+constexpr int kRowsSlotBase = kRowsAccs * kRowsAccCols;
+static_assert(kRowsSlotBase + kRowsSlots * kRowsSlotCols <= 512, "TMEM");
 constexpr int kRowsXBufs = 2;
 
 struct RowsParams {
@@ -74,6 +74,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v)
                  : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t *v)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
+}
+
 // A from TMEM (lane = row of A, a column = two neighbours in k), B from shared memory.
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
@@ -84,6 +89,17 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
         :
         : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+// One step's six products, the smallest first: split weights at TMEM columns `a`, the parts of x `part` bytes apart.
+__device__ __forceinline__ void issue_step(uint32_t d, uint32_t a, const ptx::SmemDesc &x, uint32_t at, uint32_t part, uint32_t idesc)
+{
+    mma_ts(d, a + 16, x.at(at), idesc, 0u);
+    mma_ts(d, a, x.at(at + 2 * part), idesc, 1u);
+    mma_ts(d, a + 8, x.at(at + part), idesc, 1u);
+    mma_ts(d, a + 8, x.at(at), idesc, 1u);
+    mma_ts(d, a, x.at(at + part), idesc, 1u);
+    mma_ts(d, a, x.at(at), idesc, 1u);
 }
 
 }  // namespace rows
@@ -117,15 +133,14 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
     auto w_full = [&](int s) { return bar_base + 8u * s; };
     auto w_empty = [&](int s) { return bar_base + 8u * (kRowsStages + s); };
     auto a_full = [&](int r) { return bar_base + 8u * (2 * kRowsStages + r); };
-    auto a_empty = [&](int r) { return bar_base + 8u * (2 * kRowsStages + kRowsSlots + r); };
+    auto done = [&](int r) { return bar_base + 8u * (2 * kRowsStages + kRowsSlots + r); };      // a step's instructions: its sums are there, its weights read
     constexpr int kX = 2 * kRowsStages + 2 * kRowsSlots;
     auto x_full = [&](int b) { return bar_base + 8u * (kX + b); };
     auto x_empty = [&](int b) { return bar_base + 8u * (kX + kRowsXBufs + b); };
-    auto acc_full = [&](int b) { return bar_base + 8u * (kX + 2 * kRowsXBufs + b); };
-    auto acc_empty = [&](int b) { return bar_base + 8u * (kX + 2 * kRowsXBufs + 2 + b); };
-    const uint32_t drain_bar = bar_base + 8u * (kX + 2 * kRowsXBufs + 4);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * (kX + 2 * kRowsXBufs + 5));
-    static_assert(8 * (kX + 2 * kRowsXBufs + 5) + 8 <= 512, "barriers");
+    auto acc_empty = [&](int b) { return bar_base + 8u * (kX + 2 * kRowsXBufs + b); };
+    const uint32_t drain_bar = bar_base + 8u * (kX + 2 * kRowsXBufs + kRowsAccs);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * (kX + 2 * kRowsXBufs + kRowsAccs + 1));
+    static_assert(8 * (kX + 2 * kRowsXBufs + kRowsAccs + 1) + 8 <= 512, "barriers");
     volatile uint32_t *abort_flag = tmem_slot + 1;
 
     const int warp = ptx::warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -137,17 +152,14 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
         }
         for (int r = 0; r < kRowsSlots; ++r) {
             ptx::mbar_init(a_full(r), 4);
-            ptx::mbar_init(a_empty(r), 1);
+            ptx::mbar_init(done(r), 1);
         }
         for (int b = 0; b < kRowsXBufs; ++b) {
             ptx::mbar_init(x_full(b), 4);
-            ptx::mbar_init(x_empty(b), 1);
+            ptx::mbar_init(x_empty(b), kRowsIssuers);
         }
-        for (int b = 0; b < 2; ++b) {
-            ptx::mbar_init(acc_full(b), 1);
-            ptx::mbar_init(acc_empty(b), 8);
-        }
-        ptx::mbar_init(drain_bar, 1);
+        for (int b = 0; b < kRowsAccs; ++b) ptx::mbar_init(acc_empty(b), 8);
+        ptx::mbar_init(drain_bar, kRowsIssuers);
         *abort_flag = 0u;
         ptx::fence_mbar_init();
         ptx::prefetch_tensormap(&tmap_w);
@@ -198,7 +210,7 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
 #pragma unroll
                     for (int j = 0; j < 8; ++j) rows::split3(v[2 * j], v[2 * j + 1], p0[j], p1[j], p2[j]);
                     const uint32_t r = g % kRowsSlots;
-                    if (!bounded_wait(a_empty(r), ((g / kRowsSlots) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
+                    if (!bounded_wait(done(r), ((g / kRowsSlots) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
                         ok = false;
                         break;
                     }
@@ -223,15 +235,15 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
         // ------------------------------------------------------------ sums
         const int half = (warp - 8) >> 2, quarter = warp & 3, n = quarter * 32 + lane;
         const uint32_t mine = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + half * kCols;
-        uint32_t c = 0;
+        uint32_t g = 0;
         if (p.early) grid_dependency_wait();   // y may still be read by it
         for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
             float acc[kCols];
 #pragma unroll
             for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
-            for (int ks = 0; ks < walk.steps; ks += kRowsChunk, ++c) {
-                const uint32_t b = c & 1u;
-                if (!bounded_wait(acc_full(b), (c >> 1) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
+            for (int ks = 0; ks < walk.steps; ++ks, ++g) {
+                const uint32_t b = g % kRowsAccs;
+                if (!bounded_wait(done(g % kRowsSlots), (g / kRowsSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
                     ok = false;
                     break;
                 }
@@ -346,9 +358,9 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
         // ------------------------------------------------------------ instructions
         const bool issuer = ptx::elect_one();
         const ptx::SmemDesc desc_x = ptx::smem_desc_words(x_base, 16, 1024, ptx::kLayoutSw128);
-        uint32_t g = 0, c = 0, xb = 0, ph = 0;
+        uint32_t g = 0, xb = 0, ph = 0;
+        const uint32_t turn = warp - 21;
         for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
-            uint32_t accumulate = 0;
             for (int b = 0; ok && b < walk.blocks; ++b) {
                 if (!bounded_wait(x_full(xb), ph, abort_flag, p.status, DEV_TIMEOUT_MMA_FULL)) {
                     ok = false;
@@ -356,36 +368,21 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
                 }
                 const int steps = walk.in_block(b);
                 for (int ks = 0; ks < steps; ++ks, ++g) {
-                    const int step = 4 * b + ks;
-                    const uint32_t buf = c & 1u, r = g % kRowsSlots;
-                    if (step % kRowsChunk == 0) {
-                        accumulate = 0;
-                        if (!bounded_wait(acc_empty(buf), ((c >> 1) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM)) {
-                            ok = false;
-                            break;
-                        }
-                    }
-                    if (!bounded_wait(a_full(r), (g / kRowsSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) {
+                    if (g % kRowsIssuers != turn) continue;
+                    const uint32_t buf = g % kRowsAccs, r = g % kRowsSlots;
+                    if (!bounded_wait(acc_empty(buf), ((g / kRowsAccs) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM) ||
+                        !bounded_wait(a_full(r), (g / kRowsSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) {
                         ok = false;
                         break;
                     }
                     ptx::tc_fence_after();
                     const uint32_t d = tmem + buf * kRowsAccCols, a = tmem + kRowsSlotBase + r * kRowsSlotCols, x = xb * kXBytes + ks * 32;
-                    const bool last = step % kRowsChunk == kRowsChunk - 1 || step + 1 == walk.steps;
-                    if (issuer) {   // the smallest products first
-                        rows::mma_ts(d, a + 16, desc_x.at(x), kIdesc, accumulate);
-                        rows::mma_ts(d, a, desc_x.at(x + 2 * MR * 128), kIdesc, 1u);
-                        rows::mma_ts(d, a + 8, desc_x.at(x + MR * 128), kIdesc, 1u);
-                        rows::mma_ts(d, a + 8, desc_x.at(x), kIdesc, 1u);
-                        rows::mma_ts(d, a, desc_x.at(x + MR * 128), kIdesc, 1u);
-                        rows::mma_ts(d, a, desc_x.at(x), kIdesc, 1u);
-                        ptx::mma_commit(a_empty(r));
-                        if (last) ptx::mma_commit(acc_full(buf));
-                        if (ks == steps - 1) ptx::mma_commit(x_empty(xb));
+                    if (issuer) {
+                        rows::issue_step(d, a, desc_x, x, MR * 128, kIdesc);
+                        ptx::mma_commit(done(r));
                     }
-                    accumulate = 1u;
-                    if (last) ++c;
                 }
+                if (issuer) ptx::mma_commit(x_empty(xb));
                 if (++xb == kRowsXBufs) {
                     xb = 0;
                     ph ^= 1u;
