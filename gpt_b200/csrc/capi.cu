@@ -573,6 +573,8 @@ GemmPlanInput plan_input(const gptb200_ctx *ctx, const GemmCall &c)
     in.M = c.M; in.N = c.N; in.K = c.K;
     in.a_mn = c.a_mn; in.b_mn = c.b_mn;
     in.has_epilogue = c.bias != nullptr || c.act != nullptr;
+    in.split_epilogue = true;
+    in.x3 = ctx->mode == GPTB200_MODE_3XTF32;
     in.accumulate = c.accumulate;
     in.aligned = aligned16(c.a) && aligned16(c.b) && aligned16(c.out) && (!c.act || aligned16(c.act));
     in.num_sms = ctx->max_sms > 0 ? std::min(ctx->max_sms, ctx->num_sms) : ctx->num_sms;
@@ -590,7 +592,16 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
     if (gelu_fused) *gelu_fused = false;
     GemmPlanInput in = plan_input(ctx, c);
     in.fma_only = c.fma_only;
-    const GemmPlan pl = plan_gemm(in);
+    GemmPlan pl = plan_gemm(in);
+    if (pl.kernel == KERNEL_SINGLE && pl.splits > 1 && in.has_epilogue && pl.workspace_bytes > ctx->ws_bytes) {
+        // scratch cannot be allocated while a graph is captured; a forward call that has not run before needs none otherwise
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess) cudaGetLastError();
+        if (status != cudaStreamCaptureStatusNone) {
+            in.split_epilogue = false;
+            pl = plan_gemm(in);
+        }
+    }
     if (pl.kernel == KERNEL_NONE) return GPTB200_OK;
     if (pl.kernel == KERNEL_SKINNY) return run_skinny(ctx, c, pl);
     if (pl.kernel == KERNEL_SIMT) {
@@ -766,7 +777,7 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
         const long long n4 = (1LL * c.M * c.N) >> 2;
         const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, 1LL * ctx->num_sms * 8));
         ctx->launches++;
-    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, c.out, ctx->ws, n4, splits, c.accumulate ? 1 : 0));
+    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, c.out, ctx->ws, n4, splits, c.accumulate ? 1 : 0, c.bias, c.act, c.N));
     }
     return GPTB200_OK;
 }
@@ -1025,7 +1036,7 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
         const long long n4 = (1LL * c.M * c.N) >> 2;
         const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, 1LL * ctx->num_sms * 8));
         ctx->launches++;
-    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, static_cast<float *>(c.out), ctx->ws, n4, pl.splits, 0));
+    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, static_cast<float *>(c.out), ctx->ws, n4, pl.splits, 0, nullptr, nullptr, c.N));
     }
     return GPTB200_OK;
 }

@@ -31,6 +31,8 @@ struct GemmPlanInput {
     int opt_skinny_rows;     // most rows the weight-streaming kernel takes; 0 = kPlanSkinnyMaxRows
     size_t ws_limit;         // scratch limit in bytes
     bool fma_only;           // fp32 FMAs only: no tensor-core kernel
+    bool split_epilogue;     // split-K in spite of an epilogue: the reduction applies it
+    bool x3;                 // 3xTF32
 };
 
 struct GemmPlan {
@@ -200,9 +202,12 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
     // as there are enough 256 x 256 work items to occupy most SM pairs; with fewer, 128-wide one-CTA tiles fill the
     // machine better.
     const long long pair_tiles = 1LL * ((in.M + 255) / 256) * ((in.N + 255) / 256);
-    const bool split_allowed = !in.has_epilogue;
     const size_t bytes_per_split = size_t(in.M) * size_t(in.N) * sizeof(float);
     p.num_kb = (in.K + kPlanBK - 1) / kPlanBK;
+    // A k-block of a one-CTA tile takes 0.7 us in 3xTF32 mode and 0.15 us in TF32 mode, the reduction with its epilogue 4 us: a forward call is split where the
+    // k-blocks saved are worth more.  Forward + backward, us before / now: 3xTF32, FFN down at 65 rows 104.7 / 53.7, at 300 88.5 / 59.1, at 500 104.9 / 78.3,
+    // projection at 300 rows 57.0 / 46.7; TF32, FFN down at 65 rows 42.6 / 35.9, at 300 63.5 / 39.0, at 1000 76.6 / 61.6.
+    const bool split_allowed = !in.has_epilogue || (in.split_epilogue && p.num_kb >= (in.x3 ? 16 : 40));
     const int max_pairs = std::max(1, in.num_sms / 2);
     const long long pair_kb = pair_tiles * p.num_kb;
     // pairs that can be given at least eight k-blocks each

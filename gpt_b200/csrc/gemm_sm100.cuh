@@ -717,8 +717,9 @@ static __global__ void wait_timeout_selftest_kernel(int *status, long long limit
     __syncthreads();
 }
 
-// out[i] (+)= sum_s ws[s][i], fixed order s = 0..splits-1 (deterministic split-K reduction).
-static __global__ void splitk_reduce_kernel(float *__restrict__ out, const float *__restrict__ ws, long long n4, int splits, int accumulate)
+// out[i] (+)= sum_s ws[s][i] (+ bias[i % N]), fixed order s = 0..splits-1 (deterministic split-K reduction); act = gelu_tanh(out) where there is one.
+static __global__ void splitk_reduce_kernel(float *__restrict__ out, const float *__restrict__ ws, long long n4, int splits, int accumulate, const float *__restrict__ bias, float *__restrict__ act,
+                                            int N)
 {
     grid_dependency_wait();
     grid_dependency_launch();
@@ -734,7 +735,12 @@ static __global__ void splitk_reduce_kernel(float *__restrict__ out, const float
             const float4 prev = *o;
             acc.x += prev.x; acc.y += prev.y; acc.z += prev.z; acc.w += prev.w;
         }
+        if (bias) {   // need not be 16-byte aligned
+            const float *b = bias + i % (N >> 2) * 4;
+            acc.x += __ldg(b); acc.y += __ldg(b + 1); acc.z += __ldg(b + 2); acc.w += __ldg(b + 3);
+        }
         *o = acc;
+        if (act) reinterpret_cast<float4 *>(act)[i] = make_float4(gelu_tanh(acc.x), gelu_tanh(acc.y), gelu_tanh(acc.z), gelu_tanh(acc.w));
     }
 }
 

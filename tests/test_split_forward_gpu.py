@@ -1,0 +1,69 @@
+"""Forward products that are split over k: bias and GELU ride the reduction.  And products of 9 to 64 rows in three bf16 parts."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(torch, m, k, n, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    x, w = torch.randn(m, k, device="cuda", generator=gen), torch.randn(k, n, device="cuda", generator=gen) * k ** -0.5
+    b = torch.randn(n + 1, device="cuda", generator=gen)[1:]      # not 16-byte aligned
+    return x, w, b, x.double() @ w.double() + b.double()
+
+
+@pytest.mark.parametrize("m,k,n", [(65, 3072, 768), (200, 1540, 132), (500, 2052, 260), (70, 512, 772)])
+@pytest.mark.parametrize("mode,tol", [(0, 1e-5), (1, 2e-3)])
+def test_epilogue_behind_split_k(m, k, n, mode, tol):
+    """Several parts, the last one shorter, ragged rows and columns; tolerances of the modes.  A first call inside a capture needs no scratch."""
+    import torch
+    import gpt_b200
+    x, w, b, want = _problem(torch, m, k, n, m + k + n)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    for captured in (False, True):
+        with torch.cuda.stream(stream):
+            be = gpt_b200.Backend(0, stream.cuda_stream, mode)
+            y, act = torch.full((m + 1, n), 7.0, device="cuda"), torch.full((m + 1, n), 7.0, device="cuda")
+            stream.synchronize()
+            if captured:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=stream):
+                    be.device_linear_activation_fused_forward(y, act, x, w, b, True, 1, m, k, n)
+                graph.replay()
+            else:
+                be.device_linear_activation_fused_forward(y, act, x, w, b, True, 1, m, k, n)
+            be.synchronize()
+            assert float((y[:m].double() - want).abs().max()) <= tol * float(want.abs().max())
+            assert float((act[:m].double() - torch.nn.functional.gelu(want, approximate="tanh")).abs().max()) <= tol * float(want.abs().max())
+            assert (y[m] == 7).all() and (act[m] == 7).all()
+            if captured:
+                del graph
+            be.close()
+
+
+@pytest.mark.parametrize("m", [9, 16, 17, 33, 64])
+@pytest.mark.parametrize("k,n", [(768, 2304), (1028, 1284), (36, 132), (3072, 768), (772, 19204)])
+def test_rows_in_three_parts(m, k, n):
+    """Ragged steps of 16 k, shares of k in clusters, several column tiles per block, both layouts of the weights.  At most six truncating additions (2^-23 of
+    the partial sum each) before fp32 sums of k / 16 terms: below 5e-7 of the result's size, and no worse than the fp32 FMA kernel by more than a tenth (at small
+    k the FMA kernel's few roundings are the smaller ones: 1.5e-7 is accepted there)."""
+    import torch
+    import gpt_b200
+    if m > 16 and k * n < 512 * 512:
+        pytest.skip("another kernel's size")
+    x, w, b, want = _problem(torch, m, k, n, m * 3 + k + n)
+    wt = w.t().contiguous()
+    be = gpt_b200.Backend(0, torch.cuda.current_stream().cuda_stream, 0)
+    errors = {}
+    for tensor in (1, 0):
+        be.set_option("skinny_tensor", tensor)
+        y, act, z = (torch.full((m + 1, n), 7.0, device="cuda") for _ in range(3))
+        be.device_linear_activation_fused_forward(y, act, x, w, b, True, 1, m, k, n)
+        be.device_unembedding_forward(z, x, wt, 1, m, k, n)
+        be.synchronize()
+        assert (y[m] == 7).all() and (act[m] == 7).all() and (z[m] == 7).all()
+        plain, gelu = want - b.double(), torch.nn.functional.gelu(want, approximate="tanh")
+        errors[tensor] = [float((got[:m].double() - ref).norm() / ref.norm()) for got, ref in ((y, want), (act, gelu), (z, plain))]
+    for new, old in zip(errors[1], errors[0]):
+        assert new <= 5e-7 and new <= max(1.1 * old, 1.5e-7), errors
+    be.close()
