@@ -573,7 +573,7 @@ GemmPlanInput plan_input(const gptb200_ctx *ctx, const GemmCall &c)
     in.M = c.M; in.N = c.N; in.K = c.K;
     in.a_mn = c.a_mn; in.b_mn = c.b_mn;
     in.has_epilogue = c.bias != nullptr || c.act != nullptr;
-    in.split_epilogue = true;
+    in.layers = true;
     in.x3 = ctx->mode == GPTB200_MODE_3XTF32;
     in.accumulate = c.accumulate;
     in.aligned = aligned16(c.a) && aligned16(c.b) && aligned16(c.out) && (!c.act || aligned16(c.act));
@@ -598,7 +598,7 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
         cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess) cudaGetLastError();
         if (status != cudaStreamCaptureStatusNone) {
-            in.split_epilogue = false;
+            in.layers = false;
             pl = plan_gemm(in);
         }
     }

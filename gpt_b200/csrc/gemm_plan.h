@@ -31,7 +31,7 @@ struct GemmPlanInput {
     int opt_skinny_rows;     // most rows the weight-streaming kernel takes; 0 = kPlanSkinnyMaxRows
     size_t ws_limit;         // scratch limit in bytes
     bool fma_only;           // fp32 FMAs only: no tensor-core kernel
-    bool split_epilogue;     // split-K in spite of an epilogue: the reduction applies it
+    bool layers;             // the calls of the linear layers: split-K in spite of an epilogue, which the reduction applies, and plan_one_wave
     bool x3;                 // 3xTF32
 };
 
@@ -163,6 +163,26 @@ inline DecodePlan plan_decode(int M, int N, int K, bool w_kn, bool has_epilogue,
     return d;
 }
 
+// One wave of 128 x 128 one-CTA tiles, k split as often as fits it, against CTA pairs whose ranges are cut inside tiles (`pair_kb` k-blocks each): a cut costs 15
+// - 25 us for partial tiles that travel through L2 and output that follows them.  Returns the number of parts, 0 for the pairs.  Models of us per launch,
+// fitted to GPT-2's layers at 600 - 4096 rows; measured, pairs / one wave (parts):
+//   TF32    grad_w 768 x 3072 at 600 rows 23.6 / 13.6 (1), 2048 29.7 / 22.3, 4096 41.7 / 38.0; grad_x 2048 x 768 x 2304 24.2 / 19.1 (1), 1536 rows 24.1 / 14.1 (2),
+//           3000 26.1 / 17.7 (1); FFN down forward at 1536 rows 26.6 / 16.5 (2), 3000 30.8 / 23.2 (1)
+//   3xTF32  grad_w 768 x 3072 at 600 rows 33.0 / 24.8, 1000 36.7 / 34.9, 1536 44.7 / 47.5; grad_x 1536 x 768 x 2304 38.5 / 33.2 (2), 2048 rows 38.4 / 42.6 (1)
+inline int plan_one_wave(const GemmPlanInput &in, int num_kb, long long tiles128, double pair_kb, bool split_allowed, size_t bytes_per_split)
+{
+    if (tiles128 > in.num_sms) return 0;
+    long long parts = split_allowed ? std::min<long long>(in.num_sms / tiles128, std::max(1, num_kb / 8)) : 1;
+    if (bytes_per_split > 0) parts = std::min<long long>(parts, std::max<size_t>(1, (in.ws_limit / 2) / bytes_per_split));
+    const int kb = static_cast<int>((num_kb + parts - 1) / parts);
+    parts = (num_kb + kb - 1) / kb;
+    const bool both_mn = in.a_mn && in.b_mn;
+    const double tile_kb = in.x3 ? (both_mn ? 0.78 : 0.56) : both_mn ? 0.245 : in.b_mn ? 0.16 : 0.135;
+    const double wave = (in.x3 ? 10.0 : 8.0) + tile_kb * kb + (parts > 1 ? 3.0 : 0.0);
+    const double pairs = in.x3 ? 24.0 + (both_mn ? 0.95 : 0.65) * pair_kb : both_mn ? 17.7 + 0.387 * pair_kb : 15.0 + 0.32 * pair_kb;
+    return wave < pairs ? static_cast<int>(parts) : 0;
+}
+
 inline GemmPlan plan_gemm(const GemmPlanInput &in)
 {
     GemmPlan p{};
@@ -207,7 +227,7 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
     // A k-block of a one-CTA tile takes 0.7 us in 3xTF32 mode and 0.15 us in TF32 mode, the reduction with its epilogue 4 us: a forward call is split where the
     // k-blocks saved are worth more.  Forward + backward, us before / now: 3xTF32, FFN down at 65 rows 104.7 / 53.7, at 300 88.5 / 59.1, at 500 104.9 / 78.3,
     // projection at 300 rows 57.0 / 46.7; TF32, FFN down at 65 rows 42.6 / 35.9, at 300 63.5 / 39.0, at 1000 76.6 / 61.6.
-    const bool split_allowed = !in.has_epilogue || (in.split_epilogue && p.num_kb >= (in.x3 ? 16 : 40));
+    const bool split_allowed = !in.has_epilogue || (in.layers && p.num_kb >= (in.x3 ? 16 : 40));
     const int max_pairs = std::max(1, in.num_sms / 2);
     const long long pair_kb = pair_tiles * p.num_kb;
     // pairs that can be given at least eight k-blocks each
@@ -225,6 +245,7 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
     const bool automatic = in.opt_pair == 0 && in.opt_tile_n == 0 && in.opt_stream_k == 0 && in.opt_max_splits == 0;
     const long long tiles128 = 1LL * ((in.M + kPlanBM - 1) / kPlanBM) * ((in.N + 127) / 128);
     bool force128 = false;
+    int parts = 0;   // one wave of 128 x 128 tiles with this many parts of k
     if (pair && automatic) {
         const long long kb_each = std::max<long long>(1, pair_kb / pairs_busy);
         if (!in.accumulate && p.num_kb <= 32 && tiles128 <= in.num_sms) {
@@ -245,12 +266,17 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
         const long long whole_pairs = std::min<long long>(max_pairs, pair_tiles);
         const long long rounds = (pair_tiles + whole_pairs - 1) / whole_pairs;
         const double whole_eff = double(pair_tiles) / double(rounds * pairs_busy);   // share of the usable pairs kept busy by whole tiles
-        long long pairs;
+        long long pairs = 0;
         // Whole tiles per pair when they keep at least 97 % of the usable pairs busy -- or when the tiles are short (at most 32
         // k-blocks), fit one round and occupy at least half of the pairs: the main loop a cut would save is then shorter than the
         // cut's fixed cost (FFN-up forward at 1024 rows: 22.7 against 28.5 us in TF32 mode, 37.0 against 56.2 us in 3xTF32 mode).
         const bool short_single_round = automatic && pair_tiles <= max_pairs && p.num_kb <= 32 && 2 * pair_tiles >= max_pairs;
-        if (in.opt_stream_k < 0 || (in.opt_stream_k == 0 && (whole_eff >= 0.97 || short_single_round))) {
+        if (automatic && in.layers && whole_eff < 0.97 && !short_single_round)
+            parts = plan_one_wave(in, p.num_kb, tiles128, double(pair_kb) / double(pairs_busy), split_allowed, bytes_per_split);
+        if (parts > 0) {
+            pair = false;
+            force128 = true;
+        } else if (in.opt_stream_k < 0 || (in.opt_stream_k == 0 && (whole_eff >= 0.97 || short_single_round))) {
             p.sk_unit = p.num_kb;   // whole tiles, as evenly as they go
             pairs = whole_pairs;
             p.sk_max_share = 1;
@@ -297,8 +323,10 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
             }
             if (p.sk_max_share == 1) p.workspace_bytes = 0;   // every boundary fell between tiles
         }
-        p.grid = 2 * static_cast<int>(pairs);
-        return p;
+        if (pair) {
+            p.grid = 2 * static_cast<int>(pairs);
+            return p;
+        }
     }
     int bn = in.opt_tile_n;
     if (bn != 128 && bn != 256) {
@@ -310,7 +338,7 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
     p.tiles_m = (in.M + kPlanBM - 1) / kPlanBM;
     p.tiles_n = (in.N + bn - 1) / bn;
     const long long tiles = 1LL * p.tiles_m * p.tiles_n;
-    const int splits = plan_splits(in, tiles, p.num_kb, split_allowed, bytes_per_split, in.num_sms);
+    const int splits = parts > 0 ? parts : plan_splits(in, tiles, p.num_kb, split_allowed, bytes_per_split, in.num_sms);
     p.kb_per_split = (p.num_kb + splits - 1) / splits;
     p.splits = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
     const long long items = tiles * p.splits;

@@ -126,7 +126,8 @@ int gptb200_selftest_grid_barrier(gptb200_ctx *ctx, int polls);
  * default options).  plan8 = {kernel (0 none, 1 CTA-pair tcgen05, 2 one-CTA tcgen05, 3 weight streaming, 4 SIMT), tile_n,
  * tiles_m, tiles_n, split_k, k-blocks (or k elements for kernel 3) per split, CTAs, scratch KiB}.  For kernel 1 split_k is the
  * largest number of CTA pairs that work on one 256 x 256 tile (1: every pair computes whole tiles) and the next field the
- * k-blocks per CTA pair.  (gptb200_linear_forward may split k in spite of an epilogue, which the reduction then applies; the plan here keeps it in the product.) */
+ * k-blocks per CTA pair.  (The linear layers' calls may split k in spite of an epilogue, which the reduction then applies, and may
+ * take one wave of 128 x 128 one-CTA tiles where ranges would be cut inside tiles: not shown here.) */
 int gptb200_plan_gemm(int num_sms, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate, int *plan8);
 /* For a call that gptb200_plan_gemm sends to the weight-streaming kernels (kernel 3: at most 64 rows): which of them runs with
  * default options, host logic only.  w_kn_major: the weight is stored [k][n] (linear layers) rather than [n][k] (un-embedding,

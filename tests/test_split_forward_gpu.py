@@ -67,3 +67,21 @@ def test_rows_in_three_parts(m, k, n):
     for new, old in zip(errors[1], errors[0]):
         assert new <= 5e-7 and new <= max(1.1 * old, 1.5e-7), errors
     be.close()
+
+
+@pytest.mark.parametrize("m,k,n", [(600, 768, 3072), (1540, 768, 2304), (1000, 260, 1028), (2050, 3072, 768)])
+@pytest.mark.parametrize("mode,tol", [(0, 1e-5), (1, 2e-3)])
+def test_one_wave_of_tiles_backward(m, k, n, mode, tol):
+    """Weight and input gradients as one wave of one-CTA tiles, whole and in parts of k: added to what is there, tolerances of the modes."""
+    import torch
+    import gpt_b200
+    x, w, b, _ = _problem(torch, m, k, n, m + n)
+    gy = torch.randn(m, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(m))
+    be = gpt_b200.Backend(0, torch.cuda.current_stream().cuda_stream, mode)
+    gx, gw, gb = torch.full((m + 1, k), 7.0, device="cuda"), torch.full_like(w, 3.0), torch.full((n,), 5.0, device="cuda")
+    be.device_linear_backward(gx, gw, gb, gy, x, w, 1, m, k, n)
+    be.synchronize()
+    for got, want in ((gx[:m], gy.double() @ w.double().t()), (gw, x.double().t() @ gy.double() + 3.0), (gb, gy.double().sum(0) + 5.0)):
+        assert float((got.double() - want).abs().max()) <= tol * float(want.abs().max())
+    assert (gx[m] == 7).all()
+    be.close()
