@@ -930,9 +930,10 @@ private:
             int longest = 0;
             for (int i = 0; i < n; ++i) longest = std::max(longest, parts[entry0 + i].count);
             const int blocks = s.heads * ((s.vdim + kChunkCols - 1) / kChunkCols);
-            // of the option's tokens, or shorter where the heads and requests of a step leave blocks of the machine (two per SM) idle: a chunk after the
-            // other takes 5 us, the pass for the states in front of the segments half of what it saves (three prompts of 870 tokens, 12 heads of 64)
-            constexpr int kShortestSegment = 256;
+            // of the option's tokens, or shorter where the heads and requests of a step leave blocks of the machine (two per SM) idle.  Whole prompts, us, at segments
+            // of 64 / 128 / 256 / 512 tokens: 768 wide, three of 870 tokens 1 742 / 1 702 / 1 746 / 1 877, one of 900 1 615 / 1 590 / 1 673 / 1 824, of 3000 2 960 /
+            // 2 841 / 2 787 / 2 963; 2048 wide, 4096 tokens 7 775 / 7 059 / 6 820 / 6 972
+            constexpr int kShortestSegment = 128;
             int segment = segment_tokens_;
             if (segment_auto_) {
                 const int side_by_side = std::max(1, 2 * ctx_->num_sms / (blocks * n));
@@ -940,18 +941,22 @@ private:
             }
             const int tokens = longest > segment + segment / 2 ? segment : pad_to(longest, kChunk);
             const int segments = (longest + tokens - 1) / tokens;
-            const size_t smem = size_t(chunk_smem_bytes(s.state));
+            const int tiles = chunk_state_tiles(s.state);
+            const size_t smem = size_t(chunk_smem_bytes(tiles));
             float *seg_state = nullptr, *seg_decay = nullptr;
+            const auto chunks = [&](auto kernel, int count) {
+                return launch(kernel, dim3(blocks, n, count), dim3(kChunkThreads), smem, ssm_y_, in.rows, in.ld, in.steps, in.log_decay, in.ld_decay, in.skip, s, entries_ + entry0, tokens, segments,
+                              seg_state, seg_decay);
+            };
             if (segments > 1) {
                 const size_t pieces = size_t(n) * s.heads * segments;
                 RC_TRY(scratch(pieces * (size_t(s.state) * s.vdim + 1)));
                 seg_state = scratch_;
                 seg_decay = scratch_ + pieces * s.state * s.vdim;
-                RC_TRY(launch(mamba_chunk_kernel<true>, dim3(blocks, n, segments - 1), dim3(kChunkThreads), smem, ssm_y_, in.rows, in.ld, in.steps, in.log_decay, in.ld_decay, in.skip, s,
-                              entries_ + entry0, tokens, segments, seg_state, seg_decay));
+                RC_TRY(tiles == 4 ? chunks(mamba_chunk_kernel<true, 4>, segments - 1) : chunks(mamba_chunk_kernel<true, 8>, segments - 1));
+                RC_TRY(launch(mamba_segments_kernel, dim3(s.heads * ((s.state * s.vdim + 255) / 256), n), dim3(256), 0, seg_state, seg_decay, s, entries_ + entry0, tokens, segments));
             }
-            return launch(mamba_chunk_kernel<false>, dim3(blocks, n, segments), dim3(kChunkThreads), smem, ssm_y_, in.rows, in.ld, in.steps, in.log_decay, in.ld_decay, in.skip, s,
-                          entries_ + entry0, tokens, segments, seg_state, seg_decay);
+            return tiles == 4 ? chunks(mamba_chunk_kernel<false, 4>, segments) : chunks(mamba_chunk_kernel<false, 8>, segments);
         }
     }
 

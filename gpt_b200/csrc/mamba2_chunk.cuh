@@ -4,13 +4,19 @@
 // With a_t the running sum of log-decays inside a chunk and S the state before it,
 //   y_t = exp(a_t) C_t S + sum_{s <= t} exp(a_t - a_s) dt_s (C_t . B_s) x_s + D x_t
 //   S  <- exp(a_end) S + sum_s exp(a_end - a_s) dt_s B_s x_s^T
-// One block carries one head's state for 32 of its value columns through the chunks of a request, or of a segment of it: S stays in
-// fp32 accumulators from chunk to chunk, and the next chunk's x, B and C arrive while this one is computed.  Four warps
-// compute the outputs, four the state.  x, B and C are bf16 as the convolution left them; everything that is fp32 by nature (weights with
-// decays and steps, the scaled x, the state) enters a product as the sum of two bf16 values.
+// One block carries one head's state for 64 of its value columns through the chunks of a request, or of a segment of it, and the next chunk's x, B and C
+// arrive while this one is computed.  x, B and C are bf16 as the convolution left them; everything that is fp32 by nature (weights with decays and steps, the
+// scaled x, the state) enters a product as the sum of two bf16 values.
+//
+// Four warps keep the state, 16 value columns each, transposed in fp32 accumulators: as such they are the left operand of y^T = S^T C^T, so that the state never
+// passes through shared memory and nothing waits for it.  Four warps compute the weights of the chunk's keys, C . B with decays and steps, for all of them.
+// Bound by the state warps' chain of products (two blocks per SM: tensor pipe 38 % busy).  4096 tokens, 64 heads of 64 x 128, us for all launches: 307 with 32
+// columns per block, the state handed to output warps as two bf16 terms in shared memory; 264 as now, 191 with sizes known at compile time, 171 with all tokens
+// of a chunk at once (the products of eight sums alternate, a state is split once) and the segments' initial states from a launch of their own.  Three prompts of
+// 870 tokens, 12 heads of 64 x 64: 43 / 33.
 //
 // Long requests are cut into segments that run side by side: a first launch computes what each segment alone adds to the state and by
-// how much it lets earlier state decay; in the second every block puts its segment's initial state together from those.
+// how much it lets earlier state decay, a second one turns those into the segments' initial states, the third computes the outputs.
 #pragma once
 
 #include "mamba2.cuh"
@@ -19,7 +25,7 @@ namespace gptb200 {
 namespace dec {
 
 constexpr int kChunk = 64;
-constexpr int kChunkCols = 32;       // value columns per block
+constexpr int kChunkCols = 64;       // value columns per block
 constexpr int kChunkThreads = 256;
 constexpr int kChunkMaxState = 128;
 
@@ -71,17 +77,21 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t &hi, uint32_t 
 
 }  // namespace mma16
 
-__host__ __device__ inline int chunk_smem_bytes(int state)
+// 16-wide tiles of the state's rows, a size known at compile time: with run-time bounds every product had a branch around it (2 200 instead of 1 000
+// instructions per warp and chunk).  Rows beyond the state are zeros.
+__host__ __device__ constexpr int chunk_state_tiles(int state) { return state <= 64 ? 4 : 8; }
+
+__host__ __device__ constexpr int chunk_smem_bytes(int tiles)
 {
-    const int n = (state + 15) / 16 * 16, np = (n + 8) * 2, xp = (kChunkCols + 8) * 2;
-    return 2 * kChunk * (2 * np + xp) + 2 * kChunk * xp + 2 * n * xp + 2 * 4 * kChunk * 4;
+    const int np = (16 * tiles + 8) * 2, xp = (kChunkCols + 8) * 2, wp = (kChunk + 8) * 2;
+    return 2 * kChunk * (2 * np + xp) + 2 * kChunk * wp + 2 * 4 * kChunk * 4;
 }
 
 // SEGMENT_STATES: only what a segment adds to the state, from zero, into segment_state [entry][head][segment][state][vdim] and the
 // segment's decay into segment_decay [entry][head][segment]; the last segment is left out.  Otherwise outputs and, in the last
 // segment, the request's new state.  dt null: steps of one; ld_decay: row pitch of log_decay (0: constant decays); d_skip null: none.
 // grid: (heads * column slices, entries, segments)
-template <bool SEGMENT_STATES>
+template <bool SEGMENT_STATES, int NT>
 __global__ void __launch_bounds__(kChunkThreads, 2)
 mamba_chunk_kernel(float *__restrict__ y, const __nv_bfloat16 *__restrict__ xbc, int ld_xbc, const float *__restrict__ dt, const float *__restrict__ log_decay, int ld_decay,
                    const float *__restrict__ d_skip, const RecurrentShape s, const StepEntry *__restrict__ entries, int segment_tokens, int max_segments, float *__restrict__ segment_state,
@@ -99,21 +109,24 @@ mamba_chunk_kernel(float *__restrict__ y, const __nv_bfloat16 *__restrict__ xbc,
 
     const int slices = (s.vdim + kChunkCols - 1) / kChunkCols;
     const int h = blockIdx.x / slices, p0 = (blockIdx.x % slices) * kChunkCols;
-    const int P = s.vdim, N = s.state, n16 = (N + 15) / 16, NP = n16 * 16;
+    const int P = s.vdim, N = s.state;
+    constexpr int NP = 16 * NT;
     const int g = h / (s.heads / s.groups);
     const int cols = min(kChunkCols, P - p0);
-    const int np = (NP + 8) * 2, xp = (kChunkCols + 8) * 2;   // row pitches in bytes
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool state_role = warp >= 4;
+    constexpr int np = (NP + 8) * 2, xp = (kChunkCols + 8) * 2, wp = (kChunk + 8) * 2;   // row pitches in bytes
+    const int warp = ptx::warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const bool score_role = !SEGMENT_STATES && warp >= 4;
     const int rw = warp & 3;      // warp within its role
-    // shared memory: two buffers of [B | C | x], scaled x (two terms), state (two terms), per-token values of two chunks
-    const int buf_bytes = kChunk * (2 * np + xp);
+    // shared memory: two buffers of [B | C | x], weights of the keys (two terms), per-token values of two chunks
+    // (for states alone: four buffers of [B | x], so that a chunk's copies have three chunks' time)
+    constexpr int kBufs = SEGMENT_STATES ? 4 : 2, buf_bytes = kChunk * ((SEGMENT_STATES ? 1 : 2) * np + xp);
+    static_assert(kBufs * buf_bytes <= 2 * kChunk * (2 * np + xp) + 2 * kChunk * wp, "shared memory");
     const uint32_t base = ptx::smem_u32(chunk_smem);
-    const uint32_t wx = base + 2 * buf_bytes, st = wx + 2 * kChunk * xp;
-    float *tokens = reinterpret_cast<float *>(chunk_smem + 2 * buf_bytes + 2 * kChunk * xp + 2 * NP * xp);
+    const uint32_t wt = base + kBufs * buf_bytes;
+    float *tokens = reinterpret_cast<float *>(chunk_smem + 2 * kChunk * (2 * np + xp) + 2 * kChunk * wp);
     auto tile_b = [&](int b) { return base + b * buf_bytes; };
     auto tile_c = [&](int b) { return base + b * buf_bytes + kChunk * np; };
-    auto tile_x = [&](int b) { return base + b * buf_bytes + 2 * kChunk * np; };
+    auto tile_x = [&](int b) { return base + (b + 1) * buf_bytes - kChunk * xp; };
     // running log2-decay, step, decay since the chunk's start, decay to its end times step
     auto cum = [&](int b) { return tokens + b * 4 * kChunk; };
     auto step = [&](int b) { return tokens + b * 4 * kChunk + kChunk; };
@@ -125,6 +138,7 @@ mamba_chunk_kernel(float *__restrict__ y, const __nv_bfloat16 *__restrict__ xbc,
     const float *old_state = state + e.parity * state_floats;
     const long long seg0 = (static_cast<long long>(blockIdx.y) * s.heads + h) * max_segments;
     const bool vec = P % 8 == 0 && N % 8 == 0;    // all column offsets are then multiples of 8
+    const bool whole = vec && N == NP && cols == kChunkCols;
     const int off_b = s.inner + g * N, off_c = off_b + s.groups * N;
 
     // One piece of eight columns of a row: 16-byte asynchronous copy, or plain loads where columns are unaligned or end.
@@ -143,14 +157,35 @@ mamba_chunk_kernel(float *__restrict__ y, const __nv_bfloat16 *__restrict__ xbc,
     };
     // four threads per token
     auto fetch = [&](int chunk, int b) {
+        if (chunk * kChunk >= count) {   // beyond the segment: an empty group, so that waits count alike
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            return;
+        }
         const int t = threadIdx.x >> 2, q0 = threadIdx.x & 3;
         const bool in = chunk * kChunk + t < count;
         const __nv_bfloat16 *row = xbc + static_cast<long long>(first_row + (in ? chunk * kChunk + t : 0)) * ld_xbc;
+        if (whole) {   // rows beyond the segment are filled with zeros
+            const int bytes = in ? 16 : 0;
+            auto copy = [&](uint32_t dst, const __nv_bfloat16 *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory"); };
+            const uint32_t to = tile_b(b) + t * np + q0 * 16, x_to = tile_x(b) + t * xp + q0 * 16;
+            const __nv_bfloat16 *sb = row + off_b + q0 * 8, *sc = row + off_c + q0 * 8, *sx = row + h * P + p0 + q0 * 8;
+#pragma unroll
+            for (int i = 0; i < NP / 32; ++i) {
+                copy(to + i * 64, sb + i * 32);
+                if (!SEGMENT_STATES) copy(to + kChunk * np + i * 64, sc + i * 32);
+            }
+#pragma unroll
+            for (int i = 0; i < kChunkCols / 32; ++i) copy(x_to + i * 64, sx + i * 32);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            return;
+        }
+#pragma unroll 1
         for (int q = q0; q < NP / 8; q += 4) {
             piece(tile_b(b) + t * np + q * 16, row + off_b + q * 8, in ? min(8, N - q * 8) : 0);
             if (!SEGMENT_STATES) piece(tile_c(b) + t * np + q * 16, row + off_c + q * 8, in ? min(8, N - q * 8) : 0);
         }
-        piece(tile_x(b) + t * xp + q0 * 16, row + h * P + p0 + q0 * 8, in ? min(8, cols - q0 * 8) : 0);
+#pragma unroll 1
+        for (int q = q0; q < kChunkCols / 8; q += 4) piece(tile_x(b) + t * xp + q * 16, row + h * P + p0 + q * 8, in ? min(8, cols - q * 8) : 0);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     // per-token values of a chunk by one warp, two tokens per lane: load early, finish later
@@ -180,193 +215,220 @@ mamba_chunk_kernel(float *__restrict__ y, const __nv_bfloat16 *__restrict__ xbc,
     };
 
     const int r = lane >> 2, c2 = (lane & 3) * 2;
-    // state fragments of the state warps: row tiles rw and rw + 4 of 16 state rows, four tiles of 8 columns
-    float S[2][4][4];
-    float decay_all = 1.0f;
-    fetch(0, 0);
-    if (warp == 7) load_tokens(0);
-    if (state_role) {
-        auto each = [&](auto &&f) {
+    // The state of value columns 16 rw ... of this slice: S[j] are 16 columns (rows of the fragment) by state rows 16 k0 + 8 j ...  Without outputs to compute, all
+    // eight warps keep states, half of the state rows each.
+    constexpr bool kSplitRegs = !SEGMENT_STATES && NT == 8;
+    constexpr int kTiles = SEGMENT_STATES ? NT / 2 : NT;      // of 16 state rows
+    constexpr int kBatch = kTiles < 4 ? kTiles : 4;           // tiles whose products alternate: a sum is added to every eight products
+    const int k0 = SEGMENT_STATES ? (warp >> 2) * kTiles : 0;
+    const bool idle = rw * 16 >= cols;                        // no value columns here
+    const int chunks = (count + kChunk - 1) / kChunk;
+    auto begin_chunk = [&](int ch) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 2) : "memory");
+        __syncthreads();   // this chunk's tiles and token values are there, the buffer of the chunk before and the weights are free
+        fetch(ch + kBufs - 1, (ch + kBufs - 1) % kBufs);
+        if (warp == 4 && ch + 1 < chunks) load_tokens(ch + 1);
+    };
 #pragma unroll
-            for (int k = 0; k < 2; ++k)
+    for (int i = 0; i < kBufs - 1; ++i) fetch(i, i);
+    if (warp == 4) {
+        load_tokens(0);
+        finish_tokens(0);
+    }
+    if (score_role) {
+        if (kSplitRegs) ptx::reg_dec<96>();
+        for (int ch = 0; ch < chunks; ++ch) {
+            const int b = ch & 1;
+            begin_chunk(ch);
+            // 16 rows of the chunk against its keys
+            float G[8][4] = {};
+#pragma unroll 2
+            for (int k = 0; k < NT; ++k) {
+                uint32_t a[4], f[4][4];
+                a_frag(a, tile_c(b), np, rw * 16, k * 16, lane);
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
+                    if (j <= rw) b_frag(f[j], tile_b(b), np, j * 16, k * 16, lane);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int n = (rw + 4 * k) * 16 + r + (i >> 1) * 8, p = j * 8 + c2 + (i & 1);
-                        f(S[k][j][i], n < N && p < cols, static_cast<long long>(n) * P + p);
+                for (int j = 0; j < 4; ++j)
+                    if (j <= rw) {
+                        mma(G[2 * j], a, f[j][0], f[j][1]);
+                        mma(G[2 * j + 1], a, f[j][2], f[j][3]);
                     }
-        };
-        if (SEGMENT_STATES) {
-            each([&](float &v, bool, long long) { v = 0.0f; });
-        } else {
-            each([&](float &v, bool ok, long long at) { v = ok ? old_state[at] : 0.0f; });
-            for (int i = 0; i < segment; ++i) {
-                const float keep = segment_decay[seg0 + i];
-                const float *add = segment_state + (seg0 + i) * N * P + p0;
-                each([&](float &v, bool ok, long long at) { v = ok ? fmaf(v, keep, add[at]) : 0.0f; });
             }
+            // decayed, stepped, causal
+            const int ta = rw * 16 + r, tb = ta + 8;
+            const float ca = cum(b)[ta], cb = cum(b)[tb];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (j > 2 * rw + 1) continue;
+                const int key = j * 8 + c2;
+                const float2 sk = *reinterpret_cast<const float2 *>(step(b) + key), ck = *reinterpret_cast<const float2 *>(cum(b) + key);
+                const float w00 = key <= ta ? G[j][0] * exp2f(ca - ck.x) * sk.x : 0.0f, w01 = key + 1 <= ta ? G[j][1] * exp2f(ca - ck.y) * sk.y : 0.0f;
+                const float w10 = key <= tb ? G[j][2] * exp2f(cb - ck.x) * sk.x : 0.0f, w11 = key + 1 <= tb ? G[j][3] * exp2f(cb - ck.y) * sk.y : 0.0f;
+                uint32_t hi, lo;
+                const uint32_t at = wt + ta * wp + key * 2;
+                split2(w00, w01, hi, lo);
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(hi) : "memory");
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + kChunk * wp), "r"(lo) : "memory");
+                split2(w10, w11, hi, lo);
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + 8 * wp), "r"(hi) : "memory");
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + (kChunk + 8) * wp), "r"(lo) : "memory");
+            }
+            asm volatile("bar.arrive 1, %0;" ::"n"(kChunkThreads) : "memory");
+            if (warp == 4 && ch + 1 < chunks) finish_tokens(b ^ 1);
         }
+        return;
     }
-    if (warp == 7) finish_tokens(0);
+    if (kSplitRegs) ptx::reg_inc<160>();   // 128 x 96 + 128 x 160 = 256 x 128 registers
+    float S[2 * kTiles][4] = {};
+    float decay_all = 1.0f;
+    auto each = [&](auto &&f) {
+#pragma unroll
+        for (int j = 0; j < 2 * kTiles; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int n = k0 * 16 + j * 8 + c2 + (i & 1), p = rw * 16 + r + (i >> 1) * 8;
+                f(S[j][i], n < N && p < cols, n * P + p);
+            }
+    };
+    if (!SEGMENT_STATES) {
+        const float *init = segment == 0 ? old_state : segment_state + (seg0 + segment - 1) * N * P + p0;
+        each([&](float &v, bool ok, int at) { v = ok ? init[at] : 0.0f; });
+    }
     const float skip = d_skip ? d_skip[h] : 0.0f;
-    const int chunks = (count + kChunk - 1) / kChunk;
     for (int ch = 0; ch < chunks; ++ch) {
         const int b = ch & 1, t0 = ch * kChunk;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();   // this chunk's tiles and token values are there, the other buffer is free
-        if (ch + 1 < chunks) {
-            fetch(ch + 1, b ^ 1);
-            if (warp == 7) load_tokens(ch + 1);
-        }
-        // scaled x and the state before the chunk, as two bf16 terms each
-        {
-            const float *dn = down(b);
-            for (int i = threadIdx.x; i < kChunk * (kChunkCols / 2); i += kChunkThreads) {
-                const int t = i / (kChunkCols / 2), q = i % (kChunkCols / 2);
-                uint32_t xv, hi, lo;
-                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(xv) : "r"(tile_x(b) + t * xp + q * 4) : "memory");
-                split2(dn[t] * bf16_lo(xv), dn[t] * bf16_hi(xv), hi, lo);
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(wx + t * xp + q * 4), "r"(hi) : "memory");
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(wx + kChunk * xp + t * xp + q * 4), "r"(lo) : "memory");
+        begin_chunk(ch);
+        if (!SEGMENT_STATES) {
+            float Y[8][4] = {};   // eight tokens each
+            // contribution of the state before the chunk
+#pragma unroll
+            for (int k = 0; k < kTiles; ++k) {
+                uint32_t hi[4], lo[4], f[4][4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) b_frag(f[t], tile_c(b), np, t * 16, k * 16, lane);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) split2(S[2 * k + (i >> 1)][2 * (i & 1)], S[2 * k + (i >> 1)][2 * (i & 1) + 1], hi[i], lo[i]);
+#pragma unroll
+                for (int t = 0; t < 8; ++t) mma(Y[t], hi, f[t >> 1][2 * (t & 1)], f[t >> 1][2 * (t & 1) + 1]);
+#pragma unroll
+                for (int t = 0; t < 8; ++t) mma(Y[t], lo, f[t >> 1][2 * (t & 1)], f[t >> 1][2 * (t & 1) + 1]);
             }
-        }
-        if (state_role && !SEGMENT_STATES) {
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (rw + 4 * k < n16) {
+            for (int t = 0; t < 8; ++t) {
+                const float2 u = *reinterpret_cast<const float2 *>(up(b) + t * 8 + c2);
+                Y[t][0] *= u.x;
+                Y[t][1] *= u.y;
+                Y[t][2] *= u.x;
+                Y[t][3] *= u.y;
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kChunkThreads) : "memory");   // the weights of the keys are there
+            if (!idle) {
+                // the chunk's own tokens up to each row
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                for (int kk = 0; kk < 4; ++kk) {
+                    uint32_t x[4], f[4][4];
+                    a_frag_t(x, tile_x(b), xp, kk * 16, rw * 16, lane);
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            uint32_t hi, lo;
-                            split2(S[k][j][2 * half], S[k][j][2 * half + 1], hi, lo);
-                            const uint32_t at = st + ((rw + 4 * k) * 16 + r + 8 * half) * xp + (j * 8 + c2) * 2;
-                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(hi) : "memory");
-                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + NP * xp), "r"(lo) : "memory");
+                    for (int term = 0; term < 2; ++term) {
+#pragma unroll
+                        for (int t = kk; t < 4; ++t) b_frag(f[t], wt + term * kChunk * wp, wp, t * 16, kk * 16, lane);
+#pragma unroll
+                        for (int t = 2 * kk; t < 8; ++t) mma(Y[t], x, f[t >> 1][2 * (t & 1)], f[t >> 1][2 * (t & 1) + 1]);
+                    }
+                }
+                // rows of the fragment are value columns: a quarter warp writes 32 bytes of a token
+                float *dst = y + static_cast<long long>(first_row + t0 + c2) * s.inner + h * P + p0 + rw * 16 + r;
+                const int left = count - (t0 + c2), below = cols - (rw * 16 + r);
+                const bool all = t0 + kChunk <= count && cols == kChunkCols;
+#pragma unroll
+                for (int t = 0; t < 8; t += 2) {
+                    uint32_t x[4];
+                    a_frag_t(x, tile_x(b), xp, t * 8, rw * 16, lane);
+#pragma unroll
+                    for (int q = t; q < t + 2; ++q) {
+                        float v[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const uint32_t xv = x[2 * (q & 1) + (i >> 1)];
+                            v[i] = fmaf(skip, (i & 1) ? bf16_hi(xv) : bf16_lo(xv), Y[q][i]);
                         }
-                }
-            }
-        }
-        __syncthreads();
-        if (state_role) {
-            // the state after the chunk
-            const float keep = up(b)[kChunk - 1];
-            decay_all *= keep;
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (rw + 4 * k < n16) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) S[k][j][i] *= keep;
-#pragma unroll
-                    for (int kk = 0; kk < kChunk / 16; ++kk) {
-                        uint32_t a[4], f[4];
-                        a_frag_t(a, tile_b(b), np, kk * 16, (rw + 4 * k) * 16, lane);
-#pragma unroll
-                        for (int term = 0; term < 2; ++term)
-#pragma unroll
-                            for (int j = 0; j < 2; ++j) {
-                                b_frag_t(f, wx + term * kChunk * xp, xp, kk * 16, j * 16, lane);
-                                mma(S[k][2 * j], a, f[0], f[1]);
-                                mma(S[k][2 * j + 1], a, f[2], f[3]);
-                            }
-                    }
-                }
-            }
-            if (warp == 7 && ch + 1 < chunks) finish_tokens(b ^ 1);
-            continue;
-        }
-        if (SEGMENT_STATES) continue;
-        // this warp's 16 rows of the chunk: contribution of the state, scores against the chunk's keys
-        float Y[4][4] = {}, G[8][4] = {};
-        for (int k = 0; k < n16; ++k) {
-            uint32_t a[4], f[4];
-            a_frag(a, tile_c(b), np, rw * 16, k * 16, lane);
-#pragma unroll
-            for (int term = 0; term < 2; ++term)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    b_frag_t(f, st + term * NP * xp, xp, k * 16, j * 16, lane);
-                    mma(Y[2 * j], a, f[0], f[1]);
-                    mma(Y[2 * j + 1], a, f[2], f[3]);
-                }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j <= rw) {
-                    b_frag(f, tile_b(b), np, j * 16, k * 16, lane);
-                    mma(G[2 * j], a, f[0], f[1]);
-                    mma(G[2 * j + 1], a, f[2], f[3]);
-                }
-        }
-        const int ta = rw * 16 + r, tb = ta + 8;
-        const float ua = up(b)[ta], ub = up(b)[tb], ca = cum(b)[ta], cb = cum(b)[tb];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            Y[j][0] *= ua;
-            Y[j][1] *= ua;
-            Y[j][2] *= ub;
-            Y[j][3] *= ub;
-        }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            if (kk > rw) continue;
-            // 16 keys as the A operand: decayed, stepped, causal
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int key = kk * 16 + q * 8 + c2;
-                float (&gq)[4] = G[2 * kk + q];
-                const float2 sk = *reinterpret_cast<const float2 *>(step(b) + key), ck = *reinterpret_cast<const float2 *>(cum(b) + key);
-                const float w00 = key <= ta ? gq[0] * exp2f(ca - ck.x) * sk.x : 0.0f, w01 = key + 1 <= ta ? gq[1] * exp2f(ca - ck.y) * sk.y : 0.0f;
-                const float w10 = key <= tb ? gq[2] * exp2f(cb - ck.x) * sk.x : 0.0f, w11 = key + 1 <= tb ? gq[3] * exp2f(cb - ck.y) * sk.y : 0.0f;
-                split2(w00, w01, hi[2 * q], lo[2 * q]);
-                split2(w10, w11, hi[2 * q + 1], lo[2 * q + 1]);
-            }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                uint32_t f[4];
-                b_frag_t(f, tile_x(b), xp, kk * 16, j * 16, lane);
-                mma(Y[2 * j], hi, f[0], f[1]);
-                mma(Y[2 * j], lo, f[0], f[1]);
-                mma(Y[2 * j + 1], hi, f[2], f[3]);
-                mma(Y[2 * j + 1], lo, f[2], f[3]);
-            }
-        }
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int t = half ? tb : ta;
-            if (t0 + t < count) {
-                float *dst = y + static_cast<long long>(first_row + t0 + t) * s.inner + h * P + p0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int p = j * 8 + c2;
-                    uint32_t xv;
-                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(xv) : "r"(tile_x(b) + t * xp + p * 2) : "memory");
-                    const float v0 = fmaf(skip, bf16_lo(xv), Y[j][2 * half]), v1 = fmaf(skip, bf16_hi(xv), Y[j][2 * half + 1]);
-                    if (vec && p + 1 < cols) {
-                        *reinterpret_cast<float2 *>(dst + p) = make_float2(v0, v1);
-                    } else {
-                        if (p < cols) dst[p] = v0;
-                        if (p + 1 < cols) dst[p + 1] = v1;
+                        float *even = dst, *odd = dst + s.inner;
+                        if (all) {
+                            even[0] = v[0];
+                            odd[0] = v[1];
+                            even[8] = v[2];
+                            odd[8] = v[3];
+                        } else {
+                            if (q * 8 < left && 0 < below) even[0] = v[0];
+                            if (q * 8 + 1 < left && 0 < below) odd[0] = v[1];
+                            if (q * 8 < left && 8 < below) even[8] = v[2];
+                            if (q * 8 + 1 < left && 8 < below) odd[8] = v[3];
+                        }
+                        dst += 8 * s.inner;
                     }
                 }
             }
         }
-    }
-    if (state_role && (SEGMENT_STATES || last_segment)) {
-        float *dst = SEGMENT_STATES ? segment_state + (seg0 + segment) * N * P + p0 : state + (e.parity ^ 1) * state_floats;
+        // the state after the chunk
+        const float keep = up(b)[kChunk - 1];
+        decay_all *= keep;
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
+        for (int j = 0; j < 2 * kTiles; ++j)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int i = 0; i < 4; ++i) S[j][i] *= keep;
+        if (!idle) {
+#pragma unroll SEGMENT_STATES ? 4 : 2
+            for (int kk = 0; kk < kChunk / 16; ++kk) {
+                uint32_t x[4], hi[4], lo[4];
+                a_frag_t(x, tile_x(ch % kBufs), xp, kk * 16, rw * 16, lane);
+                const float2 d0 = *reinterpret_cast<const float2 *>(down(b) + kk * 16 + c2), d1 = *reinterpret_cast<const float2 *>(down(b) + kk * 16 + 8 + c2);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int n = (rw + 4 * k) * 16 + r + (i >> 1) * 8, p = j * 8 + c2 + (i & 1);
-                    if (n < N && p < cols) dst[static_cast<long long>(n) * P + p] = S[k][j][i];
+                    const float2 d = i < 2 ? d0 : d1;
+                    split2(d.x * bf16_lo(x[i]), d.y * bf16_hi(x[i]), hi[i], lo[i]);
                 }
-        if (SEGMENT_STATES && p0 == 0 && warp == 4 && lane == 0) segment_decay[seg0 + segment] = decay_all;
+#pragma unroll
+                for (int k = 0; k < kTiles; k += kBatch) {
+                    uint32_t f[kBatch][4];
+#pragma unroll
+                    for (int j = 0; j < kBatch; ++j) b_frag_t(f[j], tile_b(ch % kBufs), np, kk * 16, (k0 + k + j) * 16, lane);
+#pragma unroll
+                    for (int term = 0; term < 2; ++term)
+#pragma unroll
+                        for (int j = 0; j < 2 * kBatch; ++j) mma(S[2 * k + j], term ? lo : hi, f[j >> 1][2 * (j & 1)], f[j >> 1][2 * (j & 1) + 1]);
+                }
+            }
+        }
+        if (SEGMENT_STATES && warp == 4 && ch + 1 < chunks) finish_tokens(b ^ 1);
+    }
+    if (SEGMENT_STATES || last_segment) {
+        float *dst = SEGMENT_STATES ? segment_state + (seg0 + segment) * N * P + p0 : state + (e.parity ^ 1) * state_floats;
+        each([&](float &v, bool ok, int at) {
+            if (ok) dst[at] = v;
+        });
+        if (SEGMENT_STATES && p0 == 0 && warp == 0 && lane == 0) segment_decay[seg0 + segment] = decay_all;
+    }
+}
+
+// What the segments add -> the states after them: segment_state[i] <- decay_i * (state before) + segment_state[i].
+// grid: (heads * blocks of 256 state values, entries)
+__global__ void mamba_segments_kernel(float *__restrict__ segment_state, const float *__restrict__ segment_decay, const RecurrentShape s, const StepEntry *__restrict__ entries,
+                                      int segment_tokens, int max_segments)
+{
+    grid_dependency_wait();
+    grid_dependency_launch();
+    const int size = s.state * s.vdim, blocks = (size + 255) / 256, h = blockIdx.x / blocks, at = blockIdx.x % blocks * 256 + threadIdx.x;
+    if (at >= size) return;
+    const StepEntry e = entries[blockIdx.y];
+    const long long seg0 = (static_cast<long long>(blockIdx.y) * s.heads + h) * max_segments;
+    const int segments = (e.count + segment_tokens - 1) / segment_tokens;
+    float v = reinterpret_cast<const float *>(e.slot + s.ssm_state)[(static_cast<long long>(e.parity) * s.heads + h) * size + at];
+    for (int i = 0; i + 1 < segments; ++i) {
+        float *add = segment_state + (seg0 + i) * size + at;
+        v = fmaf(v, segment_decay[seg0 + i], *add);
+        *add = v;
     }
 }
 

@@ -99,6 +99,20 @@ def test_large_heads_and_states(tmp_path, layers):
         model.close_model()
 
 
+@pytest.mark.parametrize("heads,vdim,state", [(2, 8, 8), (3, 72, 24), (1, 130, 40), (2, 64, 112), (1, 100, 128), (4, 5, 16)])
+def test_chunked_recurrence_of_any_slice(tmp_path, heads, vdim, state):
+    """Value columns that leave a slice of 64 or a warp's 16 partly empty, odd and even numbers of state tiles, chunks with remainders, with segments and without."""
+    c, w = build([dm.mamba(heads=heads, vdim=vdim, state=state, groups=1, norm_groups=1)], {}, {}, 24)
+    tokens = np.random.default_rng(29).integers(0, c["vocab"], 209)
+    want = budurax.forward(c, w, tokens)
+    model = load(tmp_path, c, w, "bfloat16")
+    for segment in (1024, 64, 128):
+        model.set_option("segment_tokens", segment)
+        for cuts in ((1 << 20,), (64, 8, 137)):
+            assert dm.close(whole(model, tokens, cuts), want, TOL["bfloat16"]), (segment, cuts)
+    model.close_model()
+
+
 def test_long_decoding(tmp_path):
     c, w = build(MIXED["layers"], {}, {}, 4)
     tokens = np.random.default_rng(9).integers(0, c["vocab"], 700)
