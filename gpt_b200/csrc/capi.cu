@@ -976,10 +976,11 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
                                  : launch_gemv(ctx, gemv_bf16_kernel<false>, g, std::max(1, std::min(need, ctx->num_sms * 4 / groups)), groups, size_t(c.K) * 2);
         }
         const int tiles = is_glu(c.out_kind) ? 2 : 1;   // a gate tile and its up tile
-        const int ctas = (widest + tiles * 16 - 1) / (tiles * 16);
+        int ctas = (widest + tiles * 16 - 1) / (tiles * 16);
         // fewer CTAs than two per SM: a cluster shares a tile's k, each CTA at least 512 of it
         int cluster = 1;
         while (cluster < kGemvMaxCluster && ctas * groups * cluster < 2 * ctx->num_sms && c.K / (cluster * 2) >= 512) cluster *= 2;
+        if (cluster == 1) ctas = std::min(ctas, std::max(1, 2 * ctx->num_sms / groups));   // as many as run at once
         return tiles == 2 ? launch_gemv(ctx, gemv_bf16_mma_kernel<2>, g, ctas, groups, 0, cluster) : launch_gemv(ctx, gemv_bf16_mma_kernel<1>, g, ctas, groups, 0, cluster);
     }
     const bool f32 = c.out_kind == OUT_F32;

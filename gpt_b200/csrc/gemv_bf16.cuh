@@ -181,6 +181,8 @@ gemv_bf16_kernel(const GemvParams p)
 // two products, values 0-3 the first and 4-7 the second.  While a warp multiplies, its next blocks' weights are on their way.
 // Layers with few weight rows: the CTAs of a cluster (blockIdx.z) share a tile's k, so that all SMs have loads in flight; their sums meet
 // in the first CTA's shared memory in rank order.  Eight rows of the 2048-wide models, the products of a step: 415 -> 395 us for 1.8 GB.
+// Otherwise no more CTAs than run at once, which walk over the tiles: the next tile's first weights travel while a tile's sums are added up.  Whole requests of the
+// linear-attention models, us, a CTA per tile / now: 2048 wide, eight of 32 tokens 19 100 / 17 773, three 16 908 / 15 839; 768 wide, four 10 663 / 10 341.
 // (TILES = 2 is for the gated kinds, 1 for the others.  With the kind known at compile time the gated form needs 12 registers less and a step of eight
 // sequences of the 2048-wide linear-attention model took 2 % longer.)
 constexpr int kGemvMmaUnroll = 4;   // blocks of 32 k and tiles per buffer of weights and warp: two buffers of 32 registers leave two CTAs per SM
@@ -206,15 +208,13 @@ gemv_bf16_mma_kernel(const GemvParams p)
     const int n0 = blockIdx.y * p.group_cols, N = min(p.N - n0, p.group_cols);   // this group's columns
     const int S = gridDim.z, rank = blockIdx.z;
     const uint16_t *w = p.w + static_cast<long long>(n0) * p.K;
-    // weight rows of the block's tiles
-    int row[TILES];
-#pragma unroll
-    for (int t = 0; t < TILES; ++t)
-        row[t] = is_glu(p.out_kind) ? (blockIdx.x >> 1) * 64 + (blockIdx.x & 1) * 16 + t * 32 : (blockIdx.x * TILES + t) * 16;
+    const int items = is_glu(p.out_kind) ? N / 32 : (N + TILES * 16 - 1) / (TILES * 16);
+    // weight rows of an item's tiles
+    auto row = [&](int item, int t) { return is_glu(p.out_kind) ? (item >> 1) * 64 + (item & 1) * 16 + t * 32 : (item * TILES + t) * 16; };
     const int blocks = (p.K + 31) / 32, per_warp = (blocks + 8 * S - 1) / (8 * S);
     const int first = min(blocks, (rank * 8 + warp) * per_warp), end = min(blocks, first + per_warp);
     uint4 wv[2][kUnroll][TILES][2];
-    auto fetch = [&](uint4 (&v)[kUnroll][TILES][2], int blk) {
+    auto fetch = [&](uint4 (&v)[kUnroll][TILES][2], int item, int blk) {
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
             const int k = (blk + u) * 32 + c * 8;
@@ -222,7 +222,7 @@ gemv_bf16_mma_kernel(const GemvParams p)
             for (int t = 0; t < TILES; ++t)
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    const int r = row[t] + g + 8 * half;
+                    const int r = row(item, t) + g + 8 * half;
                     v[u][t][half] = blk + u < end && k < p.K && r < N ? __ldg(reinterpret_cast<const uint4 *>(w + static_cast<long long>(r) * p.K + k)) : make_uint4(0u, 0u, 0u, 0u);
                 }
         }
@@ -246,53 +246,66 @@ gemv_bf16_mma_kernel(const GemvParams p)
             }
         }
     };
-    fetch(wv[0], first);
-    if (first + kUnroll < end) fetch(wv[1], first + kUnroll);
+    fetch(wv[0], blockIdx.x, first);
+    if (first + kUnroll < end) fetch(wv[1], blockIdx.x, first + kUnroll);
     grid_dependency_wait();
     grid_dependency_launch();
-    for (int blk = first; blk < end; blk += 2 * kUnroll) {
-        multiply(wv[0], blk);
-        if (blk + 2 * kUnroll < end) fetch(wv[0], blk + 2 * kUnroll);
-        if (blk + kUnroll < end) {
-            multiply(wv[1], blk + kUnroll);
-            if (blk + 3 * kUnroll < end) fetch(wv[1], blk + 3 * kUnroll);
+#pragma unroll 1
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {   // one item where a cluster shares k
+        const int next = item + gridDim.x;
+#pragma unroll
+        for (int t = 0; t < TILES; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[t][i] = 0.0f;
+        for (int blk = first; blk < end; blk += 2 * kUnroll) {
+            multiply(wv[0], blk);
+            if (blk + 2 * kUnroll < end)
+                fetch(wv[0], item, blk + 2 * kUnroll);
+            else if (next < items)   // the next item's first weights travel during the sums
+                fetch(wv[0], next, first);
+            if (blk + kUnroll < end) {
+                multiply(wv[1], blk + kUnroll);
+                if (blk + 3 * kUnroll < end) fetch(wv[1], item, blk + 3 * kUnroll);
+            }
+            if (blk + 2 * kUnroll >= end && next < items && first + kUnroll < end) fetch(wv[1], next, first + kUnroll);
         }
-    }
-    if (S > 1) cg::this_cluster().barrier_arrive();   // this CTA runs: its shared memory may be written once all have arrived
+        if (S > 1) cg::this_cluster().barrier_arrive();   // this CTA runs: its shared memory may be written once all have arrived
 #pragma unroll
-    for (int t = 0; t < TILES; ++t)
+        for (int t = 0; t < TILES; ++t)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sums[(warp * TILES * 16 + t * 16 + g + (i >> 1) * 8) * 8 + 2 * c + (i & 1)] = acc[t][i];
-    __syncthreads();
-    if (S > 1) {
-        cg::cluster_group cluster = cg::this_cluster();
-        cluster.barrier_wait();
-        if (rank > 0) {
-            float *there = cluster.map_shared_rank(from_others, 0) + (rank - 1) * kSums;
-            for (int i = threadIdx.x; i < kSums; i += kGemvThreads) {
+            for (int i = 0; i < 4; ++i) sums[(warp * TILES * 16 + t * 16 + g + (i >> 1) * 8) * 8 + 2 * c + (i & 1)] = acc[t][i];
+        __syncthreads();
+        if (S > 1) {
+            cg::cluster_group cluster = cg::this_cluster();
+            cluster.barrier_wait();
+            if (rank > 0) {
+                float *there = cluster.map_shared_rank(from_others, 0) + (rank - 1) * kSums;
+                for (int i = threadIdx.x; i < kSums; i += kGemvThreads) {
+                    float v = 0.0f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) v += sums[q * kSums + i];
+                    there[i] = v;
+                }
+            }
+            cluster.sync();   // nothing remote is touched after this
+            if (rank > 0) return;
+        }
+        const int outputs = is_glu(p.out_kind) ? 128 : kSums;
+        for (int i = threadIdx.x; i < outputs; i += kGemvThreads) {
+            const int r = i >> 3, m = i & 7;
+            if (m >= p.M) continue;
+            auto total = [&](int at) {
                 float v = 0.0f;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) v += sums[q * kSums + i];
-                there[i] = v;
-            }
+                for (int q = 0; q < 8; ++q) v += sums[q * kSums + at];
+                for (int q = 1; q < S; ++q) v += from_others[(q - 1) * kSums + at];
+                return v;
+            };
+            const float v = total(i), up = TILES == 2 && is_glu(p.out_kind) ? total(128 + i) : 0.0f;
+            const int n = is_glu(p.out_kind) ? row(item, 0) + r : item * TILES * 16 + r;
+            if (n < N) gemv_emit(p, m, n0 + n, v, up);
         }
-        cluster.sync();   // nothing remote is touched after this
-        if (rank > 0) return;
-    }
-    const int outputs = is_glu(p.out_kind) ? 128 : kSums;
-    for (int i = threadIdx.x; i < outputs; i += kGemvThreads) {
-        const int r = i >> 3, m = i & 7;
-        if (m >= p.M) continue;
-        auto total = [&](int at) {
-            float v = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) v += sums[q * kSums + at];
-            for (int q = 1; q < S; ++q) v += from_others[(q - 1) * kSums + at];
-            return v;
-        };
-        const float v = total(i), up = TILES == 2 && is_glu(p.out_kind) ? total(128 + i) : 0.0f;
-        const int n = is_glu(p.out_kind) ? row[0] + r : blockIdx.x * TILES * 16 + r;
-        if (n < N) gemv_emit(p, m, n0 + n, v, up);
+        if (next < items) __syncthreads();   // the sums have been read
     }
 }
 
