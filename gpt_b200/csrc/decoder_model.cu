@@ -781,7 +781,7 @@ private:
     int launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args)
     {
         const void *key = reinterpret_cast<const void *>(kernel);
-        if (smem > 48 * 1024 && !ctx_->configured.count(key)) {
+        if (smem > 40 * 1024 && !ctx_->configured.count(key)) {   // 48 KB and more need it, static shared memory included
             cudaFuncAttributes fixed{};
             CUDA_TRY(ctx_, cudaFuncGetAttributes(&fixed, kernel));
             CUDA_TRY(ctx_, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - static_cast<int>(fixed.sharedSizeBytes)));
@@ -860,8 +860,19 @@ private:
         b.entries = entries_; b.row_entry = row_entry_; b.row_list = row_list;
         if constexpr (!kF32)
             if (b.side_y && single_rows(rows)) return launch(layer_begin_row_kernel<T>, dim3(rows), dim3(pad_to(pitch_ / 4, 32)), 0, b);
-        b.tile = rows <= 512 || !b.shift ? 1 : rows <= 2048 ? 4 : 8;
-        return launch(layer_begin_kernel<T>, dim3((rows + b.tile - 1) / b.tile), dim3(row_threads(rows)), 2 * size_t(pitch_) * sizeof(float), b);
+        const int pieces = pitch_ / 4;   // of four columns; every thread has one, two, four or eight
+        const int v = pieces <= row_threads(rows) ? 1 : pieces <= 512 ? 2 : pieces <= 2048 ? 4 : 8;
+        // rows per block: a block's first row costs the one before it again, so as few blocks as run at once
+        const int per_sm = v == 1 ? 3 : v == 2 ? 2 : 1, blocks = per_sm * ctx_->num_sms;
+        b.tile = rows <= 512 || !b.shift ? 1 : std::max(4, (rows + blocks - 1) / blocks);
+        const size_t buffer = size_t(2 + std::max(0, b.n_states - 1)) * pitch_ * sizeof(float);
+        b.ahead = b.tile > 1 ? static_cast<int>(std::min<size_t>(2, size_t(216 * 1024) / per_sm / buffer)) : 0;
+        const auto begin = [&](auto kernel, int threads) { return launch(kernel, dim3((rows + b.tile - 1) / b.tile), dim3(threads), b.ahead * buffer, b); };
+        if (v == 1) return begin(layer_begin_kernel<T, 1>, row_threads(rows));
+        if (v == 2) return begin(layer_begin_kernel<T, 2>, pad_to((pieces + 1) / 2, 32));
+        if (v == 4) return begin(layer_begin_kernel<T, 4>, pad_to((pieces + 3) / 4, 32));
+        if (pieces <= 8192) return begin(layer_begin_kernel<T, 8>, std::min(1024, pad_to((pieces + 7) / 8, 32)));
+        return fail(ctx_, GPTB200_ERR_TOO_LARGE, "width %d: rows of at most 32768", c_.width);
     }
 
     int mamba(const Layer &d, const std::vector<Part> &parts, int rows)

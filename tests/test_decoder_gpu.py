@@ -113,6 +113,19 @@ def test_chunked_recurrence_of_any_slice(tmp_path, heads, vdim, state):
     model.close_model()
 
 
+@pytest.mark.parametrize("width,depth", [(72, 4), (1100, 6), (1100, 11), (2056, 3), (8200, 4)])
+def test_start_of_a_layer_of_many_rows(tmp_path, width, depth):
+    """Rows in tiles with a shorter last one: one, two, four and eight pieces per thread, two, one and no rows ahead in shared memory; fp32, whose tolerance shows
+    a row or column that is off."""
+    c, w = build([dm.mamba(heads=2, vdim=8, state=8, groups=1, norm_groups=1, ff=None)] * depth, {}, dict(width=width), 24)
+    tokens = np.random.default_rng(30).integers(0, c["vocab"], 603)
+    want = budurax.forward(c, w, tokens)
+    model = load(tmp_path, c, w, "float32")
+    for cuts in ((1 << 20,), (20, 583)):
+        assert dm.close(whole(model, tokens, cuts), want, TOL["float32"]), cuts
+    model.close_model()
+
+
 def test_long_decoding(tmp_path):
     c, w = build(MIXED["layers"], {}, {}, 4)
     tokens = np.random.default_rng(9).integers(0, c["vocab"], 700)
