@@ -919,6 +919,14 @@ private:
             RC_TRY(k == 2 ? recurrent_chunks(s, {xbc_, ld_xbc, dt_, decay_, s.heads, d.d_skip}, parts, entry0, n) : mamba_tokens(d, entry0, n, ld_xbc));
         }
         const int part = s.inner / s.norm_groups;
+        // a warp per part where those fill the machine; fewer rows: a block per part, whose loads are more
+        if (part % 4 == 0 && part <= 2048 && 1LL * rows * s.norm_groups >= 32LL * ctx_->num_sms) {
+            const auto warps = [&](auto kernel) {
+                return launch(kernel, dim3(static_cast<unsigned>((1LL * rows * s.norm_groups + kNormWarps - 1) / kNormWarps)), dim3(32 * kNormWarps), 0, act_, d.mix_out,
+                              static_cast<const float *>(ssm_y_), static_cast<const T *>(proj_), ld, static_cast<const float *>(d.mix_norm), s, static_cast<float>(c_.eps), rows);
+            };
+            return part <= 512 ? warps(mamba_gated_norm_warp_kernel<T, 4>) : warps(mamba_gated_norm_warp_kernel<T, 16>);
+        }
         return launch(mamba_gated_norm_kernel<T>, dim3(rows, s.norm_groups), dim3(std::min(rows <= 2 * ctx_->num_sms ? 1024 : 256, pad_to((part + 3) / 4, 32))), size_t(part) * sizeof(float), act_, d.mix_out,
                       static_cast<const float *>(ssm_y_), static_cast<const T *>(proj_), ld, static_cast<const float *>(d.mix_norm), s, static_cast<float>(c_.eps));
     }
