@@ -766,11 +766,12 @@ gpt_step_rows_kernel(const GptStep s)
         }
     };
 
-    // The same on the tensor cores, operands in three bf16 parts as in rows_sm100.cuh.  An item's weights go through registers to TMEM at once (lane = column, 24
+    // The same on the tensor cores, operands in three bf16 parts as in rows_sm100.cuh, a step's products in one accumulator, the leading ones last (TMEM has no room
+    // for a second one: their truncation, 2^-23 of a step's sum of 16 k, is the largest error of it).  An item's weights go through registers to TMEM at once (lane = column, 24
     // columns per step of 16 k), four warps issue the products of a step each into an accumulator of its own, and the sixteen warps add up a sixteenth of
     // all accumulators each, in fp32 and in the order of k.
     auto product_tensor = [&](const float *w, const StepPhase &ph, float *part, const float *x, const float *w_next, const StepPhase &ph_next, int item_next) {
-        constexpr int kAccs = ROWS == 64 ? 4 : 8, kAccCols = 256 / kAccs, kMine = ROWS / 4;      // accumulators, rows per warp
+        constexpr int kAccs = ROWS == 64 ? 4 : 8, kAccCols = 256 / kAccs, kSlotBase = 256, kMine = ROWS / 4;      // accumulators, split weights behind them, rows per warp
         constexpr uint32_t kIdesc = ptx::make_idesc_bf16(128, ROWS, false, false), kPart = ROWS * 128;
         const int items = ph.groups * ph.splits, set = warp >> 2, q4 = warp & 3, n = q4 * 32 + lane;
         const uint32_t lanes = static_cast<uint32_t>(q4 * 32) << 16, x_at = ptx::smem_u32(xs);
@@ -821,7 +822,7 @@ gpt_step_rows_kernel(const GptStep s)
                 uint32_t p0[8], p1[8], p2[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) rows::split3(f[2 * j], f[2 * j + 1], p0[j], p1[j], p2[j]);
-                const uint32_t slot = tmem + lanes + kRowsSlotBase + ks * kRowsSlotCols;
+                const uint32_t slot = tmem + lanes + kSlotBase + ks * kRowsSlotCols;
                 rows::tmem_st8(slot, p0);
                 rows::tmem_st8(slot + 8, p1);
                 rows::tmem_st8(slot + 16, p2);
@@ -840,7 +841,7 @@ gpt_step_rows_kernel(const GptStep s)
                     if (ptx::elect_one()) {
                         for (int a = warp; a < count; a += 4) {
                             const int ks = base + a;
-                            rows::issue_step(tmem + a * kAccCols, tmem + kRowsSlotBase + ks * kRowsSlotCols, desc_x, (ks >> 2) * 3 * kPart + (ks & 3) * 32, kPart, kIdesc);
+                            rows::issue_step(tmem + a * kAccCols, tmem + a * kAccCols, tmem + kSlotBase + ks * kRowsSlotCols, desc_x, (ks >> 2) * 3 * kPart + (ks & 3) * 32, kPart, kIdesc);
                         }
                         ptx::mma_commit(bar);
                     }

@@ -1,10 +1,12 @@
 // Products of 9 to 64 rows of fp32 with a weight matrix stored [k][n] (linear layers) or [n][k] (un-embedding, grad_x): y[m][n] = x[m][k] . w, bias and GELU,
 // on the tensor cores and no less exact than fp32 FMAs.
 //
-// Both operands are split exactly into three bf16 values (8 + 8 + 8 bits: the first truncated, the others rounded), and the six products of 2^-16 and more
-// are added: what is left out is 2^-24 of a product and less.  The tensor core adds into its accumulator with truncation, so the accumulator is handed to fp32
-// sums in registers (round to nearest) after every step of 16 k: 64 rows, k 768, n 50304 are off by 1.40e-7 of the result's size, 2.2e-7 with two steps, 4.3e-7 with
-// four (fp32 FMAs: 2.1e-7).  Infinite inputs give NaN, as in the products of more rows.
+// Both operands are split exactly into three bf16 values a0 + a1 + a2 (8 + 8 + 8 bits: the first truncated, the others rounded, so |a1| < 2^-7 |a| and |a2| <=
+// 2^-15 |a|), and all of their products but a2 . b2 (2^-30) are added.  The tensor core adds into its accumulator with truncation, so the accumulator is handed to
+// fp32 sums in registers (round to nearest) after every step of 16 k, the exact products a0 . b0 apart from the others.  Off from 64-bit sums, this / fp32 FMAs, of
+// the result's size: k 32, n 8192 4.5e-8 / 6.9e-8, 768 x 2304 8.3e-8 / 1.15e-7, 3072 x 768 1.08e-7 / 1.54e-7, 768 x 50304 1.33e-7 / 2.08e-7; sums of a single
+// product at most 6.0e-8 / 5.9e-8, where six products in one accumulator were off by 2.3e-7 (us: output layer at 64 rows 59.5, then 50; at 9 rows 35.0 and 33.0).
+// Infinite inputs give NaN, as in the products of more rows.
 //
 // A block computes 128 columns for all rows over its share of k.  The weights are the M = 128 operand; split, they never go back to shared memory: the converter
 // warps write them to TMEM, where the instructions take their A operand from.
@@ -12,7 +14,7 @@
 //   warps 8-15   sums: accumulator -> registers, half of the rows each
 //   warps 16-19  x: global -> three bf16 tiles of 64 k in shared memory (B operand)
 //   warp 20      TMA producer: 32 KB of weights per 64 k, four stages
-//   warps 21, 22 issue the instructions, every other step each: one of them took 500 cycles per step for its waits, six instructions and commits (output layer
+//   warps 21, 22 issue the instructions, every other step each: one of them took 500 cycles per step for its waits, instructions (six then) and commits (output layer
 //                55 us at 64 rows and 40 at 9; two 47 and 33, three 47 and 32).  More converters, or the instructions of several steps in turn, were slower.
 // The un-embedding has enough column tiles for all SMs (blocks walk over them); narrow layers share k in a cluster, partial tiles meet in rank order through
 // distributed shared memory.
@@ -27,10 +29,8 @@ namespace gptb200 {
 constexpr int kRowsIssuers = 2;
 constexpr int kRowsThreads = (21 + kRowsIssuers) * 32;
 constexpr int kRowsStages = 4, kRowsStageBytes = 128 * 64 * 4;
-constexpr int kRowsSlots = 8, kRowsSlotCols = 24;      // split weights of 16 k: 3 x 8 TMEM columns
-constexpr int kRowsAccs = 4, kRowsAccCols = 64;        // accumulators: with two of them the way to the sums and back was what a step took
-constexpr int kRowsSlotBase = kRowsAccs * kRowsAccCols;
-static_assert(kRowsSlotBase + kRowsSlots * kRowsSlotCols <= 512, "TMEM");
+constexpr int kRowsSlotCols = 24;                      // split weights of 16 k: 3 x 8 TMEM columns
+constexpr int kRowsMaxSlots = 8, kRowsMaxAccs = 4;
 constexpr int kRowsXBufs = 2;
 
 struct RowsParams {
@@ -41,6 +41,15 @@ struct RowsParams {
     int tiles;                 // of 128 columns
     int *status;
     int early;                 // weights may be read before the predecessor on the stream has completed
+};
+
+// TMEM of a block: accumulators (with two of them the way to the sums and back was what a step took), then split weights.
+template <int MR>
+struct RowsTmem {
+    static constexpr int kAccs = MR == 64 ? 3 : 4, kSlots = MR == 64 ? 5 : 8;
+    static constexpr int kRest = MR < 32 ? 32 : MR, kAccCols = 2 * kRest;   // leading products, and the others kRest columns on
+    static constexpr int kSlotBase = kAccs * kAccCols;
+    static_assert(kAccs <= kRowsMaxAccs && kSlots <= kRowsMaxSlots && kSlotBase + kSlots * kRowsSlotCols <= 512, "TMEM");
 };
 
 constexpr int rows_smem_bytes(int mr) { return kRowsStages * kRowsStageBytes + kRowsXBufs * 3 * mr * 128 + 1024 + 512; }
@@ -91,15 +100,18 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
         : "memory");
 }
 
-// One step's six products, the smallest first: split weights at TMEM columns `a`, the parts of x `part` bytes apart.
-__device__ __forceinline__ void issue_step(uint32_t d, uint32_t a, const ptx::SmemDesc &x, uint32_t at, uint32_t part, uint32_t idesc)
+// One step's eight products, the smallest first: split weights at TMEM columns `a`, the parts of x `part` bytes apart.  The leading products go to `d`, the others to
+// `rest`, or all of them to one accumulator.
+__device__ __forceinline__ void issue_step(uint32_t d, uint32_t rest, uint32_t a, const ptx::SmemDesc &x, uint32_t at, uint32_t part, uint32_t idesc)
 {
-    mma_ts(d, a + 16, x.at(at), idesc, 0u);
-    mma_ts(d, a, x.at(at + 2 * part), idesc, 1u);
-    mma_ts(d, a + 8, x.at(at + part), idesc, 1u);
-    mma_ts(d, a + 8, x.at(at), idesc, 1u);
-    mma_ts(d, a, x.at(at + part), idesc, 1u);
-    mma_ts(d, a, x.at(at), idesc, 1u);
+    mma_ts(rest, a + 16, x.at(at + part), idesc, 0u);
+    mma_ts(rest, a + 8, x.at(at + 2 * part), idesc, 1u);
+    mma_ts(rest, a + 16, x.at(at), idesc, 1u);
+    mma_ts(rest, a, x.at(at + 2 * part), idesc, 1u);
+    mma_ts(rest, a + 8, x.at(at + part), idesc, 1u);
+    mma_ts(rest, a + 8, x.at(at), idesc, 1u);
+    mma_ts(rest, a, x.at(at + part), idesc, 1u);
+    mma_ts(d, a, x.at(at), idesc, d == rest ? 1u : 0u);
 }
 
 }  // namespace rows
@@ -123,6 +135,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
 rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams p)
 {
     namespace cg = cooperative_groups;
+    using T = RowsTmem<MR>;
     constexpr int kXBytes = 3 * MR * 128, kCols = MR / 2;
     constexpr uint32_t kIdesc = ptx::make_idesc_bf16(128, MR, false, false);
     extern __shared__ uint8_t smem_raw[];
@@ -133,14 +146,14 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
     auto w_full = [&](int s) { return bar_base + 8u * s; };
     auto w_empty = [&](int s) { return bar_base + 8u * (kRowsStages + s); };
     auto a_full = [&](int r) { return bar_base + 8u * (2 * kRowsStages + r); };
-    auto done = [&](int r) { return bar_base + 8u * (2 * kRowsStages + kRowsSlots + r); };      // a step's instructions: its sums are there, its weights read
-    constexpr int kX = 2 * kRowsStages + 2 * kRowsSlots;
+    auto done = [&](int r) { return bar_base + 8u * (2 * kRowsStages + kRowsMaxSlots + r); };      // a step's instructions: its sums are there, its weights read
+    constexpr int kX = 2 * kRowsStages + 2 * kRowsMaxSlots;
     auto x_full = [&](int b) { return bar_base + 8u * (kX + b); };
     auto x_empty = [&](int b) { return bar_base + 8u * (kX + kRowsXBufs + b); };
     auto acc_empty = [&](int b) { return bar_base + 8u * (kX + 2 * kRowsXBufs + b); };
-    const uint32_t drain_bar = bar_base + 8u * (kX + 2 * kRowsXBufs + kRowsAccs);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * (kX + 2 * kRowsXBufs + kRowsAccs + 1));
-    static_assert(8 * (kX + 2 * kRowsXBufs + kRowsAccs + 1) + 8 <= 512, "barriers");
+    const uint32_t drain_bar = bar_base + 8u * (kX + 2 * kRowsXBufs + kRowsMaxAccs);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * (kX + 2 * kRowsXBufs + kRowsMaxAccs + 1));
+    static_assert(8 * (kX + 2 * kRowsXBufs + kRowsMaxAccs + 1) + 8 <= 512, "barriers");
     volatile uint32_t *abort_flag = tmem_slot + 1;
 
     const int warp = ptx::warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -150,7 +163,7 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
             ptx::mbar_init(w_full(s), 1);
             ptx::mbar_init(w_empty(s), 8);
         }
-        for (int r = 0; r < kRowsSlots; ++r) {
+        for (int r = 0; r < T::kSlots; ++r) {
             ptx::mbar_init(a_full(r), 4);
             ptx::mbar_init(done(r), 1);
         }
@@ -158,7 +171,7 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
             ptx::mbar_init(x_full(b), 4);
             ptx::mbar_init(x_empty(b), kRowsIssuers);
         }
-        for (int b = 0; b < kRowsAccs; ++b) ptx::mbar_init(acc_empty(b), 8);
+        for (int b = 0; b < T::kAccs; ++b) ptx::mbar_init(acc_empty(b), 8);
         ptx::mbar_init(drain_bar, kRowsIssuers);
         *abort_flag = 0u;
         ptx::fence_mbar_init();
@@ -179,7 +192,7 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
     if (warp < 8) {
         // ------------------------------------------------------------ converters
         const int set = warp >> 2, quarter = warp & 3, n = quarter * 32 + lane;
-        const uint32_t slots = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kRowsSlotBase;
+        const uint32_t slots = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + T::kSlotBase;
         uint32_t g = 0, s = 0, ph = 0;
         for (int t = blockIdx.x; ok && t < p.tiles; t += gridDim.x) {
             for (int b = 0; ok && b < walk.blocks; ++b) {
@@ -209,8 +222,8 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
                     uint32_t p0[8], p1[8], p2[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) rows::split3(v[2 * j], v[2 * j + 1], p0[j], p1[j], p2[j]);
-                    const uint32_t r = g % kRowsSlots;
-                    if (!bounded_wait(done(r), ((g / kRowsSlots) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
+                    const uint32_t r = g % T::kSlots;
+                    if (!bounded_wait(done(r), ((g / T::kSlots) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_CONVERT)) {
                         ok = false;
                         break;
                     }
@@ -242,21 +255,30 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
 #pragma unroll
             for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
             for (int ks = 0; ks < walk.steps; ++ks, ++g) {
-                const uint32_t b = g % kRowsAccs;
-                if (!bounded_wait(done(g % kRowsSlots), (g / kRowsSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
+                const uint32_t b = g % T::kAccs;
+                if (!bounded_wait(done(g % T::kSlots), (g / T::kSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {
                     ok = false;
                     break;
                 }
                 ptx::tc_fence_after();
-                uint32_t v[kCols];
+                constexpr int kPiece = kCols < 16 ? kCols : 16;
 #pragma unroll
-                for (int j = 0; j < kCols; j += 8) rows::tmem_ld8(mine + b * kRowsAccCols + j, v + j);
-                ptx::tmem_ld_wait();
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(acc_empty(b));
+                for (int c = 0; c < kCols; c += kPiece) {
+                    uint32_t v[kPiece], u[kPiece];
 #pragma unroll
-                for (int j = 0; j < kCols; ++j) acc[j] += __uint_as_float(v[j]);
+                    for (int j = 0; j < kPiece; j += 8) {
+                        rows::tmem_ld8(mine + b * T::kAccCols + c + j, v + j);
+                        rows::tmem_ld8(mine + b * T::kAccCols + T::kRest + c + j, u + j);
+                    }
+                    ptx::tmem_ld_wait();
+                    if (c + kPiece == kCols) {
+                        ptx::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(acc_empty(b));
+                    }
+#pragma unroll
+                    for (int j = 0; j < kPiece; ++j) acc[c + j] += __uint_as_float(v[j]) + __uint_as_float(u[j]);
+                }
             }
             if (!ok) break;
             if (S == 1) {
@@ -369,16 +391,16 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
                 const int steps = walk.in_block(b);
                 for (int ks = 0; ks < steps; ++ks, ++g) {
                     if (g % kRowsIssuers != turn) continue;
-                    const uint32_t buf = g % kRowsAccs, r = g % kRowsSlots;
-                    if (!bounded_wait(acc_empty(buf), ((g / kRowsAccs) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM) ||
-                        !bounded_wait(a_full(r), (g / kRowsSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) {
+                    const uint32_t buf = g % T::kAccs, r = g % T::kSlots;
+                    if (!bounded_wait(acc_empty(buf), ((g / T::kAccs) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM) ||
+                        !bounded_wait(a_full(r), (g / T::kSlots) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_CONV)) {
                         ok = false;
                         break;
                     }
                     ptx::tc_fence_after();
-                    const uint32_t d = tmem + buf * kRowsAccCols, a = tmem + kRowsSlotBase + r * kRowsSlotCols, x = xb * kXBytes + ks * 32;
+                    const uint32_t d = tmem + buf * T::kAccCols, a = tmem + T::kSlotBase + r * kRowsSlotCols, x = xb * kXBytes + ks * 32;
                     if (issuer) {
-                        rows::issue_step(d, a, desc_x, x, MR * 128, kIdesc);
+                        rows::issue_step(d, d + T::kRest, a, desc_x, x, MR * 128, kIdesc);
                         ptx::mma_commit(done(r));
                     }
                 }
