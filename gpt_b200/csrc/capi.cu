@@ -475,7 +475,7 @@ int run_rows_tensor(gptb200_ctx *ctx, const GemmCall &c)
 {
     const bool nk = !c.b_mn;
     RowsParams p{};
-    p.y = c.out; p.act = c.act; p.x = c.a; p.bias = c.bias;
+    p.y = c.out; p.act = c.act; p.x = c.a; p.w = c.b; p.bias = c.bias;
     p.M = c.M; p.N = c.N; p.K = c.K;
     p.tiles = (c.N + 127) / 128;
     p.status = ctx->d_status;

@@ -6,7 +6,8 @@
 // fp32 sums in registers (round to nearest) after every step of 16 k, the exact products a0 . b0 apart from the others.  Off from 64-bit sums, this / fp32 FMAs, of
 // the result's size: k 32, n 8192 4.5e-8 / 6.9e-8, 768 x 2304 8.3e-8 / 1.15e-7, 3072 x 768 1.08e-7 / 1.54e-7, 768 x 50304 1.33e-7 / 2.08e-7; sums of a single
 // product at most 6.0e-8 / 5.9e-8, where six products in one accumulator were off by 2.3e-7 (us: output layer at 64 rows 59.5, then 50; at 9 rows 35.0 and 33.0).
-// Infinite inputs give NaN, as in the products of more rows.
+// An infinite value splits into parts that are NaN: outputs that come out as NaN are computed again with fp32 FMAs at the end, so that they are infinite or NaN
+// as there.
 //
 // A block computes 128 columns for all rows over its share of k.  The weights are the M = 128 operand; split, they never go back to shared memory: the converter
 // warps write them to TMEM, where the instructions take their A operand from.
@@ -35,7 +36,7 @@ constexpr int kRowsXBufs = 2;
 
 struct RowsParams {
     float *y, *act;            // act: null, or gelu(y)
-    const float *x, *bias;     // bias: null for none
+    const float *x, *w, *bias; // bias: null for none
     int M, N, K;
     int slice;                 // k per block of a cluster, a multiple of 16
     int tiles;                 // of 128 columns
@@ -153,8 +154,8 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
     auto acc_empty = [&](int b) { return bar_base + 8u * (kX + 2 * kRowsXBufs + b); };
     const uint32_t drain_bar = bar_base + 8u * (kX + 2 * kRowsXBufs + kRowsMaxAccs);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + (bar_base - smem_base) + 8 * (kX + 2 * kRowsXBufs + kRowsMaxAccs + 1));
-    static_assert(8 * (kX + 2 * kRowsXBufs + kRowsMaxAccs + 1) + 8 <= 512, "barriers");
-    volatile uint32_t *abort_flag = tmem_slot + 1;
+    static_assert(8 * (kX + 2 * kRowsXBufs + kRowsMaxAccs + 1) + 12 <= 512, "barriers");
+    volatile uint32_t *abort_flag = tmem_slot + 1, *nan_flag = tmem_slot + 2;
 
     const int warp = ptx::warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int S = gridDim.y, rank = blockIdx.y;
@@ -173,7 +174,7 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
         }
         for (int b = 0; b < T::kAccs; ++b) ptx::mbar_init(acc_empty(b), 8);
         ptx::mbar_init(drain_bar, kRowsIssuers);
-        *abort_flag = 0u;
+        *abort_flag = *nan_flag = 0u;
         ptx::fence_mbar_init();
         ptx::prefetch_tensormap(&tmap_w);
     }
@@ -285,15 +286,18 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
                 const int col = t * 128 + n;
                 if (col < p.N) {
                     const float bias = p.bias ? __ldg(p.bias + col) : 0.0f;
+                    float all = 0.0f;
 #pragma unroll
                     for (int j = 0; j < kCols; ++j) {
                         const int m = half * kCols + j;
+                        all += acc[j];
                         if (m < p.M) {
                             const float v = acc[j] + bias;
                             p.y[static_cast<long long>(m) * p.N + col] = v;
                             if (p.act) p.act[static_cast<long long>(m) * p.N + col] = gelu_tanh(v);
                         }
                     }
+                    if (isnan(all)) *nan_flag = 1u;
                 }
             } else {   // the partial tile [row][column] takes the place of the weights: all of them have been converted
                 float *tile = reinterpret_cast<float *>(smem_gen);
@@ -425,6 +429,7 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
         ptx::tc_fence_after();
         ptx::tmem_dealloc(tmem, 512);
     }
+    bool nan_seen = *nan_flag != 0u;
     if (S > 1) {
         cg::cluster_group cluster = cg::this_cluster();
         cluster.sync();
@@ -455,8 +460,32 @@ rows_tensor_kernel(const __grid_constant__ CUtensorMap tmap_w, const RowsParams 
             }
             *reinterpret_cast<float4 *>(p.y + static_cast<long long>(m) * p.N + col) = sum;
             if (p.act) *reinterpret_cast<float4 *>(p.act + static_cast<long long>(m) * p.N + col) = make_float4(gelu_tanh(sum.x), gelu_tanh(sum.y), gelu_tanh(sum.z), gelu_tanh(sum.w));
+            nan_seen |= isnan(sum.x + sum.y + sum.z + sum.w);
         }
         cluster.sync();   // no block leaves while its tile may still be read
+    }
+    if (nan_seen) {
+        // rare and slow, but no work for the loops above: the four columns of a piece one after the other
+        for (int t = blockIdx.x; t < p.tiles; t += gridDim.x)
+            for (int e = rank * kRowsThreads + threadIdx.x; e < p.M * 32; e += S * kRowsThreads)
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c) {
+                    const int m = e >> 5, col = t * 128 + 4 * (e & 31) + c;
+                    const long long at = static_cast<long long>(m) * p.N + col;
+                    if (col >= p.N || !isnan(p.y[at])) continue;
+                    const float *x = p.x + static_cast<long long>(m) * p.K, *w = W_NK ? p.w + static_cast<long long>(col) * p.K : p.w + col;
+                    const long long step = W_NK ? 1 : p.N;
+                    float sum = 0.0f;
+#pragma unroll 1
+                    for (int k = 0; k < p.K && !isnan(sum); k += 4) {   // K is a multiple of 4
+                        const float4 v = __ldcg(reinterpret_cast<const float4 *>(x + k));
+                        const float u[4] = {w[k * step], w[(k + 1) * step], w[(k + 2) * step], w[(k + 3) * step]};
+                        sum = fmaf(v.w, u[3], fmaf(v.z, u[2], fmaf(v.y, u[1], fmaf(v.x, u[0], sum))));
+                    }
+                    if (p.bias) sum += __ldg(p.bias + col);
+                    p.y[at] = sum;
+                    if (p.act) p.act[at] = gelu_tanh(sum);
+                }
     }
 }
 

@@ -222,3 +222,39 @@ def test_the_form_may_change_between_steps(batch):
     one = FEW if batch <= 2 else ROWS
     assert launches[:2] == [one] * 2 and min(launches[2:4]) > ROWS and launches[4:] == [one] * 3
     assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("name,index", [("wte", (5, 7)), ("up_w", (0, 3, 9)), ("qkv_w", (0, 11, 100))])
+def test_infinite_weights_give_what_the_operators_give(name, index):
+    """One infinite weight: which logits are infinite and which are NaN is the same with products in three bf16 parts as with fp32 FMAs.  (Inside the layers an infinite
+    value meets a norm or a softmax in every form; an infinite embedding also reaches the un-embedding as a weight.)"""
+    import torch
+    import gpt_b200
+    batch, prompt, steps = 12, 5, 4
+    c = dict(max_seq_len=64, num_layers=2, vocab_size=600, **dict(GPT2, vocab_size_padded=600))
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    parts = []
+    for n, shape in _shapes(c):
+        t = torch.randn(*shape, device="cuda", generator=gen) * 0.02 + (1.0 if n in ("ln1_w", "ln2_w", "lnf_w") else 0.0)
+        if n == name:
+            t[index] = float("inf")
+        parts.append(t.reshape(-1))
+    text = torch.randint(6, 600, (batch, prompt + steps), device="cuda", dtype=torch.int32, generator=gen)
+    text[3, prompt + 1] = 5
+    got = []
+    for operators in (False, True):
+        model = gpt_b200.Model(c, 0, torch.cuda.current_stream().cuda_stream, gpt_b200.MODE_TF32, use_grad=False)
+        model.load_weights(torch.cat(parts).cpu().numpy())
+        if operators:
+            model.set_option("skinny_rows", 64)
+            model.set_option("skinny_tensor", 0)
+        model.generate_begin(text[:, :prompt].contiguous(), batch, prompt, prompt + steps)
+        out = torch.empty(steps, batch, 600, device="cuda")
+        for i in range(steps):
+            model.generate_step(text[:, prompt + i].contiguous(), out[i])
+        torch.cuda.synchronize()
+        got.append(out)
+        model.close()
+    new, old = got
+    assert torch.equal(new.isnan(), old.isnan()) and torch.equal(new.isposinf(), old.isposinf()) and torch.equal(new.isneginf(), old.isneginf())
+    assert not old.isfinite().all() and (name != "wte" or old.isposinf().any())

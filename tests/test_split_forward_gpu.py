@@ -92,6 +92,38 @@ def test_one_product_per_element(m):
     be.close()
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("m,k,n", [(9, 772, 2308), (16, 36, 132), (32, 768, 768), (64, 260, 19204)])
+def test_infinite_operands_of_some_rows(m, k, n, mode):
+    """Infinities, NaN and overflow in x, w and the last k give what fp32 FMAs give: the same infinite and NaN outputs, and the others as ever."""
+    import torch
+    import gpt_b200
+    if m > 16 and k * n < 512 * 512:
+        pytest.skip("another kernel's size")
+    x, w, b, _ = _problem(torch, m, k, n, m + k + n)
+    inf = float("inf")
+    x[1, 5], x[2, k - 1], x[m - 1, 0] = inf, -inf, float("nan")
+    x[4, 7], x[4, 8] = inf, -inf
+    x[5, 3], w[3, 10] = 3e38, 3e38                     # overflows
+    w[9, 2], w[k - 1, n - 1], w[11, 6] = -inf, inf, 0.0
+    x[6, 11], x[6, 9] = inf, 0.0                       # inf x 0 at column 6, 0 x -inf at column 2
+    be = gpt_b200.Backend(0, torch.cuda.current_stream().cuda_stream, mode)
+    got = []
+    for tensor in (1, 0):
+        be.set_option("skinny_tensor", tensor)
+        y, act, z = (torch.full((m + 1, n), 7.0, device="cuda") for _ in range(3))
+        be.device_linear_activation_fused_forward(y, act, x, w, b, True, 1, m, k, n)
+        be.device_unembedding_forward(z, x, w.t().contiguous(), 1, m, k, n)
+        be.synchronize()
+        got.append((y, act, z))
+    for new, old in zip(*got):
+        assert torch.equal(new.isnan(), old.isnan()) and torch.equal(new.isposinf(), old.isposinf()) and torch.equal(new.isneginf(), old.isneginf())
+        assert old.isposinf().any() and old.isfinite().all(1).any()
+        ok = old.abs() < 100                           # all but those of the overflowing row and column
+        assert int(ok.sum()) > old.numel() // 3 and float((new[ok] - old[ok]).abs().max()) <= 2e-6 * float(old[ok].abs().max())
+    be.close()
+
+
 @pytest.mark.parametrize("m,k,n", [(600, 768, 3072), (1540, 768, 2304), (1000, 260, 1028), (2050, 3072, 768)])
 @pytest.mark.parametrize("mode,tol", [(0, 1e-5), (1, 2e-3)])
 def test_one_wave_of_tiles_backward(m, k, n, mode, tol):
