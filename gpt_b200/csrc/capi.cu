@@ -479,7 +479,7 @@ int run_rows_tensor(gptb200_ctx *ctx, const GemmCall &c)
     p.M = c.M; p.N = c.N; p.K = c.K;
     p.tiles = (c.N + 127) / 128;
     p.status = ctx->d_status;
-    p.early = ctx->decode_early_launch ? 1 : 0;
+    p.early = ctx->decode_early_launch >= 2 ? 1 : 0;   // as for the register-tiled kernel, whose calls these are
     // the largest cluster of which one per column tile runs at once; at least 32 of k each
     int cluster = std::max(1, std::min({16, ctx->num_sms / p.tiles, (c.K + 31) / 32}));
     while (cluster > 1 && rows_clusters(ctx, cluster) < p.tiles) --cluster;

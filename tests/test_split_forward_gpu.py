@@ -140,3 +140,32 @@ def test_one_wave_of_tiles_backward(m, k, n, mode, tol):
         assert float((got.double() - want).abs().max()) <= tol * float(want.abs().max())
     assert (gx[m] == 7).all()
     be.close()
+
+
+@pytest.mark.parametrize("m", [9, 64])
+def test_weights_written_just_before_the_call(m):
+    """Option decode_early_launch = 1 covers the per-warp kernels only: products of 9 to 64 rows see weights that the launch before them wrote."""
+    import torch
+    import gpt_b200
+    k, n = 768, 19200
+    be = gpt_b200.Backend(0, torch.cuda.current_stream().cuda_stream, 0)
+    be.set_option("decode_early_launch", 1)
+    x, pre = torch.randn(m, k, device="cuda"), torch.full((n, k), 20.0, device="cuda")      # where the derivative of GELU is one
+    w, z, out = torch.empty(n, k, device="cuda"), torch.empty(m, n, device="cuda"), torch.empty(m, k, device="cuda")
+    grad = torch.randn(m, n, device="cuda")
+    for seed in range(4):
+        source = torch.randn(n, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+        w.fill_(100.0)
+        torch.cuda.synchronize()
+        be.device_activation_backward(w, source, pre, 1, n, k)
+        be.device_unembedding_forward(z, x, w, 1, m, k, n)
+        be.synchronize()
+        assert float((z.double() - x.double() @ source.double().t()).norm() / z.double().norm()) <= 1e-6
+        w.fill_(100.0)
+        torch.cuda.synchronize()
+        be.device_activation_backward(w, source, pre, 1, n, k)
+        be.linear_backward_input(out, grad, w.view(k, n), m, k, n)
+        be.synchronize()
+        want = grad.double() @ source.view(k, n).double().t()
+        assert float((out.double() - want).norm() / want.norm()) <= 1e-6
+    be.close()
