@@ -26,7 +26,7 @@ MODE_TF32 = 1
 EXPORTED_SYMBOLS = [
     "gptb200_ctx_create", "gptb200_ctx_destroy", "gptb200_ctx_set_mode", "gptb200_ctx_get_mode",
     "gptb200_ctx_set_stream", "gptb200_ctx_set_option", "gptb200_ctx_synchronize", "gptb200_ctx_launch_count", "gptb200_ctx_tensor_map_encodes", "gptb200_ctx_read_trace",
-    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_decode", "gptb200_selftest_wait_timeout", "gptb200_selftest_grid_barrier", "gptb200_plan_generate_step",
+    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_decode", "gptb200_plan_rows", "gptb200_selftest_wait_timeout", "gptb200_selftest_grid_barrier", "gptb200_plan_generate_step",
     "gptb200_linear_forward", "gptb200_linear_backward", "gptb200_linear_backward_weights", "gptb200_linear_backward_input",
     "gptb200_linear_backward_input_gelu", "gptb200_gemm_batched",
     "gptb200_gelu_backward",
@@ -80,6 +80,7 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         "gptb200_selftest_grid_barrier": (i, [vp, i]),
         "gptb200_plan_gemm": (i, [i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_plan_decode": (i, [i, i, i, i, i, i, ctypes.POINTER(i)]),
+        "gptb200_plan_rows": (i, [i, i, i, i, i, ctypes.POINTER(i), ctypes.POINTER(i)]),
         "gptb200_plan_generate_step": (i, [i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_status_string": (ctypes.c_char_p, [i]),
         "gptb200_last_error": (ctypes.c_char_p, [vp]),
@@ -174,6 +175,16 @@ def plan_decode(num_sms: int, m: int, n: int, k: int, w_kn: bool, has_epilogue: 
     d = dict(zip(["kernel", "rows", "groups", "cluster"], list(out)))
     d["kernel"] = DECODE_KERNELS[d["kernel"]]
     return d
+
+
+def plan_rows(num_sms: int, m: int, n: int, k: int, max_cluster: int = 16, clusters: list | None = None) -> dict:
+    """How the tensor-core kernel of 9 to 64 rows runs a call (host logic only); see gptb200_plan_rows in include/gptb200.h."""
+    lib = load_library()
+    out = (ctypes.c_int * 4)()
+    rc = lib.gptb200_plan_rows(num_sms, m, n, k, max_cluster, (ctypes.c_int * 17)(*clusters) if clusters else None, out)
+    if rc != 0:
+        raise GptB200Error(rc, "gptb200_plan_rows")
+    return dict(zip(["rows", "cluster", "slice", "blocks"], list(out)))
 
 
 STEP_KERNELS = {0: "operators", 1: "few", 2: "rows"}

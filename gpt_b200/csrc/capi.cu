@@ -480,16 +480,15 @@ int run_rows_tensor(gptb200_ctx *ctx, const GemmCall &c)
     p.tiles = (c.N + 127) / 128;
     p.status = ctx->d_status;
     p.early = ctx->decode_early_launch >= 2 ? 1 : 0;   // as for the register-tiled kernel, whose calls these are
-    // the largest cluster of which one per column tile runs at once; at least 32 of k each
-    int cluster = std::max(1, std::min({16, ctx->num_sms / p.tiles, (c.K + 31) / 32}));
-    while (cluster > 1 && rows_clusters(ctx, cluster) < p.tiles) --cluster;
-    p.slice = ((c.K + cluster - 1) / cluster + 15) / 16 * 16;
+    const int sms = ctx->max_sms > 0 ? std::min(ctx->max_sms, ctx->num_sms) : ctx->num_sms;
+    const RowsPlan pl = plan_rows(c.M, c.N, c.K, sms, ctx->skinny_cluster, [&](int size) { return rows_clusters(ctx, size); });
+    p.slice = pl.slice;
     CUtensorMap tw;
     const int rc = nk ? make_tmap(ctx, &tw, c.b, c.N, c.K, 32, 128, false) : make_plain_tmap(ctx, &tw, c.b, c.K, c.N);
     if (rc != GPTB200_OK) return rc;
-    const int ctas = cluster > 1 ? p.tiles : std::min(p.tiles, ctx->num_sms);
-    if (c.M <= 16) return nk ? launch_rows_tensor<16, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<16, false>(ctx, tw, p, ctas, cluster);
-    if (c.M <= 32) return nk ? launch_rows_tensor<32, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<32, false>(ctx, tw, p, ctas, cluster);
+    const int cluster = pl.cluster, ctas = pl.blocks / cluster;
+    if (pl.rows == 16) return nk ? launch_rows_tensor<16, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<16, false>(ctx, tw, p, ctas, cluster);
+    if (pl.rows == 32) return nk ? launch_rows_tensor<32, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<32, false>(ctx, tw, p, ctas, cluster);
     return nk ? launch_rows_tensor<64, true>(ctx, tw, p, ctas, cluster) : launch_rows_tensor<64, false>(ctx, tw, p, ctas, cluster);
 }
 
@@ -1371,6 +1370,14 @@ int gptb200_plan_decode(int num_sms, int m, int n, int k, int w_kn_major, int ha
     if (!plan4 || num_sms <= 0 || m <= 0 || n <= 0 || k <= 0) return GPTB200_ERR_INVALID_ARG;
     const DecodePlan d = plan_decode(m, n, k, w_kn_major != 0, has_epilogue != 0, num_sms, DecodeOptions{});
     plan4[0] = d.kernel; plan4[1] = d.rows; plan4[2] = d.groups; plan4[3] = d.cluster;
+    return GPTB200_OK;
+}
+
+int gptb200_plan_rows(int num_sms, int m, int n, int k, int max_cluster, const int *clusters, int *plan4)
+{
+    if (!plan4 || num_sms <= 0 || m <= 0 || m > 64 || n <= 0 || k <= 0) return GPTB200_ERR_INVALID_ARG;
+    const RowsPlan p = plan_rows(m, n, k, num_sms, max_cluster, [&](int size) { return clusters ? clusters[size] : num_sms / size; });
+    plan4[0] = p.rows; plan4[1] = p.cluster; plan4[2] = p.slice; plan4[3] = p.blocks;
     return GPTB200_OK;
 }
 

@@ -163,6 +163,29 @@ inline DecodePlan plan_decode(int M, int N, int K, bool w_kn, bool has_epilogue,
     return d;
 }
 
+// ---- rows_tensor_kernel: the calls of DECODE_TILE_CLUSTER, unless options ask for fp32 FMAs ------------------------------------------
+struct RowsPlan {
+    int rows;      // of x, padded: 16, 32 or 64
+    int cluster;   // blocks that share k
+    int slice;     // k per block of a cluster, a multiple of 16
+    int blocks;    // column tiles of 128, or blocks that walk over them; times cluster
+};
+
+// clusters(size): how many clusters of that many blocks run at once (they lie within a GPC, so that it is fewer than SMs / size).
+template <typename F>
+inline RowsPlan plan_rows(int M, int N, int K, int num_sms, int max_cluster, F &&clusters)
+{
+    RowsPlan p{};
+    const int tiles = (N + 127) / 128;
+    p.rows = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+    // the largest cluster of which one per column tile runs at once; at least 32 of k each
+    p.cluster = std::max(1, std::min({16, max_cluster, num_sms / tiles, (K + 31) / 32}));
+    while (p.cluster > 1 && clusters(p.cluster) < tiles) --p.cluster;
+    p.slice = ((K + p.cluster - 1) / p.cluster + 15) / 16 * 16;
+    p.blocks = p.cluster * std::min(tiles, num_sms);
+    return p;
+}
+
 // One wave of 128 x 128 one-CTA tiles, k split as often as fits it, against CTA pairs whose ranges are cut inside tiles (`pair_kb` k-blocks each): a cut costs 15
 // - 25 us for partial tiles that travel through L2 and output that follows them.  Returns the number of parts, 0 for the pairs.  Models of us per launch,
 // fitted to GPT-2's layers at 600 - 4096 rows; measured, pairs / one wave (parts):

@@ -63,9 +63,11 @@ int gptb200_ctx_set_stream(gptb200_ctx *ctx, void *cuda_stream);
  * "skinny_push" (that kernel's cluster sum: 1 = every CTA stores its part into the shared memory of the CTA that finishes it
  * (default), 0 = the finishing CTA loads the parts; same bits either way),
  * "skinny_cluster_rows" (most rows of x for which that kernel is used: default 8),
- * "skinny_tile" (more rows than the per-warp / row-wise kernels take, either weight layout: one-launch register-tiled kernel
- * whose k split also runs over a cluster: 1 = on (default), 0 = off (k-split kernel with partial sums in scratch)),
- * "skinny_tile_rows" (that kernel's row tile beyond 32 rows: 0 or 64 = one 64-row tile (default), 32 = row groups of 32),
+ * "skinny_tile" (more rows than the per-warp / row-wise kernels take, either weight layout: one launch whose k split also runs over a
+ * cluster: 1 = on (default), 0 = off (k-split kernel with partial sums in scratch)),
+ * "skinny_tensor" (... on the tensor cores with three bf16 parts per operand, no less exact: 1 = on (default), 0 = register-tiled fp32 FMAs, which
+ * "skinny_rows" also keeps),
+ * "skinny_tile_rows" (the register-tiled kernel's row tile beyond 32 rows: 0 or 64 = one 64-row tile (default), 32 = row groups of 32),
  * "skinny_pipelined" (the k-split kernel's 16-row groups fetch weights through a shared-memory ring: 1 = on (default), 0 = off),
  * "skinny_rowwise" (decode-shaped calls whose weight is stored [n][k] - the un-embedding, grad_x: one-launch kernel, a warp
  * per pair of weight rows and group of up to 16 rows of x: 1 = on (default), 0 = off (k-split kernel)),
@@ -130,10 +132,14 @@ int gptb200_selftest_grid_barrier(gptb200_ctx *ctx, int polls);
  * take one wave of 128 x 128 one-CTA tiles where ranges would be cut inside tiles: not shown here.) */
 int gptb200_plan_gemm(int num_sms, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate, int *plan8);
 /* For a call that gptb200_plan_gemm sends to the weight-streaming kernels (kernel 3: at most 64 rows): which of them runs with
- * default options, host logic only.  w_kn_major: the weight is stored [k][n] (linear layers) rather than [n][k] (un-embedding,
+ * default options, host logic only (kernel 2 stands for the tensor-core kernel of those calls: gptb200_plan_rows).  w_kn_major: the weight is stored [k][n] (linear layers) rather than [n][k] (un-embedding,
  * grad_x).  plan4 = {kernel (0 k-split with scratch, 1 per-warp cluster kernel, 2 register-tiled cluster kernel, 3 warp per
  * weight-row pair), rows of x per CTA, row groups, CTAs per cluster}; clusters of 16 are assumed to be schedulable. */
 int gptb200_plan_decode(int num_sms, int m, int n, int k, int w_kn_major, int has_epilogue, int *plan4);
+/* How rows_tensor_kernel runs a call that gptb200_plan_decode sends to kernel 2: with default options it takes those calls, the register-tiled kernel only
+ * with skinny_tensor = 0, skinny_rows or fp32 FMAs asked for.  max_cluster: option skinny_cluster; clusters: number of clusters of 1 .. 16 blocks that run at
+ * once, by size (17 entries), or NULL for num_sms / size.  plan4 = {padded rows of x, blocks per cluster, k per block, blocks}. */
+int gptb200_plan_rows(int num_sms, int m, int n, int k, int max_cluster, const int *clusters, int *plan4);
 /* How gptb200_model_generate_step runs a step at a position, called or (replayed != 0) captured into a CUDA graph, with default options (host logic
  * only).  plan10 = {0 operator by operator, 1 one launch of
  * the kernel of one or two rows, 2 one launch of the kernel of padded rows and the un-embedding; its padded rows; slices of k and k-rows per slice of

@@ -155,6 +155,24 @@ def test_decode_kernel_choice_for_gpt2_124m():
             assert p["rows"] * k <= 12288
 
 
+@pytest.mark.parametrize("sms,most", [(148, 16), (148, 8), (100, 16), (16, 16), (1, 16)])
+def test_tensor_core_kernel_of_few_rows(built_library, sms, most):
+    """gptb200_plan_rows: never more blocks than SMs (option max_sms), clusters within the option and within what runs at once, all of k covered."""
+    from gpt_b200 import plan_rows
+    at_once = [0] + [max(-1, sms // s - (s > 2)) for s in range(1, 17)]   # a few less than SMs / size, as with blocks of one GPC
+    for m, n, k in itertools.product((9, 16, 17, 33, 64), (36, 132, 768, 2304, 3072, 50304), (32, 36, 100, 768, 3072)):
+        p = plan_rows(sms, m, n, k, most, at_once)
+        tiles = -(-n // 128)
+        assert p["rows"] >= m and p["rows"] in (16, 32, 64) and (p["rows"] == 16 or p["rows"] < 2 * m)
+        assert 1 <= p["cluster"] <= most and p["blocks"] <= sms and p["blocks"] == p["cluster"] * min(tiles, sms)
+        assert p["slice"] % 16 == 0 and p["slice"] * p["cluster"] >= k
+        if p["cluster"] > 1:
+            assert at_once[p["cluster"]] >= tiles and k > 32 * (p["cluster"] - 1)
+    if sms == 148 and most == 16:
+        assert plan_rows(sms, 64, 768, 3072) == dict(rows=64, cluster=16, slice=192, blocks=96)
+        assert plan_rows(sms, 64, 50304, 768) == dict(rows=64, cluster=1, slice=768, blocks=148)
+
+
 def test_generation_step_plans(built_library):
     """Which kernel runs a generation step.  Blocks take few rounds of items (a partial sum per slice is read back), the kernel of one or two rows ends
     where its repeated attention costs more than the other kernel's padding, and sizes that no kernel takes go operator by operator."""

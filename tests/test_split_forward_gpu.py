@@ -169,3 +169,20 @@ def test_weights_written_just_before_the_call(m):
         want = grad.double() @ source.view(k, n).double().t()
         assert float((out.double() - want).norm() / want.norm()) <= 1e-6
     be.close()
+
+
+@pytest.mark.parametrize("option,value", [("max_sms", 20), ("max_sms", 1), ("skinny_cluster", 1), ("skinny_cluster", 4)])
+def test_rows_on_part_of_the_machine(option, value):
+    import torch
+    import gpt_b200
+    be = gpt_b200.Backend(0, torch.cuda.current_stream().cuda_stream, 0)
+    be.set_option(option, value)
+    for m, k, n in ((12, 772, 772), (64, 260, 5124)):
+        x, w, b, want = _problem(torch, m, k, n, m)
+        y, z = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+        be.device_linear_activation_fused_forward(y, None, x, w, b, False, 1, m, k, n)
+        be.device_unembedding_forward(z, x, w.t().contiguous(), 1, m, k, n)
+        be.synchronize()
+        for got, ref in ((y, want), (z, want - b.double())):
+            assert float((got.double() - ref).norm() / ref.norm()) <= 5e-7
+    be.close()
