@@ -117,10 +117,13 @@ int attention64_backward(gptb200_ctx *ctx, float *gqkv, float *dcache, const flo
 // device cannot give it: the caller then takes the fp32 FMA kernels, which need none.
 bool attention_scratch(gptb200_ctx *ctx, size_t bytes)
 {
-    if (bytes <= ctx->attn_ws_bytes) return true;
+    const bool in_capture = capturing(ctx);
+    if (bytes <= ctx->attn_ws_bytes) {
+        ctx->attn_ws_captured |= in_capture;
+        return true;
+    }
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;   // queued launches may still use the old buffer
-    if (ctx->attn_ws) cudaFree(ctx->attn_ws);
-    ctx->attn_ws = nullptr;
+    release_scratch(ctx, ctx->attn_ws, ctx->attn_ws_captured);
     ctx->attn_ws_bytes = 0;
     if (cudaMalloc(&ctx->attn_ws, bytes) != cudaSuccess) {
         cudaGetLastError();

@@ -25,14 +25,35 @@ using namespace gptb200;
 
 namespace gptb200 {
 
+bool capturing(gptb200_ctx *ctx)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess) cudaGetLastError();
+    return status != cudaStreamCaptureStatusNone;
+}
+
+void release_scratch(gptb200_ctx *ctx, float *&buffer, bool &captured)
+{
+    if (captured)
+        ctx->retired.push_back(buffer);
+    else if (buffer)
+        cudaFree(buffer);
+    buffer = nullptr;
+    captured = false;
+}
+
 int ensure_workspace(gptb200_ctx *ctx, size_t bytes)
 {
-    if (bytes <= ctx->ws_bytes) return GPTB200_OK;
+    const bool in_capture = capturing(ctx);
+    if (bytes <= ctx->ws_bytes) {
+        ctx->ws_captured |= in_capture;
+        return GPTB200_OK;
+    }
     if (bytes > ctx->ws_limit) return fail(ctx, GPTB200_ERR_WORKSPACE, "scratch request of %zu bytes exceeds limit %zu", bytes, ctx->ws_limit);
+    if (in_capture) return fail(ctx, GPTB200_ERR_WORKSPACE, "scratch of %zu bytes cannot be allocated while a graph is captured: call once before", bytes);
     // Growing the scratch buffer waits for queued work: earlier kernels may still read the old one.
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->ws) CUDA_TRY(ctx, cudaFree(ctx->ws));
-    ctx->ws = nullptr;
+    release_scratch(ctx, ctx->ws, ctx->ws_captured);
     ctx->ws_bytes = 0;
     const size_t rounded = (bytes + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
     CUDA_TRY(ctx, cudaMalloc(&ctx->ws, rounded));
@@ -592,14 +613,10 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
     GemmPlanInput in = plan_input(ctx, c);
     in.fma_only = c.fma_only;
     GemmPlan pl = plan_gemm(in);
-    if (pl.kernel == KERNEL_SINGLE && pl.splits > 1 && in.has_epilogue && pl.workspace_bytes > ctx->ws_bytes) {
-        // scratch cannot be allocated while a graph is captured; a forward call that has not run before needs none otherwise
-        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess) cudaGetLastError();
-        if (status != cudaStreamCaptureStatusNone) {
-            in.layers = false;
-            pl = plan_gemm(in);
-        }
+    if (pl.kernel == KERNEL_SINGLE && pl.splits > 1 && in.has_epilogue && ensure_workspace(ctx, pl.workspace_bytes) != GPTB200_OK) {
+        cudaGetLastError();   // a device without room even for the reserve: as where an epilogue cannot be split
+        in.layers = false;
+        pl = plan_gemm(in);
     }
     if (pl.kernel == KERNEL_NONE) return GPTB200_OK;
     if (pl.kernel == KERNEL_SKINNY) return run_skinny(ctx, c, pl);
@@ -1128,6 +1145,13 @@ int gptb200_ctx_create(gptb200_ctx **out, int device, void *cuda_stream, int mod
         delete ctx;
         return GPTB200_ERR_CUDA;
     }
+    // where the device has no room, scratch comes with the first call that needs it
+    if (cudaMalloc(&ctx->ws, kPlanReservedBytes) == cudaSuccess) {
+        ctx->ws_bytes = kPlanReservedBytes;
+    } else {
+        cudaGetLastError();
+        ctx->ws = nullptr;
+    }
     *out = ctx;
     return GPTB200_OK;
 }
@@ -1139,6 +1163,7 @@ int gptb200_ctx_destroy(gptb200_ctx *ctx)
     cudaStreamSynchronize(ctx->stream);
     if (ctx->ws) cudaFree(ctx->ws);
     if (ctx->attn_ws) cudaFree(ctx->attn_ws);
+    for (void *buffer : ctx->retired) cudaFree(buffer);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->d_pair_flags) cudaFree(ctx->d_pair_flags);
     if (ctx->d_trace) cudaFree(ctx->d_trace);

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <set>
 #include <unordered_map>
+#include <vector>
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -81,6 +82,9 @@ struct gptb200_ctx {
                                            // then the decode kernel's tickets (one per column block, zero between launches)
     float *ws = nullptr;  // scratch: split-K partial tiles, partial rows of column reductions
     size_t ws_bytes = 0;
+    bool ws_captured = false;   // a graph that was captured holds its address ...
+    bool attn_ws_captured = false;
+    std::vector<void *> retired;   // ... so that it is kept, beside the larger one that takes its place, until the context goes
     float *attn_ws = nullptr;   // scratch of the tensor-core attention: score and score-gradient matrices of all heads
     size_t attn_ws_bytes = 0;
     int exact3x = 2;               // 3xTF32 CTA-pair kernel: correction terms as TF32 products of fp32 low-part tiles instead of one bf16 chain:
@@ -175,6 +179,9 @@ int run_linear_f32(gptb200_ctx *ctx, float *out, const float *a, const float *w,
 
 // Grows the context's scratch buffer to at least `bytes` (waits for queued work before replacing it).
 int ensure_workspace(gptb200_ctx *ctx, size_t bytes);
+bool capturing(gptb200_ctx *ctx);
+// Frees a scratch buffer, or keeps it until the context goes where a captured graph holds its address.
+void release_scratch(gptb200_ctx *ctx, float *&buffer, bool &captured);
 
 }  // namespace gptb200
 

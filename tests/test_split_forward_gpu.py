@@ -11,10 +11,10 @@ def _problem(torch, m, k, n, seed):
     return x, w, b, x.double() @ w.double() + b.double()
 
 
-@pytest.mark.parametrize("m,k,n", [(65, 3072, 768), (200, 1540, 132), (500, 2052, 260), (70, 512, 772)])
+@pytest.mark.parametrize("m,k,n", [(65, 3072, 768), (200, 1540, 132), (500, 2052, 260), (70, 512, 772), (300, 3072, 768), (1000, 3072, 768), (1540, 3072, 768)])
 @pytest.mark.parametrize("mode,tol", [(0, 1e-5), (1, 2e-3)])
 def test_epilogue_behind_split_k(m, k, n, mode, tol):
-    """Several parts, the last one shorter, ragged rows and columns; tolerances of the modes.  A first call inside a capture needs no scratch."""
+    """Several parts, the last one shorter, ragged rows and columns; tolerances of the modes.  A first call may be inside a capture and gives the same bits there."""
     import torch
     import gpt_b200
     x, w, b, want = _problem(torch, m, k, n, m + k + n)
@@ -37,8 +37,50 @@ def test_epilogue_behind_split_k(m, k, n, mode, tol):
             assert float((act[:m].double() - torch.nn.functional.gelu(want, approximate="tanh")).abs().max()) <= tol * float(want.abs().max())
             assert (y[m] == 7).all() and (act[m] == 7).all()
             if captured:
+                assert torch.equal(y, eager[0]) and torch.equal(act, eager[1])
                 del graph
+            eager = y, act
             be.close()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_scratch_of_a_captured_call_outlives_its_growth(mode):
+    """Warm up, capture, a call that needs more scratch than there is, replay: the graph still owns the memory that it writes.  And scratch that would have to grow
+    inside a capture is an error that leaves the capture valid."""
+    import torch
+    import gpt_b200
+    m, k, n, big = 300, 3072, 768, (128, 768, 50304)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert gpt_b200.plan_gemm(sms, big[0], big[2], big[1], False, False)["scratch_kib"] > 32 << 10
+    x, w, b, _ = _problem(torch, m, k, n, mode)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        be = gpt_b200.Backend(0, stream.cuda_stream, mode)
+        y, act, want = (torch.empty(m, n, device="cuda") for _ in range(3))
+        h, wte, logits = torch.randn(*big[:2], device="cuda"), torch.randn(big[2], big[1], device="cuda"), torch.empty(big[0], big[2], device="cuda")
+        call = lambda: be.device_linear_activation_fused_forward(y, act, x, w, b, True, 1, m, k, n)
+        large = lambda: be.device_unembedding_forward(logits, h, wte, 1, *big)
+        call()
+        want.copy_(y)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            with pytest.raises(gpt_b200.GptB200Error):
+                large()
+            call()
+        large()
+        stream.synchronize()
+        fill = [torch.full((4 << 20,), float("nan"), device="cuda") for _ in range(16)]     # takes what was freed
+        y.zero_()
+        graph.replay()
+        be.synchronize()
+        assert torch.equal(y, want) and all(t.isnan().all() for t in fill)
+        large()
+        be.synchronize()
+        assert float((logits.double() - h.double() @ wte.double().t()).abs().max()) <= (1e-5 if mode == 0 else 2e-3) * float(logits.abs().max())
+        del graph
+        be.close()
 
 
 @pytest.mark.parametrize("m", [9, 16, 17, 33, 64])
