@@ -20,10 +20,12 @@
 // MMA thread issues  lo.hi + hi.lo + hi.hi  per k-step.
 //
 // Accumulator precision: every tcgen05.mma adds into the fp32 accumulator with truncation, which biases
-// long sums (measured: relative error grows by about 2^-24 per MMA).  In 3xTF32 mode the MMA thread
-// therefore hands the accumulator to the epilogue warps every kChunkKB k-blocks; they add the chunk into
-// a running sum kept in registers with round-to-nearest fp32 adds, so the truncation never sees more than
-// one chunk.  In plain TF32 mode the operand truncation (2^-11) dominates and a tile is one chunk.
+// long sums (measured: relative error grows by about 2^-24 per MMA).  The MMA thread therefore hands the
+// accumulator to the epilogue warps every kChunkKB k-blocks; they add the chunk into a running sum kept in
+// registers with round-to-nearest fp32 adds, so the truncation never sees more than one chunk.  In TF32 mode,
+// where the operand truncation (2^-11) dominates, every kChunkTf32KB k-blocks (sums of 3072 positive products
+// off by 1.4e-6 instead of 2.2e-5, for 3 - 6 % of the launch: 2048 x 768 x 2304 19.0 us, 17.9 without), and in
+// tiles of 256 columns, which have no registers left, a tile is one chunk.
 #pragma once
 
 #include <cstdint>
@@ -157,12 +159,14 @@ constexpr int kUmmaK = 8;                     // K per tcgen05.mma kind::tf32
 constexpr int kATileBytes = kBM * kBK * 4;    // 16 KiB
 constexpr int kBoxBytesMN = kBK * 32 * 4;     // one [32 k-rows x 32 floats] box of an MN-major operand
 constexpr int kChunkKB = 4;                   // 3xTF32: k-blocks per accumulator hand-off (K = 128)
+constexpr int kChunkTf32KB = 8;               // TF32, 128-column tiles
 constexpr int kStageTileBytes = 32 * 32 * 4;  // one [32 rows x 32 cols] output staging tile
 constexpr long long kWaitTimeoutCycles = 2000000000LL;  // about one second
 
 template <int BN, bool X3>
 struct GemmCfg {
-    static constexpr bool kChunked = X3;
+    static constexpr bool kChunked = X3 || BN == 128;
+    static constexpr int kChunk = X3 ? kChunkKB : kChunkTf32KB;
     static constexpr int kEpiWarps = (X3 && BN == 256) ? 8 : 4;   // chunked: 128 running sums per thread
     static constexpr int kColsPerEpiWarp = BN / (kEpiWarps / 4);
     static constexpr int kStageBufsPerWarp = kEpiWarps == 8 ? 1 : 2;
@@ -316,6 +320,18 @@ __device__ __forceinline__ void stage_row(uint32_t buf, int lane, const float (&
     }
 }
 
+__device__ __forceinline__ void load_row(uint32_t buf, int lane, float (&v)[32])
+{
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float4 f = ptx::lds128(buf + lane * 128 + ((j ^ (lane & 7)) << 4));
+        v[4 * j] = f.x;
+        v[4 * j + 1] = f.y;
+        v[4 * j + 2] = f.z;
+        v[4 * j + 3] = f.w;
+    }
+}
+
 template <int BN, bool A_MN, bool B_MN, bool X3>
 __global__ void __launch_bounds__(GemmCfg<BN, X3>::kThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -389,7 +405,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     };
 
     if (warp < 4) {
-        if (C::kChunked) ptx::reg_dec<56>();
+        if (X3) ptx::reg_dec<56>();
         if (warp == 0) {
             // ------------------------------------------------------------ TMA producer: one elected lane issues
             const bool issuer = ptx::elect_one();
@@ -452,7 +468,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 decode(w, tm, tn, kb0, kb1, split);
                 int kb = kb0;
                 while (ok && kb < kb1) {
-                    const int kend = C::kChunked ? min(kb + kChunkKB, kb1) : kb1;
+                    const int kend = C::kChunked ? min(kb + C::kChunk, kb1) : kb1;
                     const uint32_t buf = g & 1u;
                     const uint32_t use = (g >> 1) & 1u;
                     if (!bounded_wait(tmem_empty_bar(buf), use ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA_TMEM)) {
@@ -511,7 +527,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
     } else if (warp < kFirstConvWarp) {
         // ------------------------------------------------------------ epilogue
-        if (C::kChunked) ptx::reg_inc<C::kEpiWarps == 8 ? 184 : 200>();
+        if (X3) ptx::reg_inc<C::kEpiWarps == 8 ? 184 : 200>();
         const int e = warp - kFirstEpiWarp;
         const int q = warp & 3;  // TMEM lane quarter this warp may read (warp index mod 4)
         const int col_base = (e >> 2) * C::kColsPerEpiWarp;
@@ -522,14 +538,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         uint32_t g = 0;
         bool ok = true;
 
-        float held[32];   // gate columns of the gated kinds
         // bias / GELU, staging, TMA store of one [32 rows x 32 cols] piece of the tile
         auto emit = [&](float (&v)[32], int row0, int col0, int split) {
             if constexpr (!A_MN && !B_MN && !X3) {
                 if (p.out_kind != OUT_F32 && p.epi_mode == EPI_STORE) {
                     uint32_t w[16];
                     int word0;
+                    // gate columns of the gated kinds wait for their up columns in the staging tile: every lane reads its own row again
+                    const bool gate = is_glu(p.out_kind) && !(col0 & 32);
+                    float held[32];
+                    if (is_glu(p.out_kind) && !gate) {
+                        load_row(ring.acquire(lane), lane, held);
+                        __syncwarp();
+                    }
                     const bool some = piece_to_bf16(p, v, held, row0, col0, lane, w, word0);
+                    if (gate) {
+                        stage_row(ring.acquire(lane), lane, held);
+                        return;
+                    }
                     if (__any_sync(0xffffffffu, some)) {
                         const uint32_t buf = ring.acquire(lane);
                         stage_row_bf16(buf, lane, w);
@@ -589,7 +615,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 float acc[128];
 #pragma unroll
                 for (int j = 0; j < 128; ++j) acc[j] = 0.0f;
-                for (int kb = kb0; ok && kb < kb1; kb += kChunkKB, ++g) {
+                for (int kb = kb0; ok && kb < kb1; kb += C::kChunk, ++g) {
                     const uint32_t buf = g & 1u;
                     const uint32_t use = (g >> 1) & 1u;
                     if (!bounded_wait(tmem_full_bar(buf), use, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE)) {

@@ -228,3 +228,23 @@ def test_rows_on_part_of_the_machine(option, value):
         for got, ref in ((y, want), (z, want - b.double())):
             assert float((got.double() - ref).norm() / ref.norm()) <= 5e-7
     be.close()
+
+
+@pytest.mark.parametrize("m,k,n,which", [(600, 768, 3072, "y gx gw"), (1540, 3072, 768, "y gw"), (2048, 768, 2304, "gx gw"), (3000, 3072, 768, "y gw")])
+def test_one_wave_of_tf32_tiles_keeps_its_chains_short(m, k, n, which):
+    """Operands that TF32 holds exactly, all positive: a chain of 32 truncating additions (at most 2^-23 of the partial sum each) before the fp32 sums, 16 on average over
+    a growing sum, and 1e-6 for those: below 3e-6 of the result.  Chains of a whole k of 3072 are off by 2.2e-5.  The products that one wave of tiles takes."""
+    import torch
+    import gpt_b200
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    exact = lambda *shape: (torch.rand(*shape, device="cuda", generator=gen).view(torch.int32) & -8192).view(torch.float32)
+    x, w, gy = exact(m, k), exact(k, n), exact(m, n)
+    be = gpt_b200.Backend(0, torch.cuda.current_stream().cuda_stream, 1)
+    y, gx, gw, gb = torch.empty(m, n, device="cuda"), torch.empty(m, k, device="cuda"), torch.zeros(k, n, device="cuda"), torch.zeros(n, device="cuda")
+    be.device_linear_activation_fused_forward(y, None, x, w, torch.zeros(n, device="cuda"), False, 1, m, k, n)
+    be.device_linear_backward(gx, gw, gb, gy, x, w, 1, m, k, n)
+    be.synchronize()
+    for name, got, want in (("y", y, x.double() @ w.double()), ("gx", gx, gy.double() @ w.double().t()), ("gw", gw, x.double().t() @ gy.double())):
+        if name in which.split():
+            assert float((got.double() - want).norm() / want.norm()) <= 3e-6, name
+    be.close()
