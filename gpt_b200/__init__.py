@@ -26,7 +26,7 @@ MODE_TF32 = 1
 EXPORTED_SYMBOLS = [
     "gptb200_ctx_create", "gptb200_ctx_destroy", "gptb200_ctx_set_mode", "gptb200_ctx_get_mode",
     "gptb200_ctx_set_stream", "gptb200_ctx_set_option", "gptb200_ctx_synchronize", "gptb200_ctx_launch_count", "gptb200_ctx_tensor_map_encodes", "gptb200_ctx_read_trace",
-    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_decode", "gptb200_plan_rows", "gptb200_selftest_wait_timeout", "gptb200_selftest_grid_barrier", "gptb200_plan_generate_step",
+    "gptb200_status_string", "gptb200_last_error", "gptb200_plan_gemm", "gptb200_plan_layer", "gptb200_plan_bf16", "gptb200_plan_decode", "gptb200_plan_rows", "gptb200_selftest_wait_timeout", "gptb200_selftest_grid_barrier", "gptb200_plan_generate_step",
     "gptb200_linear_forward", "gptb200_linear_backward", "gptb200_linear_backward_weights", "gptb200_linear_backward_input",
     "gptb200_linear_backward_input_gelu", "gptb200_gemm_batched",
     "gptb200_gelu_backward",
@@ -79,6 +79,8 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         "gptb200_selftest_wait_timeout": (i, [vp, i]),
         "gptb200_selftest_grid_barrier": (i, [vp, i]),
         "gptb200_plan_gemm": (i, [i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
+        "gptb200_plan_layer": (i, [i, i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
+        "gptb200_plan_bf16": (i, [i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_plan_decode": (i, [i, i, i, i, i, i, ctypes.POINTER(i)]),
         "gptb200_plan_rows": (i, [i, i, i, i, i, ctypes.POINTER(i), ctypes.POINTER(i)]),
         "gptb200_plan_generate_step": (i, [i, i, i, i, i, i, i, i, ctypes.POINTER(i)]),
@@ -151,11 +153,32 @@ PLAN_KERNELS = {0: "none", 1: "pair", 2: "single", 3: "skinny", 4: "simt"}
 
 def plan_gemm(num_sms: int, m: int, n: int, k: int, a_mn: bool, b_mn: bool, has_epilogue: bool = False, accumulate: bool = False) -> dict:
     """Launch plan of one GEMM (host logic only, no GPU needed); see gptb200_plan_gemm in include/gptb200.h."""
-    lib = load_library()
     out = (ctypes.c_int * 8)()
-    rc = lib.gptb200_plan_gemm(num_sms, m, n, k, int(a_mn), int(b_mn), int(has_epilogue), int(accumulate), out)
+    rc = load_library().gptb200_plan_gemm(num_sms, m, n, k, int(a_mn), int(b_mn), int(has_epilogue), int(accumulate), out)
     if rc != 0:
         raise GptB200Error(rc, "gptb200_plan_gemm")
+    return _gemm_plan(out)
+
+
+def plan_layer(num_sms: int, mode: int, m: int, n: int, k: int, a_mn: bool, b_mn: bool, has_epilogue: bool = False, accumulate: bool = False) -> dict:
+    """Launch plan of a call of a linear layer or the un-embedding; see gptb200_plan_layer in include/gptb200.h."""
+    out = (ctypes.c_int * 8)()
+    rc = load_library().gptb200_plan_layer(num_sms, mode, m, n, k, int(a_mn), int(b_mn), int(has_epilogue), int(accumulate), out)
+    if rc != 0:
+        raise GptB200Error(rc, "gptb200_plan_layer")
+    return _gemm_plan(out)
+
+
+def plan_bf16(num_sms: int, m: int, n: int, k: int, gated: bool = False, plain_f32: bool = False) -> dict:
+    """How a bf16 product of more than a few rows runs; see gptb200_plan_bf16 in include/gptb200.h."""
+    out = (ctypes.c_int * 2)()
+    rc = load_library().gptb200_plan_bf16(num_sms, m, n, k, int(gated), int(plain_f32), out)
+    if rc != 0:
+        raise GptB200Error(rc, "gptb200_plan_bf16")
+    return dict(columns=out[0], split_k=bool(out[1]))
+
+
+def _gemm_plan(out) -> dict:
     keys = ["kernel", "tile_n", "tiles_m", "tiles_n", "splits", "k_per_split", "grid", "scratch_kib"]
     d = dict(zip(keys, list(out)))
     d["kernel"] = PLAN_KERNELS[d["kernel"]]

@@ -1373,20 +1373,51 @@ int gptb200_selftest_wait_timeout(gptb200_ctx *ctx, int limit_us)
     return GPTB200_OK;
 }
 
-int gptb200_plan_gemm(int num_sms, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate, int *plan8)
+namespace {
+
+int report_plan(const GemmPlanInput &in, int *plan8)
 {
-    if (!plan8 || num_sms <= 0 || m < 0 || n < 0 || k < 0) return GPTB200_ERR_INVALID_ARG;
-    GemmPlanInput in{};
-    in.M = m; in.N = n; in.K = k;
-    in.a_mn = a_mn_major != 0; in.b_mn = b_mn_major != 0;
-    in.has_epilogue = has_epilogue != 0; in.accumulate = accumulate != 0; in.aligned = true;
-    in.num_sms = num_sms; in.opt_skinny = true; in.ws_limit = size_t(1) << 30;
     const GemmPlan p = plan_gemm(in);
     const long long ws = static_cast<long long>(p.workspace_bytes);
     const int pairs = p.kernel == KERNEL_PAIR ? p.grid / 2 : 1;
     const int kb_each = p.kernel == KERNEL_PAIR ? static_cast<int>((p.sk_total + pairs - 1) / pairs) : p.kb_per_split;
     const int out[8] = {p.kernel, p.tile_n, p.tiles_m, p.tiles_n, p.kernel == KERNEL_PAIR ? p.sk_max_share : p.splits, kb_each, p.grid, static_cast<int>(std::min<long long>(ws >> 10, 0x7fffffff))};
     for (int i = 0; i < 8; ++i) plan8[i] = out[i];
+    return GPTB200_OK;
+}
+
+GemmPlanInput default_plan_input(int num_sms, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate)
+{
+    GemmPlanInput in{};
+    in.M = m; in.N = n; in.K = k;
+    in.a_mn = a_mn_major != 0; in.b_mn = b_mn_major != 0;
+    in.has_epilogue = has_epilogue != 0; in.accumulate = accumulate != 0; in.aligned = true;
+    in.num_sms = num_sms; in.opt_skinny = true; in.ws_limit = size_t(1) << 30;
+    return in;
+}
+
+}  // namespace
+
+int gptb200_plan_gemm(int num_sms, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate, int *plan8)
+{
+    if (!plan8 || num_sms <= 0 || m < 0 || n < 0 || k < 0) return GPTB200_ERR_INVALID_ARG;
+    return report_plan(default_plan_input(num_sms, m, n, k, a_mn_major, b_mn_major, has_epilogue, accumulate), plan8);
+}
+
+int gptb200_plan_layer(int num_sms, int mode, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate, int *plan8)
+{
+    if (!plan8 || num_sms <= 0 || m < 0 || n < 0 || k < 0 || (mode != GPTB200_MODE_3XTF32 && mode != GPTB200_MODE_TF32)) return GPTB200_ERR_INVALID_ARG;
+    GemmPlanInput in = default_plan_input(num_sms, m, n, k, a_mn_major, b_mn_major, has_epilogue, accumulate);
+    in.layers = true;
+    in.x3 = mode == GPTB200_MODE_3XTF32;
+    return report_plan(in, plan8);
+}
+
+int gptb200_plan_bf16(int num_sms, int m, int n, int k, int gated, int plain_f32, int *plan2)
+{
+    if (!plan2 || num_sms <= 0 || m <= 0 || n <= 0 || k <= 0) return GPTB200_ERR_INVALID_ARG;
+    const Bf16Plan p = plan_bf16(m, n, k, num_sms, gated != 0, plain_f32 != 0, size_t(1) << 30);
+    plan2[0] = p.columns; plan2[1] = p.split_k ? 1 : 0;
     return GPTB200_OK;
 }
 

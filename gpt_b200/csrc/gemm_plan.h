@@ -19,7 +19,7 @@ enum GemmKernelKind : int {
 struct GemmPlanInput {
     int M, N, K;             // D[M x N] = A[M x K] . B[K x N]
     bool a_mn, b_mn;         // operand stored with the free index contiguous
-    bool has_epilogue;       // bias and / or GELU output: split-K is not possible
+    bool has_epilogue;       // bias and / or GELU output: split-K only for `layers`, whose reduction applies it
     bool accumulate;         // out += result
     bool aligned;            // base pointers 16-byte aligned
     int num_sms;

@@ -56,7 +56,8 @@ int gptb200_ctx_set_stream(gptb200_ctx *ctx, void *cuda_stream);
 /* Tuning knobs, for benchmarking: key "tile_n" (0 = automatic, 128, 256), "max_splits" (0 = automatic),
  * "pair" (CTA-pair kernel with 256 x 256 tiles: 1 = always, 0 = heuristic, -1 = never),
  * "stream_k" (CTA-pair kernel: give every pair the same number of k-blocks by letting a pair's range begin and end inside a
- * tile, partial tiles summed through scratch: 1 = always, 0 = when whole tiles would leave SMs idle, -1 = never),
+ * tile, partial tiles summed through scratch: 1 = always, 0 = when whole tiles would leave SMs idle, -1 = never; fp32 products
+ * only: gptb200_linear_bf16 gives its pairs whole tiles),
  * "skinny" (weight-streaming kernel for decode-shaped calls, up to 64 rows: 1 = on (default), 0 = off),
  * "skinny_rows" (most rows that kernel takes: 0 = 64 (default), 1 .. 64),
  * "skinny_cluster" (decode-shaped calls whose weight is stored [k][n]: one launch that splits k over the warps of a CTA and
@@ -131,9 +132,15 @@ int gptb200_selftest_grid_barrier(gptb200_ctx *ctx, int polls);
  * default options).  plan8 = {kernel (0 none, 1 CTA-pair tcgen05, 2 one-CTA tcgen05, 3 weight streaming, 4 SIMT), tile_n,
  * tiles_m, tiles_n, split_k, k-blocks (or k elements for kernel 3) per split, CTAs, scratch KiB}.  For kernel 1 split_k is the
  * largest number of CTA pairs that work on one 256 x 256 tile (1: every pair computes whole tiles) and the next field the
- * k-blocks per CTA pair.  (The linear layers' calls may split k in spite of an epilogue, which the reduction then applies, and may
- * take one wave of 128 x 128 one-CTA tiles where ranges would be cut inside tiles: not shown here.) */
+ * k-blocks per CTA pair.  This is the plan of a product whose mode is not known and whose epilogue cannot be split (a forward call when the device has no room
+ * for scratch); what the calls of this header run is gptb200_plan_layer. */
 int gptb200_plan_gemm(int num_sms, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate, int *plan8);
+/* The same for a call of a linear layer or the un-embedding in a mode (gptb200_mode): k may be split in spite of an epilogue, which the reduction then applies, and
+ * one wave of 128 x 128 one-CTA tiles may take the place of CTA pairs whose ranges would be cut inside tiles. */
+int gptb200_plan_layer(int num_sms, int mode, int m, int n, int k, int a_mn_major, int b_mn_major, int has_epilogue, int accumulate, int *plan8);
+/* How gptb200_linear_bf16 runs more than gemv_rows rows: plan2 = {columns per 256-row tile of a CTA pair, 1 for split-K over one-CTA tiles instead}.  gated: the
+ * kinds with gate and up columns; plain_f32: contiguous fp32 output without a bias. */
+int gptb200_plan_bf16(int num_sms, int m, int n, int k, int gated, int plain_f32, int *plan2);
 /* For a call that gptb200_plan_gemm sends to the weight-streaming kernels (kernel 3: at most 64 rows): which of them runs with
  * default options, host logic only (kernel 2 stands for the tensor-core kernel of those calls: gptb200_plan_rows).  w_kn_major: the weight is stored [k][n] (linear layers) rather than [n][k] (un-embedding,
  * grad_x).  plan4 = {kernel (0 k-split with scratch, 1 per-warp cluster kernel, 2 register-tiled cluster kernel, 3 warp per

@@ -118,6 +118,80 @@ def test_plan_invariants_over_a_sweep(plan, sms):
                 assert m <= 64 and p["tiles_m"] == (m + 15) // 16 and not acc and p["splits"] * p["k_per_split"] >= k and p["k_per_split"] % 4 == 0
 
 
+@pytest.mark.parametrize("sms", [148, 132, 16])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_layer_plan_invariants_over_a_sweep(built_library, mode, sms):
+    """What the layers' calls run (gptb200_plan_layer): parts that cover k, none of them empty or shorter than eight k-blocks, one wave where products are taken from the
+    pairs, and for forward calls no scratch beyond the 32 MB that every context holds."""
+    from gpt_b200 import plan_layer
+    dims_m = [65, 100, 129, 300, 600, 1000, 1537, 2048, 3000, 5000, 8192, 32768]
+    dims_nk = [32, 100, 132, 260, 768, 2304, 3072, 50304]
+    seen = set()
+    for m, n, k in itertools.product(dims_m, dims_nk, dims_nk):
+        for form, (a_mn, b_mn, epi, acc) in dict(forward=(False, True, True, False), grad_x=(False, False, False, False), grad_w=(True, True, False, True)).items():
+            M, N, K = (n, k, m) if form == "grad_w" else (m, n, k)
+            if M * N >= 2 ** 31 or M * K >= 2 ** 31:
+                continue
+            p = plan_layer(sms, mode, M, N, K, a_mn, b_mn, epi, acc)
+            num_kb = -(-K // 32)
+            assert p["grid"] >= 1
+            if epi:
+                assert p["scratch_kib"] <= 32 << 10
+            if p["kernel"] == "single":
+                tiles = p["tiles_m"] * p["tiles_n"]
+                assert p["tile_n"] in (128, 256) and p["tiles_m"] == -(-M // 128) and p["tiles_n"] == -(-N // p["tile_n"])
+                assert p["grid"] == min(sms, tiles * p["splits"])
+                assert p["splits"] * p["k_per_split"] >= num_kb > (p["splits"] - 1) * p["k_per_split"]
+                if p["splits"] > 1:
+                    assert p["k_per_split"] >= 8 and p["scratch_kib"] * 1024 > p["splits"] * M * N * 4 - 1024
+                    if epi:
+                        assert num_kb >= (16 if mode == 0 else 40)
+                        seen.add("split epilogue")
+                else:
+                    assert p["scratch_kib"] == 0
+                general = _general(sms, M, N, K, a_mn, b_mn, epi, acc)
+                if general["kernel"] == "pair":     # taken from pairs whose ranges would be cut inside tiles
+                    one_wave = tiles * p["splits"] <= sms
+                    assert general["splits"] > 1 and p["tile_n"] == 128
+                    assert one_wave or (epi and p["splits"] > 1 and general["grid"] >= 2 * 4 * -(-M // 256) * -(-N // 256))   # ... or four pairs and more to a tile
+                    seen |= {"one wave"} if one_wave else set()
+            elif p["kernel"] == "pair":
+                assert p == _general(sms, M, N, K, a_mn, b_mn, epi, acc)
+    assert seen == {"split epilogue", "one wave"}
+
+
+def _general(*args):
+    import gpt_b200
+    return gpt_b200.plan_gemm(*args)
+
+
+def test_layer_plans_of_gpt2(built_library):
+    from gpt_b200 import plan_layer
+    D, F = 768, 3072
+    assert plan_layer(SMS, 1, 1000, 3 * D, D, False, True, True)["splits"] == 1                        # 24 k-blocks: not worth the reduction in TF32 mode
+    down = plan_layer(SMS, 0, 300, D, F, False, True, True)
+    assert down["kernel"] == "single" and down["splits"] == 8 and down["scratch_kib"] == 8 * 300 * D * 4 // 1024
+    dw = plan_layer(SMS, 1, D, F, 1000, True, True, False, True)                                        # one wave of 144 tiles
+    assert dw["kernel"] == "single" and dw["splits"] == 1 and dw["grid"] == 144
+    assert plan_layer(SMS, 0, D, F, 2048, True, True, False, True)["kernel"] == "pair"                  # 3xTF32: the pairs' main loop is worth its cuts
+    assert plan_layer(SMS, 0, 8192, F, D, False, True, True) == _general(SMS, 8192, F, D, False, True, True)
+
+
+def test_bf16_plans(built_library):
+    """Columns per tile and split-K of bf16 products (gptb200_plan_bf16): both sides of the lines that plan_bf16's comment gives figures for."""
+    from gpt_b200 import plan_bf16
+    assert plan_bf16(SMS, 4096, 10304, 2048) == dict(columns=256, split_k=False)
+    assert plan_bf16(SMS, 2611, 768, 3072) == dict(columns=128, split_k=False)
+    assert plan_bf16(SMS, 2611, 3072, 768) == dict(columns=256, split_k=False)
+    assert plan_bf16(SMS, 16, 2048, 8192, plain_f32=True)["split_k"] and not plan_bf16(SMS, 16, 2048, 8192)["split_k"]
+    assert plan_bf16(SMS, 300, 768, 3072, plain_f32=True)["split_k"] and not plan_bf16(SMS, 300, 768, 1536, plain_f32=True)["split_k"]
+    assert not plan_bf16(SMS, 512, 2048, 8192, plain_f32=True)["split_k"]
+    for m, n, k, sms in itertools.product((9, 64, 257, 2611, 9000), (64, 776, 2048, 10304), (64, 768, 8192), (148, 20, 1)):
+        assert plan_bf16(sms, m, n, k, gated=True)["columns"] in (128, 256)
+        assert plan_bf16(sms, m, n, k, plain_f32=True)["columns"] in (64, 128, 256)
+        assert not plan_bf16(sms, m, n + 2, k, plain_f32=True)["split_k"]      # rows of partial sums are whole 16-byte pieces
+
+
 def test_decode_kernel_choice_for_gpt2_124m():
     """Which weight-streaming kernel a decode-shaped call runs (gptb200_plan_decode, default options)."""
     import gpt_b200
