@@ -158,10 +158,18 @@ bool gpt_step_replayed(const gptb200_ctx *ctx)
 //   1600, 3                4165 / 3859, 4071      4380 / 4276, 4436      4648 / 4889, 5060      4991 / 5779, 6003
 //   512, 3                 288 / 258, 312         317 / 285, 337         355 / 322, 378         418 / 381, 443
 //   768, 8                 477 / 522, 599         534 / 712, 755         589 / 915, 961         693 / 1139, 1201
-// and beyond width 1600 their products are long enough to hide the launches (2048, eight layers, position 96, 300, 480; 16 rows 1188 / 1429, 1551):
+// and beyond width 1600 their products are long enough to hide the launches (2048, eight layers, position 96, 300, 480):
 //   2048, 2 (8 passes)     -                      -                      1117 / 1026, 1066
 //   2048, 4                994 / 759, 798         1080 / 990, 1022       1135 / 1116, 1152
 //   2048, 8                1124 / 1053, 1101      1223 / 1233, 1280      1283 / 1368, 1415
+// From nine rows on both sides run on the tensor cores.  The step's padding and its partial sums grow with the rows, the operators' launches do not: from width 1600
+// on they take more than 16 rows (positions 64, 256, 480; operators replayed, called; 1280 beyond 32 rows is left with the step, which they would beat there too):
+//   768, 16       446 / 684, 707      580 / 935, 963      698 / 1202, 1191       64      624 / 862, 865      893 / 1190, 1213     1211 / 1564, 1586
+//   1024, 16      580 / 797, 822      718 / 1054, 1087    834 / 1331, 1327       64      851 / 1015, 1013    1199 / 1392, 1446    1542 / 1778, 1876
+//   1280, 32      860 / 917, 952      1129 / 1226, 1276   1489 / 1583, 1718      64      1262 / 1110, 1128   1902 / 1531, 1702    2534 / 1978, 2322
+//   1600, 16      990 / 978, 1022     1143 / 1245, 1300   1301 / 1549, 1581      17      1121 / 1034, 1086   1367 / 1305, 1368    1713 / 1601, 1654
+//   1600, 32      1166 / 1100, 1131   1508 / 1431, 1515   1961 / 1805, 2049      64      1717 / 1380, 1395   2468 / 1846, 2058    3174 / 2354, 2576
+//   2048, 16 (8)  851 / 820, 863      966 / 1013, 1062    1088 / 1250, 1252      64 (8)  1498 / 1206, 1224   2189 / 1607, 1872    2520 / 2028, 2253
 const GptStep *gpt_step_form(const GptStepForms &f, int position, bool replayed)
 {
     if (f.few_fits) {
@@ -171,6 +179,7 @@ const GptStep *gpt_step_form(const GptStepForms &f, int position, bool replayed)
     }
     if (!f.many_fits) return nullptr;
     const int batch = f.many.batch, d = f.many.d;
+    if (d >= 1600 && batch > 16) return nullptr;
     if (d > 1600 && position < (batch <= 2 ? 640 : batch <= 4 ? 480 : batch <= 8 ? 256 : 0)) return nullptr;
     if (batch <= 2 && position * 5 < d) return nullptr;
     // a graph is replayed at the positions up to the cache's end

@@ -276,6 +276,9 @@ def test_generation_step_plans(built_library):
     for batch, line in ((1, 640), (2, 640), (4, 480), (8, 256)):
         assert of(batch, 2048, 32, line - 1) == "operators" and of(batch, 2048, 32, line) == "rows"
     assert of(9, 2048, 32, 5) == "rows"
+    for d, heads in ((1600, 25), (2048, 32)):
+        assert of(16, d, heads, 5) == "rows" and of(17, d, heads, 1000) == "operators" and of(64, d, heads, 5) == "operators"
+    assert of(64, 1280, 20, 5) == "rows"
     assert step(SMS, 17, 768, 3072, 12, 256, 64)["rows"] == 32 and step(SMS, 64, 768, 3072, 12, 256, 64)["rows"] == 64
     # sizes that neither takes: more rows, other head sizes, odd widths, offsets within a layer's matrix beyond an int, scores beyond shared memory
     for args in ((65, 768, 3072, 12, 256), (1, 768, 3072, 8, 256), (1, 768, 3072, 768 // 4, 256), (1, 770, 3072, 77, 256), (1, 768, 3070, 12, 256),
