@@ -793,7 +793,7 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
         const long long n4 = (1LL * c.M * c.N) >> 2;
         const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, 1LL * ctx->num_sms * 8));
         ctx->launches++;
-    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, c.out, ctx->ws, n4, splits, c.accumulate ? 1 : 0, c.bias, c.act, c.N));
+        CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, c.out, ctx->ws, n4, splits, c.accumulate ? 1 : 0, c.bias, c.act, c.N));
     }
     return GPTB200_OK;
 }
@@ -1053,7 +1053,7 @@ int run_linear_bf16_impl(gptb200_ctx *ctx, const Bf16Linear &c)
         const long long n4 = (1LL * c.M * c.N) >> 2;
         const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, 1LL * ctx->num_sms * 8));
         ctx->launches++;
-    CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, static_cast<float *>(c.out), ctx->ws, n4, pl.splits, 0, nullptr, nullptr, c.N));
+        CUDA_TRY(ctx, launch_chained(ctx, splitk_reduce_kernel, dim3(blocks), dim3(256), 0, static_cast<float *>(c.out), ctx->ws, n4, pl.splits, 0, nullptr, nullptr, c.N));
     }
     return GPTB200_OK;
 }

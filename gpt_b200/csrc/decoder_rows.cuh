@@ -138,8 +138,9 @@ struct LayerBegin {
 // (nothing is exchanged between blocks), or comes from the sequence's state.
 //
 // Every thread keeps V pieces of four columns in registers, and its columns of the next two rows (residual, token input, the earlier layers' results; one row
-// where two don't fit) are copied to shared memory during the three sums over a row.  Bound by memory, 0.26 GB in the
-// mean layer of 4096 rows of 2048: 75 us with one row after the other, 63 now; prompt of 3000 tokens of the 768-wide model 2 819 / 2 555 us.
+// where two don't fit) are copied to shared memory during the three sums over a row.  0.26 GB in the
+// mean layer of 4096 rows of 2048: 75 us with one row after the other, 63 now, 0.62 of the copy bandwidth (what is left is a row's chain of three sums with a
+// barrier each); prompt of 3000 tokens of the 768-wide model 2 819 / 2 555 us.
 constexpr int layer_begin_threads(int v) { return v == 2 ? 256 : v == 4 ? 512 : 1024; }
 
 template <typename T, int V>

@@ -4,7 +4,7 @@
 // 128-byte swizzle) per stage; one thread of the leader issues 256 x BN x 16 instructions into one of two accumulators in TMEM.  Whole tiles, as evenly as
 // they go, m fastest (the pairs that run together share rows of w in L2).
 //
-// What bounds it: the tensor pipe and the power limit at large sizes (4096 x 10304 x 2048: 1 588 TFLOP/s, 113 us; loads alone 57 us, instructions alone
+// What bounds it: the tensor pipe and the power limit at large sizes (4096 x 10304 x 2048: 1 530 TFLOP/s, 113 us; loads alone 57 us, instructions alone
 // 86 us), the last wave and the first loads at small ones.  The general pair kernel (gemm_sm100_pair.cuh) took 167 us: it built two 64-bit descriptors per
 // instruction in the issuing thread, waited with cluster-scope acquires, and cut tiles between pairs, which costs more than it saves while a tile's main
 // loop is a few microseconds (2611 x 3072 x 768: 33 us against 15 us).

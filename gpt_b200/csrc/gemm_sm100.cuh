@@ -140,7 +140,7 @@ struct GemmParams {
 constexpr int kTraceSlots = 128;
 enum TraceEvent : int {
     TRACE_LOAD_ISSUE = 0,   // producer: stage free, loads about to be issued
-    TRACE_CONV_BEGIN = 1,   // converter (first warp of the group): raw tile landed, low-part buffer free
+    TRACE_CONV_BEGIN = 1,   // first converter warp: raw tile landed, low-part buffer free
     TRACE_CONV_END = 2,     // converter: tiles written and published
     TRACE_MMA_FULL = 3,     // MMA thread: raw tile landed
     TRACE_MMA_READY = 4,    // MMA thread: converted tiles of both CTAs ready

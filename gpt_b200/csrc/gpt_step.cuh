@@ -3,7 +3,8 @@
 // As one launch per operator a step of 12 layers is a chain of 89 launches of 3 - 16 us for 0.5 GB of weights (75 us of HBM
 // time): bound by launches, not by memory.  Here one block per SM stays for the whole step.  Phases meet at grid barriers
 // (arrivals counted in device memory, a cooperative launch keeps all blocks resident), and while a block waits at one its weights of the
-// next phase are already on their way: they depend on nothing.  All arithmetic is fp32 FMAs; sums have a fixed order.
+// next phase are already on their way: they depend on nothing.  Arithmetic is fp32 FMAs, the products of 16 padded rows and more three bf16 parts per operand
+// on the tensor cores with fp32 sums; sums have a fixed order.
 #pragma once
 
 #include <cfloat>

@@ -108,7 +108,7 @@ int gptb200_ctx_set_stream(gptb200_ctx *ctx, void *cuda_stream);
 int gptb200_ctx_set_option(gptb200_ctx *ctx, const char *key, int value);
 /* Kernel-phase trace (option "trace" = 1): the most recent CTA-pair GEMM launch recorded the SM clock at 11 events,
  * [event][slot] with 128 slots per event.  Events 0-5 are taken in the launch's first CTA, slot = k-block (the first 128):
- * 0 loads issued, 1 conversion begins (first converter warp of the group, 3xTF32), 2 conversion published, 3 MMA thread at the
+ * 0 loads issued, 1 conversion begins (first converter warp, 3xTF32), 2 conversion published, 3 MMA thread at the
  * k-block, 4 MMA thread has the operands, 5 MMAs and commits issued.  Events 6 / 7: a tile's output begins / its stores are
  * issued (slot = tile, 3xTF32).  Events 8-10: events 0-2 in the pair's second CTA (another SM: its clock is a different
  * counter, compare durations only).  Copies up to `capacity` samples (11 * 128 in all; 0 = not recorded) after waiting for
