@@ -122,14 +122,13 @@ bool attention_scratch(gptb200_ctx *ctx, size_t bytes)
         ctx->attn_ws_captured |= in_capture;
         return true;
     }
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;   // queued launches may still use the old buffer
-    release_scratch(ctx, ctx->attn_ws, ctx->attn_ws_captured);
+    if (release_scratch(ctx, ctx->attn_ws, ctx->attn_ws_captured, in_capture) != cudaSuccess) return false;
     ctx->attn_ws_bytes = 0;
-    if (cudaMalloc(&ctx->attn_ws, bytes) != cudaSuccess) {
+    if (allocate_scratch(&ctx->attn_ws, bytes, in_capture) != cudaSuccess) {
         cudaGetLastError();
-        ctx->attn_ws = nullptr;
         return false;
     }
+    ctx->attn_ws_captured = in_capture;
     ctx->attn_ws_bytes = bytes;
     return true;
 }

@@ -32,14 +32,30 @@ bool capturing(gptb200_ctx *ctx)
     return status != cudaStreamCaptureStatusNone;
 }
 
-void release_scratch(gptb200_ctx *ctx, float *&buffer, bool &captured)
+cudaError_t release_scratch(gptb200_ctx *ctx, float *&buffer, bool &captured, bool in_capture)
 {
-    if (captured)
+    if (!in_capture) {   // queued launches may still use it
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return e;
+    }
+    cudaError_t e = cudaSuccess;
+    if (buffer && (captured || in_capture))
         ctx->retired.push_back(buffer);
     else if (buffer)
-        cudaFree(buffer);
+        e = cudaFree(buffer);
     buffer = nullptr;
     captured = false;
+    return e;
+}
+
+cudaError_t allocate_scratch(float **buffer, size_t bytes, bool in_capture)
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // allocation is not a part of the graph
+    if (in_capture) cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaMalloc(buffer, bytes);
+    if (in_capture) cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) *buffer = nullptr;
+    return e;
 }
 
 int ensure_workspace(gptb200_ctx *ctx, size_t bytes)
@@ -50,14 +66,12 @@ int ensure_workspace(gptb200_ctx *ctx, size_t bytes)
         return GPTB200_OK;
     }
     if (bytes > ctx->ws_limit) return fail(ctx, GPTB200_ERR_WORKSPACE, "scratch request of %zu bytes exceeds limit %zu", bytes, ctx->ws_limit);
-    if (in_capture) return fail(ctx, GPTB200_ERR_WORKSPACE, "scratch of %zu bytes cannot be allocated while a graph is captured: call once before", bytes);
-    // Growing the scratch buffer waits for queued work: earlier kernels may still read the old one.
-    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    release_scratch(ctx, ctx->ws, ctx->ws_captured);
+    CUDA_TRY(ctx, release_scratch(ctx, ctx->ws, ctx->ws_captured, in_capture));
     ctx->ws_bytes = 0;
     const size_t rounded = (bytes + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
-    CUDA_TRY(ctx, cudaMalloc(&ctx->ws, rounded));
+    CUDA_TRY(ctx, allocate_scratch(&ctx->ws, rounded, in_capture));
     ctx->ws_bytes = rounded;
+    ctx->ws_captured = in_capture;
     return GPTB200_OK;
 }
 
@@ -614,7 +628,7 @@ int run_gemm(gptb200_ctx *ctx, const GemmCall &c, bool *dbias_fused = nullptr, b
     in.fma_only = c.fma_only;
     GemmPlan pl = plan_gemm(in);
     if (pl.kernel == KERNEL_SINGLE && pl.splits > 1 && in.has_epilogue && ensure_workspace(ctx, pl.workspace_bytes) != GPTB200_OK) {
-        cudaGetLastError();   // a device without room even for the reserve: as where an epilogue cannot be split
+        cudaGetLastError();   // a device without room for it: as where an epilogue cannot be split
         in.layers = false;
         pl = plan_gemm(in);
     }
@@ -1144,13 +1158,6 @@ int gptb200_ctx_create(gptb200_ctx **out, int device, void *cuda_stream, int mod
         if (ctx->d_status) cudaFree(ctx->d_status);
         delete ctx;
         return GPTB200_ERR_CUDA;
-    }
-    // where the device has no room, scratch comes with the first call that needs it
-    if (cudaMalloc(&ctx->ws, kPlanReservedBytes) == cudaSuccess) {
-        ctx->ws_bytes = kPlanReservedBytes;
-    } else {
-        cudaGetLastError();
-        ctx->ws = nullptr;
     }
     *out = ctx;
     return GPTB200_OK;

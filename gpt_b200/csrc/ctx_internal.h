@@ -180,8 +180,9 @@ int run_linear_f32(gptb200_ctx *ctx, float *out, const float *a, const float *w,
 // Grows the context's scratch buffer to at least `bytes` (waits for queued work before replacing it).
 int ensure_workspace(gptb200_ctx *ctx, size_t bytes);
 bool capturing(gptb200_ctx *ctx);
-// Frees a scratch buffer, or keeps it until the context goes where a captured graph holds its address.
-void release_scratch(gptb200_ctx *ctx, float *&buffer, bool &captured);
+// Frees a scratch buffer that has become too small, or keeps it until the context goes where a captured graph (or the one being captured) holds its address.
+cudaError_t release_scratch(gptb200_ctx *ctx, float *&buffer, bool &captured, bool in_capture);
+cudaError_t allocate_scratch(float **buffer, size_t bytes, bool in_capture);
 
 }  // namespace gptb200
 

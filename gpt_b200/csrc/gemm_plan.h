@@ -50,21 +50,18 @@ struct GemmPlan {
 };
 
 constexpr size_t kPairSlotBytes = 256 * 256 * sizeof(float);
-// Scratch that every context holds from the start: what the plans of forward calls ask for (one partial tile per CTA pair, or the parts of a product that is
-// split in spite of its epilogue) lies within it, so that a first call may be one that is captured into a graph and takes the plan of any other.
-constexpr size_t kPlanReservedBytes = size_t(32) << 20;
 
 constexpr int kPlanBM = 128;
 constexpr int kPlanBK = 32;
 constexpr int kPlanSkinnyMaxRows = 64;   // beyond this the fp32 FMAs of the weight-streaming kernel cost more than a tensor-core tile
 
 // `units`: number of CTAs (or CTA pairs) that run concurrently
-inline int plan_splits(const GemmPlanInput &in, long long tiles, int num_kb, bool allowed, size_t bytes_per_split, size_t limit, int units)
+inline int plan_splits(const GemmPlanInput &in, long long tiles, int num_kb, bool allowed, size_t bytes_per_split, int units)
 {
     if (!allowed) return 1;
     int cap = in.opt_max_splits > 0 ? in.opt_max_splits : 16;
     cap = std::min(cap, std::max(1, num_kb / 8));  // at least 8 k-blocks per split
-    if (bytes_per_split > 0) cap = static_cast<int>(std::min<size_t>(cap, std::max<size_t>(1, limit / bytes_per_split)));
+    if (bytes_per_split > 0) cap = static_cast<int>(std::min<size_t>(cap, std::max<size_t>(1, (in.ws_limit / 2) / bytes_per_split)));
     if (in.opt_max_splits > 0) return std::max(1, cap);
     int best = 1;
     double best_eff = 0.0;
@@ -364,8 +361,7 @@ inline GemmPlan plan_gemm(const GemmPlanInput &in)
     p.tiles_m = (in.M + kPlanBM - 1) / kPlanBM;
     p.tiles_n = (in.N + bn - 1) / bn;
     const long long tiles = 1LL * p.tiles_m * p.tiles_n;
-    const size_t limit = in.has_epilogue ? std::min(in.ws_limit / 2, kPlanReservedBytes) : in.ws_limit / 2;
-    const int splits = parts > 0 ? parts : plan_splits(in, tiles, p.num_kb, split_allowed, bytes_per_split, limit, in.num_sms);
+    const int splits = parts > 0 ? parts : plan_splits(in, tiles, p.num_kb, split_allowed, bytes_per_split, in.num_sms);
     p.kb_per_split = (p.num_kb + splits - 1) / splits;
     p.splits = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
     const long long items = tiles * p.splits;
@@ -408,7 +404,7 @@ inline Bf16Plan plan_bf16(int M, int N, int K, int num_sms, bool gated, bool pla
         in.ws_limit = ws_limit;
         const GemmPlan s = plan_gemm(in);
         const long long waves = (1LL * s.tiles_m * s.tiles_n * s.splits + num_sms - 1) / num_sms;
-        p.split_k = s.kernel == KERNEL_SINGLE && s.splits > 1 && s.workspace_bytes <= kPlanReservedBytes && 8000 + waves * s.kb_per_split * 485 < 6000 + least * ((K + 63) / 64);
+        p.split_k = s.kernel == KERNEL_SINGLE && s.splits > 1 && 8000 + waves * s.kb_per_split * 485 < 6000 + least * ((K + 63) / 64);
     }
     return p;
 }

@@ -45,9 +45,8 @@ typedef enum gptb200_mode {
 } gptb200_mode;
 
 /* ---- context: stands in for cublasCreate / cublasDestroy (cuda_backend.cu:6, :17)
- * A context holds 32 MB of scratch from the start (if the device has room), which covers every forward layer: those may be captured into a graph without a call
- * before.  Calls that need more grow it, outside of captures only (GPTB200_ERR_WORKSPACE inside one); a buffer that a captured call uses is kept beside the larger
- * one until the context is destroyed, and graphs must not be replayed after that. ---- */
+ * A context's scratch grows with the calls that need it, captured ones included; a buffer that a captured call uses is kept beside the larger one until the context
+ * is destroyed, and graphs must not be replayed after that. ---- */
 int gptb200_ctx_create(gptb200_ctx **out, int device, void *cuda_stream, int mode);
 int gptb200_ctx_destroy(gptb200_ctx *ctx);
 int gptb200_ctx_set_mode(gptb200_ctx *ctx, int mode);
