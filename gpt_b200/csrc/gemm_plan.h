@@ -1,6 +1,6 @@
 // Host-side planning of one GEMM call: which kernel, which tile, how many split-K parts, how many CTAs and how much
 // scratch.  Plain C++ without CUDA so that the same code is used by the launcher (capi.cu) and exercised by CPU
-// tests through gptb200_plan_gemm.
+// tests through gptb200_plan_gemm, gptb200_plan_layer, gptb200_plan_bf16, gptb200_plan_decode and gptb200_plan_rows.
 #pragma once
 
 #include <algorithm>
